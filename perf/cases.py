@@ -135,24 +135,24 @@ def _tokens(case, cfg, seed):
 STD = 0.02
 
 
-def _raw(cfg, g, n, k):
-    """A random matrix of standard deviation 0.02 as its checkpoint stores it."""
+def _raw(cfg, g, n, k, std=STD):
+    """A random matrix of standard deviation ``std`` as its checkpoint stores it."""
     m = cfg.quant.method
     if m == "cubic":
         codes = (torch.randn(n, k, device="cuda", generator=g) * 2.6).round_().clamp_(-7, 7).to(torch.int8)
         u = torch.rand(3, n, k // 128, device="cuda", generator=g)
-        return {"codes": codes, "scale": STD * 7 / 2.6 * (0.8 + 0.4 * u[0]), "a": (0.9 + 0.2 * u[1]).half(), "b": (0.2 * u[2] - 0.1).half()}
+        return {"codes": codes, "scale": std * 7 / 2.6 * (0.8 + 0.4 * u[0]), "a": (0.9 + 0.2 * u[1]).half(), "b": (0.2 * u[2] - 0.1).half()}
     if m == "gguf":
         codes = (torch.randn(n, k, device="cuda", generator=g) * 2.6 + 8).round_().clamp_(0, 15).to(torch.uint8)
         u = torch.rand(2, n, k // 32, device="cuda", generator=g)
-        scale = (STD / 2.6 * (0.8 + 0.4 * u[0])).bfloat16().float()
-        return {"codes": codes, "scale": scale, "offset": (STD * (0.1 * u[1] - 0.05)).bfloat16().float() - 8 * scale}
+        scale = (std / 2.6 * (0.8 + 0.4 * u[0])).bfloat16().float()
+        return {"codes": codes, "scale": scale, "offset": (std * (0.1 * u[1] - 0.05)).bfloat16().float() - 8 * scale}
     if m == "nvfp4":
         packed = torch.randint(0, 256, (n, k // 2), device="cuda", generator=g, dtype=torch.uint8)
         scale = (32 + 64 * torch.rand(n, k // 16, device="cuda", generator=g)).to(torch.float8_e4m3fn)
-        return {"packed": packed, "scale": scale, "global": STD / 2.9 / 64}
+        return {"packed": packed, "scale": scale, "global": std / 2.9 / 64}
     w = (torch.randn(n, k, device="cuda", generator=g) * 100).clamp_(-448, 448).to(torch.float8_e4m3fn)
-    return {"weight": w, "scale": STD / 100 * (0.8 + 0.4 * torch.rand(-(-n // 128), -(-k // 128), device="cuda", generator=g))}
+    return {"weight": w, "scale": std / 100 * (0.8 + 0.4 * torch.rand(-(-n // 128), -(-k // 128), device="cuda", generator=g))}
 
 
 def _pack(cfg, r):
@@ -202,8 +202,12 @@ class _Layer:
     def __init__(self, cfg, seed, i):
         self.cfg, self.seed, self.i = cfg, seed, i
 
-    def raw(self, part, n, k):
-        return _raw(self.cfg, _generator(self.seed, 2, self.i, part), n, k)
+    def raw(self, part, n, k, std=STD):
+        return _raw(self.cfg, _generator(self.seed, 2, self.i, part), n, k, std)
+
+    def added(self, part, n, k):
+        """A matrix whose results join the residual stream: smaller with the depth of the whole model, as networks start out."""
+        return self.raw(part, n, k, STD * (2 * NAMED_CONFIGS[self.cfg.name]().num_layers) ** -0.5)
 
     def small(self, part, *shape):
         return torch.randn(*shape, device="cuda", generator=_generator(self.seed, 3, self.i, part))
@@ -213,7 +217,7 @@ class _Layer:
         return self.raw(0, c.q_size + 2 * c.kv_size, c.hidden_size)
 
     def o(self):
-        return self.raw(1, self.cfg.hidden_size, self.cfg.q_size)
+        return self.added(1, self.cfg.hidden_size, self.cfg.q_size)
 
     def gate(self):
         return self.raw(2, self.cfg.q_size, self.cfg.hidden_size)
@@ -225,8 +229,8 @@ class _Layer:
     def down(self):
         c = self.cfg
         if c.is_moe:
-            return self.raw(4, c.num_experts * c.hidden_size, c.moe_intermediate_size)
-        return self.raw(4, c.hidden_size, c.intermediate_size)
+            return self.added(4, c.num_experts * c.hidden_size, c.moe_intermediate_size)
+        return self.added(4, c.hidden_size, c.intermediate_size)
 
     def router(self):
         return _bf16(_generator(self.seed, 4, self.i), self.cfg.num_experts, self.cfg.hidden_size, STD)
@@ -236,7 +240,7 @@ class _Layer:
         hk, hv, H = c.gdn_k_heads, c.gdn_v_heads, c.hidden_size
         return {"in_proj": self.raw(5, (2 * hk + 2 * hv) * 128, H), "in_ba": self.small(6, 2 * hv, H).mul_(STD).bfloat16(),
                 "conv": self.small(7, (2 * hk + hv) * 128, 4) * 0.3, "a_log": self.small(8, hv) * 0.5, "dt_bias": self.small(9, hv) * 0.5,
-                "out": self.raw(10, H, hv * 128)}
+                "out": self.added(10, H, hv * 128)}
 
 
 def _embedding(cfg, seed):
@@ -361,10 +365,9 @@ def work(case):
 
 
 def tolerance(case):
-    # bf16 activations through all layers, and codes of the cache that turn over: against ``exact`` the paths are 0.007
-    # (moe-30b-a3b, six layers) to 0.03 off, with 8-bit activations, whose codes turn over too, 0.05; two orders of the
-    # same sums differ by a part of that
-    return {"rel": 0.03, "max": 0.5}
+    # bf16 activations through all layers, and codes of the cache (and of 8-bit activations) that turn over: against ``exact``
+    # the paths are 0.005 (two layers) to 0.011 (twelve) off, and about 0.7 of that against other orders of the same sums
+    return {"rel": 0.03, "max": 0.2}
 
 
 # ------------------------------------------------------------------------------------------------- in 64 bits
