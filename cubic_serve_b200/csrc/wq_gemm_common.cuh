@@ -295,6 +295,55 @@ __device__ __forceinline__ void store_wide4(const WqGemmParams& p, int m, int n0
       if (n0 + j < p.N) dst[j] = __float2bfloat16(v[j]);
   }
 }
+// Four consecutive output features n0..n0+3 of row m from unscaled fp32 accumulators: scale, add the residual,
+// round once to bf16, store locally or (scatter-push) into the receive buffer of the rank that owns row m.
+template <int FMT>
+__device__ __forceinline__ void sk_store4(const WqGemmParams& p, int m, int n0, const float4 v) {
+  if (n0 >= p.N) return;
+  float o4[4] = {v.x * p.alpha, v.y * p.alpha, v.z * p.alpha, v.w * p.alpha};
+  if constexpr (FMT == kFmtBf16) {
+    if (p.wide) {
+      store_wide4(p, m, n0, o4);
+      return;
+    }
+  }
+  __nv_bfloat16* dst;
+  const __nv_bfloat16* res = nullptr;
+  bool vec;
+  if (p.tp.mode & kTpScatterPush) {
+    const int o = m / p.tp.rows_per_rank;
+    const int lr = m - o * p.tp.rows_per_rank;
+    dst = p.tp.recv[o] + (static_cast<size_t>(p.tp.rank) * p.tp.rows_per_rank + lr) * p.N + n0;
+    vec = (p.N & 3) == 0;
+  } else {
+    const size_t off = static_cast<size_t>(m) * p.ldy + n0;
+    dst = p.y + off;
+    if (p.residual) res = p.residual + off;
+    vec = (p.ldy & 3) == 0;
+  }
+  if (vec && n0 + 3 < p.N) {
+    if (res) {
+      const uint2 rv = *reinterpret_cast<const uint2*>(res);
+      const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&rv);
+      const float2 a0 = __bfloat1622float2(rp[0]), a1 = __bfloat1622float2(rp[1]);
+      o4[0] += a0.x; o4[1] += a0.y; o4[2] += a1.x; o4[3] += a1.y;
+    }
+    uint2 ov;
+    ov.x = pack_bf16x2(o4[0], o4[1]);
+    ov.y = pack_bf16x2(o4[2], o4[3]);
+    *reinterpret_cast<uint2*>(dst) = ov;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (n0 + j < p.N) {
+        float w = o4[j];
+        if (res) w += __bfloat162float(res[j]);
+        dst[j] = __float2bfloat16(w);
+      }
+    }
+  }
+}
+
 // offset of activation feature j (0..63) of a tile inside a 128-float tile row: gate value there, up value 16 on
 __device__ __forceinline__ int act_gate_col(int j) { return ((j >> 4) << 5) + (j & 15); }
 

@@ -1595,7 +1595,7 @@ _MIXER_SOURCES = {DeltaSpec: ("delta_rule.cu",), LatentSpec: ("latent_attn.cu",)
 
 def kernel_sources(cfg: LayeredConfig) -> set[str]:
     """Sources of ``csrc`` whose kernels a model of this configuration launches: products, rows, pages, sampling, and its mixers'."""
-    out = {"wq_gemm.cu", "wq_gemm_sk.cu", "elementwise.cu", "kv_cache.cu", "sampling.cu", "guard.cu", "layered.cu"}
+    out = {"wq_gemm.cu", "wq_gemm_sk.cu", "wq_gemm_skinny.cu", "elementwise.cu", "kv_cache.cu", "sampling.cu", "guard.cu", "layered.cu"}
     for l in cfg.layers:
         for part in l.mixer.parts:
             out.update(_MIXER_SOURCES[type(part)])

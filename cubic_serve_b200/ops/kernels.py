@@ -13,7 +13,7 @@ from dataclasses import dataclass
 import torch
 
 from . import native
-from .wq_pack import FMT_BF16, FMT_CUBIC4, FMT_FP8, FMT_FP8_BLOCK, PackedWeight
+from .wq_pack import FMT_AFFINE4, FMT_BF16, FMT_CUBIC4, FMT_FP8, FMT_FP8_BLOCK, FMT_NVFP4, PackedWeight
 
 PAGE_TOKENS = 16
 
@@ -154,6 +154,44 @@ def use_stream_k(m: int, n: int, fmt: int, sms: int = 148, k: int = 4096) -> boo
     return m <= g.stream_k_max_rows or (fmt == FMT_BF16 and g.stream_k_bf16)
 
 
+def skinny_fits(w: PackedWeight, x: torch.Tensor) -> bool:
+    """Whether ``csrc/wq_gemm_skinny.cu`` takes the operands (the rows aside): whole iterations of K columns, one scale group
+    for all columns of a lane, 16-byte chunks of the activations."""
+    if w.fmt == FMT_BF16:
+        whole = w.k % 128 == 0
+    elif w.fmt in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
+        whole = w.k % 256 == 0 and (w.fmt != FMT_CUBIC4 or w.group_k % 128 == 0)
+    else:
+        return False
+    return whole and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+
+
+def use_skinny(m: int, w: PackedWeight, x: torch.Tensor) -> bool:
+    """Which batches the kernel without decoded tiles takes.  Its products run on ``mma.sync`` eight rows at a time, so its time
+    grows with the rows where the tcgen05 kernels' stays: 4-bit weights of 24576 x 4096 take 22 / 26 / 43 us at 8 / 16 / 32 rows
+    against 34 / 34 / 35, 4096 x 4096 6.4 / 8.2 / 14 against 10.1 / 10.2 / 10.6.  bf16 weights have nothing to decode: with more
+    weight tiles than SMs they stream at 65 / 68 / 74 us against 98 / 98 / 102 (50688 x 4096), with fewer the split tiles of the
+    other kernel are as good from 16 rows on (8.0 / 10.4 against 9.2 / 9.2, 4096 x 4096).  (One B200, weights not in L2.)"""
+    if w.fmt == FMT_BF16:
+        most = 32 if -(-w.n // 128) > 148 else 8
+    else:
+        most = 16
+    return m <= most and skinny_fits(w, x)
+
+
+# Rows an expert gets on average up to which the grouped launches take that kernel: 6 / 12 / 16 / 24 rows of 128 experts of 1536 x
+# 2048 (NVFP4) take 82 / 103 / 107 / 134 us against 125 us of the tcgen05 kernel at any of them
+SKINNY_ROWS_PER_EXPERT = 16
+
+
+def _wq_gemm_skinny(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, residual: torch.Tensor | None, ws: "Workspace", swiglu: bool) -> torch.Tensor:
+    code = native.lib().cb_wq_gemm_skinny(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(), out.stride(0),
+                                          _ptr(residual), float(w.alpha), x.shape[0], w.n, w.k, w.group_k, int(swiglu), ws.gemm.data_ptr(),
+                                          ws.gemm.numel(), ws.gemm_counters.data_ptr(), ws.status.data_ptr(), _stream())
+    native.check(code, "cb_wq_gemm_skinny")
+    return out
+
+
 @dataclass
 class Fp8Act:
     """Activations quantized per token for the fp8 GEMMs: e4m3 bytes ``q [M, K]`` and fp32 scales ``scale [M]``."""
@@ -261,8 +299,8 @@ def wq_gemm(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = None,
             ws: Workspace | None = None, link=None, min_units: int | None = None) -> torch.Tensor:
     """``out[M, N] = x[M, K] @ W[N, K]^T * alpha (+ residual)`` with W in packed form.
 
-    Two kernels: one CTA per (weight tile, K split) (``csrc/wq_gemm.cu``) and the persistent stream-K kernel
-    (``csrc/wq_gemm_sk.cu``).  With neither ``splits`` nor ``min_units`` given the faster one for the shape is
+    Three kernels: one CTA per (weight tile, K split) (``csrc/wq_gemm.cu``), the persistent stream-K kernel
+    (``csrc/wq_gemm_sk.cu``), and one for few rows (``csrc/wq_gemm_skinny.cu``, see ``use_skinny``).  With neither ``splits`` nor ``min_units`` given the faster one for the shape is
     used (``use_stream_k``).  ``splits`` forces the first with that split-K factor; ``min_units`` forces the
     second (0 = its own schedule, > 0 = the smallest run of k-blocks a CTA is dealt).
     """
@@ -278,6 +316,8 @@ def wq_gemm(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = None,
     ws = ws or workspace(x.device)
     if w.fmt in (FMT_FP8, FMT_FP8_BLOCK):
         return _wq_gemm_fp8(x, w, out, residual, splits, ws, link, False, min_units)
+    if splits is None and min_units is None and link is None and use_skinny(m, w, x):
+        return _wq_gemm_skinny(x, w, out, residual, ws, False)
     l = native.lib()
     if splits is None and min_units is None and link is None and TUNED_PLANS:
         tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:0")
@@ -327,6 +367,8 @@ def wq_gemm_act(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = Non
     ws = ws or workspace(x.device)
     if w.fmt in (FMT_FP8, FMT_FP8_BLOCK):
         return _wq_gemm_fp8(x, w, out, None, splits, ws, link, True, min_units)
+    if splits is None and min_units is None and link is None and use_skinny(m, w, x):
+        return _wq_gemm_skinny(x, w, out, None, ws, True)
     l = native.lib()
     if splits is None and min_units is None and link is None and TUNED_PLANS:
         tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:1")
@@ -614,6 +656,13 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
                                                    sc.tiles.data_ptr(), sc.max_items, sc.mb, w.codes.shape[0], int(swiglu),
                                                    ws.status.data_ptr(), _stream())
         native.check(code, "cb_wq_gemm_fp8_grouped")
+        return out
+    per = rows / w.codes.shape[0]
+    if per <= SKINNY_ROWS_PER_EXPERT and w.fmt != FMT_BF16 and skinny_fits(w, x):
+        code = native.lib().cb_wq_gemm_skinny_grouped(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(),
+                                                      out.stride(0), float(w.alpha), rows, w.n, w.k, w.group_k, int(swiglu), sc.tiles.data_ptr(),
+                                                      8 if per <= 2 else 16 if per <= 8 else 32, code_stride, meta_stride, ws.status.data_ptr(), _stream())
+        native.check(code, "cb_wq_gemm_skinny_grouped")
         return out
     entry = native.lib().cb_wq_gemm_grouped_act if swiglu else native.lib().cb_wq_gemm_grouped
     code = entry(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta),

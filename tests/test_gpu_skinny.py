@@ -1,0 +1,98 @@
+"""The weight GEMM for few batch rows (csrc/wq_gemm_skinny.cu) against the dense matrix and against the per-tile kernel."""
+import pytest
+import torch
+
+from cubic_serve_b200.ops import wq_pack
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _weight(fmt, n, k, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rand = lambda *s: torch.rand(*s, device=DEV, generator=g)  # noqa: E731
+    if fmt == "cubic":
+        codes = torch.randint(-7, 8, (n, k), device=DEV, generator=g, dtype=torch.int8)
+        return wq_pack.pack_cubic4(codes, rand(n, k // 128) * 0.05, 0.5 + rand(n, k // 128), rand(n, k // 128) - 0.5, 128)
+    if fmt == "affine":
+        q = torch.randint(0, 16, (n, k), device=DEV, generator=g, dtype=torch.uint8)
+        return wq_pack.pack_affine4(q, rand(n, k // 32) * 0.02, -rand(n, k // 32) * 0.2, 32)
+    if fmt == "nvfp4":
+        q = torch.randint(0, 256, (n, k // 2), device=DEV, generator=g, dtype=torch.uint8)
+        return wq_pack.pack_nvfp4(q, (rand(n, k // 16) * 8).to(torch.float8_e4m3fn), 0.01)
+    return wq_pack.pack_bf16((rand(n, k) - 0.5) * 0.1)
+
+
+def _close(y, y0, k):
+    """Both kernels multiply the same bf16 operands into fp32 sums of another order (2^-24 of the sum of magnitudes for each of K
+    terms, well below a bf16 step of the largest results) and round once: a step of bf16 apart at most, near zero that of the scale."""
+    y, y0 = y.float(), y0.float()
+    return ((y - y0).abs() <= 2.0 ** -7 * y0.abs() + 2.0 ** -9 * y0.square().mean().sqrt()).all()
+
+
+@pytest.mark.parametrize("fmt", ["cubic", "affine", "nvfp4", "bf16"])
+@pytest.mark.parametrize("n,k", [
+    (128, 256),            # one tile, one iteration (two for bf16)
+    (200, 768),            # a tile with 72 rows of padding, three parts
+    (1000, 1280),          # five parts of a tile, the last tile short
+    (4096, 2048),          # aligned runs
+    (24576, 1024),         # runs that straddle tiles
+])
+def test_skinny_gemm(fmt, n, k):
+    from cubic_serve_b200.ops import kernels as K
+    w = _weight(fmt, n, k, n + k)
+    dense = wq_pack.unpack_to_dense(w)[:n]
+    g = torch.Generator(device=DEV).manual_seed(1)
+    for m in (1, 2, 7, 8, 9, 15, 16) + ((17, 31, 32) if fmt == "bf16" and n > 148 * 128 else ()):
+        wide = torch.randn(m, k + 64, device=DEV, generator=g).bfloat16()
+        x, res = wide[:, :k], torch.randn(m, n, device=DEV, generator=g).bfloat16()
+        assert m <= 8 or fmt != "bf16" or n > 148 * 128 or not K.use_skinny(m, w, x)
+        ref = x.float() @ dense.t()
+        out = torch.full((m, n + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+        K.wq_gemm(x, w, out=out[:, :n])
+        assert (out[:, n:] == 7).all()
+        assert _close(out[:, :n], K.wq_gemm(x, w, splits=1), k)
+        assert ((out[:, :n].float() - ref).norm() / ref.norm()).item() < 6e-3        # rounding of decode arithmetic and result
+        got = K.wq_gemm(x, w, residual=res)
+        assert _close(got, K.wq_gemm(x, w, residual=res, splits=1), k)
+        assert torch.equal(got, K.wq_gemm(x, w, residual=res))                       # parts are summed in their order
+    K.workspace(torch.device(DEV, 0)).check_status()
+    assert not K.workspace(torch.device(DEV, 0)).gemm_counters.any()
+
+
+@pytest.mark.parametrize("fmt", ["cubic", "affine", "nvfp4"])
+@pytest.mark.parametrize("m,inter,k", [(1, 128, 512), (8, 192, 256), (16, 12288, 512)])
+def test_skinny_gemm_gated_epilogue(fmt, m, inter, k):
+    from cubic_serve_b200.ops import kernels as K
+    w = wq_pack.swiglu_interleave(_weight(fmt, 2 * inter, k, inter))
+    x = torch.randn(m, k, device=DEV, generator=torch.Generator(device=DEV).manual_seed(2)).bfloat16()
+    plain = wq_pack.PackedWeight(w.fmt, w.n, w.k, w.group_k, w.codes, w.meta, w.alpha)
+    gu = torch.empty(m, 2 * inter, device=DEV, dtype=torch.bfloat16)
+    gu[:, wq_pack.swiglu_row_order(inter).to(DEV)] = K.wq_gemm(x, plain)
+    assert torch.equal(K.wq_gemm_act(x, w), K.swiglu(gu))
+
+
+@pytest.mark.parametrize("tokens", [1, 5, 40, 90])
+@pytest.mark.parametrize("skew", [False, True])
+def test_skinny_grouped_gemm(tokens, skew):
+    """Few rows an expert; with ``skew`` every token goes to the same eight experts, whose items take several passes."""
+    from cubic_serve_b200.models.moe import MoeLayer, stack_experts
+    from cubic_serve_b200.ops import kernels as K
+    E, H, I = 64, 512, 256
+    gu, c0, m0 = stack_experts([_weight("nvfp4", 2 * I, H, e) for e in range(E)])
+    dn, c1, m1 = stack_experts([_weight("nvfp4", H, I, 100 + e) for e in range(E)])
+    router = torch.randn(E, H, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)) * 0.1
+    x = torch.randn(tokens, H, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4)).bfloat16()
+    if skew:
+        x[:, 0] = 8.0
+        router[:8, 0] += 10.0
+    layer = MoeLayer(wq_pack.pack_bf16(router), gu, dn, (c0, m0, c1, m1), E, 8, 0, E, True)
+    layer.fuse_activation()
+    got = layer.forward(x).clone()
+    limit, K.SKINNY_ROWS_PER_EXPERT = K.SKINNY_ROWS_PER_EXPERT, 0
+    try:
+        want = layer.forward(x)
+    finally:
+        K.SKINNY_ROWS_PER_EXPERT = limit
+    # two chained products: a flipped rounding of an activation moves a result by a part of a bf16 step
+    assert ((got.float() - want.float()).norm() / want.float().norm()).item() < 2e-3
