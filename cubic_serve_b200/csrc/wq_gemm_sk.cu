@@ -44,6 +44,7 @@ static constexpr int kSkFirstDecodeWarp = 7;
 static constexpr int kSkThreads = (kSkFirstDecodeWarp + kSkDecodeWarps) * 32;   // 736
 static constexpr int kSkMaxAx = 6;
 static constexpr int kSkMaxC = 8;
+static_assert(kSkMaxC == 2 * kSkDecodeGroups, "code ring");
 __host__ __device__ constexpr int sk_cstage_bytes(int fmt) { return kCodeBytes + meta_bytes(fmt); }
 
 // One contiguous run of k-blocks of one tile, as dealt to a CTA.
@@ -1094,7 +1095,11 @@ int launch_streamk(int fmt, const CUtensorMap& tx, const CUtensorMap& tw, WqGemm
     S = static_cast<int>((budget - 4 * kSkCStageBytes) / ax);
     if (S > kSkMaxAx) S = kSkMaxAx;
     NC = static_cast<int>((budget - S * ax) / kSkCStageBytes);
-    if (NC > kSkMaxC) NC = kSkMaxC;
+    // A whole number of rounds of the decode groups: a slot then always belongs to the same group, whose wait for k-block j cannot
+    // come before k-block j - NC has landed and been decoded.  Otherwise the copies of two neighbouring k-blocks that land in
+    // reverse order let a group wait for a phase two ahead of the barrier, which a parity cannot tell from one that has passed:
+    // it decoded codes that were not there and released the slot (launch failures at 5 slots: 176 rows of NVFP4, 240 of Cubic).
+    NC = NC >= kSkMaxC ? kSkMaxC : NC >= kSkDecodeGroups ? kSkDecodeGroups : 0;
   }
   if (S > kSkMaxAx) S = kSkMaxAx;
   if (S < 2 || (!fmt_is_direct(fmt) && NC < 2)) return -14;
