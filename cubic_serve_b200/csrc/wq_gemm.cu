@@ -46,6 +46,7 @@ struct __align__(8) SmemCtl {
   uint32_t tmem_base;
   uint32_t abort_flag;
   uint32_t is_last;
+  uint32_t issued;         // k-blocks whose copies have been issued
 };
 
 template <int FMT>
@@ -110,6 +111,7 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
     }
     ctl->abort_flag = 0;
     ctl->is_last = 0;
+    ctl->issued = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -135,6 +137,7 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
         uint8_t* st = smem + static_cast<size_t>(s) * stage_bytes;
         const uint32_t bar = smem_u32(&ctl->full[s]);
         mbar_expect_tx(bar, tx);
+        *static_cast<volatile uint32_t*>(&ctl->issued) = static_cast<uint32_t>(i) + 1u;
         if (kDirect) {
           tma_load_2d(smem_u32(st + x_bytes), &tmap_w, kb * kBK, w_row0 + n_tile * kTileN, bar);
         } else {
@@ -254,6 +257,10 @@ wq_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x,
       int s = grp % S;                  // k-block i lives in stage i % S, phase (i / S) & 1
       uint32_t ph = static_cast<uint32_t>(grp / S) & 1u;
       for (int i = grp; i < iters; i += 4) {
+        // A slot's k-blocks go round the groups unless the ring has four or eight slots, so this group may come here before
+        // another group's k-block i - S has even landed (copies land in any order), and then the barrier is still one phase
+        // further back than a parity can tell: the copies of k-block i are only issued once i - S has been multiplied.
+        if (i >= S && !wait_above(&ctl->issued, static_cast<uint32_t>(i), abort_flag)) break;
         if (!mbar_wait_park(smem_u32(&ctl->full[s]), ph, abort_flag)) break;
         CB_STAMP(dq == 0, i * 8 + 2);
         uint8_t* st = smem + static_cast<size_t>(s) * stage_bytes;

@@ -155,6 +155,21 @@ __device__ __forceinline__ bool wait_counter(const uint32_t* p, uint32_t target,
   return true;
 }
 
+// Bounded wait until a counter in this CTA's shared memory is above `value`.
+__device__ __forceinline__ bool wait_above(volatile uint32_t* p, uint32_t value, volatile uint32_t* abort_flag) {
+  if (*p > value) return true;
+  const long long t0 = clock64();
+  while (*p <= value) {
+    if (*abort_flag) return false;
+    if (clock64() - t0 > kWaitBudgetCycles) {
+      *abort_flag = 1;
+      return false;
+    }
+    __nanosleep(32);
+  }
+  return true;
+}
+
 // The same for a counter that CTAs of THIS kernel raise (device scope), reaching at least `target`.
 __device__ __forceinline__ bool wait_counter_gpu(const uint32_t* p, uint32_t target, volatile uint32_t* abort_flag) {
   const long long t0 = clock64();
