@@ -370,6 +370,7 @@ wq_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
 #pragma unroll
             for (int c = 0; c < 4; ++c) f(mine[(nb * 8 + (c & 1)) * kSnRedStride + rt * 16 + (c >> 1) * 8], acc[rt][nb][c]);
     };
+    sn_bar();                                  // the previous segment's sums have been read: nothing else holds a warp back that is a run ahead
     if (kg == 1) each([](float& m, float v) { m = v; });
     sn_bar();
     if (kg == 0) each([](float& m, float v) { m += v; });
