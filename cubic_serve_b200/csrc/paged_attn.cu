@@ -18,6 +18,7 @@
 #include "ptx.cuh"
 #include "launch.cuh"
 #include "kv_layout.cuh"
+#include <type_traits>
 
 namespace cb {
 
@@ -84,6 +85,51 @@ struct WarpState {
   float l[2];       // running partial sum (this lane's columns only)
   float o[16][4];   // O accumulators: n-tile (cg*4 + sub) x {row g: 2 cols, row g+8: 2 cols}
 };
+
+// Fills `p` from the arguments of the C entries; 0 or a negative argument error.
+static inline int make_attn_params(AttnParams& p, const void* q, void* out, const void* cache, const void* page_table, const void* rb_req, const void* rb_qstart,
+                                   const void* rb_qcount, const void* rb_ctx, int Hq, int Hkv, int D, int max_pages, int k_bits, int v_bits, float scale, int splits,
+                                   void* partial, void* counters, void* status) {
+  if (D != kD || Hkv <= 0 || Hq % Hkv != 0) return -10;
+  const int G = Hq / Hkv;
+  if (G > 16 || (16 % G) != 0) return -11;
+  if (splits < 1) splits = 1;
+  if (splits > 1 && (!partial || !counters)) return -12;
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.cache = static_cast<const uint8_t*>(cache);
+  p.page_table = static_cast<const int*>(page_table);
+  p.rb_req = static_cast<const int*>(rb_req);
+  p.rb_qstart = static_cast<const int*>(rb_qstart);
+  p.rb_qcount = static_cast<const int*>(rb_qcount);
+  p.rb_ctx = static_cast<const int*>(rb_ctx);
+  p.partial = static_cast<float*>(partial);
+  p.counters = static_cast<uint32_t*>(counters);
+  p.status = static_cast<uint32_t*>(status);
+  p.Hq = Hq; p.Hkv = Hkv; p.G = G; p.max_pages = max_pages; p.splits = splits;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.lay = make_kv_layout(D, k_bits, v_bits);
+  return 0;
+}
+
+// Calls `f` with the bits of K and V as constants; -13 for widths that the cache does not have.
+template <typename F>
+static inline int with_kv_bits(int k_bits, int v_bits, F&& f) {
+  auto with_v = [&](auto kb) {
+    switch (v_bits) {
+      case 8: return f(kb, std::integral_constant<int, 8>());
+      case 6: return f(kb, std::integral_constant<int, 6>());
+      case 4: return f(kb, std::integral_constant<int, 4>());
+      default: return -13;
+    }
+  };
+  switch (k_bits) {
+    case 8: return with_v(std::integral_constant<int, 8>());
+    case 6: return with_v(std::integral_constant<int, 6>());
+    case 4: return with_v(std::integral_constant<int, 4>());
+    default: return -13;
+  }
+}
 
 // UPPER = false: MMA rows 8..15 of the block hold no query (decode: one position x G <= 8 heads), so their scores,
 // softmax state and output rescaling are skipped; the tensor-core instructions still compute them, at no cost.
@@ -481,6 +527,326 @@ paged_attn_kernel(const AttnParams p) {
   if (threadIdx.x == 0 && abort_word) atomicExch(p.status, static_cast<uint32_t>(kErrBarrierTimeout));
 }
 
+// Decode form: row blocks of at most eight rows (one position of up to eight query heads per key / value head, or a few positions of
+// fewer).  The cache is the MMA's 16-row operand -- S^T = K Q^T, O^T = V^T P^T -- so a page takes 16 MMAs where the general kernel
+// takes 32 of which half the rows are empty, the output needs 32 registers a lane instead of 64, and four CTAs run on an SM
+// instead of two; that is what the time hangs on, since a warp spends most of a page's life waiting for its own loads.  The
+// code words are the same: what is a column pair's B operand there is a row's A operand here.  Probabilities change
+// lanes by a matrix transpose after the V scale and the rounding to f16, the point where the general kernel rounds them.
+// KV splits that would give a warp less than two pages are not used: one row over 700 tokens took 46 us in 32 splits, 7 in 6.
+//
+// Measured, INT8 K and V, 32 / 8 heads (general kernel -> this one): 256 rows of 1280 tokens 164 -> 124 us (753 MB: 6.1 TB/s), 48
+// rows of 560 to 1500 33.5 -> 30.7, 7 of 900 to 2100 25.8 -> 13, 1 of 700 46 -> 7.
+static constexpr int kDecStages = 3;
+static constexpr int kDecRows = 8;
+static constexpr int kDecMinPages = 2 * kAttnWarps;
+
+__device__ __forceinline__ uint32_t transpose8(uint32_t a) {
+  uint32_t r;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(a));
+  return r;
+}
+
+struct DecState {
+  float m[2], l[2];          // rows 2 t and 2 t + 1: running max (log2 domain), this lane's part of the sum
+  float o[8][4];             // [32-channel group * 2 + h]: channels 32 cg + 4 g + 2 h and the next one x the two rows
+};
+
+template <int KBITS, int VBITS>
+__device__ __forceinline__ void decode_page(const uint8_t* blob, const KvLayout& lay, const uint32_t (&qf)[8][2], DecState& st, int tok0, const int (&limit)[2], int visible,
+                                            int g, int t) {
+  const uint8_t* vcodes = blob + lay.v_code_off;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};                     // tokens g and g + 8 x rows 2 t, 2 t + 1
+  const float4 kl = *reinterpret_cast<const float4*>(blob + lay.k_scale_off + g * 16), kh = *reinterpret_cast<const float4*>(blob + lay.k_scale_off + (g + 8) * 16);
+#pragma unroll
+  for (int cg = 0; cg < 4; ++cg) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    if constexpr (KBITS == 8) {
+#pragma unroll
+      for (int jh = 0; jh < 2; ++jh) {
+        const int j = cg * 2 + jh;
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(blob + j * 256 + g * 16 + t * 4), w1 = *reinterpret_cast<const uint32_t*>(blob + j * 256 + (g + 8) * 16 + t * 4);
+        const uint32_t a[4] = {u8x2_to_f16x2(w0, 0x5140u, 0x64806480u), u8x2_to_f16x2(w1, 0x5140u, 0x64806480u), u8x2_to_f16x2(w0, 0x5342u, 0x64806480u),
+                               u8x2_to_f16x2(w1, 0x5342u, 0x64806480u)};
+        mma_f16(acc, a, qf[j][0], qf[j][1]);
+      }
+    } else {
+      constexpr uint32_t bias = KBITS == 6 ? 0x64206420u : 0x64086408u;
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(blob + cg * 256 + g * 16 + t * 4), w1 = *reinterpret_cast<const uint32_t*>(blob + cg * 256 + (g + 8) * 16 + t * 4);
+      uint32_t l0 = w0 & 0x0F0F0F0Fu, h0 = (w0 >> 4) & 0x0F0F0F0Fu, l1 = w1 & 0x0F0F0F0Fu, h1 = (w1 >> 4) & 0x0F0F0F0Fu;
+      if constexpr (KBITS == 6) {
+        const uint32_t hb = *reinterpret_cast<const uint32_t*>(blob + kPageTokens * kD / 2 + cg * 128 + g * 16 + t * 4);
+        l0 |= hb & 0x30303030u;
+        h0 |= (hb >> 2) & 0x30303030u;
+        l1 |= (hb << 4) & 0x30303030u;
+        h1 |= (hb << 2) & 0x30303030u;
+      }
+      const uint32_t a[4] = {u8x2_to_f16x2(l0, 0x5140u, bias), u8x2_to_f16x2(l1, 0x5140u, bias), u8x2_to_f16x2(l0, 0x5342u, bias), u8x2_to_f16x2(l1, 0x5342u, bias)};
+      const uint32_t b[4] = {u8x2_to_f16x2(h0, 0x5140u, bias), u8x2_to_f16x2(h1, 0x5140u, bias), u8x2_to_f16x2(h0, 0x5342u, bias), u8x2_to_f16x2(h1, 0x5342u, bias)};
+      mma_f16(acc, a, qf[cg * 2][0], qf[cg * 2][1]);
+      mma_f16(acc, b, qf[cg * 2 + 1][0], qf[cg * 2 + 1][1]);
+    }
+    const float k0 = (&kl.x)[cg], k1 = (&kh.x)[cg];
+    s[0] = fmaf(acc[0], k0, s[0]); s[1] = fmaf(acc[1], k0, s[1]);
+    s[2] = fmaf(acc[2], k1, s[2]); s[3] = fmaf(acc[3], k1, s[3]);
+  }
+  float alpha[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    if (tok0 + g >= limit[r]) s[r] = -INFINITY;
+    if (tok0 + g + 8 >= limit[r]) s[2 + r] = -INFINITY;
+    float mx = fmaxf(s[r], s[2 + r]);
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+    const float m = fmaxf(st.m[r], mx), use = m == -INFINITY ? 0.f : m;
+    alpha[r] = fast_exp2(st.m[r] - use);
+    st.m[r] = m;
+    s[r] = fast_exp2(s[r] - use);
+    s[2 + r] = fast_exp2(s[2 + r] - use);
+    st.l[r] = fmaf(st.l[r], alpha[r], s[r] + s[2 + r]);
+  }
+  if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) st.o[n][c] *= alpha[c & 1];
+  }
+  // slots past the longest visible length may hold stale bytes (even NaN bit patterns): their scale counts as zero
+  float4 vl = make_float4(0.f, 0.f, 0.f, 0.f), vh = vl;
+  if (tok0 + g < visible) vl = *reinterpret_cast<const float4*>(blob + lay.v_scale_off + g * 16);
+  if (tok0 + g + 8 < visible) vh = *reinterpret_cast<const float4*>(blob + lay.v_scale_off + (g + 8) * 16);
+#pragma unroll
+  for (int cg = 0; cg < 4; ++cg) {
+    const float v0 = (&vl.x)[cg], v1 = (&vh.x)[cg];
+    const uint32_t b0 = transpose8(pack_f16x2(s[0] * v0, s[1] * v0)), b1 = transpose8(pack_f16x2(s[2] * v1, s[3] * v1));
+    const int chunk = (cg * 8 + g) ^ (t << 2);
+    uint32_t lo[4], hi[4];                                // token pairs t and t + 4 of four channels
+    if constexpr (VBITS == 8) {
+      const uint2 l = *reinterpret_cast<const uint2*>(vcodes + t * 256 + chunk * 8), h = *reinterpret_cast<const uint2*>(vcodes + (t + 4) * 256 + chunk * 8);
+      lo[0] = u8x2_to_f16x2(l.x, 0x5140u, 0x64806480u); lo[1] = u8x2_to_f16x2(l.x, 0x5342u, 0x64806480u);
+      lo[2] = u8x2_to_f16x2(l.y, 0x5140u, 0x64806480u); lo[3] = u8x2_to_f16x2(l.y, 0x5342u, 0x64806480u);
+      hi[0] = u8x2_to_f16x2(h.x, 0x5140u, 0x64806480u); hi[1] = u8x2_to_f16x2(h.x, 0x5342u, 0x64806480u);
+      hi[2] = u8x2_to_f16x2(h.y, 0x5140u, 0x64806480u); hi[3] = u8x2_to_f16x2(h.y, 0x5342u, 0x64806480u);
+    } else {
+      constexpr uint32_t bias = VBITS == 6 ? 0x64206420u : 0x64086408u;
+      const uint32_t l = *reinterpret_cast<const uint32_t*>(vcodes + t * 128 + chunk * 4), h = *reinterpret_cast<const uint32_t*>(vcodes + (t + 4) * 128 + chunk * 4);
+      uint32_t le = l & 0x0F0F0F0Fu, lod = (l >> 4) & 0x0F0F0F0Fu, he = h & 0x0F0F0F0Fu, hod = (h >> 4) & 0x0F0F0F0Fu;
+      if constexpr (VBITS == 6) {
+        const uint32_t hw = *reinterpret_cast<const uint32_t*>(vcodes + kPageTokens * kD / 2 + t * 128 + chunk * 4);
+        le |= hw & 0x30303030u;
+        lod |= (hw >> 2) & 0x30303030u;
+        he |= (hw << 4) & 0x30303030u;
+        hod |= (hw << 2) & 0x30303030u;
+      }
+      const uint32_t l01 = prmt(le, lod, 0x5140u), l23 = prmt(le, lod, 0x7362u), h01 = prmt(he, hod, 0x5140u), h23 = prmt(he, hod, 0x7362u);
+      lo[0] = u8x2_to_f16x2(l01, 0x5140u, bias); lo[1] = u8x2_to_f16x2(l01, 0x5342u, bias);
+      lo[2] = u8x2_to_f16x2(l23, 0x5140u, bias); lo[3] = u8x2_to_f16x2(l23, 0x5342u, bias);
+      hi[0] = u8x2_to_f16x2(h01, 0x5140u, bias); hi[1] = u8x2_to_f16x2(h01, 0x5342u, bias);
+      hi[2] = u8x2_to_f16x2(h23, 0x5140u, bias); hi[3] = u8x2_to_f16x2(h23, 0x5342u, bias);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t a[4] = {lo[2 * h], lo[2 * h + 1], hi[2 * h], hi[2 * h + 1]};
+      mma_f16(st.o[cg * 2 + h], a, b0, b1);
+    }
+  }
+}
+
+template <int KBITS, int VBITS>
+__global__ void __launch_bounds__(kAttnWarps * 32, 4)
+paged_decode_kernel(const AttnParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int RS = kD + 2;
+  __shared__ __align__(8) uint64_t bars[kAttnWarps * kDecStages];
+  __shared__ uint32_t abort_word, is_last;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int kvh = blockIdx.x, rb = blockIdx.y, split = blockIdx.z;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int qcount = p.rb_qcount[rb];
+  if (qcount <= 0) return;                                // padding block (uniform across the CTA)
+  const int req = p.rb_req[rb], qstart = p.rb_qstart[rb], ctx = p.rb_ctx[rb];
+  const int G = p.G;
+  const int total = ctx + qcount - 1, pages = (total + kPageTokens - 1) / kPageTokens;
+  const int splits = max(1, min(p.splits, (pages + kDecMinPages - 1) / kDecMinPages));
+  const int per = (pages + splits - 1) / splits;
+  const int used = (pages + per - 1) / per;               // splits that have pages
+  if (split >= used) return;
+  if (qcount * G > kDecRows) {                            // the caller's promise does not hold: said, not computed wrongly
+    if (tid == 0) atomicExch(p.status, static_cast<uint32_t>(kErrBadArgument));
+    return;
+  }
+  const int stride = (p.lay.blob_bytes + 127) & ~127;
+  uint8_t* stages = smem + static_cast<size_t>(warp) * kDecStages * stride;
+  uint64_t* my = bars + warp * kDecStages;
+  volatile uint32_t* abort_flag = &abort_word;
+  if (tid == 0) abort_word = 0;
+  if (lane == 0) {
+    for (int s = 0; s < kDecStages; ++s) mbar_init(smem_u32(&my[s]), 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  const int lo = split * per, hi = min(pages, lo + per), first = lo + warp;
+  const int n = first < hi ? (hi - first + kAttnWarps - 1) / kAttnWarps : 0;
+  const int* ptab = p.page_table + static_cast<size_t>(req) * p.max_pages;
+  auto issue = [&](int i, int page) {
+    const int s = i % kDecStages;
+    const uint32_t bar = smem_u32(&my[s]);
+    mbar_expect_tx(bar, p.lay.blob_bytes);
+    bulk_g2s(smem_u32(stages + s * stride), p.cache + (static_cast<size_t>(page) * p.Hkv + kvh) * p.lay.blob_bytes, p.lay.blob_bytes, bar);
+  };
+  if (lane == 0) {
+    int pg[kDecStages];
+#pragma unroll
+    for (int i = 0; i < kDecStages; ++i) pg[i] = i < n ? ptab[first + i * kAttnWarps] : 0;
+#pragma unroll
+    for (int i = 0; i < kDecStages; ++i)
+      if (i < n) issue(i, pg[i]);
+  }
+  int limit[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int qp = (2 * t + r) / G;
+    limit[r] = qp < qcount ? ctx + qp : 0;
+  }
+  uint32_t qf[8][2];
+  {
+    const int qp = g / G, hh = g - qp * G;
+    const bool valid = qp < qcount;
+    const __nv_bfloat16* q = p.q + (static_cast<size_t>(qstart + qp) * p.Hq + kvh * G + hh) * kD;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      uint2 w = make_uint2(0u, 0u);
+      if (valid) w = *reinterpret_cast<const uint2*>(q + j * 16 + t * 4);
+      const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.x)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.y));
+      qf[j][0] = pack_f16x2(x.x * p.scale_log2, x.y * p.scale_log2);
+      qf[j][1] = pack_f16x2(y.x * p.scale_log2, y.y * p.scale_log2);
+    }
+  }
+  DecState st;
+  st.m[0] = st.m[1] = -INFINITY;
+  st.l[0] = st.l[1] = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) st.o[i][c] = 0.f;
+  int page_next = (lane == 0 && kDecStages < n) ? ptab[first + kDecStages * kAttnWarps] : 0;
+  bool ok = true;
+  int slot = 0;
+  uint32_t phase = 0;
+  for (int i = 0; i < n; ++i) {
+    ok = __all_sync(0xffffffffu, mbar_wait_t<20>(smem_u32(&my[slot]), phase, abort_flag));
+    if (!ok) break;
+    const int page_after = (lane == 0 && i + 1 + kDecStages < n) ? ptab[first + (i + 1 + kDecStages) * kAttnWarps] : 0;
+    decode_page<KBITS, VBITS>(stages + slot * stride, p.lay, qf, st, (first + i * kAttnWarps) * kPageTokens, limit, total, g, t);
+    __syncwarp();
+    if (lane == 0 && i + kDecStages < n) issue(i + kDecStages, page_next);
+    page_next = page_after;
+    if (++slot == kDecStages) { slot = 0; phase ^= 1u; }
+  }
+  if (!ok && lane == 0) {
+    // a wait gave up: copies may still be in flight, they get a bounded time to land
+    for (int s = 0; s < kDecStages; ++s) {
+      const long long t0 = clock64();
+      while (!mbar_try_wait(smem_u32(&my[s]), 0) && !mbar_try_wait(smem_u32(&my[s]), 1) && clock64() - t0 < kWaitBudgetCycles / 8) {
+      }
+    }
+    atomicExch(p.status, static_cast<uint32_t>(kErrBarrierTimeout));
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    st.l[r] += __shfl_xor_sync(0xffffffffu, st.l[r], 4);
+    st.l[r] += __shfl_xor_sync(0xffffffffu, st.l[r], 8);
+    st.l[r] += __shfl_xor_sync(0xffffffffu, st.l[r], 16);
+  }
+  __syncthreads();                                        // all warps are done with their stages
+  // the warps meet in shared memory: [warp][8 rows][D | max, sum]
+  float* mg = reinterpret_cast<float*>(smem);
+  float* mine = mg + warp * kDecRows * RS;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      *reinterpret_cast<float2*>(mine + (2 * t + c) * RS + (i >> 1) * 32 + 4 * g + 2 * (i & 1)) = make_float2(st.o[i][c], st.o[i][2 + c]);
+  if (g == 0) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) *reinterpret_cast<float2*>(mine + (2 * t + r) * RS + kD) = make_float2(st.m[r], st.l[r]);
+  }
+  __syncthreads();
+  const int row = tid >> 4, cb = (tid & 15) * 8;          // eight channels of a row
+  float m = -INFINITY, l = 0.f, o[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) o[c] = 0.f;
+#pragma unroll
+  for (int w = 0; w < kAttnWarps; ++w) m = fmaxf(m, mg[(w * kDecRows + row) * RS + kD]);
+#pragma unroll
+  for (int w = 0; w < kAttnWarps; ++w) {
+    const float* x = mg + (w * kDecRows + row) * RS;
+    const float f = x[kD] == -INFINITY ? 0.f : fast_exp2(x[kD] - m);
+    l = fmaf(f, x[kD + 1], l);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) o[c] = fmaf(f, x[cb + c], o[c]);
+  }
+  if (used > 1) {
+    // parts of the row block: [split][8 rows][D], then [split][8 rows]{max, sum}; the last split to arrive merges them in order
+    const size_t idx = static_cast<size_t>(rb) * p.Hkv + kvh;
+    float* part = p.partial + idx * p.splits * 16 * RS;
+    float* ml = part + static_cast<size_t>(used) * kDecRows * kD;
+    float* to = part + (static_cast<size_t>(split) * kDecRows + row) * kD + cb;
+    __stcg(reinterpret_cast<float4*>(to), make_float4(o[0], o[1], o[2], o[3]));
+    __stcg(reinterpret_cast<float4*>(to + 4), make_float4(o[4], o[5], o[6], o[7]));
+    if (cb == 0) __stcg(reinterpret_cast<float2*>(ml + (split * kDecRows + row) * 2), make_float2(m, l));
+    __syncthreads();
+    if (tid == 0) {
+      const uint32_t prev = atom_add_acq_rel_gpu(p.counters + idx, 1u);
+      is_last = prev == static_cast<uint32_t>(used) - 1u;
+      if (is_last) p.counters[idx] = 0;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    float2* sml = reinterpret_cast<float2*>(mg);
+    for (int i = tid; i < used * kDecRows; i += kAttnWarps * 32) sml[i] = __ldcg(reinterpret_cast<const float2*>(ml) + i);
+    __syncthreads();
+    m = -INFINITY; l = 0.f;
+    for (int s = 0; s < used; ++s) m = fmaxf(m, sml[s * kDecRows + row].x);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) o[c] = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < used; ++s) {
+      const float* x = part + (static_cast<size_t>(s) * kDecRows + row) * kD + cb;
+      const float4 a = __ldcg(reinterpret_cast<const float4*>(x)), b = __ldcg(reinterpret_cast<const float4*>(x + 4));
+      const float2 e = sml[s * kDecRows + row];
+      const float f = e.x == -INFINITY ? 0.f : fast_exp2(e.x - m);
+      l = fmaf(f, e.y, l);
+      o[0] = fmaf(f, a.x, o[0]); o[1] = fmaf(f, a.y, o[1]); o[2] = fmaf(f, a.z, o[2]); o[3] = fmaf(f, a.w, o[3]);
+      o[4] = fmaf(f, b.x, o[4]); o[5] = fmaf(f, b.y, o[5]); o[6] = fmaf(f, b.z, o[6]); o[7] = fmaf(f, b.w, o[7]);
+    }
+  }
+  const int qp = row / G, hh = row - qp * G;
+  if (qp >= qcount) return;
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  *reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(qstart + qp) * p.Hq + kvh * G + hh) * kD + cb) =
+      make_uint4(pack_bf16x2(o[0] * inv, o[1] * inv), pack_bf16x2(o[2] * inv, o[3] * inv), pack_bf16x2(o[4] * inv, o[5] * inv), pack_bf16x2(o[6] * inv, o[7] * inv));
+}
+
+template <int KB, int VB>
+static int launch_decode(const AttnParams& p, int row_blocks, cudaStream_t st) {
+  const int stride = (p.lay.blob_bytes + 127) & ~127;
+  size_t smem = static_cast<size_t>(kAttnWarps) * kDecStages * stride;
+  const size_t merge = static_cast<size_t>(kAttnWarps) * kDecRows * (kD + 2) * 4;      // also holds {max, sum} of 64 splits
+  if (smem < merge) smem = merge;
+  static bool configured[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -18;
+  if (!configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(paged_decode_kernel<KB, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured[dev] = true;
+  }
+  return static_cast<int>(launch(paged_decode_kernel<KB, VB>, dim3(p.Hkv, row_blocks, p.splits), dim3(kAttnWarps * 32), smem, st, p));
+}
+
 template <int KB, int VB>
 static int launch_attn(const AttnParams& p, dim3 grid, size_t smem, cudaStream_t st) {
   static bool configured = false;
@@ -507,42 +873,32 @@ int cb_paged_attn(const void* q, void* out, const void* cache, const void* page_
                   void* counters, void* status, void* stream) {
   using namespace cb;
   if (row_blocks <= 0) return 0;
-  if (D != kD || Hkv <= 0 || Hq % Hkv != 0) return -10;
-  const int G = Hq / Hkv;
-  if (G > 16 || (16 % G) != 0) return -11;
-  if (splits < 1) splits = 1;
-  if (splits > 1 && (!partial || !counters)) return -12;
   AttnParams p;
-  p.q = static_cast<const __nv_bfloat16*>(q);
-  p.out = static_cast<__nv_bfloat16*>(out);
-  p.cache = static_cast<const uint8_t*>(cache);
-  p.page_table = static_cast<const int*>(page_table);
-  p.rb_req = static_cast<const int*>(rb_req);
-  p.rb_qstart = static_cast<const int*>(rb_qstart);
-  p.rb_qcount = static_cast<const int*>(rb_qcount);
-  p.rb_ctx = static_cast<const int*>(rb_ctx);
-  p.partial = static_cast<float*>(partial);
-  p.counters = static_cast<uint32_t*>(counters);
-  p.status = static_cast<uint32_t*>(status);
-  p.Hq = Hq; p.Hkv = Hkv; p.G = G; p.max_pages = max_pages; p.splits = splits;
-  p.scale_log2 = scale * 1.4426950408889634f;
-  p.lay = make_kv_layout(D, k_bits, v_bits);
+  const int bad = make_attn_params(p, q, out, cache, page_table, rb_req, rb_qstart, rb_qcount, rb_ctx, Hq, Hkv, D, max_pages, k_bits, v_bits, scale, splits, partial, counters,
+                                   status);
+  if (bad) return bad;
   const int stage_stride = (p.lay.blob_bytes + 127) & ~127;
   size_t smem = static_cast<size_t>(kAttnWarps) * kAttnStages * stage_stride + kAttnWarps * kAttnStages * 8;
   const size_t merge = static_cast<size_t>(kAttnWarps) * 16 * (kD + 2) * 4;
   if (smem < merge) smem = merge;
-  dim3 grid(Hkv, row_blocks, splits);
+  dim3 grid(Hkv, row_blocks, p.splits);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (k_bits == 8 && v_bits == 8) return launch_attn<8, 8>(p, grid, smem, st);
-  if (k_bits == 4 && v_bits == 8) return launch_attn<4, 8>(p, grid, smem, st);
-  if (k_bits == 4 && v_bits == 4) return launch_attn<4, 4>(p, grid, smem, st);
-  if (k_bits == 8 && v_bits == 4) return launch_attn<8, 4>(p, grid, smem, st);
-  if (k_bits == 6 && v_bits == 6) return launch_attn<6, 6>(p, grid, smem, st);
-  if (k_bits == 6 && v_bits == 8) return launch_attn<6, 8>(p, grid, smem, st);
-  if (k_bits == 8 && v_bits == 6) return launch_attn<8, 6>(p, grid, smem, st);
-  if (k_bits == 4 && v_bits == 6) return launch_attn<4, 6>(p, grid, smem, st);
-  if (k_bits == 6 && v_bits == 4) return launch_attn<6, 4>(p, grid, smem, st);
-  return -13;
+  return with_kv_bits(k_bits, v_bits, [&](auto kb, auto vb) { return launch_attn<decltype(kb)::value, decltype(vb)::value>(p, grid, smem, st); });
+}
+
+// Arguments as cb_paged_attn; every row block holds at most eight rows (positions x query heads per key / value head), splits <= 64.
+int cb_paged_decode(const void* q, void* out, const void* cache, const void* page_table, const void* rb_req, const void* rb_qstart, const void* rb_qcount,
+                    const void* rb_ctx, int row_blocks, int Hq, int Hkv, int D, int max_pages, int k_bits, int v_bits, float scale, int splits, void* partial,
+                    void* counters, void* status, void* stream) {
+  using namespace cb;
+  if (row_blocks <= 0) return 0;
+  AttnParams p;
+  const int bad = make_attn_params(p, q, out, cache, page_table, rb_req, rb_qstart, rb_qcount, rb_ctx, Hq, Hkv, D, max_pages, k_bits, v_bits, scale, splits, partial, counters,
+                                   status);
+  if (bad) return bad;
+  if (p.G > kDecRows || p.splits > 64) return -14;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return with_kv_bits(k_bits, v_bits, [&](auto kb, auto vb) { return launch_decode<decltype(kb)::value, decltype(vb)::value>(p, row_blocks, st); });
 }
 
 }  // extern "C"

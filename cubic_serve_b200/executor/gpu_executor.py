@@ -115,10 +115,15 @@ class BatchBuilder:
         self.device = device
         self._page_rows: list[tuple[int, int]] = [(-2, 0)] * max_rows
 
-    def _splits(self, row_blocks: int) -> int:
+    def _splits(self, row_blocks: int, decode: bool = False) -> int:
+        """KV splits of a step.  Four CTAs of the decode form run on an SM where the general kernel has two, so from one
+        CTA an SM on twice as many are wanted (48 rows x 8 heads: 33.6 us in one split, 30.7 in two, 33.1 in four); with
+        fewer the merge of more splits costs what they gain."""
         from ..ops.strategies import active
         a = active().attention
         ctas = max(1, row_blocks * self.kv_heads)
+        if decode and ctas * 2 >= a.target_ctas:
+            ctas = -(-ctas // 2)
         return int(min(a.max_splits, max(1, -(-a.target_ctas // ctas))))
 
     def fill(self, segs: list[Segment], pad_rows_to: int | None = None):
@@ -147,7 +152,7 @@ class BatchBuilder:
         st = self.stage
         h = st.h
         qb = self.qb
-        axes, embeds = False, []
+        axes, embeds, decode = False, [], False
         for s in segs:
             self._sync_page_row(s)
         if all(len(s.token_ids) == 1 for s in segs):
@@ -171,6 +176,7 @@ class BatchBuilder:
             h["seg_pos0"][:n] = starts
             t = rb = nseg = n
             rows = 0
+            decode = self.qb >= 2                                 # one position of at most eight heads per row block
             if all(s.sample for s in segs):
                 h["row_slot"][:n] = h["rb_req"][:n]
                 h["budget_init"][:n] = [s.budget_init for s in segs]
@@ -247,11 +253,12 @@ class BatchBuilder:
         else:
             rows_cap = rows
         d = st.d
-        splits = self._splits(rb)
+        splits = self._splits(rb, decode)
         return StepBatch(num_tokens=t, num_row_blocks=rb, num_logit_rows=rows_cap, token_ids=d["token_ids"],
                          positions=d["positions"], slots=d["slots"], page_table=d["page_table"], rb_req=d["rb_req"],
                          rb_qstart=d["rb_qstart"], rb_qcount=d["rb_qcount"], rb_ctx=d["rb_ctx"],
                          logit_rows=d["logit_rows"], attn_splits=splits,
+                         attn_decode=decode,
                          segments=K.GdnSegments(d["seg_row0"], d["seg_count"], d["seg_slot"], d["seg_pos0"], nseg),
                          positions_hw=(d["positions_h"], d["positions_w"]) if axes else None,
                          embeds=[(first, feat.to(self.device, torch.bfloat16, non_blocking=True))

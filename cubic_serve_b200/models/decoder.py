@@ -265,6 +265,7 @@ class StepBatch:
     rb_ctx: torch.Tensor
     logit_rows: torch.Tensor     # int64 [R] rows of the hidden state that feed lm_head
     attn_splits: int = 1
+    attn_decode: bool = False    # no row block holds more than eight rows (K.paged_attention, ``form``)
     segments: object | None = None   # K.GdnSegments: the step's rows grouped by request (Gated DeltaNet layers)
     # multimodal prefill steps (one GPU): row- and column-axis rotary positions int32 [T] each (``positions`` is then
     # the temporal axis) and encoder feature rows ``[(first row, bf16 [n, H])]`` that replace token embeddings
@@ -424,6 +425,12 @@ class DecoderRunner(StepRunner):
                     eps_norm=self.cfg.rms_eps, commit=rec is None)
         return out
 
+    def _attend(self, b: StepBatch, q: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, rb0: int, rb1: int) -> None:
+        """Attention of the row blocks ``[rb0, rb1)``."""
+        K.paged_attention(q, out, kv, b.page_table, b.rb_req[rb0:rb1], b.rb_qstart[rb0:], b.rb_qcount[rb0:], b.rb_ctx[rb0:], self.hq, self.hkv,
+                          self.D, self.k_bits, self.v_bits, scale=self.cfg.attention_scale, splits=b.attn_splits, ws=self.ws,
+                          form="decode" if b.attn_decode else "")
+
     def begin_gdn_review(self, rows: int) -> None:
         """The next ``forward_hidden`` is a speculative review pass over ``rows`` token rows: Gated DeltaNet layers
         leave their state untouched and keep their projections for ``fold_gdn``."""
@@ -512,9 +519,7 @@ class DecoderRunner(StepRunner):
                                 self.D, self.k_bits, self.v_bits, q_norm=lw.q_norm, k_norm=lw.k_norm, eps=cfg.rms_eps,
                                 rotary_dim=cfg.rotary_dim, rotate=self.kv_rotation, positions_hw=hw,
                                 mrope_section=cfg.mrope_section if hw is not None else None, qkv_bias=lw.qkv_bias)
-                K.paged_attention(q_all, attn_all, self.kv[li], b.page_table, b.rb_req[rb0:rb1], b.rb_qstart[rb0:],
-                                  b.rb_qcount[rb0:], b.rb_ctx[rb0:], self.hq, self.hkv, self.D, self.k_bits, self.v_bits,
-                                  scale=cfg.attention_scale, splits=b.attn_splits, ws=self.ws)
+                self._attend(b, q_all, attn_all, self.kv[li], rb0, rb1)
                 n += 4
                 if self.kv_rotation:
                     K.hadamard(attn)
@@ -596,9 +601,7 @@ class DecoderRunner(StepRunner):
             K.rope_kv_write(qkv, q, self.kv[li], b.positions, b.slots, self.inv_freq, self.hq, self.hkv, self.D,
                             self.k_bits, self.v_bits, q_norm=lw.q_norm, k_norm=lw.k_norm, eps=cfg.rms_eps,
                             rotary_dim=cfg.rotary_dim, rotate=self.kv_rotation, qkv_bias=lw.qkv_bias)
-            K.paged_attention(q.view(T, self.hq, self.D), attn.view(T, self.hq, self.D), self.kv[li], b.page_table,
-                              b.rb_req[:b.num_row_blocks], b.rb_qstart, b.rb_qcount, b.rb_ctx, self.hq, self.hkv,
-                              self.D, self.k_bits, self.v_bits, scale=cfg.attention_scale, splits=b.attn_splits, ws=self.ws)
+            self._attend(b, q.view(T, self.hq, self.D), attn.view(T, self.hq, self.D), self.kv[li], 0, b.num_row_blocks)
             if self.kv_rotation:
                 K.hadamard(attn)
                 n += 1

@@ -520,20 +520,24 @@ def copy_rows(t: torch.Tensor, src: torch.Tensor, dst: torch.Tensor) -> None:
 def paged_attention(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, page_table: torch.Tensor,
                     rb_req: torch.Tensor, rb_qstart: torch.Tensor, rb_qcount: torch.Tensor, rb_ctx: torch.Tensor,
                     hq: int, hkv: int, head_dim: int, k_bits: int, v_bits: int, scale: float | None = None,
-                    splits: int = 1, ws: Workspace | None = None) -> torch.Tensor:
-    """Attention of row blocks over the paged quantized cache (see ``csrc/paged_attn.cu``)."""
+                    splits: int = 1, ws: Workspace | None = None, form: str = "") -> torch.Tensor:
+    """Attention of row blocks over the paged quantized cache (see ``csrc/paged_attn.cu``).
+
+    ``form``: what the caller knows of the row blocks.  ``"decode"``: none holds more than eight rows (positions x query heads
+    per key / value head)."""
     rbs = rb_req.numel()
     ws = ws or workspace(q.device)
     l = native.lib()
+    entry = {"": "cb_paged_attn", "decode": "cb_paged_decode"}[form]
     if splits > 1:
         ws.ensure_attn(l.cb_paged_attn_partial_floats(rbs, hkv, splits))
         assert rbs * hkv <= ws.attn_counters.numel()
-    code = l.cb_paged_attn(q.data_ptr(), out.data_ptr(), cache.data_ptr(), page_table.data_ptr(), rb_req.data_ptr(),
-                           rb_qstart.data_ptr(), rb_qcount.data_ptr(), rb_ctx.data_ptr(), rbs, hq, hkv, head_dim,
-                           page_table.shape[1], k_bits, v_bits,
-                           float(scale if scale is not None else 1.0 / math.sqrt(head_dim)), splits,
-                           ws.attn.data_ptr(), ws.attn_counters.data_ptr(), ws.status.data_ptr(), _stream())
-    native.check(code, "cb_paged_attn")
+    code = getattr(l, entry)(q.data_ptr(), out.data_ptr(), cache.data_ptr(), page_table.data_ptr(), rb_req.data_ptr(),
+                             rb_qstart.data_ptr(), rb_qcount.data_ptr(), rb_ctx.data_ptr(), rbs, hq, hkv, head_dim,
+                             page_table.shape[1], k_bits, v_bits,
+                             float(scale if scale is not None else 1.0 / math.sqrt(head_dim)), splits,
+                             ws.attn.data_ptr(), ws.attn_counters.data_ptr(), ws.status.data_ptr(), _stream())
+    native.check(code, entry)
     return out
 
 

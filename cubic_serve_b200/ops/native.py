@@ -250,8 +250,9 @@ def _declare(l: ctypes.CDLL) -> None:
     l.cb_copy_pages.restype = i
     l.cb_paged_attn_partial_floats.argtypes = [i, i, i]
     l.cb_paged_attn_partial_floats.restype = ll
-    l.cb_paged_attn.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, f, i, vp, vp, vp, vp]
-    l.cb_paged_attn.restype = i
+    for entry in (l.cb_paged_attn, l.cb_paged_decode):
+        entry.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, f, i, vp, vp, vp, vp]
+        entry.restype = i
     l.cb_sample.argtypes = [vp, i, i, vp, i, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp]
     l.cb_sample.restype = i
     l.cb_verify_greedy.argtypes = [vp, vp, vp, i, vp, vp, vp, i, vp]

@@ -1,0 +1,87 @@
+"""The decode form of paged attention against the general kernel (itself tested against the dense oracle) and, for one layout,
+against the oracle."""
+
+import pytest
+import torch
+
+from cubic_serve_b200.ops import eager
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+D = 128
+
+
+def _cache(tokens, hkv, kb, vb, seed):
+    """Pages of random codes; token slots past a request's length hold NaN scales.  Returns the cache and the page table."""
+    g = torch.Generator().manual_seed(seed)
+    lay = eager.blob_layout(D, kb, vb)
+    per = [-(-n // 16) for n in tokens]
+    order = torch.randperm(sum(per), generator=g).tolist()
+    blob = torch.randint(0, 256, (sum(per), hkv, lay["bytes"]), dtype=torch.uint8, generator=g)
+    table = torch.zeros(len(tokens), max(per), dtype=torch.int32)
+    at = 0
+    for r, n in enumerate(tokens):
+        for j in range(per[r]):
+            page = order[at]
+            at += 1
+            table[r, j] = page
+            for name, end, s in (("k_scale", "v_code", 0.05), ("v_scale", "bytes", 0.02)):
+                scale = (torch.rand(hkv, 16, D // 32, generator=g) + 0.5) * s * 127 / ((1 << ((kb if name == "k_scale" else vb) - 1)) - 1)
+                scale[:, max(0, n - 16 * j):] = float("nan")
+                blob[page, :, lay[name]:lay[end]] = scale.reshape(hkv, -1).contiguous().view(torch.uint8).reshape(hkv, -1)
+    return blob.to(DEV), table.to(DEV)
+
+
+def _run(form, q, cache, table, blocks, hq, hkv, kb, vb, splits):
+    from cubic_serve_b200.ops import kernels as K
+    rb = [torch.tensor(c, dtype=torch.int32, device=DEV) for c in zip(*blocks)]
+    out = torch.full_like(q, 7.0)
+    K.paged_attention(q, out, cache, table, *rb, hq, hkv, D, kb, vb, scale=0.05, splits=splits, form=form)
+    ws = K.workspace(torch.device(DEV, 0))
+    ws.check_status()
+    assert not ws.attn_counters.any()
+    return out
+
+
+def _close(a, b):
+    """Probabilities are rounded to f16 (2^-11) relative to another running maximum, sums run in another order, results are rounded
+    to bf16 (2^-8): two steps of the value, or of a small part of the row's scale."""
+    a, b = a.float(), b.float()
+    assert torch.isfinite(a).all()
+    return ((a - b).abs() <= 2.0 ** -7 * b.abs() + 2.0 ** -8 * b.square().mean(-1, keepdim=True).sqrt()).all()
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (4, 8), (6, 6), (4, 4), (8, 4), (6, 8), (8, 6), (4, 6), (6, 4)])
+@pytest.mark.parametrize("group", [1, 4, 8])
+def test_decode_form(kb, vb, group):
+    hkv = 2
+    tokens = [1, 15, 16, 17, 47, 129, 1000, 300]
+    cache, table = _cache(tokens, hkv, kb, vb, kb * vb + group)
+    q = torch.randn(len(tokens), group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)).bfloat16()
+    blocks = [(r, r, 0 if r == 5 else 1, n) for r, n in enumerate(tokens)]                # request 5 is padding
+    want = _run("", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
+    for splits in (1, 2, 7, 32):
+        got = _run("decode", q, cache, table, blocks, group * hkv, hkv, kb, vb, splits)
+        assert (got[5] == 7).all() and _close(got[:5], want[:5]) and _close(got[6:], want[6:])
+
+
+def test_decode_form_against_the_oracle():
+    hkv, group, n = 2, 4, 333
+    cache, table = _cache([n], hkv, 8, 8, 5)
+    q = torch.randn(1, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)).bfloat16()
+    kv = [[eager.decode_cache_page(cache[p, h].cpu(), D, 8, 8) for h in range(hkv)] for p in table[0].tolist()]
+    k, v = (torch.stack([torch.cat([page[h][i] for page in kv])[:n] for h in range(hkv)], 1) for i in (0, 1))
+    ref = eager.attention_rows(q.cpu(), k, v, torch.tensor([n]), 0.05)
+    assert _close(_run("decode", q, cache, table, [(0, 0, 1, n)], group * hkv, hkv, 8, 8, 2).cpu(), ref)
+
+
+def test_decode_form_reports_too_many_rows():
+    from cubic_serve_b200.ops import kernels as K
+    from cubic_serve_b200.ops.native import NativeLibraryError
+    cache, table = _cache([40], 1, 8, 8, 6)
+    q = torch.randn(4, 4, D, device=DEV).bfloat16()
+    with pytest.raises(NativeLibraryError):
+        _run("decode", q, cache, table, [(0, 0, 4, 37)], 4, 1, 8, 8, 1)
+    with pytest.raises(NativeLibraryError):
+        K.paged_attention(q.view(1, 16, D), torch.empty(1, 16, D, device=DEV, dtype=torch.bfloat16), cache, table, *(torch.ones(1, dtype=torch.int32, device=DEV) for _ in range(4)),
+                          16, 1, D, 8, 8, form="decode")
