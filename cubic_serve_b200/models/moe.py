@@ -61,6 +61,7 @@ class MoeLayer:
     shared_gate_up: wq_pack.PackedWeight | None = None    # [2 Is(/tp), H]
     shared_down: wq_pack.PackedWeight | None = None       # [H, Is(/tp)]
     shared_gate: wq_pack.PackedWeight | None = None       # bf16 [8, H]: row 0 is the gate vector, the others zero
+    least_rows: int = 0                                   # rows of a work item of a small step (set with the scratch)
 
     def fuse_activation(self) -> None:
         """Re-order every expert's ``[gate; up]`` rows so that the grouped GEMM applies SwiGLU in its epilogue."""
@@ -99,6 +100,7 @@ class MoeLayer:
             big = max_tokens * self.top_k >= pol.large_routes_per_expert * self.expert_count
             mb = pol.rows_per_item_large if big else pol.rows_per_item_small
             self.scratch = K.MoeScratch(max_tokens, self.top_k, hidden, self.gate_up.n, self.expert_count, mb, device)
+            self.least_rows = mb
             self.logits = torch.empty(max_tokens, self.num_experts, dtype=torch.bfloat16, device=device)
             self.out = torch.empty(max_tokens, hidden, dtype=torch.bfloat16, device=device)
             if self.shared_gate_up is not None:
@@ -119,6 +121,7 @@ class MoeLayer:
         t, h = x.shape
         sc = self.ensure_scratch(runner.max_tokens if runner is not None else t, h, x.device)
         ws = runner.ws if runner is not None else None
+        sc.mb = K.rows_per_work_item(t * self.top_k, self.num_experts, self.least_rows)
         logits = K.wq_gemm(x, self.router, out=self.logits[:t], ws=ws)
         K.moe_route(logits, x, self.top_k, sc, self.normalize, self.expert_lo, self.expert_count)
         rows = t * self.top_k

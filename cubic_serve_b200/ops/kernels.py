@@ -611,7 +611,8 @@ class MoeScratch:
 
     def __init__(self, max_tokens: int, top_k: int, hidden: int, inter2: int, local_experts: int, mb: int, device) -> None:
         routes = max_tokens * top_k
-        self.mb = mb
+        self.mb = mb                         # rows of a work item; a step may take more (``rows_per_item``)
+        self.local_experts = local_experts
         self.max_items = -(-routes // mb) + local_experts
         i32 = dict(dtype=torch.int32, device=device)
         self.topk_ids = torch.empty(max_tokens, top_k, **i32)
@@ -623,11 +624,30 @@ class MoeScratch:
         self.tiles = torch.zeros(1 + 3 * self.max_items, **i32)
         self.route_pos = torch.empty(max_tokens, top_k, **i32)
         bf = dict(dtype=torch.bfloat16, device=device)
-        # + mb rows of slack: a work item's TMA tile may run past the last route (those rows are never stored)
-        self.xs = torch.zeros(routes + mb, hidden, **bf)
-        self.gu = torch.zeros(routes + mb, inter2, **bf)
-        self.act = torch.zeros(routes + mb, inter2 // 2, **bf)
-        self.y = torch.zeros(routes + mb, hidden, **bf)
+        # + 256 rows of slack: a work item's TMA tile may run past the last route (those rows are never stored)
+        slack = max(mb, 256)
+        self.xs = torch.zeros(routes + slack, hidden, **bf)
+        self.gu = torch.zeros(routes + slack, inter2, **bf)
+        self.act = torch.zeros(routes + slack, inter2 // 2, **bf)
+        self.y = torch.zeros(routes + slack, hidden, **bf)
+
+    def items(self, rows: int) -> int:
+        """Most work items that ``rows`` routes can make.  The per-tile kernel launches a CTA for every one of them and weight
+        tile: sized by the scratch (8192 tokens), a decode step's launch was nine tenths CTAs that found nothing to do."""
+        return min(self.max_items, rows // self.mb + min(self.local_experts, rows))
+
+
+def rows_per_work_item(rows: int, experts: int, least: int) -> int:
+    """Rows of a work item of the grouped tcgen05 GEMM for ``rows`` routes over ``experts``.  A work item's weights are decoded once
+    whatever its rows, and the decode sets the pace up to 200 of them, so an item should hold all rows of an expert with an
+    average load (three standard deviations of a random routing above the mean), or an even part of them.  Gate / up and down of
+    128 experts (1536 x 2048, 2048 x 768, NVFP4), items of 64 rows -> of this size: 1024 tokens 188 + 109 -> 137 + 92 us (96),
+    2048 tokens 299 + 179 -> 156 + 136 (160), 4096 tokens 531 + 320 -> 291 + 267 (160), 8192 tokens 1000 + 610 -> 514 + 486 (192)."""
+    mean = rows / experts
+    want = mean + 3.0 * math.sqrt(mean)
+    if want <= least:
+        return least
+    return max(least, -(-math.ceil(want / math.ceil(want / 256)) // 16) * 16)
 
 
 def moe_route(router_logits: torch.Tensor, x: torch.Tensor, top_k: int, sc: MoeScratch, normalize: bool = True,
@@ -657,7 +677,7 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
         code = native.lib().cb_wq_gemm_fp8_grouped(a.q.data_ptr(), a.q.stride(0), a.scale.data_ptr(), w.codes.data_ptr(),
                                                    w.meta.data_ptr(), int(w.fmt == FMT_FP8_BLOCK), out.data_ptr(),
                                                    out.stride(0), rows, w.n, w.k,
-                                                   sc.tiles.data_ptr(), sc.max_items, sc.mb, w.codes.shape[0], int(swiglu),
+                                                   sc.tiles.data_ptr(), sc.items(rows), sc.mb, w.codes.shape[0], int(swiglu),
                                                    ws.status.data_ptr(), _stream())
         native.check(code, "cb_wq_gemm_fp8_grouped")
         return out
@@ -671,7 +691,7 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
     entry = native.lib().cb_wq_gemm_grouped_act if swiglu else native.lib().cb_wq_gemm_grouped
     code = entry(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta),
                                            out.data_ptr(), out.stride(0), float(w.alpha), rows, w.n, w.k, w.group_k,
-                                           sc.tiles.data_ptr(), sc.max_items, sc.mb, w.codes.shape[0], code_stride, meta_stride,
+                                           sc.tiles.data_ptr(), sc.items(rows), sc.mb, w.codes.shape[0], code_stride, meta_stride,
                                            ws.status.data_ptr(), _stream())
     native.check(code, "cb_wq_gemm_grouped")
     return out
