@@ -3,13 +3,20 @@
 // One launch after the QKV GEMM replaces the reference's separate q/k norm,
 // M-RoPE (position/qwen_mrope.py:25) and cache quantization kernels
 // (cache_quantization_native.cu:49).  One warp handles one (token, head) at a
-// time; lane l holds channels l, l+32, l+64, l+96, so a rotate-half RoPE pair
-// (c, c+64) and a 32-channel quantization group (c/32) are both warp-local.
+// time; lane l holds channels 4 l .. 4 l + 3: one 8-byte load and store for q, the
+// eight lanes of a 32-channel quantization group are neighbours (three exchanges
+// for its maximum), a rotate-half pair (c, c + 64) is lanes l and l ^ 16, and the
+// four codes are one word of the K planes and one chunk of the V planes.
+//
+// What bounds it: with a channel of every 32 per lane (2-byte accesses, byte and
+// per-code atomic stores) it was instruction issue: 4096 tokens of 32 + 8 + 8 heads 55 us, 41 us so.
 #include "ptx.cuh"
 #include "kv_layout.cuh"
 #include "launch.cuh"
 
 namespace cb {
+
+static constexpr int kHeadDim = 128;
 
 struct KvWriteParams {
   const __nv_bfloat16* qkv;    // [T, (Hq + 2*Hkv) * D]
@@ -31,8 +38,8 @@ struct KvWriteParams {
   KvLayout lay;
 };
 
-// Normalised Walsh-Hadamard transform of a 128-vector held as v[a] = x[lane + 32 a]: index bits 5-6 are the
-// register index, bits 0-4 the lane.  fp32 stages, the caller rounds once (reference:
+// Normalised Walsh-Hadamard transform of a 128-vector held as v[a] = x[4 lane + a] (the transform treats all index bits alike,
+// so any four of them may be the registers).  fp32 stages, the caller rounds once (reference:
 // ops/cuda/cache_rotation_native.cu:12).  The transform is its own inverse, and q . k is unchanged when both are
 // transformed, so attention over a rotated cache needs only the transform of its output (V's rotation undone).
 __device__ __forceinline__ void hadamard128(float (&v)[4], int lane) {
@@ -50,98 +57,116 @@ __device__ __forceinline__ void hadamard128(float (&v)[4], int lane) {
   for (int k = 0; k < 4; ++k) v[k] *= 0.08838834764831845f;     // 1 / sqrt(128)
 }
 
+// four bytes, or four nibble fields at the bytes' bit `shift`, of a word that other tokens' writers share
+__device__ __forceinline__ void merge_word(uint8_t* at, uint32_t mask, uint32_t bits) {
+  atomicAnd(reinterpret_cast<uint32_t*>(at), ~mask);
+  atomicOr(reinterpret_cast<uint32_t*>(at), bits);
+}
+
+// `v`: channels 4 lane .. 4 lane + 3 of a K or V head vector of token slot `tok` (layout: kv_layout.cuh).
 __device__ __forceinline__ void quantize_store(const float (&v)[4], int bits, bool is_v, uint8_t* blob,
                                                const KvLayout& lay, int tok, int lane) {
   const float qmax = bits == 8 ? 127.f : (bits == 6 ? 31.f : 7.f);
   const int bias = bits == 8 ? 128 : (bits == 6 ? 32 : 8);
   uint8_t* codes = blob + (is_v ? lay.v_code_off : 0);
   float* scales = reinterpret_cast<float*>(blob + (is_v ? lay.v_scale_off : lay.k_scale_off));
+  float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+  const float scale = amax > 0.f ? amax / qmax : 1.f;
+  uint32_t word = 0;                                     // the four codes, a byte each
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const float amax = warp_max(fabsf(v[k]));
-    const float scale = amax > 0.f ? amax / qmax : 1.f;
-    float c = rintf(v[k] / scale);
-    c = fminf(fmaxf(c, -qmax), qmax);
-    uint32_t code = static_cast<uint32_t>(static_cast<int>(c) + bias);
-    const int ch = lane + 32 * k;
-    int shift;
-    if (bits == 6) {
-      // two high bits into the second plane (the fields of one 32-bit word come from several lanes and from
-      // several tokens = several warps: atomics), low nibble as a 4-bit code below
-      const int pos = is_v ? v_hi_pos(lay.head_dim, tok, ch, &shift) : k_hi_pos(lay.head_dim, tok, ch, &shift);
-      uint32_t* word = reinterpret_cast<uint32_t*>(codes + pos);
-      atomicAnd(word, ~(0x3u << shift));
-      atomicOr(word, (code >> 4) << shift);
-      code &= 15u;
-    }
+    const float c = fminf(fmaxf(rintf(v[k] / scale), -qmax), qmax);
+    word |= static_cast<uint32_t>(static_cast<int>(c) + bias) << (8 * k);
+  }
+  const int blk = lane >> 3, t = lane & 3;
+  if ((lane & 7) == 0) scales[tok * (kHeadDim / kKvGroup) + blk] = scale;
+  if (!is_v) {
     if (bits == 8) {
-      const int pos = is_v ? v_code_pos(8, lay.head_dim, tok, ch, &shift) : k_code_pos(8, tok, ch, &shift);
-      codes[pos] = static_cast<uint8_t>(code);
-    } else if (!is_v) {
-      // channels c and c+16 of a 32-block share a byte: lanes l and l+16
-      const uint32_t other = __shfl_down_sync(0xffffffffu, code, 16);
-      if (lane < 16) {
-        const int pos = k_code_pos(4, tok, ch, &shift);
-        codes[pos] = static_cast<uint8_t>(code | (other << 4));
-      }
-    } else {
-      // even/odd tokens share a byte and may be written by different warps
-      const int pos = v_code_pos(4, lay.head_dim, tok, ch, &shift);
-      uint32_t* word = reinterpret_cast<uint32_t*>(codes + (pos & ~3));
-      const int bit = (pos & 3) * 8 + shift;
-      atomicAnd(word, ~(0xFu << bit));
-      atomicOr(word, code << bit);
+      *reinterpret_cast<uint32_t*>(codes + (lane >> 2) * 256 + tok * 16 + t * 4) = word;
+      return;
     }
-    if (lane == 0) scales[tok * (lay.head_dim / kKvGroup) + k] = scale;
+    // lanes t and t + 4 of a block: channels c and c + 16 share bytes
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, word, 4);
+    if (lane & 4) return;
+    *reinterpret_cast<uint32_t*>(codes + blk * 256 + tok * 16 + t * 4) = (word & 0x0F0F0F0Fu) | ((other & 0x0F0F0F0Fu) << 4);
+    if (bits == 6) {
+      const uint32_t hi = (word & 0x30303030u) | ((other & 0x30303030u) << 2);        // bits 4..7 of every byte
+      merge_word(codes + kPageTokens * kHeadDim / 2 + blk * 128 + (tok & 7) * 16 + t * 4, tok < 8 ? 0xF0F0F0F0u : 0x0F0F0F0Fu, tok < 8 ? hi : hi >> 4);
+    }
+    return;
+  }
+  const int pair = tok >> 1, chunk = lane ^ ((pair & 3) << 2);
+  if (bits == 8) {
+    uint8_t* at = codes + pair * (kHeadDim * 2) + chunk * 8 + (tok & 1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) at[2 * k] = static_cast<uint8_t>(word >> (8 * k));
+    return;
+  }
+  // even and odd tokens share bytes
+  const int odd = tok & 1;
+  merge_word(codes + pair * kHeadDim + chunk * 4, odd ? 0xF0F0F0F0u : 0x0F0F0F0Fu, odd ? (word & 0x0F0F0F0Fu) << 4 : word & 0x0F0F0F0Fu);
+  if (bits == 6) {
+    const int shift = (pair < 4 ? 0 : 4) - 2 * odd;      // bits 4, 5 of a code to bit 4 or 0, two further for odd tokens
+    const uint32_t hi = word & 0x30303030u;
+    merge_word(codes + kPageTokens * kHeadDim / 2 + (pair & 3) * kHeadDim + chunk * 4, shift >= 0 ? 0x30303030u >> shift : 0x30303030u << -shift,
+               shift >= 0 ? hi >> shift : hi << -shift);
   }
 }
 
 static constexpr int kRopeWarps = 8;
 
 // One CTA per token; its eight warps share the token's heads (warp w takes heads w, w + 8, ...).  The rotary
-// angles depend on (position, channel) only, so each lane computes its two sin / cos pairs ONCE and reuses them
-// for every head of the token: full-precision sincosf on arguments of thousands of radians is the expensive
-// part of this kernel, and one warp per (token, head) paid it 6x as often.
+// angles depend on (position, channel) only, so the CTA computes its sin / cos pairs ONCE, a thread each, and reuses them
+// for every head of the token: full-precision sincosf on arguments of thousands of radians is expensive.
 __global__ void __launch_bounds__(kRopeWarps * 32)
 rope_kv_write_kernel(const KvWriteParams p) {
+  __shared__ __align__(16) float sn_s[64], cs_s[64];
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int heads = p.Hq + 2 * p.Hkv;
-  const int D = p.lay.head_dim;  // == 128
   const int half = p.rotary_dim >> 1;
-  const float pos = static_cast<float>(p.positions[t]);
-  // three-axis form: frequency slot j turns by the position on its axis (interleaved layout: temporal by default, the
-  // row axis on slots 1, 4, 7, .., the column axis on 2, 5, 8, .. as far as their counts reach)
-  auto slot_pos = [&](int j) -> float {
-    if (p.pos_h == nullptr) return pos;
-    const int r = j % 3;
-    if (r == 1 && j < 3 * p.mrope_h) return static_cast<float>(p.pos_h[t]);
-    if (r == 2 && j < 3 * p.mrope_w) return static_cast<float>(p.pos_w[t]);
-    return pos;
-  };
-  float sn[2] = {0.f, 0.f}, cs[2] = {1.f, 1.f};
-  if (half == 64) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) sincosf(slot_pos(lane + 32 * k) * p.inv_freq[lane + 32 * k], &sn[k], &cs[k]);
-  } else if (half == 32) {
-    sincosf(slot_pos(lane) * p.inv_freq[lane], &sn[0], &cs[0]);
+  if (threadIdx.x < half) {
+    // three-axis form: frequency slot j turns by the position on its axis (interleaved layout: temporal by default, the
+    // row axis on slots 1, 4, 7, .., the column axis on 2, 5, 8, .. as far as their counts reach)
+    const int j = threadIdx.x, r = j % 3;
+    int pos = p.positions[t];
+    if (p.pos_h != nullptr) {
+      if (r == 1 && j < 3 * p.mrope_h) pos = p.pos_h[t];
+      if (r == 2 && j < 3 * p.mrope_w) pos = p.pos_w[t];
+    }
+    sincosf(static_cast<float>(pos) * p.inv_freq[j], &sn_s[j], &cs_s[j]);
   }
   const int slot = p.slots[t];
+  __syncthreads();
+  // lane's frequency slots: its channels modulo the rotated half
+  const bool turns = 4 * lane < p.rotary_dim, upper = 4 * lane >= half;
+  float4 sn = make_float4(0.f, 0.f, 0.f, 0.f), cs = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (turns) {
+    sn = *reinterpret_cast<const float4*>(sn_s + (4 * lane - (upper ? half : 0)));
+    cs = *reinterpret_cast<const float4*>(cs_s + (4 * lane - (upper ? half : 0)));
+    if (!upper) sn = make_float4(-sn.x, -sn.y, -sn.z, -sn.w);      // a cos - b sin below, b cos + a sin above
+  }
+  const int pair_lane = half >> 2;                                 // lanes between the two channels of a pair
+#pragma unroll 2
   for (int h = warp; h < heads; h += kRopeWarps) {
-    const __nv_bfloat16* src = p.qkv + (static_cast<size_t>(t) * heads + h) * D;
     float v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __bfloat162float(src[lane + 32 * k]);
+    {
+      const uint2 raw = *reinterpret_cast<const uint2*>(p.qkv + (static_cast<size_t>(t) * heads + h) * kHeadDim + 4 * lane);
+      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+      v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+    }
     if (p.qkv_bias != nullptr) {
       // the projection's output was rounded to bf16 by the GEMM; the sum is rounded again, as an unfused add would
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        v[k] = __bfloat162float(__float2bfloat16(v[k] + __bfloat162float(p.qkv_bias[h * D + lane + 32 * k])));
+        v[k] = __bfloat162float(__float2bfloat16(v[k] + __bfloat162float(p.qkv_bias[h * kHeadDim + 4 * lane + k])));
     }
-
     const bool is_q = h < p.Hq;
     const bool is_k = !is_q && h < p.Hq + p.Hkv;
     if (is_q || is_k) {
@@ -149,33 +174,27 @@ rope_kv_write_kernel(const KvWriteParams p) {
       if (nw) {
         float ss = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
         ss = warp_sum(ss);
-        const float inv = rsqrtf(ss / static_cast<float>(D) + p.eps);
+        const float inv = rsqrtf(ss / static_cast<float>(kHeadDim) + p.eps);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           // round to bf16 after the norm, as an unfused norm kernel would
-          v[k] = __bfloat162float(__float2bfloat16(v[k] * inv * __bfloat162float(nw[lane + 32 * k])));
+          v[k] = __bfloat162float(__float2bfloat16(v[k] * inv * __bfloat162float(nw[4 * lane + k])));
         }
       }
-      // pairs (c, c + half) for c < half; with D = 128 and half = 64: (l, l+64), (l+32, l+96)
-      if (half == 64) {
+      if (half) {
+        float o[4];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const float a = v[k], b = v[k + 2];
-          v[k] = a * cs[k] - b * sn[k];
-          v[k + 2] = b * cs[k] + a * sn[k];
+        for (int k = 0; k < 4; ++k) o[k] = __shfl_xor_sync(0xffffffffu, v[k], pair_lane);
+        if (turns) {
+          v[0] = v[0] * cs.x + o[0] * sn.x; v[1] = v[1] * cs.y + o[1] * sn.y;
+          v[2] = v[2] * cs.z + o[2] * sn.z; v[3] = v[3] * cs.w + o[3] * sn.w;
         }
-      } else if (half == 32) {
-        // partial rotary over the first 64 channels: pairs (l, l+32)
-        const float a = v[0], b = v[1];
-        v[0] = a * cs[0] - b * sn[0];
-        v[1] = b * cs[0] + a * sn[0];
       }
     }
     if (p.rotate) hadamard128(v, lane);
+    const uint2 bf = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
     if (is_q) {
-      __nv_bfloat16* dst = p.q_out + (static_cast<size_t>(t) * p.Hq + h) * D;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) dst[lane + 32 * k] = __float2bfloat16(v[k]);
+      *reinterpret_cast<uint2*>(p.q_out + (static_cast<size_t>(t) * p.Hq + h) * kHeadDim + 4 * lane) = bf;
       continue;
     }
     if (slot < 0) continue;
@@ -183,9 +202,9 @@ rope_kv_write_kernel(const KvWriteParams p) {
     const int page = slot >> 4, tok = slot & 15;
     uint8_t* blob = p.cache + (static_cast<size_t>(page) * p.Hkv + kvh) * p.lay.blob_bytes;
     // the cache stores what attention will see: bf16-rounded values
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __bfloat162float(__float2bfloat16(v[k]));
-    quantize_store(v, is_k ? p.lay.k_bits : p.lay.v_bits, !is_k, blob, p.lay, tok, lane);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&bf.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&bf.y));
+    const float r[4] = {lo.x, lo.y, hi.x, hi.y};
+    quantize_store(r, is_k ? p.lay.k_bits : p.lay.v_bits, !is_k, blob, p.lay, tok, lane);
   }
 }
 
@@ -203,11 +222,11 @@ hadamard_kernel(const __nv_bfloat16* __restrict__ x, int ldx, __nv_bfloat16* __r
   const __nv_bfloat16* src = x + static_cast<size_t>(r) * ldx + h * 128;
   __nv_bfloat16* dst = y + static_cast<size_t>(r) * ldy + h * 128;
   float v[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) v[k] = __bfloat162float(src[lane + 32 * k]);
+  const uint2 raw = *reinterpret_cast<const uint2*>(src + 4 * lane);
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
   hadamard128(v, lane);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) dst[lane + 32 * k] = __float2bfloat16(v[k]);
+  *reinterpret_cast<uint2*>(dst + 4 * lane) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
 }
 
 // Copy whole pages (all kv heads) src -> dst: copy-on-write of a shared page.

@@ -63,41 +63,4 @@ __host__ __device__ inline KvLayout make_kv_layout(int head_dim, int k_bits, int
   return l;
 }
 
-// byte offset (and nibble shift for 4-bit) of K element (tok, ch) inside the K code region
-__host__ __device__ inline int k_code_pos(int bits, int tok, int ch, int* shift) {
-  if (bits == 8) {
-    *shift = 0;
-    return (ch >> 4) * 256 + tok * 16 + (ch & 15);
-  }
-  const int blk = ch >> 5, c = ch & 31;
-  *shift = (c >= 16) ? 4 : 0;
-  return blk * 256 + tok * 16 + (c & 15);
-}
-
-// 6-bit: byte offset of the 32-bit word of high bits (relative to the START of the code region, i.e. past the
-// nibble plane) and the bit position of the two high bits of element (tok, ch)
-__host__ __device__ inline int k_hi_pos(int head_dim, int tok, int ch, int* shift) {
-  const int blk = ch >> 5, c = ch & 31;
-  *shift = 8 * (c & 3) + ((tok >= 8) ? 0 : 4) + ((c >= 16) ? 2 : 0);
-  return kPageTokens * head_dim / 2 + blk * 128 + (tok & 7) * 16 + ((c & 15) >> 2) * 4;
-}
-__host__ __device__ inline int v_hi_pos(int head_dim, int tok, int ch, int* shift) {
-  const int p = tok >> 1;
-  const int chunk = (ch >> 2) ^ ((p & 3) << 2);
-  *shift = 8 * (ch & 3) + ((p >= 4) ? 0 : 4) + ((tok & 1) ? 2 : 0);
-  return kPageTokens * head_dim / 2 + (p & 3) * head_dim + chunk * 4;
-}
-
-// byte offset (and nibble shift) of V element (tok, ch) inside the V code region
-__host__ __device__ inline int v_code_pos(int bits, int head_dim, int tok, int ch, int* shift) {
-  const int p = tok >> 1;
-  const int chunk = (ch >> 2) ^ ((p & 3) << 2);
-  if (bits == 8) {
-    *shift = 0;
-    return p * (head_dim * 2) + chunk * 8 + (ch & 3) * 2 + (tok & 1);
-  }
-  *shift = (tok & 1) ? 4 : 0;
-  return p * head_dim + chunk * 4 + (ch & 3);
-}
-
 }  // namespace cb
