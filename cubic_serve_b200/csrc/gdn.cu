@@ -21,6 +21,7 @@
 // Reference counterparts: ops/cuda/linear_attention/causal_conv_native.cu:13, gated_delta_native.cu:36,
 // gated_delta_coefficients_native.cu:17 and the oracle ops/eager/hybrid.py:255-548 (fp32 recurrence branch).
 #include "ptx.cuh"
+#include "segments.cuh"
 
 namespace cb {
 
@@ -33,52 +34,85 @@ struct GdnSegments {
   const int* pos0;      // [S] absolute position of the first row (0 = fresh state)
 };
 
-// grid (ceil(C / 128), segments); one thread per channel walks the segment's rows in order.
+// Tiles of kConvRows rows of a segment x 128 threads of V neighbouring channels.  The convolution has no chain: a tile takes the
+// three inputs before its first row from the rows themselves.  (One thread walking a channel's whole segment left 3000 rows of
+// 8192 channels to 320 blocks with four loads in flight each: 290 us where the bytes take 15.)  Only the first tile of a segment
+// touches the request's state: it has read the old inputs before it writes the new ones.
+static constexpr int kConvRows = 32;
+
+template <int V>
 __global__ void __launch_bounds__(128)
 gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, __nv_bfloat16* __restrict__ y, int ldy,
                 const float* __restrict__ w,            // [C, 4], tap 3 multiplies the current input
                 const float* __restrict__ bias,         // [C] or null
                 __nv_bfloat16* __restrict__ state,      // [slots, 3, C]
-                GdnSegments seg, int C, int commit) {
-  const int c = blockIdx.x * 128 + threadIdx.x;
-  const int s = blockIdx.y;
+                Segments seg, int C, int commit) {
+  int s, off;
+  if (!find_tile(seg, kConvRows, blockIdx.y, s, off)) return;
+  const int c = (blockIdx.x * 128 + threadIdx.x) * V;
+  if (c >= C) return;
   const int n = seg.count[s];
-  if (c >= C || n <= 0) return;
-  const int row0 = seg.row0[s];
+  const __nv_bfloat16* xp = x + static_cast<size_t>(seg.row0[s]) * ldx + c;
+  __nv_bfloat16* yp = y + static_cast<size_t>(seg.row0[s]) * ldy + c;
   __nv_bfloat16* st = state + static_cast<size_t>(seg.slot[s]) * 3 * C + c;
-  float h0 = 0.f, h1 = 0.f, h2 = 0.f;                   // inputs at t-3, t-2, t-1
-  if (seg.pos0[s] > 0) {
-    h0 = __bfloat162float(st[0]);
-    h1 = __bfloat162float(st[static_cast<size_t>(C)]);
-    h2 = __bfloat162float(st[static_cast<size_t>(2) * C]);
+  struct Chan { float v[V]; };
+  auto load = [](const __nv_bfloat16* at) {
+    Chan r;
+    if constexpr (V == 2) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(at));
+      r.v[0] = f.x; r.v[1] = f.y;
+    } else {
+      r.v[0] = __bfloat162float(*at);
+    }
+    return r;
+  };
+  auto store = [](__nv_bfloat16* at, const Chan& r) {
+    if constexpr (V == 2) *reinterpret_cast<__nv_bfloat162*>(at) = __floats2bfloat162_rn(r.v[0], r.v[1]);
+    else *at = __float2bfloat16(r.v[0]);
+  };
+  float4 wv[V];
+  float b[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    wv[i] = *reinterpret_cast<const float4*>(w + static_cast<size_t>(c + i) * 4);
+    b[i] = bias ? bias[c + i] : 0.f;
   }
-  const float4 wv = *reinterpret_cast<const float4*>(w + static_cast<size_t>(c) * 4);
-  const float b = bias ? bias[c] : 0.f;
-  const __nv_bfloat16* xp = x + static_cast<size_t>(row0) * ldx + c;
-  __nv_bfloat16* yp = y + static_cast<size_t>(row0) * ldy + c;
-  // four rows per trip: the loads do not depend on the arithmetic, so they are issued together
-  int t = 0;
-  for (; t + 4 <= n; t += 4) {
-    float v[4];
+  Chan h[3] = {};                                       // inputs at t - 3, t - 2, t - 1
+  if (off > 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = __bfloat162float(xp[static_cast<size_t>(t + j) * ldx]);
+    for (int j = 0; j < 3; ++j) h[j] = load(xp + static_cast<size_t>(off - 3 + j) * ldx);
+  } else if (seg.pos0[s] > 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float a = b + wv.x * h0 + wv.y * h1 + wv.z * h2 + wv.w * v[j];
-      yp[static_cast<size_t>(t + j) * ldy] = __float2bfloat16(silu_fast(a));
-      h0 = h1; h1 = h2; h2 = v[j];
+    for (int j = 0; j < 3; ++j) h[j] = load(st + static_cast<size_t>(j) * C);
+  }
+  if (off == 0 && commit) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int t = n - 3 + j;                          // an input before the segment's first is one of the old three
+      const Chan v = t >= 0 ? load(xp + static_cast<size_t>(t) * ldx) : t == -1 ? h[2] : h[1];
+      store(st + static_cast<size_t>(j) * C, v);
     }
   }
-  for (; t < n; ++t) {
-    const float v = __bfloat162float(xp[static_cast<size_t>(t) * ldx]);
-    const float a = b + wv.x * h0 + wv.y * h1 + wv.z * h2 + wv.w * v;
-    yp[static_cast<size_t>(t) * ldy] = __float2bfloat16(silu_fast(a));
-    h0 = h1; h1 = h2; h2 = v;
+  const int end = min(n, off + kConvRows);
+  // eight rows per trip: the loads do not depend on the arithmetic, so they are issued together
+  for (int t = off; t < end; t += 8) {
+    Chan v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (t + j < end) v[j] = load(xp + static_cast<size_t>(t + j) * ldx);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (t + j >= end) break;
+      Chan o;
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const float a = b[i] + wv[i].x * h[0].v[i] + wv[i].y * h[1].v[i] + wv[i].z * h[2].v[i] + wv[i].w * v[j].v[i];
+        o.v[i] = silu_fast(a);
+      }
+      store(yp + static_cast<size_t>(t + j) * ldy, o);
+      h[0] = h[1]; h[1] = h[2]; h[2] = v[j];
+    }
   }
-  if (!commit) return;
-  st[0] = __float2bfloat16(h0);
-  st[static_cast<size_t>(C)] = __float2bfloat16(h1);
-  st[static_cast<size_t>(2) * C] = __float2bfloat16(h2);
 }
 
 struct GdnDeltaParams {
@@ -109,7 +143,7 @@ struct GdnDeltaParams {
 // other's arithmetic.
 //
 // A segment is walked in blocks of 16 tokens, three phases per block:
-//   A (parallel, four warp tasks per token)  L2-normalised q / k, v, z, beta and decay of the block's tokens into shared memory
+//   A (parallel, three warp tasks per token)  L2-normalised q / k, v, z, beta and decay of the block's tokens into shared memory
 //   B (the recurrence, no CTA barrier inside)  per token: decay, S k, delta, rank-one update, S q; outputs to shared memory
 //   C (parallel, a warp per token)  gated RMSNorm of the block's outputs, coalesced stores
 // so the token-serial part is only the arithmetic that really depends on the state.
@@ -133,20 +167,24 @@ gdn_delta_kernel(const GdnDeltaParams p) {
   __shared__ float vs[kGdnBlock][kGdnDim];
   __shared__ float os[kGdnBlock][kGdnDim];
   __shared__ float zs[kGdnBlock][kGdnDim];
-  __shared__ float2 coef[kGdnBlock];                      // {beta, decay}
+  __shared__ float4 coef[kGdnBlock];                      // {beta, decay, k . q}
 
   float* sp = p.state + ((static_cast<size_t>(p.seg.slot[s]) * p.Hv + head) * kGdnDim + vrow) * kGdnDim + l8 * 4;
-  float4 S[4][4];                                        // [row i][chunk c]: columns 4 (l8 + 8 c) .. + 3
+  float2 S[4][4][2];                                     // [row i][chunk c]: columns 4 (l8 + 8 c) .. + 3
   if (p.seg.pos0[s] > 0) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) S[i][c] = *reinterpret_cast<const float4*>(sp + (4 * i) * kGdnDim + 32 * c);
+      for (int c = 0; c < 4; ++c) {
+        const float4 e = *reinterpret_cast<const float4*>(sp + (4 * i) * kGdnDim + 32 * c);
+        S[i][c][0] = make_float2(e.x, e.y);
+        S[i][c][1] = make_float2(e.z, e.w);
+      }
   } else {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) S[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int c = 0; c < 4; ++c) S[i][c][0] = S[i][c][1] = make_float2(0.f, 0.f);
   }
   const float neg_exp_a = -__expf(p.a_log[head]);
   const float dtb = p.dt_bias[head];
@@ -157,28 +195,33 @@ gdn_delta_kernel(const GdnDeltaParams p) {
 
   for (int t0 = 0; t0 < n; t0 += kGdnBlock) {
     const int nb = min(kGdnBlock, n - t0);
-    // ---- A: operands of the block's tokens.  Four independent tasks per token (q, k, v + z, coefficients) dealt
-    // to the eight warps, so that a one-token decode step still uses four warps at once
-    for (int task = warp; task < nb * 4; task += 8) {
-      const int j = task >> 2, part = task & 3;
+    // ---- A: operands of the block's tokens.  Three independent tasks per token (q and k, v and z, coefficients) dealt
+    // to the eight warps, so that a one-token decode step still uses three warps at once
+    for (int task = warp; task < nb * 3; task += 8) {
+      const int j = task / 3, part = task - j * 3;
       const size_t r = static_cast<size_t>(row0 + t0 + j);
       const __nv_bfloat16* row = p.qkv + r * p.ldqkv;
-      if (part < 2) {
+      if (part == 0) {
         // stored boundary of the oracle: normalised q / k are rounded to bf16; q carries the 1 / sqrt(d_k) scale
-        const __nv_bfloat16* src = row + (part == 0 ? q_off : k_off);
-        float x[4];
-        float ss = 0.f;
+        float q[4], k[4], qq = 0.f, kk = 0.f, kq = 0.f;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-          x[a] = __bfloat162float(src[lane + 32 * a]);
-          ss = fmaf(x[a], x[a], ss);
+          q[a] = __bfloat162float(row[q_off + lane + 32 * a]);
+          k[a] = __bfloat162float(row[k_off + lane + 32 * a]);
+          qq = fmaf(q[a], q[a], qq);
+          kk = fmaf(k[a], k[a], kk);
         }
-        const float inv = rsqrtf(warp_sum(ss) + p.eps_l2);
-        float* dst = part == 0 ? qs[j] : ks[j];
-        const float scale = part == 0 ? 0.08838834764831845f : 1.f;
+        const float qi = rsqrtf(warp_sum(qq) + p.eps_l2), ki = rsqrtf(warp_sum(kk) + p.eps_l2);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) dst[lane + 32 * a] = __bfloat162float(__float2bfloat16(x[a] * inv)) * scale;
-      } else if (part == 2) {
+        for (int a = 0; a < 4; ++a) {
+          const float qn = __bfloat162float(__float2bfloat16(q[a] * qi)) * 0.08838834764831845f, kn = __bfloat162float(__float2bfloat16(k[a] * ki));
+          qs[j][lane + 32 * a] = qn;
+          ks[j][lane + 32 * a] = kn;
+          kq = fmaf(kn, qn, kq);
+        }
+        kq = warp_sum(kq);
+        if (lane == 0) coef[j].z = kq;
+      } else if (part == 1) {
         const __nv_bfloat16* zrow = p.z + r * p.ldz + head * kGdnDim;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
@@ -189,56 +232,55 @@ gdn_delta_kernel(const GdnDeltaParams p) {
         const float bb = __bfloat162float(p.ba[r * p.ldba + head]);
         const float x = __bfloat162float(p.ba[r * p.ldba + p.Hv + head]) + dtb;
         const float softplus = x > 20.f ? x : log1pf(__expf(x));
-        coef[j] = make_float2(1.f / (1.f + __expf(-bb)), __expf(neg_exp_a * softplus));
+        coef[j].x = 1.f / (1.f + __expf(-bb));
+        coef[j].y = __expf(neg_exp_a * softplus);
       }
     }
     __syncthreads();
-    // ---- B: the recurrence
+    // ---- B: the recurrence.  The read-out is taken from the decayed state, S q = S' q + (k . q) delta, so that a token has one
+    // reduction over the eight lanes instead of two; fp32 arithmetic two at a time
     for (int j = 0; j < nb; ++j) {
-      const float beta = coef[j].x, decay = coef[j].y;
-      float4 kv[4];
+      const float4 co = coef[j];
+      const float2 decay = make_float2(co.y, co.y);
+      float4 kv[4], qv[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) kv[c] = *reinterpret_cast<const float4*>(&ks[j][4 * (l8 + 8 * c)]);
-      float mem[4];
+      for (int c = 0; c < 4; ++c) {
+        kv[c] = *reinterpret_cast<const float4*>(&ks[j][4 * (l8 + 8 * c)]);
+        qv[c] = *reinterpret_cast<const float4*>(&qs[j][4 * (l8 + 8 * c)]);
+      }
+      float mem[4], o[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float m = 0.f;
+        float2 m = make_float2(0.f, 0.f), a = m;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          float4& e = S[i][c];
-          e.x *= decay; e.y *= decay; e.z *= decay; e.w *= decay;
-          m = fmaf(e.x, kv[c].x, m); m = fmaf(e.y, kv[c].y, m); m = fmaf(e.z, kv[c].z, m); m = fmaf(e.w, kv[c].w, m);
+          S[i][c][0] = __fmul2_rn(S[i][c][0], decay);
+          S[i][c][1] = __fmul2_rn(S[i][c][1], decay);
+          m = __ffma2_rn(S[i][c][0], make_float2(kv[c].x, kv[c].y), m);
+          a = __ffma2_rn(S[i][c][0], make_float2(qv[c].x, qv[c].y), a);
+          m = __ffma2_rn(S[i][c][1], make_float2(kv[c].z, kv[c].w), m);
+          a = __ffma2_rn(S[i][c][1], make_float2(qv[c].z, qv[c].w), a);
         }
-        mem[i] = m;
+        mem[i] = m.x + m.y;
+        o[i] = a.x + a.y;
       }
 #pragma unroll
       for (int sh = 1; sh < 8; sh <<= 1)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mem[i] += __shfl_xor_sync(0xffffffffu, mem[i], sh);
-      float4 qv[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) qv[c] = *reinterpret_cast<const float4*>(&qs[j][4 * (l8 + 8 * c)]);
-      float o[4];
+        for (int i = 0; i < 4; ++i) {
+          mem[i] += __shfl_xor_sync(0xffffffffu, mem[i], sh);
+          o[i] += __shfl_xor_sync(0xffffffffu, o[i], sh);
+        }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float delta = (vs[j][vrow + 4 * i] - mem[i]) * beta;
-        float acc = 0.f;
+        const float delta = (vs[j][vrow + 4 * i] - mem[i]) * co.x;
+        const float2 d = make_float2(delta, delta);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          float4& e = S[i][c];
-          e.x = fmaf(delta, kv[c].x, e.x); e.y = fmaf(delta, kv[c].y, e.y);
-          e.z = fmaf(delta, kv[c].z, e.z); e.w = fmaf(delta, kv[c].w, e.w);
-          acc = fmaf(e.x, qv[c].x, acc); acc = fmaf(e.y, qv[c].y, acc); acc = fmaf(e.z, qv[c].z, acc); acc = fmaf(e.w, qv[c].w, acc);
+          S[i][c][0] = __ffma2_rn(d, make_float2(kv[c].x, kv[c].y), S[i][c][0]);
+          S[i][c][1] = __ffma2_rn(d, make_float2(kv[c].z, kv[c].w), S[i][c][1]);
         }
-        o[i] = acc;
-      }
-#pragma unroll
-      for (int sh = 1; sh < 8; sh <<= 1)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] += __shfl_xor_sync(0xffffffffu, o[i], sh);
-      if (l8 == 0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) os[j][vrow + 4 * i] = __bfloat162float(__float2bfloat16(o[i]));   // stored in bf16
+        if (l8 == 0) os[j][vrow + 4 * i] = __bfloat162float(__float2bfloat16(fmaf(delta, co.z, o[i])));   // stored in bf16
       }
     }
     __syncthreads();
@@ -267,7 +309,8 @@ gdn_delta_kernel(const GdnDeltaParams p) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) *reinterpret_cast<float4*>(sp + (4 * i) * kGdnDim + 32 * c) = S[i][c];
+    for (int c = 0; c < 4; ++c) 
+      *reinterpret_cast<float4*>(sp + (4 * i) * kGdnDim + 32 * c) = make_float4(S[i][c][0].x, S[i][c][0].y, S[i][c][1].x, S[i][c][1].y);
 }
 
 // out = x * sigmoid(gate): the output gate of the hybrid family's full-attention layers (bf16, in place allowed)
@@ -295,15 +338,22 @@ struct CbGdnSegments {
   int num;
 };
 
+// `rows`: rows of the step; x and y do not overlap.
 int cb_gdn_conv(const void* x, int ldx, void* y, int ldy, const void* w, const void* bias, void* state,
-                const CbGdnSegments* seg, int C, int commit, void* stream) {
-  if (!seg || seg->num <= 0 || C <= 0 || seg->num > 65535) return -60;
-  cb::GdnSegments s{static_cast<const int*>(seg->row0), static_cast<const int*>(seg->count),
-                    static_cast<const int*>(seg->slot), static_cast<const int*>(seg->pos0)};
-  dim3 grid((C + 127) / 128, seg->num);
-  cb::gdn_conv_kernel<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy, static_cast<const float*>(w),
-      static_cast<const float*>(bias), static_cast<__nv_bfloat16*>(state), s, C, commit);
+                const CbGdnSegments* seg, int C, int rows, int commit, void* stream) {
+  if (!seg || seg->num <= 0 || C <= 0 || seg->num > 65535 || rows < 0) return -60;
+  if (rows == 0) return 0;
+  const cb::Segments s{static_cast<const int*>(seg->row0), static_cast<const int*>(seg->count), static_cast<const int*>(seg->slot),
+                       static_cast<const int*>(seg->pos0), seg->num, 0};
+  const int tiles = cb::max_tiles(rows, seg->num, cb::kConvRows);
+  if (tiles > 65535) return -60;
+  const bool pairs = C % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(state)) & 3) == 0;
+  const int cols = pairs ? 256 : 128;
+  const dim3 grid((C + cols - 1) / cols, tiles);
+  auto kernel = pairs ? cb::gdn_conv_kernel<2> : cb::gdn_conv_kernel<1>;
+  kernel<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy,
+                                                              static_cast<const float*>(w), static_cast<const float*>(bias),
+                                                              static_cast<__nv_bfloat16*>(state), s, C, commit);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -734,7 +734,7 @@ def gdn_conv(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, seg: GdnSegm
     assert state.dtype == torch.bfloat16 and state.shape[1:] == (3, c) and state.is_contiguous()
     st = seg.struct()
     code = native.lib().cb_gdn_conv(x.data_ptr(), x.stride(0), out.data_ptr(), out.stride(0), w.data_ptr(), _ptr(bias),
-                                    state.data_ptr(), ctypes.byref(st), c, int(commit), _stream())
+                                    state.data_ptr(), ctypes.byref(st), c, x.shape[0], int(commit), _stream())
     native.check(code, "cb_gdn_conv")
     return out
 
