@@ -468,6 +468,8 @@ class GpuExecutor:
         dst = torch.tensor([p[1] for p in pairs], dtype=torch.int32, device=self.device)
         with torch.cuda.stream(self.stream):
             self.runner.copy_state(src, dst)
+        for t in (src, dst):
+            t.record_stream(self.stream)       # read there after this call has returned
 
     def copy_pages(self, pairs) -> None:
         """Copy-on-write page copies (all layers) ahead of a step."""
@@ -478,6 +480,8 @@ class GpuExecutor:
         with torch.cuda.stream(self.stream):
             for cache in self.runner.kv:
                 K.copy_pages(cache, src, dst)
+        for t in (src, dst):
+            t.record_stream(self.stream)       # read there after this call has returned
 
     def execute(self, segs: list[Segment]) -> np.ndarray:
         """Run one step and return the sampled token id of every sampling segment (host array)."""
