@@ -265,7 +265,10 @@ class StepBatch:
     rb_ctx: torch.Tensor
     logit_rows: torch.Tensor     # int64 [R] rows of the hidden state that feed lm_head
     attn_splits: int = 1
-    attn_decode: bool = False    # no row block holds more than eight rows (K.paged_attention, ``form``)
+    # what the attention kernels are told of the row blocks (K.paged_attention, ``form``): none holds more than eight rows;
+    # blocks [lo, hi) belong to portions of prompts
+    attn_decode: bool = False
+    attn_prompts: tuple[int, int] = (0, 0)
     segments: object | None = None   # K.GdnSegments: the step's rows grouped by request (Gated DeltaNet layers)
     # multimodal prefill steps (one GPU): row- and column-axis rotary positions int32 [T] each (``positions`` is then
     # the temporal axis) and encoder feature rows ``[(first row, bf16 [n, H])]`` that replace token embeddings
@@ -425,11 +428,20 @@ class DecoderRunner(StepRunner):
                     eps_norm=self.cfg.rms_eps, commit=rec is None)
         return out
 
-    def _attend(self, b: StepBatch, q: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, rb0: int, rb1: int) -> None:
-        """Attention of the row blocks ``[rb0, rb1)``."""
-        K.paged_attention(q, out, kv, b.page_table, b.rb_req[rb0:rb1], b.rb_qstart[rb0:], b.rb_qcount[rb0:], b.rb_ctx[rb0:], self.hq, self.hkv,
-                          self.D, self.k_bits, self.v_bits, scale=self.cfg.attention_scale, splits=b.attn_splits, ws=self.ws,
-                          form="decode" if b.attn_decode else "")
+    def _attend(self, b: StepBatch, q: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, rb0: int, rb1: int) -> int:
+        """Attention of the row blocks ``[rb0, rb1)``: portions of prompts in one launch, what is before and after them in
+        one each.  Returns the launches."""
+        lo, hi = max(b.attn_prompts[0], rb0), min(b.attn_prompts[1], rb1)
+        if lo >= hi:
+            lo = hi = rb1
+        other, n = "decode" if b.attn_decode else "", 0
+        for first, end, form in ((rb0, lo, other), (lo, hi, "prefill"), (hi, rb1, other)):
+            if first < end:
+                K.paged_attention(q, out, kv, b.page_table, b.rb_req[first:end], b.rb_qstart[first:], b.rb_qcount[first:], b.rb_ctx[first:], self.hq, self.hkv,
+                                  self.D, self.k_bits, self.v_bits, scale=self.cfg.attention_scale, splits=1 if form == "prefill" else b.attn_splits,
+                                  ws=self.ws, form=form)
+                n += 1
+        return n
 
     def begin_gdn_review(self, rows: int) -> None:
         """The next ``forward_hidden`` is a speculative review pass over ``rows`` token rows: Gated DeltaNet layers
@@ -519,8 +531,7 @@ class DecoderRunner(StepRunner):
                                 self.D, self.k_bits, self.v_bits, q_norm=lw.q_norm, k_norm=lw.k_norm, eps=cfg.rms_eps,
                                 rotary_dim=cfg.rotary_dim, rotate=self.kv_rotation, positions_hw=hw,
                                 mrope_section=cfg.mrope_section if hw is not None else None, qkv_bias=lw.qkv_bias)
-                self._attend(b, q_all, attn_all, self.kv[li], rb0, rb1)
-                n += 4
+                n += 3 + self._attend(b, q_all, attn_all, self.kv[li], rb0, rb1)
                 if self.kv_rotation:
                     K.hadamard(attn)
                     n += 1
@@ -601,7 +612,7 @@ class DecoderRunner(StepRunner):
             K.rope_kv_write(qkv, q, self.kv[li], b.positions, b.slots, self.inv_freq, self.hq, self.hkv, self.D,
                             self.k_bits, self.v_bits, q_norm=lw.q_norm, k_norm=lw.k_norm, eps=cfg.rms_eps,
                             rotary_dim=cfg.rotary_dim, rotate=self.kv_rotation, qkv_bias=lw.qkv_bias)
-            self._attend(b, q.view(T, self.hq, self.D), attn.view(T, self.hq, self.D), self.kv[li], 0, b.num_row_blocks)
+            n += self._attend(b, q.view(T, self.hq, self.D), attn.view(T, self.hq, self.D), self.kv[li], 0, b.num_row_blocks) - 1
             if self.kv_rotation:
                 K.hadamard(attn)
                 n += 1

@@ -524,11 +524,11 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, pag
     """Attention of row blocks over the paged quantized cache (see ``csrc/paged_attn.cu``).
 
     ``form``: what the caller knows of the row blocks.  ``"decode"``: none holds more than eight rows (positions x query heads
-    per key / value head)."""
+    per key / value head); ``"prefill"``: they mostly follow one another in one request (``csrc/paged_prefill.cu``, one split)."""
     rbs = rb_req.numel()
     ws = ws or workspace(q.device)
     l = native.lib()
-    entry = {"": "cb_paged_attn", "decode": "cb_paged_decode"}[form]
+    entry = {"": "cb_paged_attn", "decode": "cb_paged_decode", "prefill": "cb_paged_prefill"}[form]
     if splits > 1:
         ws.ensure_attn(l.cb_paged_attn_partial_floats(rbs, hkv, splits))
         assert rbs * hkv <= ws.attn_counters.numel()

@@ -250,7 +250,7 @@ def _declare(l: ctypes.CDLL) -> None:
     l.cb_copy_pages.restype = i
     l.cb_paged_attn_partial_floats.argtypes = [i, i, i]
     l.cb_paged_attn_partial_floats.restype = ll
-    for entry in (l.cb_paged_attn, l.cb_paged_decode):
+    for entry in (l.cb_paged_attn, l.cb_paged_decode, l.cb_paged_prefill):
         entry.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, f, i, vp, vp, vp, vp]
         entry.restype = i
     l.cb_sample.argtypes = [vp, i, i, vp, i, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp]

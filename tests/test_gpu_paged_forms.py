@@ -1,5 +1,5 @@
-"""The decode form of paged attention against the general kernel (itself tested against the dense oracle) and, for one layout,
-against the oracle."""
+"""The decode and prompt forms of paged attention against the general kernel (itself tested against the dense oracle) and, for one
+layout, against the oracle."""
 
 import pytest
 import torch
@@ -44,7 +44,7 @@ def _run(form, q, cache, table, blocks, hq, hkv, kb, vb, splits):
 
 
 def _close(a, b):
-    """Probabilities are rounded to f16 (2^-11) relative to another running maximum, sums run in another order, results are rounded
+    """Probabilities are rounded to f16 (2^-11) relative to another running maximum (up to four times lower), sums run in another order, results are rounded
     to bf16 (2^-8): two steps of the value, or of a small part of the row's scale."""
     a, b = a.float(), b.float()
     assert torch.isfinite(a).all()
@@ -65,14 +65,36 @@ def test_decode_form(kb, vb, group):
         assert (got[5] == 7).all() and _close(got[:5], want[:5]) and _close(got[6:], want[6:])
 
 
-def test_decode_form_against_the_oracle():
+@pytest.mark.parametrize("kb,vb", [(8, 8), (4, 8), (6, 6), (4, 4), (8, 4), (6, 8), (8, 6), (4, 6), (6, 4)])
+@pytest.mark.parametrize("group", [1, 4, 8, 16])
+def test_prompt_form(kb, vb, group):
+    hkv, qb = 2, 16 // group
+    portions = [(0, 1), (0, 3 * qb + 1), (37, 5), (0, 64), (15, 50), (500, 70), (0, 129)]   # (start, tokens) of every request
+    cache, table = _cache([s + n for s, n in portions], hkv, kb, vb, kb * vb + group)
+    T = sum(n for _, n in portions)
+    q = torch.randn(T, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(2)).bfloat16()
+    blocks, t = [], 0
+    for r, (s, n) in enumerate(portions):
+        blocks += [(r, t + i, min(qb, n - i), s + i + 1) for i in range(0, n, qb)]
+        if r == 2:
+            blocks.append((0, 0, 0, 0))                                                    # a padding block in between
+        t += n
+    want = _run("", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
+    assert _close(_run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1), want)
+
+
+@pytest.mark.parametrize("form", ["decode", "prefill"])
+def test_forms_against_the_oracle(form):
     hkv, group, n = 2, 4, 333
     cache, table = _cache([n], hkv, 8, 8, 5)
-    q = torch.randn(1, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)).bfloat16()
+    rows = 1 if form == "decode" else 40
+    q = torch.randn(rows, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)).bfloat16()
     kv = [[eager.decode_cache_page(cache[p, h].cpu(), D, 8, 8) for h in range(hkv)] for p in table[0].tolist()]
     k, v = (torch.stack([torch.cat([page[h][i] for page in kv])[:n] for h in range(hkv)], 1) for i in (0, 1))
-    ref = eager.attention_rows(q.cpu(), k, v, torch.tensor([n]), 0.05)
-    assert _close(_run("decode", q, cache, table, [(0, 0, 1, n)], group * hkv, hkv, 8, 8, 2).cpu(), ref)
+    first = n - rows
+    ref = eager.attention_rows(q.cpu(), k, v, torch.arange(first + 1, n + 1), 0.05)
+    blocks = [(0, 0, 1, n)] if form == "decode" else [(0, i, min(4, rows - i), first + i + 1) for i in range(0, rows, 4)]
+    assert _close(_run(form, q, cache, table, blocks, group * hkv, hkv, 8, 8, 2 if form == "decode" else 1).cpu(), ref)
 
 
 def test_decode_form_reports_too_many_rows():
