@@ -29,6 +29,7 @@ static constexpr int kPfPages = 4;                       // pages of a step
 static constexpr int kPfTok = kPfPages * kPageTokens;    // 64
 static constexpr int kPfThreads = 288;
 static constexpr float kPfGrowth = 2.f;
+static constexpr uint32_t kPfWild = 1;                   // a V scale of the step is not finite
 static constexpr uint32_t kPfTmemCols = 512, kPfTmemO = 256;      // four score tiles of 64 columns, then 128 columns of output
 
 struct PfRun {
@@ -40,6 +41,7 @@ struct __align__(1024) PfSmem {
   uint8_t k[2][2 * kPfTok * 128];                        // f16 [stage][64-channel half][token]
   uint8_t v[2][kD * 128];                                // f16 [stage][channel][64 tokens]
   float ks[2][4 * kPfTok], vs[2][4 * kPfTok];            // [stage][channel group][token]
+  uint32_t vs_kind[2][2];                                // [stage][half of the tokens] kPfWild
   uint64_t raw_full[2], kv_full[2], kv_free[2], s_full, s_free, p_full, pv_done;
   PfRun run[kPfBlocks];
   int runs, steps;
@@ -153,6 +155,11 @@ __device__ __forceinline__ void pf_convert(PfSmem& sm, int b, const uint8_t* raw
       s = *reinterpret_cast<const float4*>(raw + pg * stride + (is_v ? lay.v_scale_off : lay.k_scale_off) + (tok & 15) * 16);
     float* dst = (is_v ? sm.vs[b] : sm.ks[b]) + tok;
     dst[0] = s.x; dst[kPfTok] = s.y; dst[2 * kPfTok] = s.z; dst[3 * kPfTok] = s.w;
+    if (is_v) {                                          // both warps of V
+      const bool tame = fabsf(s.x) < INFINITY && fabsf(s.y) < INFINITY && fabsf(s.z) < INFINITY && fabsf(s.w) < INFINITY;
+      const uint32_t kind = __all_sync(0xffffffffu, tame) ? 0u : kPfWild;
+      if ((tid & 31) == 0) sm.vs_kind[b][(tid >> 5) & 1] = kind;
+    }
   }
 }
 
@@ -336,11 +343,15 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
     float m = -INFINITY, l = 0.f;
     PfWalk at;
     for (int i = 0; i < steps; ++i) {
-      const int b = i & 1, tok0 = at.step * kPfTok;
-      const PfRun& r = sm.run[at.run];
-      const int sees = (blk >= r.first && blk < r.end) ? limit - tok0 : 0;       // tokens of the step that this row sees
+      const int b = i & 1;
+      auto visible = [&](int run, int step) {            // tokens of the step that this row sees
+        const PfRun& r = sm.run[run];
+        return (blk >= r.first && blk < r.end) ? limit - step * kPfTok : 0;
+      };
+      const int sees = visible(at.run, at.step);
       at.advance(sm);
       if (ok) ok = mbar_wait_park(smem_u32(&sm.kv_full[b]), (i >> 1) & 1, abort_flag);      // the scales
+      const uint32_t vs_kind = sm.vs_kind[b][0] | sm.vs_kind[b][1];
       if (ok) ok = mbar_wait_park(smem_u32(&sm.s_full), i & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
@@ -420,6 +431,21 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
           *reinterpret_cast<uint4*>(sm.p[cg] + tid * 128 + ((c ^ (tid & 7)) << 4)) =
               make_uint4(pack_f16x2(w0.x, w0.y), pack_f16x2(w1.x, w1.y), pack_f16x2(w2.x, w2.y), pack_f16x2(w3.x, w3.y));
         }
+      // zero times a scale that is not finite, perhaps another request's, is not zero: tokens that a row does not see become zeros
+      if (vs_kind & kPfWild) {
+        // how many it sees is worked out again: the kernel has no register to hold it up to here
+        const int n = at.step == 0 ? visible(at.run - 1, sm.run[at.run - 1].steps - 1) : visible(at.run, at.step - 1);
+#pragma unroll 1
+        for (int c = max(n, 0) >> 3; c < 8; ++c) {
+          const int keep = min(max(n - 8 * c, 0), 8);                // tokens of the chunk
+#pragma unroll 1
+          for (int cg = 0; cg < 4; ++cg) {
+            uint32_t* at4 = reinterpret_cast<uint32_t*>(sm.p[cg] + tid * 128 + ((c ^ (tid & 7)) << 4));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) at4[k] &= keep >= 2 * k + 2 ? 0xFFFFFFFFu : keep == 2 * k + 1 ? 0xFFFFu : 0u;
+          }
+        }
+      }
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();

@@ -107,3 +107,33 @@ def test_decode_form_reports_too_many_rows():
     with pytest.raises(NativeLibraryError):
         K.paged_attention(q.view(1, 16, D), torch.empty(1, 16, D, device=DEV, dtype=torch.bfloat16), cache, table, *(torch.ones(1, dtype=torch.int32, device=DEV) for _ in range(4)),
                           16, 1, D, 8, 8, form="decode")
+
+
+def _scales(cache, kb, vb):
+    """V scales of the cache as floats [page][head][token of the page][group]."""
+    lay = eager.blob_layout(D, kb, vb)
+    return cache[:, :, lay["v_scale"]:lay["bytes"]].view(torch.float32).view(cache.shape[0], cache.shape[1], 16, D // 32)
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (4, 8), (6, 6), (8, 4)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_prompt_form_keeps_values_to_those_who_see_them(kb, vb, bad):
+    """An infinite value of one request reaches neither the requests that share a CTA with it nor earlier positions of its own."""
+    hkv, group, qb = 2, 4, 4
+    portions = [(0, 30), (20, 21), (0, 17), (5, 70)]
+    cache, table = _cache([s + n for s, n in portions], hkv, kb, vb, 11)
+    T = sum(n for _, n in portions)
+    q = torch.randn(T, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)).bfloat16()
+    blocks, t, rows = [], 0, []
+    for r, (s, n) in enumerate(portions):
+        blocks += [(r, t + i, min(qb, n - i), s + i + 1) for i in range(0, n, qb)]
+        rows += [(r, s + i) for i in range(n)]
+        t += n
+    want = _run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
+    for req, tok in ((1, 33), (3, 0), (3, 74)):
+        hit = cache.clone()
+        _scales(hit, kb, vb)[int(table[req, tok // 16]), :, tok % 16] = bad
+        got = _run("prefill", q, hit, table, blocks, group * hkv, hkv, kb, vb, 1)
+        sees = torch.tensor([r == req and p >= tok for r, p in rows], device=DEV)
+        assert torch.equal(got[~sees], want[~sees])
+        assert not torch.isfinite(got[sees].float()).all(-1).any()
