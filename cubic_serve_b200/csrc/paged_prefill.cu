@@ -17,7 +17,8 @@
 // The scores of step i + 1 are computed while the softmax of step i runs.  Row blocks of several requests may meet in a CTA: it walks
 // their steps one request after the other, rows of another request taking part with probability zero.  The output accumulator stays
 // in tensor memory and is rescaled only when a row's maximum has grown by more than a factor of four (2 in the log2 domain): until
-// then probabilities relative to the older maximum are at most 4.
+// then probabilities relative to the older maximum are at most 4.  A step with a V scale of which four times is more than f16 holds
+// rescales at any growth, so that scaled probabilities have the range that they have in the general kernel.
 // Every wait is bounded; on a timeout the roles run through without waiting, the status word is set and tensor memory is freed.
 #include "paged_attn.cuh"
 
@@ -29,7 +30,8 @@ static constexpr int kPfPages = 4;                       // pages of a step
 static constexpr int kPfTok = kPfPages * kPageTokens;    // 64
 static constexpr int kPfThreads = 288;
 static constexpr float kPfGrowth = 2.f;
-static constexpr uint32_t kPfWild = 1;                   // a V scale of the step is not finite
+static constexpr float kPfGrowthScale = 65504.f / 4.f;   // largest V scale of a step with probabilities up to 4
+static constexpr uint32_t kPfWild = 1, kPfLarge = 2;     // a V scale of the step is not finite, is finite and above that
 static constexpr uint32_t kPfTmemCols = 512, kPfTmemO = 256;      // four score tiles of 64 columns, then 128 columns of output
 
 struct PfRun {
@@ -41,7 +43,7 @@ struct __align__(1024) PfSmem {
   uint8_t k[2][2 * kPfTok * 128];                        // f16 [stage][64-channel half][token]
   uint8_t v[2][kD * 128];                                // f16 [stage][channel][64 tokens]
   float ks[2][4 * kPfTok], vs[2][4 * kPfTok];            // [stage][channel group][token]
-  uint32_t vs_kind[2][2];                                // [stage][half of the tokens] kPfWild
+  uint32_t vs_kind[2][2];                                // [stage][half of the tokens] kPfWild, kPfLarge
   uint64_t raw_full[2], kv_full[2], kv_free[2], s_full, s_free, p_full, pv_done;
   PfRun run[kPfBlocks];
   int runs, steps;
@@ -156,8 +158,8 @@ __device__ __forceinline__ void pf_convert(PfSmem& sm, int b, const uint8_t* raw
     float* dst = (is_v ? sm.vs[b] : sm.ks[b]) + tok;
     dst[0] = s.x; dst[kPfTok] = s.y; dst[2 * kPfTok] = s.z; dst[3 * kPfTok] = s.w;
     if (is_v) {                                          // both warps of V
-      const bool tame = fabsf(s.x) < INFINITY && fabsf(s.y) < INFINITY && fabsf(s.z) < INFINITY && fabsf(s.w) < INFINITY;
-      const uint32_t kind = __all_sync(0xffffffffu, tame) ? 0u : kPfWild;
+      auto of = [](float x) { return fabsf(x) <= kPfGrowthScale ? 0u : fabsf(x) < INFINITY ? kPfLarge : kPfWild; };
+      const uint32_t kind = __reduce_or_sync(0xffffffffu, of(s.x) | of(s.y) | of(s.z) | of(s.w));
       if ((tid & 31) == 0) sm.vs_kind[b][(tid >> 5) & 1] = kind;
     }
   }
@@ -389,7 +391,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
       for (int j = 0; j < kPfTok / 2; ++j) mx[j & 3] = fmaxf(mx[j & 3], fmaxf(s[j].x, s[j].y));
       const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       float alpha = 1.f;
-      const bool grew = top > m + kPfGrowth || (m == -INFINITY && top > m);
+      const bool grew = top > m + (vs_kind & kPfLarge ? 0.f : kPfGrowth) || (m == -INFINITY && top > m);
       if (grew) {
         alpha = fast_exp2(m - top);
         m = top;

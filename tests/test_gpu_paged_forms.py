@@ -137,3 +137,17 @@ def test_prompt_form_keeps_values_to_those_who_see_them(kb, vb, bad):
         sees = torch.tensor([r == req and p >= tok for r, p in rows], device=DEV)
         assert torch.equal(got[~sees], want[~sees])
         assert not torch.isfinite(got[sees].float()).all(-1).any()
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (8, 4)])
+@pytest.mark.parametrize("top", [16000.0, 16400.0, 40000.0, 65000.0])
+def test_prompt_form_has_the_range_of_f16_for_scales(kb, vb, top):
+    """Scales up to the largest f16: probabilities are at most one where four times a scale would not fit."""
+    hkv, group, n = 2, 4, 700
+    cache, table = _cache([n], hkv, kb, vb, 12)
+    s = _scales(cache, kb, vb)
+    s.mul_(top / s.nan_to_num().max())
+    q = torch.randn(n, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4)).bfloat16()
+    blocks = [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)]
+    want = _run("", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
+    assert torch.isfinite(want.float()).all() and _close(_run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1), want)
