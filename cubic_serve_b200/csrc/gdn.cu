@@ -37,18 +37,20 @@ struct GdnSegments {
 // Tiles of kConvRows rows of a segment x 128 threads of V neighbouring channels.  The convolution has no chain: a tile takes the
 // three inputs before its first row from the rows themselves.  (One thread walking a channel's whole segment left 3000 rows of
 // 8192 channels to 320 blocks with four loads in flight each: 290 us where the bytes take 15.)  Only the first tile of a segment
-// touches the request's state: it has read the old inputs before it writes the new ones.
+// touches the request's state: it has read the old inputs before it writes the new ones.  Rows that are written over the rows that
+// are read (`x` and `y` are not __restrict__) take tiles as long as the step: one thread then walks its channels of a whole segment, every row
+// read before it is written.
 static constexpr int kConvRows = 32;
 
 template <int V>
 __global__ void __launch_bounds__(128)
-gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, __nv_bfloat16* __restrict__ y, int ldy,
+gdn_conv_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy,
                 const float* __restrict__ w,            // [C, 4], tap 3 multiplies the current input
                 const float* __restrict__ bias,         // [C] or null
                 __nv_bfloat16* __restrict__ state,      // [slots, 3, C]
-                Segments seg, int C, int commit) {
+                Segments seg, int tile_rows, int C, int commit) {
   int s, off;
-  if (!find_tile(seg, kConvRows, blockIdx.y, s, off)) return;
+  if (!find_tile(seg, tile_rows, blockIdx.y, s, off)) return;
   const int c = (blockIdx.x * 128 + threadIdx.x) * V;
   if (c >= C) return;
   const int n = seg.count[s];
@@ -93,7 +95,7 @@ gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, __nv_bfloat16* __r
       store(st + static_cast<size_t>(j) * C, v);
     }
   }
-  const int end = min(n, off + kConvRows);
+  const int end = off + min(n - off, tile_rows);
   // eight rows per trip: the loads do not depend on the arithmetic, so they are issued together
   for (int t = off; t < end; t += 8) {
     Chan v[8];
@@ -338,22 +340,33 @@ struct CbGdnSegments {
   int num;
 };
 
-// `rows`: rows of the step; x and y do not overlap.
+// Whether the columns [0, C) of `rows` rows of x and of y share elements.
+static bool conv_overlap(const void* x, int ldx, const void* y, int ldy, int C, int rows) {
+  const long long a = static_cast<long long>(reinterpret_cast<uintptr_t>(x)), b = static_cast<long long>(reinterpret_cast<uintptr_t>(y)), cols = 2ll * C;
+  const long long x_end = a + 2ll * (rows - 1) * ldx + cols, y_end = b + 2ll * (rows - 1) * ldy + cols;
+  if (x_end <= b || y_end <= a) return false;
+  if (ldx != ldy || ldx < C) return true;
+  const long long pitch = 2ll * ldx, shift = ((b - a) % pitch + pitch) % pitch;       // neighbouring columns of one buffer
+  return shift < cols || shift > pitch - cols;
+}
+
+// `rows`: rows of the step.  y may be x.
 int cb_gdn_conv(const void* x, int ldx, void* y, int ldy, const void* w, const void* bias, void* state,
                 const CbGdnSegments* seg, int C, int rows, int commit, void* stream) {
   if (!seg || seg->num <= 0 || C <= 0 || seg->num > 65535 || rows < 0) return -60;
   if (rows == 0) return 0;
   const cb::Segments s{static_cast<const int*>(seg->row0), static_cast<const int*>(seg->count), static_cast<const int*>(seg->slot),
                        static_cast<const int*>(seg->pos0), seg->num, 0};
-  const int tiles = cb::max_tiles(rows, seg->num, cb::kConvRows);
-  if (tiles > 65535) return -60;
+  int tile_rows = conv_overlap(x, ldx, y, ldy, C, rows) || rows < cb::kConvRows ? rows : cb::kConvRows;
+  while (cb::max_tiles(rows, seg->num, tile_rows) > 65535) tile_rows = tile_rows > rows / 2 ? rows : 2 * tile_rows;     // at `rows` a tile a segment
+  const int tiles = cb::max_tiles(rows, seg->num, tile_rows);
   const bool pairs = C % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(state)) & 3) == 0;
   const int cols = pairs ? 256 : 128;
   const dim3 grid((C + cols - 1) / cols, tiles);
   auto kernel = pairs ? cb::gdn_conv_kernel<2> : cb::gdn_conv_kernel<1>;
   kernel<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy,
                                                               static_cast<const float*>(w), static_cast<const float*>(bias),
-                                                              static_cast<__nv_bfloat16*>(state), s, C, commit);
+                                                              static_cast<__nv_bfloat16*>(state), s, tile_rows, C, commit);
   return static_cast<int>(cudaGetLastError());
 }
 

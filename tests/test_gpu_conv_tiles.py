@@ -34,3 +34,25 @@ def test_conv_tiles(lengths, channels, wide, commit):
         if commit:
             want_state[slots[i]] = st
     assert torch.equal(got_state.cpu(), want_state)
+
+
+@pytest.mark.parametrize("channels,longest", [(4096, 20000), (131, 100000)])
+def test_conv_over_its_input(channels, longest):
+    """``out`` is ``x``: rows that later tiles look back at have been overwritten when there are more tiles than the GPU runs at once."""
+    from cubic_serve_b200.ops import kernels as K
+    g = torch.Generator(device=DEV).manual_seed(channels)
+    lengths = [longest, 1, 300, 90]
+    T, n = sum(lengths), len(lengths)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    seg = K.GdnSegments(i32([sum(lengths[:i]) for i in range(n)]), i32(lengths), i32([2, 0, 3, 1]), i32([0, 7, 0, 9]), n)
+    wide = torch.randn(T, 2 * channels, device=DEV, generator=g).bfloat16()
+    w = torch.randn(channels, 4, device=DEV, generator=g) * 0.5
+    state = torch.randn(n, 3, channels, device=DEV, generator=g).bfloat16()
+    x = wide[:, :channels]
+    want, want_state = torch.empty(T, channels, dtype=torch.bfloat16, device=DEV), state.clone()
+    K.gdn_conv(x, w, want_state, seg, want)
+    beside, beside_state = wide.clone(), state.clone()           # neighbouring columns of one buffer share no element
+    K.gdn_conv(beside[:, :channels], w, beside_state, seg, beside[:, channels:])
+    assert torch.equal(beside[:, channels:], want) and torch.equal(beside[:, :channels], x) and torch.equal(beside_state, want_state)
+    K.gdn_conv(x, w, state, seg, x)
+    assert torch.equal(x, want) and torch.equal(state, want_state)
