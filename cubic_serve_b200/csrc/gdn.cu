@@ -22,6 +22,7 @@
 // gated_delta_coefficients_native.cu:17 and the oracle ops/eager/hybrid.py:255-548 (fp32 recurrence branch).
 #include "ptx.cuh"
 #include "segments.cuh"
+#include <type_traits>
 
 namespace cb {
 
@@ -80,7 +81,7 @@ __device__ __forceinline__ bool conv_tile(const Segments& sg, int rows, int tile
 }
 
 template <int V>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 10)
 gdn_conv_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy,
                 const float* __restrict__ w,            // [C, 4], tap 3 multiplies the current input
                 const float* __restrict__ bias,         // [C] or null
@@ -95,16 +96,19 @@ gdn_conv_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy,
   __nv_bfloat16* yp = y + static_cast<size_t>(tile.row0) * ldy + c;
   __nv_bfloat16* st = state + static_cast<size_t>(tile.slot) * 3 * C + c;
   struct Chan { float v[V]; };
-  auto load = [](const __nv_bfloat16* at) {
+  using Raw = std::conditional_t<V == 2, __nv_bfloat162, __nv_bfloat16>;      // rows in flight stay packed: registers are what bounds a decode step
+  auto fetch = [](const __nv_bfloat16* at) { return *reinterpret_cast<const Raw*>(at); };
+  auto widen = [](Raw x) {
     Chan r;
     if constexpr (V == 2) {
-      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(at));
+      const float2 f = __bfloat1622float2(x);
       r.v[0] = f.x; r.v[1] = f.y;
     } else {
-      r.v[0] = __bfloat162float(*at);
+      r.v[0] = __bfloat162float(x);
     }
     return r;
   };
+  auto load = [&](const __nv_bfloat16* at) { return widen(fetch(at)); };
   auto store = [](__nv_bfloat16* at, const Chan& r) {
     if constexpr (V == 2) *reinterpret_cast<__nv_bfloat162*>(at) = __floats2bfloat162_rn(r.v[0], r.v[1]);
     else *at = __float2bfloat16(r.v[0]);
@@ -124,33 +128,43 @@ gdn_conv_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy,
 #pragma unroll
     for (int j = 0; j < 3; ++j) h[j] = load(st + static_cast<size_t>(j) * C);
   }
-  if (off == 0 && commit) {
+  // the segment's last three inputs: of a longer segment from its rows, else they are in registers at the end (to fetch them here made
+  // a step of four rows wait for memory twice, 11 us instead of 9)
+  commit &= off == 0;
+  if (commit && n > tile_rows) {
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int t = n - 3 + j;                          // an input before the segment's first is one of the old three
-      const Chan v = t >= 0 ? load(xp + static_cast<size_t>(t) * ldx) : t == -1 ? h[2] : h[1];
-      store(st + static_cast<size_t>(j) * C, v);
-    }
+    for (int j = 0; j < 3; ++j) store(st + static_cast<size_t>(j) * C, load(xp + static_cast<size_t>(n - 3 + j) * ldx));
   }
   const int end = off + min(n - off, tile_rows);
-  // eight rows per trip: the loads do not depend on the arithmetic, so they are issued together
-  for (int t = off; t < end; t += 8) {
-    Chan v[8];
+  // N rows at a time: the loads do not depend on the arithmetic, so they are issued together.  A decode step runs the code of one row only:
+  // its instructions come from memory too.
+  int t = off;
+  auto rows = [&](auto count) {
+    constexpr int N = decltype(count)::value;
+    Raw v[N];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (t + j < end) v[j] = load(xp + static_cast<size_t>(t + j) * ldx);
+    for (int j = 0; j < N; ++j) v[j] = fetch(xp + static_cast<size_t>(t + j) * ldx);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (t + j >= end) break;
+    for (int j = 0; j < N; ++j) {
       Chan o;
+      const Chan x0 = widen(v[j]);
 #pragma unroll
       for (int i = 0; i < V; ++i) {
-        const float a = b[i] + wv[i].x * h[0].v[i] + wv[i].y * h[1].v[i] + wv[i].z * h[2].v[i] + wv[i].w * v[j].v[i];
+        const float a = b[i] + wv[i].x * h[0].v[i] + wv[i].y * h[1].v[i] + wv[i].z * h[2].v[i] + wv[i].w * x0.v[i];
         o.v[i] = silu_fast(a);
       }
       store(yp + static_cast<size_t>(t + j) * ldy, o);
-      h[0] = h[1]; h[1] = h[2]; h[2] = v[j];
+      h[0] = h[1]; h[1] = h[2]; h[2] = x0;
     }
+    t += N;
+  };
+  while (t + 8 <= end) rows(std::integral_constant<int, 8>());
+  if (t + 4 <= end) rows(std::integral_constant<int, 4>());
+  if (t + 2 <= end) rows(std::integral_constant<int, 2>());
+  if (t < end) rows(std::integral_constant<int, 1>());
+  if (commit && n <= tile_rows) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) store(st + static_cast<size_t>(j) * C, h[j]);
   }
 }
 
