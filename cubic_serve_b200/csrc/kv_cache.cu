@@ -38,6 +38,29 @@ struct KvWriteParams {
   KvLayout lay;
 };
 
+// Four neighbouring channels; eight bytes at once where every row starts on a multiple of eight (WIDE).
+template <bool WIDE>
+__device__ __forceinline__ void load4(const __nv_bfloat16* at, float (&v)[4]) {
+  if constexpr (WIDE) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(at);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = __bfloat162float(at[k]);
+  }
+}
+template <bool WIDE>
+__device__ __forceinline__ void store4(__nv_bfloat16* at, uint2 v) {
+  if constexpr (WIDE) {
+    *reinterpret_cast<uint2*>(at) = v;
+  } else {
+    const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&v.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&v.y);
+    at[0] = lo.x; at[1] = lo.y; at[2] = hi.x; at[3] = hi.y;
+  }
+}
+static inline bool on8(const void* a, const void* b) { return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 7) == 0; }
+
 // Normalised Walsh-Hadamard transform of a 128-vector held as v[a] = x[4 lane + a] (the transform treats all index bits alike,
 // so any four of them may be the registers).  fp32 stages, the caller rounds once (reference:
 // ops/cuda/cache_rotation_native.cu:12).  The transform is its own inverse, and q . k is unchanged when both are
@@ -121,6 +144,7 @@ static constexpr int kRopeWarps = 8;
 // One CTA per token; its eight warps share the token's heads (warp w takes heads w, w + 8, ...).  The rotary
 // angles depend on (position, channel) only, so the CTA computes its sin / cos pairs ONCE, a thread each, and reuses them
 // for every head of the token: full-precision sincosf on arguments of thousands of radians is expensive.
+template <bool WIDE>
 __global__ void __launch_bounds__(kRopeWarps * 32)
 rope_kv_write_kernel(const KvWriteParams p) {
   __shared__ __align__(16) float sn_s[64], cs_s[64];
@@ -156,11 +180,7 @@ rope_kv_write_kernel(const KvWriteParams p) {
 #pragma unroll 2
   for (int h = warp; h < heads; h += kRopeWarps) {
     float v[4];
-    {
-      const uint2 raw = *reinterpret_cast<const uint2*>(p.qkv + (static_cast<size_t>(t) * heads + h) * kHeadDim + 4 * lane);
-      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-      v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
-    }
+    load4<WIDE>(p.qkv + (static_cast<size_t>(t) * heads + h) * kHeadDim + 4 * lane, v);
     if (p.qkv_bias != nullptr) {
       // the projection's output was rounded to bf16 by the GEMM; the sum is rounded again, as an unfused add would
 #pragma unroll
@@ -194,7 +214,7 @@ rope_kv_write_kernel(const KvWriteParams p) {
     if (p.rotate) hadamard128(v, lane);
     const uint2 bf = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
     if (is_q) {
-      *reinterpret_cast<uint2*>(p.q_out + (static_cast<size_t>(t) * p.Hq + h) * kHeadDim + 4 * lane) = bf;
+      store4<WIDE>(p.q_out + (static_cast<size_t>(t) * p.Hq + h) * kHeadDim + 4 * lane, bf);
       continue;
     }
     if (slot < 0) continue;
@@ -210,6 +230,7 @@ rope_kv_write_kernel(const KvWriteParams p) {
 
 // Walsh-Hadamard transform of `vectors` consecutive 128-vectors per row (in place allowed): undoes the rotation of
 // V on the attention output.  One warp per vector.
+template <bool WIDE>
 __global__ void __launch_bounds__(256)
 hadamard_kernel(const __nv_bfloat16* __restrict__ x, int ldx, __nv_bfloat16* __restrict__ y, int ldy, int vectors,
                 int rows) {
@@ -222,11 +243,9 @@ hadamard_kernel(const __nv_bfloat16* __restrict__ x, int ldx, __nv_bfloat16* __r
   const __nv_bfloat16* src = x + static_cast<size_t>(r) * ldx + h * 128;
   __nv_bfloat16* dst = y + static_cast<size_t>(r) * ldy + h * 128;
   float v[4];
-  const uint2 raw = *reinterpret_cast<const uint2*>(src + 4 * lane);
-  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-  v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+  load4<WIDE>(src + 4 * lane, v);
   hadamard128(v, lane);
-  *reinterpret_cast<uint2*>(dst + 4 * lane) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+  store4<WIDE>(dst + 4 * lane, make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])));
 }
 
 // Copy whole pages (all kv heads) src -> dst: copy-on-write of a shared page.
@@ -293,7 +312,8 @@ int cb_rope_kv_write_axes(const void* qkv, void* q_out, void* cache, const void*
   p.inv_freq = static_cast<const float*>(inv_freq);
   p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.rotary_dim = rotary_dim; p.eps = eps; p.rotate = rotate;
   p.lay = make_kv_layout(D, k_bits, v_bits);
-  return static_cast<int>(launch(rope_kv_write_kernel, dim3(static_cast<unsigned>(T)), dim3(kRopeWarps * 32), 0,
+  // rows are multiples of 256 bytes, so the first decides for all
+  return static_cast<int>(launch(on8(qkv, q_out) ? rope_kv_write_kernel<true> : rope_kv_write_kernel<false>, dim3(static_cast<unsigned>(T)), dim3(kRopeWarps * 32), 0,
                                  static_cast<cudaStream_t>(stream), p));
 }
 
@@ -301,7 +321,8 @@ int cb_rope_kv_write_axes(const void* qkv, void* q_out, void* cache, const void*
 int cb_hadamard(const void* x, int ldx, void* y, int ldy, int vectors, int rows, void* stream) {
   if (rows <= 0 || vectors <= 0) return 0;
   const long long warps = static_cast<long long>(rows) * vectors;
-  return static_cast<int>(cb::launch(cb::hadamard_kernel, dim3(static_cast<unsigned>((warps + 7) / 8)), dim3(256), 0,
+  const bool wide = cb::on8(x, y) && (rows == 1 || ((ldx | ldy) & 3) == 0);
+  return static_cast<int>(cb::launch(wide ? cb::hadamard_kernel<true> : cb::hadamard_kernel<false>, dim3(static_cast<unsigned>((warps + 7) / 8)), dim3(256), 0,
                                      static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x), ldx,
                                      static_cast<__nv_bfloat16*>(y), ldy, vectors, rows));
 }
