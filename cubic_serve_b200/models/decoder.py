@@ -266,7 +266,7 @@ class StepBatch:
     logit_rows: torch.Tensor     # int64 [R] rows of the hidden state that feed lm_head
     attn_splits: int = 1
     # what the attention kernels are told of the row blocks (K.paged_attention, ``form``): none holds more than eight rows;
-    # blocks [lo, hi) belong to portions of prompts
+    # blocks [lo, hi) belong to portions of prompts and take one split; ``attn_splits`` is for the others
     attn_decode: bool = False
     attn_prompts: tuple[int, int] = (0, 0)
     segments: object | None = None   # K.GdnSegments: the step's rows grouped by request (Gated DeltaNet layers)

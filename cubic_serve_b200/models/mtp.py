@@ -121,9 +121,8 @@ class MtpRunner:
         K.rope_kv_write(qkv, q, self.kv, b.positions, b.slots, t.inv_freq, t.hq, t.hkv, t.D, t.k_bits, t.v_bits,
                         q_norm=lw.q_norm, k_norm=lw.k_norm, eps=cfg.rms_eps, rotary_dim=cfg.rotary_dim,
                         rotate=t.kv_rotation)
-        K.paged_attention(q.view(T, t.hq, t.D), attn.view(T, t.hq, t.D), self.kv, b.page_table,
-                          b.rb_req[:b.num_row_blocks], b.rb_qstart, b.rb_qcount, b.rb_ctx, t.hq, t.hkv, t.D, t.k_bits,
-                          t.v_bits, scale=t.cfg.attention_scale, splits=b.attn_splits, ws=t.ws)
+        # as the target's layers: `attn_splits` is for the row blocks outside `attn_prompts` only
+        attended = t._attend(b, q.view(T, t.hq, t.D), attn.view(T, t.hq, t.D), self.kv, 0, b.num_row_blocks)
         if t.kv_rotation:
             K.hadamard(attn)
         if tp is None:
@@ -143,7 +142,7 @@ class MtpRunner:
             K.wq_gemm(act, lw.down, out=part, ws=t.ws)
             tp.all_reduce(part)
             h.add_(part)
-        self.launches = 16 - fused + (4 if tp is not None else 0)
+        self.launches = 15 + attended - fused + (4 if tp is not None else 0)
         return h
 
     def logits(self, hidden: torch.Tensor, rows: int, out: torch.Tensor) -> torch.Tensor:
