@@ -1,7 +1,7 @@
 """Measured launch plans for the weight GEMMs of a model.
 
-``kernels.wq_gemm`` picks between its two kernels and a split-K factor by rules fitted to a handful of shapes
-(``use_stream_k`` / ``choose_splits``).  This module replaces the rules by measurement for the shapes a model actually
+``kernels.wq_gemm`` picks between its kernels and a split-K factor by rules fitted to a handful of shapes
+(``use_skinny`` / ``use_stream_k`` / ``choose_splits``).  This module replaces the rules by measurement for the shapes a model actually
 has: every projection of the model, at every decode capacity the executor captures, is timed inside a CUDA graph with
 a cold L2 under each candidate launch form, and the fastest is recorded.  The result is a JSON plan
 (``"fmt:m:n:k:act" -> {"kernel": "tile" | "stream_k", "splits": s}``); ``install`` makes ``kernels`` consult it before

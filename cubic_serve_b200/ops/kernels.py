@@ -171,17 +171,29 @@ def use_skinny(m: int, w: PackedWeight, x: torch.Tensor) -> bool:
     grows with the rows where the tcgen05 kernels' stays: 4-bit weights of 24576 x 4096 take 22 / 26 / 43 us at 8 / 16 / 32 rows
     against 34 / 34 / 35, 4096 x 4096 6.4 / 8.2 / 14 against 10.1 / 10.2 / 10.6.  bf16 weights have nothing to decode: with more
     weight tiles than SMs they stream at 65 / 68 / 74 us against 98 / 98 / 102 (50688 x 4096), with fewer the split tiles of the
-    other kernel are as good from 16 rows on (8.0 / 10.4 against 9.2 / 9.2, 4096 x 4096).  (One B200, weights not in L2.)"""
-    if w.fmt == FMT_BF16:
-        most = 32 if -(-w.n // 128) > 148 else 8
+    other kernel are as good from 16 rows on (8.0 / 10.4 against 9.2 / 9.2, 4096 x 4096).  (One B200, weights not in L2.)
+    The thresholds live in the operator configuration (``few_rows_*``); an installed plan comes before them."""
+    from .strategies import active
+    g = active().gemm
+    if w.fmt != FMT_BF16:
+        most = g.few_rows_quantized
+    elif m <= g.few_rows_bf16:
+        most = m
     else:
-        most = 16
+        most = g.few_rows_bf16_streamed if -(-w.n // 128) > (sm_count(x.device) if x.is_cuda else 148) else 0
     return m <= most and skinny_fits(w, x)
 
 
-# Rows an expert gets on average up to which the grouped launches take that kernel: 6 / 12 / 16 / 24 rows of 128 experts of 1536 x
-# 2048 (NVFP4) take 82 / 103 / 107 / 134 us against 125 us of the tcgen05 kernel at any of them
-SKINNY_ROWS_PER_EXPERT = 16
+# Rows an expert gets on average up to which the grouped launches take that kernel; None: the operator configuration's
+# ``moe.few_rows_per_expert``
+SKINNY_ROWS_PER_EXPERT: int | None = None
+
+
+def skinny_rows_per_expert() -> int:
+    """6 / 12 / 16 / 24 rows of 128 experts of 1536 x 2048 (NVFP4) take 82 / 103 / 107 / 134 us against 125 us of the tcgen05 kernel at
+    any of them."""
+    from .strategies import active
+    return active().moe.few_rows_per_expert if SKINNY_ROWS_PER_EXPERT is None else SKINNY_ROWS_PER_EXPERT
 
 
 def _wq_gemm_skinny(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, residual: torch.Tensor | None, ws: "Workspace", swiglu: bool) -> torch.Tensor:
@@ -300,8 +312,8 @@ def wq_gemm(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = None,
     """``out[M, N] = x[M, K] @ W[N, K]^T * alpha (+ residual)`` with W in packed form.
 
     Three kernels: one CTA per (weight tile, K split) (``csrc/wq_gemm.cu``), the persistent stream-K kernel
-    (``csrc/wq_gemm_sk.cu``), and one for few rows (``csrc/wq_gemm_skinny.cu``, see ``use_skinny``).  With neither ``splits`` nor ``min_units`` given the faster one for the shape is
-    used (``use_stream_k``).  ``splits`` forces the first with that split-K factor; ``min_units`` forces the
+    (``csrc/wq_gemm_sk.cu``), and one for few rows (``csrc/wq_gemm_skinny.cu``).  With neither ``splits`` nor ``min_units`` given an
+    installed plan decides, else ``use_skinny`` and ``use_stream_k``.  ``splits`` forces the first with that split-K factor; ``min_units`` forces the
     second (0 = its own schedule, > 0 = the smallest run of k-blocks a CTA is dealt).
     """
     assert isinstance(x, Fp8Act) or (x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1)
@@ -316,13 +328,13 @@ def wq_gemm(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = None,
     ws = ws or workspace(x.device)
     if w.fmt in (FMT_FP8, FMT_FP8_BLOCK):
         return _wq_gemm_fp8(x, w, out, residual, splits, ws, link, False, min_units)
-    if splits is None and min_units is None and link is None and use_skinny(m, w, x):
-        return _wq_gemm_skinny(x, w, out, residual, ws, False)
-    l = native.lib()
-    if splits is None and min_units is None and link is None and TUNED_PLANS:
-        tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:0")
+    if splits is None and min_units is None and link is None:
+        tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:0") if TUNED_PLANS else None
         if tuned is not None:
             splits, min_units = (None, 0) if tuned[0] else (tuned[1], None)
+        elif use_skinny(m, w, x):
+            return _wq_gemm_skinny(x, w, out, residual, ws, False)
+    l = native.lib()
     if splits is None and min_units is None and use_stream_k(m, w.n, w.fmt, sm_count(x.device), k):
         from .strategies import active
         min_units = active().gemm.stream_k_min_units
@@ -367,13 +379,13 @@ def wq_gemm_act(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = Non
     ws = ws or workspace(x.device)
     if w.fmt in (FMT_FP8, FMT_FP8_BLOCK):
         return _wq_gemm_fp8(x, w, out, None, splits, ws, link, True, min_units)
-    if splits is None and min_units is None and link is None and use_skinny(m, w, x):
-        return _wq_gemm_skinny(x, w, out, None, ws, True)
-    l = native.lib()
-    if splits is None and min_units is None and link is None and TUNED_PLANS:
-        tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:1")
+    if splits is None and min_units is None and link is None:
+        tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:1") if TUNED_PLANS else None
         if tuned is not None:
             splits, min_units = (None, 0) if tuned[0] else (tuned[1], None)
+        elif use_skinny(m, w, x):
+            return _wq_gemm_skinny(x, w, out, None, ws, True)
+    l = native.lib()
     stream_k = splits is None and (min_units is not None or use_stream_k(m, w.n, w.fmt, sm_count(x.device), k))
     if stream_k and min_units is None:
         from .strategies import active
@@ -611,7 +623,7 @@ class MoeScratch:
 
     def __init__(self, max_tokens: int, top_k: int, hidden: int, inter2: int, local_experts: int, mb: int, device) -> None:
         routes = max_tokens * top_k
-        self.mb = mb                         # rows of a work item; a step may take more (``rows_per_item``)
+        self.mb = mb                         # rows of a work item; a step may take more (``rows_per_work_item``)
         self.local_experts = local_experts
         self.max_items = -(-routes // mb) + local_experts
         i32 = dict(dtype=torch.int32, device=device)
@@ -642,7 +654,11 @@ def rows_per_work_item(rows: int, experts: int, least: int) -> int:
     whatever its rows, and the decode sets the pace up to 200 of them, so an item should hold all rows of an expert with an
     average load (three standard deviations of a random routing above the mean), or an even part of them.  Gate / up and down of
     128 experts (1536 x 2048, 2048 x 768, NVFP4), items of 64 rows -> of this size: 1024 tokens 188 + 109 -> 137 + 92 us (96),
-    2048 tokens 299 + 179 -> 156 + 136 (160), 4096 tokens 531 + 320 -> 291 + 267 (160), 8192 tokens 1000 + 610 -> 514 + 486 (192)."""
+    2048 tokens 299 + 179 -> 156 + 136 (160), 4096 tokens 531 + 320 -> 291 + 267 (160), 8192 tokens 1000 + 610 -> 514 + 486 (192).
+    The operator configuration can pin them (``moe.rows_per_item_by_load``)."""
+    from .strategies import active
+    if not active().moe.rows_per_item_by_load:
+        return least
     mean = rows / experts
     want = mean + 3.0 * math.sqrt(mean)
     if want <= least:
@@ -682,7 +698,7 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
         native.check(code, "cb_wq_gemm_fp8_grouped")
         return out
     per = rows / w.codes.shape[0]
-    if per <= SKINNY_ROWS_PER_EXPERT and w.fmt != FMT_BF16 and skinny_fits(w, x):
+    if per <= skinny_rows_per_expert() and w.fmt != FMT_BF16 and skinny_fits(w, x):
         code = native.lib().cb_wq_gemm_skinny_grouped(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(),
                                                       out.stride(0), float(w.alpha), rows, w.n, w.k, w.group_k, int(swiglu), sc.tiles.data_ptr(),
                                                       8 if per <= 2 else 16 if per <= 8 else 32, code_stride, meta_stride, ws.status.data_ptr(), _stream())

@@ -4,10 +4,11 @@ Role of the reference's immutable operator config (``ops/strategies.py:276`` ``O
 ``launch``, ``linear``, ``moe``, ``collective``): one validated object that every launch policy reads, so that a
 deployment can pin or change a policy without touching code.  Here the families are:
 
-``gemm``       which weight-GEMM kernel serves a shape (``ops/kernels.py::use_stream_k``), the split-K bounds of
-               the per-tile kernel, a forced run length for the persistent kernel
+``gemm``       which weight-GEMM kernel serves a shape (``ops/kernels.py::use_skinny``, ``use_stream_k``), the split-K bounds
+               of the per-tile kernel, a forced run length for the persistent kernel
 ``attention``  how many KV splits a decode step uses for a given number of row blocks
-``moe``        rows per work item of the grouped expert GEMMs
+``moe``        rows per work item of the grouped expert GEMMs (a lower bound while they follow the load), and which steps
+               take the kernel for few rows
 
 ``load_operator_config(path)`` reads ``{"gemm": {...}, "attention": {...}, "moe": {...}, "profiles": [...]}``; unknown
 families or keys are errors (a typo must not silently keep the default).  Profiles override the base by device name,
@@ -32,6 +33,9 @@ class GemmPolicy:
     fuse_swiglu: bool = True            # SwiGLU in the epilogue of the gate/up GEMM (weight rows re-ordered at load)
     cta_pairs: bool = True              # persistent kernel on CTA pairs (cta_group::2) above stream_k_max_rows ...
     pair_min_blocks: int = 80           # ... when every pair gets at least this many k-blocks (else one CTA per tile)
+    few_rows_quantized: int = 16        # kernel without decoded tiles up to this many batch rows (0: never), 4-bit weights ...
+    few_rows_bf16: int = 8              # ... bf16 weights
+    few_rows_bf16_streamed: int = 32    # ... bf16 weights with more tiles than SMs (lm_head)
 
 
 @dataclass(frozen=True)
@@ -45,6 +49,8 @@ class MoePolicy:
     rows_per_item_small: int = 32       # rows per grouped-GEMM work item while routes < threshold x experts
     rows_per_item_large: int = 64
     large_routes_per_expert: int = 32
+    rows_per_item_by_load: bool = True  # larger work items where a step gives an expert more rows; false: exactly the above
+    few_rows_per_expert: int = 16       # mean rows of an expert up to which 4-bit experts take the kernel without decoded tiles (0: never)
 
 
 @dataclass(frozen=True)
@@ -59,6 +65,8 @@ class OperatorConfig:
             raise ValueError("gemm policy out of range")
         if g.stream_k_min_tile_ratio <= 0:
             raise ValueError("gemm.stream_k_min_tile_ratio must be positive")
+        if not all(0 <= v <= 32 for v in (g.few_rows_quantized, g.few_rows_bf16, g.few_rows_bf16_streamed)):
+            raise ValueError("gemm.few_rows_* must be in [0, 32]")
         if a.target_ctas < 1 or not 1 <= a.max_splits <= 64:
             raise ValueError("attention policy out of range")
         for v in (m.rows_per_item_small, m.rows_per_item_large):
@@ -66,6 +74,8 @@ class OperatorConfig:
                 raise ValueError("moe rows per item must be a multiple of 16 in [16, 256]")
         if m.large_routes_per_expert < 1:
             raise ValueError("moe.large_routes_per_expert must be positive")
+        if m.few_rows_per_expert < 0:
+            raise ValueError("moe.few_rows_per_expert must not be negative")
 
 
 def _family(cls, data: object, name: str):

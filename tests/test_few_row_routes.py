@@ -1,0 +1,77 @@
+"""Which kernel a weight GEMM of few rows is given to (host side: the native library is a list of the calls made)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from cubic_serve_b200.ops import autotune, kernels as K, native, strategies, wq_pack
+
+
+class Calls:
+    def __init__(self):
+        self.made = []
+
+    def __getattr__(self, name):
+        def call(*args):
+            if name.startswith("cb_wq_gemm_workspace"):
+                return 1 << 20
+            self.made.append((name, args))
+            return 0
+        return call
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    c = Calls()
+    monkeypatch.setattr(native, "lib", lambda: c)
+    monkeypatch.setattr(K, "_stream", lambda: 0)
+    monkeypatch.setattr(K, "sm_count", lambda _: 148)
+    return c
+
+
+def _ws(gemm=64 << 20, counters=1 << 16):
+    return SimpleNamespace(gemm=torch.empty(gemm, dtype=torch.uint8), gemm_counters=torch.zeros(counters, dtype=torch.int32), status=torch.zeros(1, dtype=torch.int32))
+
+
+def _route(calls, m, w, act=False, **kw):
+    x = torch.zeros(m, w.k, dtype=torch.bfloat16)
+    kw.setdefault("ws", _ws())
+    (K.wq_gemm_act if act else K.wq_gemm)(x, w, **kw)
+    return calls.made.pop()[0]
+
+
+def _weight(fmt=wq_pack.FMT_CUBIC4, n=512, k=1024, act=False):
+    return autotune._random_weight(fmt, n, k, act, "cpu")
+
+
+@pytest.mark.parametrize("m", [1, 8, 16])
+@pytest.mark.parametrize("act", [False, True])
+def test_an_installed_plan_comes_before_the_rule(calls, m, act):
+    w = _weight(act=act)
+    assert _route(calls, m, w, act) == "cb_wq_gemm_skinny"
+    try:
+        autotune.install({autotune.plan_key(w.fmt, m, w.n, w.k, act): {"use": True, "kernel": "tile", "splits": 3}})
+        assert _route(calls, m, w, act) == ("cb_wq_gemm_act" if act else "cb_wq_gemm_tp")
+        autotune.install({autotune.plan_key(w.fmt, m, w.n, w.k, act): {"use": True, "kernel": "stream_k", "splits": 0}})
+        assert _route(calls, m, w, act) == ("cb_wq_gemm_act" if act else "cb_wq_gemm_sk")
+        autotune.install({autotune.plan_key(w.fmt, m + 1, w.n, w.k, act): {"use": True, "kernel": "tile", "splits": 3}})
+        assert _route(calls, m, w, act) == "cb_wq_gemm_skinny"
+    finally:
+        autotune.install(None)
+
+
+def test_the_operator_configuration_sets_the_thresholds(calls):
+    w, head, small = _weight(), _weight(wq_pack.FMT_BF16, 19072, 128), _weight(wq_pack.FMT_BF16, 512, 128)
+    routes = lambda: [_route(calls, m, a) == "cb_wq_gemm_skinny" for a, m in ((w, 16), (w, 17), (head, 32), (head, 33), (small, 8), (small, 9))]  # noqa: E731
+    assert routes() == [True, False] * 3
+    old = strategies.active()
+    try:
+        strategies.install(strategies.operator_config_from_dict({"gemm": {"few_rows_quantized": 0, "few_rows_bf16": 9, "few_rows_bf16_streamed": 0},
+                                                                 "moe": {"few_rows_per_expert": 3, "rows_per_item_by_load": False}}))
+        assert routes() == [False, False, False, False, True, True]
+        assert K.skinny_rows_per_expert() == 3 and K.rows_per_work_item(8192, 128, 64) == 64
+    finally:
+        strategies.install(old)
+    for bad in ({"gemm": {"few_rows_quantized": 33}}, {"gemm": {"few_rows_bf16": -1}}, {"moe": {"few_rows_per_expert": -1}}):
+        with pytest.raises(ValueError):
+            strategies.operator_config_from_dict(bad)
