@@ -154,19 +154,31 @@ def use_stream_k(m: int, n: int, fmt: int, sms: int = 148, k: int = 4096) -> boo
     return m <= g.stream_k_max_rows or (fmt == FMT_BF16 and g.stream_k_bf16)
 
 
-def skinny_fits(w: PackedWeight, x: torch.Tensor) -> bool:
+def skinny_fits(w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None, residual: torch.Tensor | None = None,
+                ws: "Workspace | None" = None) -> bool:
     """Whether ``csrc/wq_gemm_skinny.cu`` takes the operands (the rows aside): whole iterations of K columns, one scale group
-    for all columns of a lane, 16-byte chunks of the activations."""
+    for all columns of a lane, 16-byte chunks of the activations.  Results and residual are moved four at a time where rows are a
+    multiple of four apart, so they have to start on eight bytes then; and the workspace holds two partial tiles of every CTA and a
+    counter of every weight tile.  The other kernels do with less."""
     if w.fmt == FMT_BF16:
         whole = w.k % 128 == 0
     elif w.fmt in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
         whole = w.k % 256 == 0 and (w.fmt != FMT_CUBIC4 or w.group_k % 128 == 0)
     else:
         return False
-    return whole and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+    if not whole or x.stride(0) % 8 or x.data_ptr() % 16:
+        return False
+    if out is not None and out.stride(0) % 4 == 0 and (out.data_ptr() | (0 if residual is None else residual.data_ptr())) % 8:
+        return False
+    if ws is not None:
+        m = x.shape[0]
+        parts = 2 * 2 * (sm_count(x.device) if x.is_cuda else 148) * (8 if m <= 8 else 16 if m <= 16 else 32) * 128 * 4
+        return parts <= ws.gemm.numel() and -(-w.n // 128) <= ws.gemm_counters.numel()
+    return True
 
 
-def use_skinny(m: int, w: PackedWeight, x: torch.Tensor) -> bool:
+def use_skinny(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None, residual: torch.Tensor | None = None,
+               ws: "Workspace | None" = None) -> bool:
     """Which batches the kernel without decoded tiles takes.  Its products run on ``mma.sync`` eight rows at a time, so its time
     grows with the rows where the tcgen05 kernels' stays: 4-bit weights of 24576 x 4096 take 22 / 26 / 43 us at 8 / 16 / 32 rows
     against 34 / 34 / 35, 4096 x 4096 6.4 / 8.2 / 14 against 10.1 / 10.2 / 10.6.  bf16 weights have nothing to decode: with more
@@ -181,7 +193,7 @@ def use_skinny(m: int, w: PackedWeight, x: torch.Tensor) -> bool:
         most = m
     else:
         most = g.few_rows_bf16_streamed if -(-w.n // 128) > (sm_count(x.device) if x.is_cuda else 148) else 0
-    return m <= most and skinny_fits(w, x)
+    return m <= most and skinny_fits(w, x, out, residual, ws)
 
 
 # Rows an expert gets on average up to which the grouped launches take that kernel; None: the operator configuration's
@@ -332,7 +344,7 @@ def wq_gemm(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = None,
         tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:0") if TUNED_PLANS else None
         if tuned is not None:
             splits, min_units = (None, 0) if tuned[0] else (tuned[1], None)
-        elif use_skinny(m, w, x):
+        elif use_skinny(m, w, x, out, residual, ws):
             return _wq_gemm_skinny(x, w, out, residual, ws, False)
     l = native.lib()
     if splits is None and min_units is None and use_stream_k(m, w.n, w.fmt, sm_count(x.device), k):
@@ -383,7 +395,7 @@ def wq_gemm_act(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = Non
         tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:1") if TUNED_PLANS else None
         if tuned is not None:
             splits, min_units = (None, 0) if tuned[0] else (tuned[1], None)
-        elif use_skinny(m, w, x):
+        elif use_skinny(m, w, x, out, None, ws):
             return _wq_gemm_skinny(x, w, out, None, ws, True)
     l = native.lib()
     stream_k = splits is None and (min_units is not None or use_stream_k(m, w.n, w.fmt, sm_count(x.device), k))
@@ -698,7 +710,7 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
         native.check(code, "cb_wq_gemm_fp8_grouped")
         return out
     per = rows / w.codes.shape[0]
-    if per <= skinny_rows_per_expert() and w.fmt != FMT_BF16 and skinny_fits(w, x):
+    if per <= skinny_rows_per_expert() and w.fmt != FMT_BF16 and skinny_fits(w, x, out):
         code = native.lib().cb_wq_gemm_skinny_grouped(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(),
                                                       out.stride(0), float(w.alpha), rows, w.n, w.k, w.group_k, int(swiglu), sc.tiles.data_ptr(),
                                                       8 if per <= 2 else 16 if per <= 8 else 32, code_stride, meta_stride, ws.status.data_ptr(), _stream())

@@ -75,3 +75,22 @@ def test_the_operator_configuration_sets_the_thresholds(calls):
     for bad in ({"gemm": {"few_rows_quantized": 33}}, {"gemm": {"few_rows_bf16": -1}}, {"moe": {"few_rows_per_expert": -1}}):
         with pytest.raises(ValueError):
             strategies.operator_config_from_dict(bad)
+
+
+@pytest.mark.parametrize("m,need", [(1, 2424832), (8, 2424832), (9, 4849664), (16, 4849664)])
+def test_a_workspace_too_small_for_the_parts_takes_the_other_kernels(calls, m, need):
+    w = _weight()
+    assert _route(calls, m, w, ws=_ws(gemm=need)) == "cb_wq_gemm_skinny" and _route(calls, m, w, ws=_ws(gemm=need - 1)) == "cb_wq_gemm_tp"
+    assert _route(calls, m, w, ws=_ws(counters=4)) == "cb_wq_gemm_skinny" and _route(calls, m, w, ws=_ws(counters=3)) == "cb_wq_gemm_tp"
+    act = _weight(act=True)
+    assert _route(calls, m, act, True, ws=_ws(gemm=need - 1)) == "cb_wq_gemm_act"
+
+
+@pytest.mark.parametrize("stride,at,takes", [(512, 0, True), (516, 4, True), (516, 1, False), (516, 2, False), (514, 1, True), (513, 3, True)])
+def test_results_that_start_anywhere(calls, stride, at, takes):
+    """Only rows a multiple of four elements apart are written four elements at a time."""
+    w = _weight()
+    out = torch.empty(at + 8 * stride, dtype=torch.bfloat16)[at:].view(8, stride)[:, :512]
+    even = torch.empty(8 * stride, dtype=torch.bfloat16).view(8, stride)[:, :512]
+    assert _route(calls, 8, w, out=out) == ("cb_wq_gemm_skinny" if takes else "cb_wq_gemm_tp")
+    assert _route(calls, 8, w, out=even, residual=out) == ("cb_wq_gemm_skinny" if takes else "cb_wq_gemm_tp")
