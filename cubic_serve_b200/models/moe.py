@@ -99,7 +99,7 @@ class MoeLayer:
             pol = active().moe
             big = max_tokens * self.top_k >= pol.large_routes_per_expert * self.expert_count
             mb = pol.rows_per_item_large if big else pol.rows_per_item_small
-            self.scratch = K.MoeScratch(max_tokens, self.top_k, hidden, self.gate_up.n, self.expert_count, mb, device)
+            self.scratch = K.MoeScratch(max_tokens, self.top_k, hidden, self.gate_up.n, self.expert_count, mb, device, experts=self.num_experts)
             self.least_rows = mb
             self.logits = torch.empty(max_tokens, self.num_experts, dtype=torch.bfloat16, device=device)
             self.out = torch.empty(max_tokens, hidden, dtype=torch.bfloat16, device=device)

@@ -633,8 +633,10 @@ def verify_sampled(q_val: torch.Tensor, q_id: torch.Tensor, p_val: torch.Tensor,
 class MoeScratch:
     """Fixed-address routing buffers for up to ``max_tokens`` tokens (graph-capturable)."""
 
-    def __init__(self, max_tokens: int, top_k: int, hidden: int, inter2: int, local_experts: int, mb: int, device) -> None:
+    def __init__(self, max_tokens: int, top_k: int, hidden: int, inter2: int, local_experts: int, mb: int, device, experts: int | None = None) -> None:
+        """``experts``: of the whole model, over which a step's routes spread (None: the local ones are all)."""
         routes = max_tokens * top_k
+        self.experts = experts or local_experts
         self.mb = mb                         # rows of a work item; a step may take more (``rows_per_work_item``)
         self.local_experts = local_experts
         self.max_items = -(-routes // mb) + local_experts
@@ -709,7 +711,7 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
                                                    ws.status.data_ptr(), _stream())
         native.check(code, "cb_wq_gemm_fp8_grouped")
         return out
-    per = rows / w.codes.shape[0]
+    per = rows / sc.experts                  # routes of all experts, wherever they live
     if per <= skinny_rows_per_expert() and w.fmt != FMT_BF16 and skinny_fits(w, x, out):
         code = native.lib().cb_wq_gemm_skinny_grouped(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(),
                                                       out.stride(0), float(w.alpha), rows, w.n, w.k, w.group_k, int(swiglu), sc.tiles.data_ptr(),

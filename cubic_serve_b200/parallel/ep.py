@@ -100,7 +100,7 @@ class FusedEp:
         self.experts_per_rank = num_experts // self.size
         virt = self.size * bufs.cap                                   # received records are the permutation's "tokens"
         mb = 64 if virt * bufs.top_k >= 32 * self.experts_per_rank else 32
-        self.sc = K.MoeScratch(virt, bufs.top_k, bufs.hidden, inter2, self.experts_per_rank, mb, device)
+        self.sc = K.MoeScratch(virt, bufs.top_k, bufs.hidden, inter2, self.experts_per_rank, mb, device, experts=num_experts)
         i32 = dict(dtype=torch.int32, device=device)
         self.local_cnt = torch.zeros(self.size, **i32)
         self.sent = torch.full((bufs.cap, self.size), -1, **i32)

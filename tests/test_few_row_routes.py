@@ -94,3 +94,14 @@ def test_results_that_start_anywhere(calls, stride, at, takes):
     even = torch.empty(8 * stride, dtype=torch.bfloat16).view(8, stride)[:, :512]
     assert _route(calls, 8, w, out=out) == ("cb_wq_gemm_skinny" if takes else "cb_wq_gemm_tp")
     assert _route(calls, 8, w, out=even, residual=out) == ("cb_wq_gemm_skinny" if takes else "cb_wq_gemm_tp")
+
+
+@pytest.mark.parametrize("ranks", [1, 2, 8])
+@pytest.mark.parametrize("tokens,entry", [(16, "cb_wq_gemm_skinny_grouped"), (64, "cb_wq_gemm_skinny_grouped"), (65, "cb_wq_gemm_grouped"), (200, "cb_wq_gemm_grouped")])
+def test_rows_of_an_expert_count_over_all_ranks(calls, ranks, tokens, entry):
+    """32 experts, 8 a token: 16 rows an expert at 64 tokens, whichever rank owns them."""
+    local, rows = 32 // ranks, tokens * 8
+    w = wq_pack.PackedWeight(wq_pack.FMT_NVFP4, 128, 256, 16, torch.zeros(local, 16), torch.zeros(local, 16), 1.0)
+    sc = K.MoeScratch(tokens, 8, 256, 128, local, 32, "cpu", experts=32)
+    K.wq_gemm_grouped(torch.zeros(rows, 256, dtype=torch.bfloat16), w, torch.empty(rows, 128, dtype=torch.bfloat16), rows, sc, 16, 16, _ws())
+    assert calls.made.pop()[0] == entry
