@@ -129,10 +129,16 @@ class BatchBuilder:
     def _prompts(self, blocks: list[int]) -> tuple[int, int]:
         """The longest run of neighbouring segments with at least four row blocks each, as row blocks ``[lo, hi)`` for the prompt
         kernel (a CTA takes eight blocks and walks the steps of one request at a time; with fewer of a request most of its rows
-        idle).  Both kernels' times follow the tokens that the row blocks see, the prompt kernel's with a smaller factor and a
-        tail of half its longest CTA, for it has no KV splits: few blocks behind a long context stay with the general kernel.
-        Measured: 24400 against 16000 tokens x heads a us, 3.2 us a step of 64 tokens (8 x 1024 tokens, 32 over 8 heads, 498 against
-        703 us; one prompt of 331, 26 against 19)."""
+        idle), if that is the faster one by a tenth of its estimated time.
+
+        Prompt kernel: 3 us a step of 64 tokens, and as much as four steps around them for every CTA; CTAs start last blocks first, so that
+        with more of them than SMs the step ends with the longest, with one that starts late behind the load before it, or with two that
+        have to share an SM.  General kernel: 0.128 us a page and SM, 2.1 us a CTA and SM, 0.06 us a page of the longest split, and
+        14.5 us for its launch, which is there anyway when there are other row blocks and twice when they are on both sides.
+        Fitted to 180 steps of 8 shapes of heads (1 to 32 key / value heads, groups of 1 to 16; 1 to 40 portions of 20 to 6000 tokens behind 0
+        to 8000): mean errors 3 and 7 %; without the margin some steps would be up to 1.26 times slower than with the general kernel, with
+        it none is, nor of 60 steps that have decode or review rows beside the portions (2 % at most).  E.g. 32 over 8 heads: 8 x 1024 tokens
+        513 against 707 us, one prompt of 331 33 against 29, 40 x 20 tokens behind 300 106 against 67.  (One B200.)"""
         best, at, lo = (0, 0), 0, 0
         for n in blocks + [0]:
             if n < 4:
@@ -143,10 +149,25 @@ class BatchBuilder:
         lo, hi = best
         if lo == hi:
             return 0, 0
-        ctx = self.stage.h["rb_ctx"][lo:hi]
-        seen = int(ctx.sum()) * self.kv_heads                 # tokens over all row blocks and heads
-        prompt = seen / 24400 + 1.6 * (int(ctx.max()) // 64 + 1)
-        return best if prompt < seen / 16000 else (0, 0)
+        from ..ops.strategies import active
+        h, n, heads, sms = self.stage.h, hi - lo, self.kv_heads, max(1, active().attention.target_ctas // 2)
+        seen, req = h["rb_ctx"][lo:hi] + h["rb_qcount"][lo:hi] - 1, h["rb_req"][lo:hi]
+        last = np.ones(n, dtype=bool)                         # the last block of a request in its CTA sees most
+        last[:-1] = (req[1:] != req[:-1]) | (np.arange(1, n) % 8 == 0)
+        steps = np.add.reduceat(np.where(last, -(-seen // 64), 0), np.arange(0, n, 8)) + 4
+        longest = float(steps.max())
+        if steps.size * heads > sms:
+            order, ranked = steps[::-1], np.sort(steps)[::-1]
+            before = (np.cumsum(order) - order) * (heads / sms)
+            longest = max(longest, float((before + order).max() - 0.5 * steps.mean()), float(ranked[(sms - 1) // heads] + ranked[sms // heads]))
+        pages, splits = -(-seen // 16), self._splits(n)
+        general = (0.128 * int(pages.sum()) * heads + 2.1 * n * heads * splits) / sms + 0.06 * int(pages.max()) / splits
+        prompt, sides = 3.9 + 2.96 * longest, (lo > 0) + (hi < sum(blocks))
+        if sides == 0:
+            general += 14.5
+        elif sides == 2:
+            prompt += 14.5
+        return best if prompt < 0.9 * general else (0, 0)
 
     def fill(self, segs: list[Segment], pad_rows_to: int | None = None):
         return self._fill(segs, pad_rows_to)

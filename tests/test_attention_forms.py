@@ -13,13 +13,15 @@ from cubic_serve_b200.ops.strategies import active
 
 def _fill(portions, hq=32, hkv=8, pad=None):
     """A step of ``(context, tokens)`` portions."""
-    bb = BatchBuilder(max_rows=max(len(portions), pad or 0), max_tokens=8192, max_model_len=9000, group=hq // hkv, kv_heads=hkv, device="cpu")
+    bb = BatchBuilder(max_rows=max(len(portions), pad or 0), max_tokens=9000, max_model_len=9000, group=hq // hkv, kv_heads=hkv, device="cpu")
     segs, page = [], 0
     for r, (start, n) in enumerate(portions):
         per = -(-(start + n) // 16)
         segs.append(Segment(r, [1] * n, start, list(range(page, page + per)), uid=r))
         page += per
-    return bb.fill(segs, pad_rows_to=pad)[0]
+    b = bb.fill(segs, pad_rows_to=pad)[0]
+    bb.stage.upload()
+    return b
 
 
 @pytest.fixture
@@ -70,3 +72,63 @@ def test_partial_sums_of_target_and_draft_head_stay_small(monkeypatch, launches,
     assert sum(n for n, *_ in target) == b.num_row_blocks
     # splits that fill the machine once (twice for the decode form, whose splits are rounded up from half as many blocks)
     assert all(s == 1 or n * hkv * s <= 4 * active().attention.target_ctas for n, _, _, s in target)
+
+
+@pytest.mark.parametrize("hq,hkv,portions,prompt", [
+    (32, 8, [(0, 1024)] * 8, True), (32, 8, [(2048, 256)] * 4, True), (32, 8, [(0, 2048)], True), (32, 8, [(0, 64)] * 16, True), (32, 8, [(0, 331)], False),
+    (32, 8, [(240, 104)] * 7, False), (32, 8, [(300, 20)] * 40, False), (32, 8, [(4000, 64)], False), (32, 32, [(240, 104)] * 7, False), (32, 32, [(0, 2048)], True),
+    (64, 4, [(1000, 128)] * 2, True), (64, 4, [(4000, 64)], False), (16, 2, [(0, 2048)], True), (16, 2, [(0, 700)], False), (16, 1, [(0, 2048)], True),
+    (8, 1, [(0, 1100)], False), (8, 8, [(0, 200)] * 30, False), (8, 8, [(3000, 1000)], False)])
+def test_prompts_take_the_kernel_that_was_measured_faster(hq, hkv, portions, prompt):
+    b = _fill(portions, hq, hkv)
+    assert b.attn_prompts == ((0, b.num_row_blocks) if prompt else (0, 0)) and not b.attn_decode
+
+
+@pytest.mark.parametrize("hq,hkv,portions,prompts", [
+    (32, 8, [(1000, 1)] * 64 + [(0, 512)] * 2, (64, 320)), (32, 4, [(700, 1)] * 20 + [(0, 512)] * 2 + [(700, 1)] * 20, (0, 0)),
+    (16, 1, [(1000, 4)] * 32 + [(0, 1024)] * 4, (0, 0)),               # the long review CTAs would start last
+    (8, 8, [(1000, 4)] * 32 + [(0, 1024)] * 4, (0, 0)), (32, 8, [(1000, 4)] * 32 + [(0, 1024)] * 4, (32, 1056)), (8, 8, [(1000, 1)] * 64 + [(0, 1024)] * 7, (0, 0))])
+def test_prompts_beside_other_rows(hq, hkv, portions, prompts):
+    assert _fill(portions, hq, hkv).attn_prompts == prompts
+
+
+DECODE, PROMPT = (900, 1), (0, 1024)
+
+
+@pytest.mark.parametrize("hq,hkv", [(32, 8), (16, 1)])              # blocks of four positions and of one
+@pytest.mark.parametrize("portions,first", [([PROMPT] * 8, 0), ([DECODE] * 5 + [PROMPT] * 8, 5), ([PROMPT] * 8 + [DECODE] * 5, 0), ([DECODE] * 3 + [PROMPT] * 8 + [(10, 2)] + [DECODE], 3),
+                                            ([PROMPT] + [DECODE] + [PROMPT] * 6 + [(5, 3)] + [PROMPT], 2)])
+def test_a_step_of_prompts_and_other_rows_is_cut_once(launches, portions, first, hq, hkv):
+    """The longest run of prompts in one launch, what is before and after it in one each, with the splits of those alone."""
+    b = _fill(portions, hq, hkv)
+    qb = 16 // (hq // hkv)
+    blocks = [-(-n // qb) for _, n in portions]
+    run = 6 if PROMPT in portions[:1] and DECODE in portions[1:2] else 8
+    lo, hi = sum(blocks[:first]), sum(blocks[:first + run])
+    assert b.attn_prompts == (lo, hi)
+    rest = b.num_row_blocks - (hi - lo)
+    splits = min(active().attention.max_splits, max(1, -(-active().attention.target_ctas // max(1, rest * hkv))))
+    q = torch.zeros(b.num_tokens, hq, 128)
+    made = [(n, form, s) for n, form, s in ((lo, "", splits), (hi - lo, "prefill", 1), (b.num_row_blocks - hi, "", splits)) if n]
+    assert DecoderRunner._attend(_runner(hq, hkv), b, q, q, None, 0, b.num_row_blocks) == len(made)
+    assert [(n, form, s) for n, _, form, s in launches] == made
+    # lanes of a pipeline stage: any cut gives every block to the same form
+    form_of = ["prefill" if lo <= i < hi else "" for i in range(b.num_row_blocks)]
+    for cut in (1, lo, lo + 9, hi - 1, hi, b.num_row_blocks - 1):
+        launches.clear()
+        for rb0, rb1 in ((0, cut), (cut, b.num_row_blocks)):
+            DecoderRunner._attend(_runner(hq, hkv), b, q, q, None, rb0, rb1)
+        got = [form for n, _, form, _ in launches for _ in range(n)]
+        assert got == form_of
+        at = 0
+        for n, qstart, _, _ in launches:
+            assert qstart == int(b.rb_qstart[at])
+            at += n
+
+
+def test_decode_steps_take_the_decode_form(launches):
+    for hq, hkv, form in ((32, 8, "decode"), (8, 8, "decode"), (16, 1, "")):
+        b = _fill([(100 + i, 1) for i in range(7)], hq, hkv, pad=8)
+        q = torch.zeros(8, hq, 128)
+        assert DecoderRunner._attend(_runner(hq, hkv), b, q, q, None, 0, 8) == 1
+        assert launches.pop()[:3] == (8, 0, form)
