@@ -74,6 +74,11 @@ struct __align__(8) SkCtl {
   SkSegment deferred[2];
 };
 
+// What the two rings share, and at least as many activation slots as decode groups at every tile: a group that has decoded k-block
+// j - groups knows that j - groups - slots has been multiplied, so its wait for j - slots is at most one phase ahead of the barrier.
+static constexpr size_t kSkRingBytes = 232448 - 1024 - 1024 - sizeof(SkCtl) - kSkEpiScratchBytes;
+static_assert((kSkRingBytes - kSkDecodeGroups * sk_cstage_bytes(kFmtCubic4)) / (256 * 128 + kATileBytes) >= kSkDecodeGroups, "activation ring");
+
 // The deal.  Identical arithmetic on every thread of every role, so all roles of a CTA walk the same list.
 struct SkIter {
   // 32-bit arithmetic throughout: the streamed region has at most one tile per SM, so units * CTAs < 2^31
@@ -1085,14 +1090,14 @@ int launch_streamk(int fmt, const CUtensorMap& tx, const CUtensorMap& tw, WqGemm
   if (grid < 1) return -17;
 
   const size_t ax = static_cast<size_t>(p.pair ? p.mb >> 1 : p.mb) * 128 + kATileBytes;
-  const size_t budget = 232448 - 1024 - 1024 - sizeof(SkCtl) - kSkEpiScratchBytes;
+  const size_t budget = kSkRingBytes;
   const size_t kSkCStageBytes = static_cast<size_t>(sk_cstage_bytes(fmt));
   int S, NC;
   if (fmt_is_direct(fmt)) {
     NC = 0;
     S = static_cast<int>(budget / ax);
   } else {
-    S = static_cast<int>((budget - 4 * kSkCStageBytes) / ax);
+    S = static_cast<int>((budget - kSkDecodeGroups * kSkCStageBytes) / ax);
     if (S > kSkMaxAx) S = kSkMaxAx;
     NC = static_cast<int>((budget - S * ax) / kSkCStageBytes);
     // A whole number of rounds of the decode groups: a slot then always belongs to the same group, whose wait for k-block j cannot
@@ -1102,7 +1107,7 @@ int launch_streamk(int fmt, const CUtensorMap& tx, const CUtensorMap& tw, WqGemm
     NC = NC >= kSkMaxC ? kSkMaxC : NC >= kSkDecodeGroups ? kSkDecodeGroups : 0;
   }
   if (S > kSkMaxAx) S = kSkMaxAx;
-  if (S < 2 || (!fmt_is_direct(fmt) && NC < 2)) return -14;
+  if (S < 2 || (!fmt_is_direct(fmt) && (S < kSkDecodeGroups || NC == 0))) return -14;
   if (fmt == kFmtFp8Block) return -14;            // block scales need the per-stage promotion of the per-tile kernel
   p.ax_stages = S;
   p.c_stages = NC;
