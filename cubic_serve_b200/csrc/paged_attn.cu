@@ -566,8 +566,8 @@ paged_decode_kernel(const AttnParams p) {
   const int G = p.G;
   const int total = ctx + qcount - 1, pages = (total + kPageTokens - 1) / kPageTokens;
   const int splits = max(1, min(p.splits, (pages + kDecMinPages - 1) / kDecMinPages));
-  const int per = (pages + splits - 1) / splits;
-  const int used = (pages + per - 1) / per;               // splits that have pages
+  const int per = max(1, (pages + splits - 1) / splits);
+  const int used = max(1, (pages + per - 1) / per);       // splits that have pages; rows that see no token are written, as zeros
   if (split >= used) return;
   if (qcount * G > kDecRows) {                            // the caller's promise does not hold: said, not computed wrongly
     if (tid == 0) atomicExch(p.status, static_cast<uint32_t>(kErrBadArgument));

@@ -453,7 +453,12 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm.p_full));
     }
-    if (steps > 0) {
+    if (steps == 0) {                                    // no row sees a token
+      if (out_row != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) reinterpret_cast<uint4*>(out_row)[j] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    } else {
       if (ok) ok = mbar_wait_park(smem_u32(&sm.pv_done), (steps - 1) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();

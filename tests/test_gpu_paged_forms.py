@@ -151,3 +151,14 @@ def test_prompt_form_has_the_range_of_f16_for_scales(kb, vb, top):
     blocks = [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)]
     want = _run("", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
     assert torch.isfinite(want.float()).all() and _close(_run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1), want)
+
+
+@pytest.mark.parametrize("form,splits", [("", 1), ("decode", 1), ("decode", 4), ("prefill", 1)])
+def test_rows_that_see_no_token_are_zero(form, splits):
+    """Alone in their CTA and beside rows that see something."""
+    cache, table = _cache([70, 70], 1, 8, 8, 7)
+    q = torch.randn(12, 4, D, device=DEV).bfloat16()
+    for blocks in ([(0, 0, 1, 0)], [(0, 0, 1, 0), (1, 1, 1, 50)], [(0, 4 * i, 1, 0) for i in range(3)]):
+        out = _run(form, q, cache, table, blocks, 4, 1, 8, 8, splits)
+        assert all((out[t] == 0).all() for _, t, _, ctx in blocks if ctx == 0)
+        assert all((out[t] != 0).any() and torch.isfinite(out[t].float()).all() for _, t, _, ctx in blocks if ctx)
