@@ -372,6 +372,14 @@ class DecoderRunner(StepRunner):
             from ..parallel.ep import FusedEp, symmetric_ep_buffers
             bufs = symmetric_ep_buffers(tp.group, H, cfg.experts_per_token, tp.fused.b.max_tokens, dev)
             self.ep = FusedEp(bufs, dev, cfg.num_experts, 2 * cfg.moe_intermediate_size, ws=self.ws)
+        else:
+            # one set of expert buffers for all layers, made here: 0.84 GB at 8192 tokens of 8 experts (hidden 2048), and a set a
+            # layer cost the first step 10 to 50 ms of allocations for six layers
+            made = []
+            for lw in weights.layers:
+                if lw.moe is not None:
+                    lw.moe.share_scratch(made, max_tokens, H, dev)
+                    made.append(lw.moe)
 
     def copy_state(self, src: torch.Tensor, dst: torch.Tensor) -> None:
         """Bit-preserving copies of whole recurrent-state rows ``src[i] -> dst[i]`` (int32 device tensors) in every

@@ -112,6 +112,22 @@ class MoeLayer:
                 self.sh_sig = torch.empty(max_tokens, 1, **bf)
         return self.scratch
 
+    def share_scratch(self, others: list["MoeLayer"], max_tokens: int, hidden: int, device) -> None:
+        """Buffers of a layer in ``others`` with the same shapes, else own ones.  Layers of a runner follow one another on its
+        stream, so that one set serves them all; ``out`` is read before the next layer's experts run."""
+        for o in others:
+            mine, its = self._buffer_shapes(), o._buffer_shapes()
+            if mine == its and o.scratch is not None and o.scratch.topk_ids.shape[0] >= max_tokens:
+                self.scratch, self.least_rows, self.logits, self.out = o.scratch, o.least_rows, o.logits, o.out
+                if self.shared_gate_up is not None:
+                    self.sh_gu, self.sh_act, self.sh_out, self.sh_logit, self.sh_sig = o.sh_gu, o.sh_act, o.sh_out, o.sh_logit, o.sh_sig
+                return
+        self.ensure_scratch(max_tokens, hidden, device)
+
+    def _buffer_shapes(self) -> tuple:
+        shared = None if self.shared_gate_up is None else (self.shared_gate_up.n, self.shared_gate.n)
+        return self.top_k, self.gate_up.n, self.gate_up.k, self.expert_count, self.num_experts, shared
+
     def forward(self, x: torch.Tensor, runner=None, residual: torch.Tensor | None = None,
                 out: torch.Tensor | None = None) -> torch.Tensor:
         """``x``: normalised activations ``[T, H]``; returns this rank's (partial) FFN output ``[T, H]``.
