@@ -11,7 +11,10 @@
 //   * it calls pdl_wait() before its first access to global memory that another kernel writes, and before its
 //     first global write (an earlier kernel may still be reading the destination);
 //   * before pdl_wait() it touches only shared / tensor memory and operands that no kernel writes (the weights);
-//   * pdl_launch_dependents() comes after pdl_wait(), so completion stays transitive along the stream.
+//   * no CTA is finished before a pdl_wait() of its own has returned, so completion stays transitive along the stream:
+//     whoever waits for this kernel waits for its predecessors as well.  Most kernels call pdl_launch_dependents() after
+//     pdl_wait(); the weight GEMMs call it first, because what their dependents do before their own pdl_wait() (set-up, weights
+//     into their own shared memory) may overlap with a predecessor's predecessor too.
 // A kernel launched without the attribute (PyTorch's own, or with the switch off) orders itself after the
 // whole predecessor as usual; pdl_wait() then returns at once.  The attribute is captured into CUDA graphs
 // as a programmatic dependency edge.

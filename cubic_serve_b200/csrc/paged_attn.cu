@@ -11,8 +11,11 @@
 //     plus one packed subtract; group scales are applied to the 4 fp32
 //     accumulators of a channel group (K) or folded into P (V), never per code;
 //   * a row block is 16 MMA rows = (16 / G) consecutive query positions x G
-//     query heads of one kv head, so the same kernel serves decode (one
-//     position), speculative review rows and causal prefill chunks.
+//     query heads of one kv head, so one general kernel serves speculative
+//     review rows, short portions of prompts and decode rows beside them.
+//
+// Steps of decode rows alone, up to eight rows a block, take the decode form below (paged_decode_kernel); longer portions of prompts
+// take paged_prefill.cu where the caller estimates that it is the faster one.
 //
 // Waits are bounded; on a timeout the CTA records Status and exits cleanly.
 #include "paged_attn.cuh"

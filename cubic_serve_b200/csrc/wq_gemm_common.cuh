@@ -1,6 +1,7 @@
 // Shared pieces of the weight-quantized GEMM kernels: formats, tile constants, the tensor-parallel link,
 // launch parameters, the packed bf16x2 decoders and the tensor-map helper.  Included by wq_gemm.cu (one CTA
-// per tile: grouped expert GEMMs, explicit split-K) and wq_gemm_sk.cu (persistent stream-K kernel).
+// per tile: grouped expert GEMMs, explicit split-K), wq_gemm_sk.cu (persistent stream-K kernel) and wq_gemm_skinny.cu
+// (few batch rows).
 #pragma once
 #include "ptx.cuh"
 #include <cuda.h>

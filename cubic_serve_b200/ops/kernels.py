@@ -377,8 +377,8 @@ def wq_gemm_act(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = Non
                 ws: Workspace | None = None, min_units: int | None = None, link=None) -> torch.Tensor:
     """Gate/up projection with SwiGLU in the GEMM epilogue: ``out[M, N/2] = silu(x Wg^T) * (x Wu^T)``.
 
-    ``w`` is the ``[gate; up]`` matrix in the interleaved row order (``wq_pack.swiglu_interleave``).  The projection
-    ``link`` (gather-wait only) as in ``wq_gemm``.  The projection is rounded to bf16 before the activation, as when ``wq_gemm`` and ``swiglu`` run as two kernels, so both paths
+    ``w`` is the ``[gate; up]`` matrix in the interleaved row order (``wq_pack.swiglu_interleave``); ``link`` (gather-wait
+    only) as in ``wq_gemm``.  The projection is rounded to bf16 before the activation, as when ``wq_gemm`` and ``swiglu`` run as two kernels, so both paths
     give the same values; the ``[M, N]`` intermediate is never written.  Kernel choice as in ``wq_gemm``.
     """
     assert w.act_interleaved, "weight rows are not in the SwiGLU order"
