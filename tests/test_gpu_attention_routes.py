@@ -50,7 +50,7 @@ def test_prompt_steps_of_a_speculative_executor():
     from cubic_serve_b200.models.mtp import MtpRunner, random_mtp_weights
     from cubic_serve_b200.ops import kernels as K
     dev = torch.device("cuda")
-    cfg = ModelConfig(name="routes", num_layers=2, hidden_size=512, num_q_heads=8, num_kv_heads=2, head_dim=128, intermediate_size=1024, vocab_size=2048,
+    cfg = ModelConfig(name="routes", num_layers=2, hidden_size=512, num_q_heads=16, num_kv_heads=4, head_dim=128, intermediate_size=1024, vocab_size=2048,
                       rope_theta=1e6, quant=QuantSpec("cubic", 4, 128))
     n, pages = 1024, 66
     runner = DecoderRunner(cfg, random_decoder_weights(cfg, dev, seed=0, std=0.05), num_pages=8 * pages, max_tokens=8192)
