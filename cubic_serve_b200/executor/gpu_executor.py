@@ -139,29 +139,36 @@ class BatchBuilder:
         to 8000): mean errors 3 and 7 %; without the margin some steps would be up to 1.26 times slower than with the general kernel, with
         it none is, nor of 60 steps that have decode or review rows beside the portions (2 % at most).  E.g. 32 over 8 heads: 8 x 1024 tokens
         513 against 707 us, one prompt of 331 33 against 29, 40 x 20 tokens behind 300 106 against 67.  (One B200.)"""
-        best, at, lo = (0, 0), 0, 0
-        for n in blocks + [0]:
+        best, at, lo, first, of = (0, 0), 0, 0, 0, (0, 0)
+        for i, n in enumerate(blocks + [0]):
             if n < 4:
                 if at - lo > best[1] - best[0]:
-                    best = (lo, at)
-                lo = at + n
+                    best, of = (lo, at), (first, i)
+                lo, first = at + n, i + 1
             at += n
         lo, hi = best
         if lo == hi:
             return 0, 0
         from ..ops.strategies import active
-        h, n, heads, sms = self.stage.h, hi - lo, self.kv_heads, max(1, active().attention.target_ctas // 2)
-        seen, req = h["rb_ctx"][lo:hi] + h["rb_qcount"][lo:hi] - 1, h["rb_req"][lo:hi]
-        last = np.ones(n, dtype=bool)                         # the last block of a request in its CTA sees most
-        last[:-1] = (req[1:] != req[:-1]) | (np.arange(1, n) % 8 == 0)
-        steps = np.add.reduceat(np.where(last, -(-seen // 64), 0), np.arange(0, n, 8)) + 4
-        longest = float(steps.max())
+        h, qb, heads, sms = self.stage.h, self.qb, self.kv_heads, max(1, active().attention.target_ctas // 2)
+        # tokens that a CTA's last block sees, in steps; a request that ends inside a CTA adds its own
+        last = np.minimum(np.arange(lo + 7, hi + 7, 8), hi - 1)
+        steps = (h["rb_ctx"][last] + h["rb_qcount"][last] + 62) // 64 + 4
+        pages, at, most = 0.0, lo, 0
+        for i in range(*of):
+            n, start, nb = int(h["seg_count"][i]), int(h["seg_pos0"][i]), blocks[i]
+            at += nb
+            most = max(most, start + n)
+            pages += (nb * start + qb * nb * (nb + 1) // 2 - (nb * qb - n)) / 16 + nb * 15 / 32
+            if at < hi and (at - lo) % 8:
+                steps[(at - lo) // 8] += -(-(start + n) // 64)
+        n, longest = hi - lo, float(steps.max())
         if steps.size * heads > sms:
             order, ranked = steps[::-1], np.sort(steps)[::-1]
-            before = (np.cumsum(order) - order) * (heads / sms)
-            longest = max(longest, float((before + order).max() - 0.5 * steps.mean()), float(ranked[(sms - 1) // heads] + ranked[sms // heads]))
-        pages, splits = -(-seen // 16), self._splits(n)
-        general = (0.128 * int(pages.sum()) * heads + 2.1 * n * heads * splits) / sms + 0.06 * int(pages.max()) / splits
+            start = np.cumsum(order) * (heads / sms) + order * (1 - heads / sms)          # the load before a CTA and the CTA
+            longest = max(longest, float(start.max()) - 0.5 * float(steps.sum()) / steps.size, float(ranked[(sms - 1) // heads] + ranked[sms // heads]))
+        splits = self._splits(n)
+        general = (0.128 * pages * heads + 2.1 * n * heads * splits) / sms + 0.06 * most / 16 / splits
         prompt, sides = 3.9 + 2.96 * longest, (lo > 0) + (hi < sum(blocks))
         if sides == 0:
             general += 14.5

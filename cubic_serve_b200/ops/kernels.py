@@ -185,6 +185,8 @@ def use_skinny(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | Non
     weight tiles than SMs they stream at 65 / 68 / 74 us against 98 / 98 / 102 (50688 x 4096), with fewer the split tiles of the
     other kernel are as good from 16 rows on (8.0 / 10.4 against 9.2 / 9.2, 4096 x 4096).  (One B200, weights not in L2.)
     The thresholds live in the operator configuration (``few_rows_*``); an installed plan comes before them."""
+    if m > 32:
+        return False
     from .strategies import active
     g = active().gemm
     if w.fmt != FMT_BF16:
