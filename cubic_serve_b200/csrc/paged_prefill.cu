@@ -8,9 +8,10 @@
 // rounding to f16 (V), as in the general kernel.  So a step makes four score tiles in tensor memory, one per channel group, and four
 // scaled copies of the probabilities; what is left to pay is that arithmetic: 256 fp32 multiply-adds, 256 multiplications, 128
 // packings and 64 exponentials a row and step.
-// One softmax warp a scheduler pays it, and waits for its own tensor-memory loads besides: about 5800 cycles a step.  General kernel -> this one,
-// 32 heads over 8: 8 x 1024 tokens 703 -> 498 us, 4 x 256 behind 2048 267 -> 223; K4 V8, 32 over 4, 2 x 2048 549 -> 400; 6 bit, 64 over 4,
-// 3 x 500 168 -> 118; one prompt of 331 tokens 19 -> 26, which the caller leaves to the general kernel.
+// One softmax warp a scheduler pays it, and waits for its own tensor-memory loads besides: about 5800 cycles a step.  General kernel -> this one
+// (with 8 us of launch and cold operands), 32 heads over 8: 8 x 1024 tokens 707 -> 513 us, 4 x 256 behind 2048 284 -> 234; 6 bit, 64 over 4,
+// 3 x 500 195 -> 136; one prompt of 331 tokens 29 -> 33, which the caller leaves to the general kernel.  What keeps values that are not finite
+// to those who see them, and scaled probabilities in the range of f16, costs 0.5 % of it.
 //
 // Roles: warps 0-3 own a row a thread (softmax needs no exchange: tensor-memory lane = row); warps 4-7 convert raw pages, which warp 4
 // copies two steps ahead, to the swizzled operands (K as [token][channel], V transposed as [channel][token]); warp 8 issues the MMAs.
@@ -165,6 +166,29 @@ __device__ __forceinline__ void pf_convert(PfSmem& sm, int b, const uint8_t* raw
   }
 }
 
+// A step with a V scale that is not finite: zero times it, and it may be another request's, is not zero.  The warp of the MMAs clears the
+// tokens that a row does not see before it multiplies (in the softmax warps, which have no register left for it, the check alone was 1 % of the kernel).
+// `rb_qcount`, `rb_ctx`: of the CTA's first row block; `blocks`: from there to the last; `i`: the step.
+__device__ __noinline__ void pf_unseen(PfSmem& sm, const int* rb_qcount, const int* rb_ctx, int blocks, int G, int i, int lane) {
+  int run = 0;
+  while (i >= sm.run[run].steps) i -= sm.run[run++].steps;
+  for (int row = lane; row < kPfRows; row += 32) {
+    const int blk = row >> 4, qp = (row & 15) / G;
+    int sees = 0;
+    if (blk >= sm.run[run].first && blk < sm.run[run].end && blk < blocks && qp < rb_qcount[blk]) sees = rb_ctx[blk] + qp - i * kPfTok;
+    for (int c = max(sees, 0) >> 3; c < 8; ++c) {
+      const int keep = min(max(sees - 8 * c, 0), 8);                 // tokens of the chunk
+      for (int cg = 0; cg < 4; ++cg) {
+        uint32_t* at = reinterpret_cast<uint32_t*>(sm.p[cg] + row * 128 + ((c ^ (row & 7)) << 4));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) at[k] &= keep >= 2 * k + 2 ? 0xFFFFFFFFu : keep == 2 * k + 1 ? 0xFFFFu : 0u;
+      }
+    }
+  }
+  fence_proxy_async_smem();
+  __syncwarp();
+}
+
 template <int KBITS, int VBITS>
 __global__ void __launch_bounds__(kPfThreads, 1)
 paged_prefill_kernel(const AttnParams p, const int row_blocks) {
@@ -285,6 +309,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
       const int b = i & 1;
       if (ok) ok = mbar_wait_park(smem_u32(&sm.p_full), i & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
+      if ((sm.vs_kind[b][0] | sm.vs_kind[b][1]) & kPfWild) pf_unseen(sm, p.rb_qcount + rb0, p.rb_ctx + rb0, row_blocks - rb0, p.G, i, lane);
       tc_fence_after();
       if (ok && leader) {
 #pragma unroll
@@ -345,15 +370,11 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
     float m = -INFINITY, l = 0.f;
     PfWalk at;
     for (int i = 0; i < steps; ++i) {
-      const int b = i & 1;
-      auto visible = [&](int run, int step) {            // tokens of the step that this row sees
-        const PfRun& r = sm.run[run];
-        return (blk >= r.first && blk < r.end) ? limit - step * kPfTok : 0;
-      };
-      const int sees = visible(at.run, at.step);
+      const int b = i & 1, tok0 = at.step * kPfTok;
+      const PfRun& r = sm.run[at.run];
+      const int sees = (blk >= r.first && blk < r.end) ? limit - tok0 : 0;       // tokens of the step that this row sees
       at.advance(sm);
       if (ok) ok = mbar_wait_park(smem_u32(&sm.kv_full[b]), (i >> 1) & 1, abort_flag);      // the scales
-      const uint32_t vs_kind = sm.vs_kind[b][0] | sm.vs_kind[b][1];
       if (ok) ok = mbar_wait_park(smem_u32(&sm.s_full), i & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       tc_fence_after();
@@ -391,7 +412,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
       for (int j = 0; j < kPfTok / 2; ++j) mx[j & 3] = fmaxf(mx[j & 3], fmaxf(s[j].x, s[j].y));
       const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       float alpha = 1.f;
-      const bool grew = top > m + (vs_kind & kPfLarge ? 0.f : kPfGrowth) || (m == -INFINITY && top > m);
+      const bool grew = top > m + ((sm.vs_kind[b][0] | sm.vs_kind[b][1]) & kPfLarge ? 0.f : kPfGrowth) || (m == -INFINITY && top > m);
       if (grew) {
         alpha = fast_exp2(m - top);
         m = top;
@@ -433,21 +454,6 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
           *reinterpret_cast<uint4*>(sm.p[cg] + tid * 128 + ((c ^ (tid & 7)) << 4)) =
               make_uint4(pack_f16x2(w0.x, w0.y), pack_f16x2(w1.x, w1.y), pack_f16x2(w2.x, w2.y), pack_f16x2(w3.x, w3.y));
         }
-      // zero times a scale that is not finite, perhaps another request's, is not zero: tokens that a row does not see become zeros
-      if (vs_kind & kPfWild) {
-        // how many it sees is worked out again: the kernel has no register to hold it up to here
-        const int n = at.step == 0 ? visible(at.run - 1, sm.run[at.run - 1].steps - 1) : visible(at.run, at.step - 1);
-#pragma unroll 1
-        for (int c = max(n, 0) >> 3; c < 8; ++c) {
-          const int keep = min(max(n - 8 * c, 0), 8);                // tokens of the chunk
-#pragma unroll 1
-          for (int cg = 0; cg < 4; ++cg) {
-            uint32_t* at4 = reinterpret_cast<uint32_t*>(sm.p[cg] + tid * 128 + ((c ^ (tid & 7)) << 4));
-#pragma unroll
-            for (int k = 0; k < 4; ++k) at4[k] &= keep >= 2 * k + 2 ? 0xFFFFFFFFu : keep == 2 * k + 1 ? 0xFFFFu : 0u;
-          }
-        }
-      }
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
