@@ -19,8 +19,8 @@
 //
 // Measured, weights not in L2 (floor = packed bytes / 6.65 TB/s), Cubic weights, 8 rows: 24576 x 4096 22.3 us (floor 9.5, tcgen05
 // kernels 34), 4096 x 12288 12.8 (4.7, 21.5), 6144 x 4096 9.1 (2.4, 14.8), 4096 x 4096 6.4 (1.6, 10.1); bf16 50688 x 4096 65 (62,
-// 98).  What is left above the floor is the decode (integer pipe 45 % busy, four warps a scheduler) and 5 us of start, last
-// loads and the sum of the parts.
+// 98).  What is left above the floor is the decode (integer pipe 38 % busy, four warps a scheduler that issue in 37 % of the cycles) and
+// 5 us of start, last loads and the sum of the parts.
 #include "wq_gemm_common.cuh"
 #include "launch.cuh"
 
