@@ -176,8 +176,8 @@ class BatchBuilder:
             prompt += 14.5
         return best if prompt < 0.9 * general else (0, 0)
 
-    def fill(self, segs: list[Segment], pad_rows_to: int | None = None):
-        return self._fill(segs, pad_rows_to)
+    def fill(self, segs: list[Segment], pad_rows_to: int | None = None, review: bool = False):
+        return self._fill(segs, pad_rows_to, review)
 
     def _sync_page_row(self, s: Segment) -> None:
         """Bring row ``request_slot`` of the host page table up to date (only the new tail is written)."""
@@ -198,7 +198,9 @@ class BatchBuilder:
         for slot in slots:
             self._page_rows[slot] = (-2, 0)
 
-    def _fill(self, segs: list[Segment], pad_rows_to: int | None = None) -> StepBatch:
+    def _fill(self, segs: list[Segment], pad_rows_to: int | None = None, review: bool = False) -> StepBatch:
+        """``review``: the segments are drafts to be verified.  Their pass is captured once for a number of requests and replayed behind
+        any contexts, so nothing that its launches depend on may follow the contexts of this step: the general kernel takes them."""
         st = self.stage
         h = st.h
         qb = self.qb
@@ -304,7 +306,7 @@ class BatchBuilder:
         else:
             rows_cap = rows
         d = st.d
-        prompts = self._prompts(blocks)
+        prompts = (0, 0) if review else self._prompts(blocks)
         splits = self._splits(rb - (prompts[1] - prompts[0]), decode)
         return StepBatch(num_tokens=t, num_row_blocks=rb, num_logit_rows=rows_cap, token_ids=d["token_ids"],
                          positions=d["positions"], slots=d["slots"], page_table=d["page_table"], rb_req=d["rb_req"],

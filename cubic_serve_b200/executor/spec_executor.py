@@ -225,12 +225,12 @@ class SpeculativeGpuExecutor(GpuExecutor):
             c *= 2
         return c
 
-    def _staged(self, segs, pad_rows_to=None):
+    def _staged(self, segs, pad_rows_to=None, review=False):
         """``_fill`` + upload, after the previous upload has left the pinned staging buffer (with captured passes the
         host runs far ahead of the device)."""
         if self._upload_pending:
             self._uploaded.synchronize()
-        b, _ = self._fill(segs, pad_rows_to=pad_rows_to)
+        b, _ = self._fill(segs, pad_rows_to=pad_rows_to, review=review)
         return b
 
     def _upload(self) -> int:
@@ -325,7 +325,7 @@ class SpeculativeGpuExecutor(GpuExecutor):
             pad_slot = self.max_rows                       # a page-table row no request uses
             review = [Segment(s.request_slot, [s.token_ids[0]] + [0] * Kd, s.start, s.pages, True, uid=s.uid) for s in segs]
             review += [Segment(pad_slot, [0] * (Kd + 1), 0, [0], True, uid=-1) for _ in range(cap - R)]
-            b = self._staged(review)
+            b = self._staged(review, review=True)
             T, Tr = cap * (Kd + 1), R * (Kd + 1)
             h = self.stage.h
             nb = -(-(Kd + 1) // self.builder.qb)
@@ -405,7 +405,7 @@ class SpeculativeGpuExecutor(GpuExecutor):
         r, dev = self.runner, self.device
         R = len(segs)
         review = [Segment(s.request_slot, [s.token_ids[0]] + [0] * Kd, s.start, s.pages, True, uid=s.uid) for s in segs]
-        b, _ = self._fill(review)
+        b, _ = self._fill(review, review=True)
         T = R * (Kd + 1)
         self.stage.h["logit_rows"][:T] = np.arange(T)
         self.stage.h["temperature"][:T] = 0

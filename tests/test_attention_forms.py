@@ -11,7 +11,7 @@ from cubic_serve_b200.ops import kernels as K
 from cubic_serve_b200.ops.strategies import active
 
 
-def _fill(portions, hq=32, hkv=8, pad=None):
+def _fill(portions, hq=32, hkv=8, pad=None, review=False):
     """A step of ``(context, tokens)`` portions."""
     bb = BatchBuilder(max_rows=max(len(portions), pad or 0), max_tokens=9000, max_model_len=9000, group=hq // hkv, kv_heads=hkv, device="cpu")
     segs, page = [], 0
@@ -19,7 +19,7 @@ def _fill(portions, hq=32, hkv=8, pad=None):
         per = -(-(start + n) // 16)
         segs.append(Segment(r, [1] * n, start, list(range(page, page + per)), uid=r))
         page += per
-    b = bb.fill(segs, pad_rows_to=pad)[0]
+    b = bb.fill(segs, pad_rows_to=pad, review=review)[0]
     bb.stage.upload()
     return b
 
@@ -90,6 +90,13 @@ def test_prompts_take_the_kernel_that_was_measured_faster(hq, hkv, portions, pro
     (8, 8, [(1000, 4)] * 32 + [(0, 1024)] * 4, (0, 0)), (32, 8, [(1000, 4)] * 32 + [(0, 1024)] * 4, (32, 1056)), (8, 8, [(1000, 1)] * 64 + [(0, 1024)] * 7, (0, 0))])
 def test_prompts_beside_other_rows(hq, hkv, portions, prompts):
     assert _fill(portions, hq, hkv).attn_prompts == prompts
+
+
+@pytest.mark.parametrize("hq,hkv,depth,requests", [(64, 4, 3, 64), (32, 4, 7, 64), (16, 2, 7, 128), (32, 2, 3, 128), (32, 8, 3, 8)])
+def test_review_rows_are_launched_alike_behind_any_context(hq, hkv, depth, requests):
+    """A captured review pass serves later rounds, whose contexts are longer."""
+    steps = [_fill([(c, depth + 1)] * requests, hq, hkv, review=True) for c in (20, 100, 1000, 4000)]
+    assert all(b.attn_prompts == (0, 0) and not b.attn_decode and b.attn_splits == steps[0].attn_splits for b in steps)
 
 
 DECODE, PROMPT = (900, 1), (0, 1024)

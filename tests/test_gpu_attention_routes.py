@@ -86,3 +86,36 @@ def test_prompt_steps_of_a_speculative_executor():
     for got, want in zip(hidden[:2] + heads[:2], hidden[2:] + heads[2:]):
         # a flipped rounding of an activation or a cache code moves what follows by parts of a bf16 step, layer after layer
         assert ((got - want).norm() / want.norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_review_passes_take_the_general_kernel(graphs):
+    """16 query heads a key / value head: the rows of a review fill four row blocks a request, which portions of prompts of that length
+    would leave to the prompt kernel behind short contexts."""
+    from cubic_serve_b200.executor.gpu_executor import Segment
+    from cubic_serve_b200.executor.spec_executor import SpeculativeGpuExecutor
+    from cubic_serve_b200.models.decoder import random_decoder_weights
+    from cubic_serve_b200.models.mtp import MtpRunner, random_mtp_weights
+    from cubic_serve_b200.ops import kernels as K
+    dev = torch.device("cuda")
+    cfg = ModelConfig(name="review", num_layers=1, hidden_size=512, num_q_heads=64, num_kv_heads=4, head_dim=128, intermediate_size=512, vocab_size=512,
+                      rope_theta=1e6, quant=QuantSpec("cubic", 4, 128))
+    requests, pages = 64, 4
+    runner = DecoderRunner(cfg, random_decoder_weights(cfg, dev, seed=0), num_pages=requests * pages, max_tokens=1024)
+    ex = SpeculativeGpuExecutor(runner, MtpRunner(runner, random_mtp_weights(cfg, dev)), 3, max_rows=requests, max_prefill_tokens=1024, max_model_len=16 * pages,
+                                round_graphs=graphs)
+    table = [list(range(r * pages, (r + 1) * pages)) for r in range(requests)]
+    ex.execute([Segment(r, list(range(16)), 0, table[r], True, uid=r) for r in range(requests)])
+    made, attend = [], K.paged_attention
+
+    def attention(*a, form="", **k):
+        made.append(form)
+        return attend(*a, form=form, **k)
+    try:
+        K.paged_attention = attention
+        ex.execute_speculative([Segment(r, [5], 16, table[r], True, uid=r) for r in range(requests)])
+    finally:
+        K.paged_attention = attend
+    runner.ws.check_status()
+    assert made and set(made) == {""}
+    assert ex.stats["graphed_rounds"] == int(graphs)
