@@ -200,7 +200,8 @@ class BatchBuilder:
 
     def _fill(self, segs: list[Segment], pad_rows_to: int | None = None, review: bool = False) -> StepBatch:
         """``review``: the segments are drafts to be verified.  Their pass is captured once for a number of requests and replayed behind
-        any contexts, so nothing that its launches depend on may follow the contexts of this step: the general kernel takes them."""
+        any contexts, so nothing that its launches depend on may follow the contexts of this step: the general kernel takes them.
+        (64 requests of four rows, 64 over 4 heads: 29 us behind 100 tokens against 25 of the prompt kernel, but 268 against 390 behind 4000.)"""
         st = self.stage
         h = st.h
         qb = self.qb
