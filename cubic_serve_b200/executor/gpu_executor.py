@@ -534,7 +534,8 @@ class GpuExecutor:
         dst = torch.tensor([p[1] for p in pairs], dtype=torch.int32, device=self.device)
         with torch.cuda.stream(self.stream):
             for cache in self.runner.kv:
-                K.copy_pages(cache, src, dst)
+                if cache.shape[0]:                 # recurrent layers have no pages
+                    K.copy_pages(cache, src, dst)
         for t in (src, dst):
             t.record_stream(self.stream)       # read there after this call has returned
 
