@@ -9,7 +9,7 @@ list, so variable routing needs no host round trip and is CUDA-graph safe.
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 
 import torch
 
@@ -62,6 +62,7 @@ class MoeLayer:
     shared_down: wq_pack.PackedWeight | None = None       # [H, Is(/tp)]
     shared_gate: wq_pack.PackedWeight | None = None       # bf16 [8, H]: row 0 is the gate vector, the others zero
     least_rows: int = 0                                   # rows of a work item of a small step (set with the scratch)
+    replaced: list = field(default_factory=list)          # buffers of an earlier, smaller runner: its captured graphs may hold their addresses
 
     def fuse_activation(self) -> None:
         """Re-order every expert's ``[gate; up]`` rows so that the grouped GEMM applies SwiGLU in its epilogue."""
@@ -95,6 +96,8 @@ class MoeLayer:
 
     def ensure_scratch(self, max_tokens: int, hidden: int, device) -> K.MoeScratch:
         if self.scratch is None or self.scratch.topk_ids.shape[0] < max_tokens:
+            if self.scratch is not None:
+                self.replaced.append(self._buffers())
             from ..ops.strategies import active
             pol = active().moe
             big = max_tokens * self.top_k >= pol.large_routes_per_expert * self.expert_count
@@ -118,11 +121,17 @@ class MoeLayer:
         for o in others:
             mine, its = self._buffer_shapes(), o._buffer_shapes()
             if mine == its and o.scratch is not None and o.scratch.topk_ids.shape[0] >= max_tokens:
+                if self.scratch is not None and self.scratch is not o.scratch:
+                    self.replaced.append(self._buffers())
                 self.scratch, self.least_rows, self.logits, self.out = o.scratch, o.least_rows, o.logits, o.out
                 if self.shared_gate_up is not None:
                     self.sh_gu, self.sh_act, self.sh_out, self.sh_logit, self.sh_sig = o.sh_gu, o.sh_act, o.sh_out, o.sh_logit, o.sh_sig
                 return
         self.ensure_scratch(max_tokens, hidden, device)
+
+    def _buffers(self) -> tuple:
+        shared = () if self.shared_gate_up is None else (self.sh_gu, self.sh_act, self.sh_out, self.sh_logit, self.sh_sig)
+        return self.scratch, self.logits, self.out, *shared
 
     def _buffer_shapes(self) -> tuple:
         shared = None if self.shared_gate_up is None else (self.shared_gate_up.n, self.shared_gate.n)

@@ -1,4 +1,5 @@
 """Routing and activation buffers of expert layers: one set a runner, made with it."""
+import weakref
 from types import SimpleNamespace
 
 import pytest
@@ -27,6 +28,22 @@ def test_layers_of_the_same_shapes_share_buffers():
     more = _layer()
     more.share_scratch(layers, 17, 64, "cpu")
     assert more.scratch is not layers[0].scratch and more.scratch.topk_ids.shape[0] == 17
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_buffers_of_a_smaller_runner_stay(shared):
+    """A larger runner over the same weights: the graphs of the first one still write where they were captured."""
+    layers = [_layer(shared=shared) for _ in range(3)]
+    for i, l in enumerate(layers):
+        l.share_scratch(layers[:i], 16, 64, "cpu")
+    first = [weakref.ref(t) for t in (layers[0].scratch, layers[0].logits, layers[0].out, *((layers[0].sh_act, layers[0].sh_sig) if shared else ()))]
+    for i, l in enumerate(layers):
+        l.share_scratch(layers[:i], 32, 64, "cpu")
+    assert all(l.scratch is layers[0].scratch and l.scratch.topk_ids.shape[0] == 32 for l in layers)
+    assert all(r() is not None for r in first)
+    for i, l in enumerate(layers):                      # the same runner again, or a smaller one: nothing new
+        l.share_scratch(layers[:i], 16, 64, "cpu")
+    assert [len(l.replaced) for l in layers] == [1, 1, 1]
 
 
 @pytest.mark.gpu
