@@ -12,6 +12,8 @@ chunks (variable token counts) launch the same kernels eagerly.
 """
 from __future__ import annotations
 
+import contextlib
+import gc
 import logging
 from dataclasses import dataclass, field, replace
 
@@ -99,6 +101,20 @@ class _Staging:
         n = self.nbytes if nbytes is None else nbytes
         self.dev[:n].copy_(self.host[:n], non_blocking=True)
         return n
+
+
+@contextlib.contextmanager
+def capturing(graph: "torch.cuda.CUDAGraph", stream: "torch.cuda.Stream"):
+    """``torch.cuda.graph`` without a garbage collection inside: one that finds the graphs of an executor that is gone destroys
+    them, and that ends a capture under way."""
+    collects = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            yield
+    finally:
+        if collects:
+            gc.enable()
 
 
 class BatchBuilder:
@@ -449,7 +465,7 @@ class GpuExecutor:
                     self._body(b)
                 self.stream.synchronize()
                 g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g, stream=self.stream):
+                with capturing(g, self.stream):
                     self._body(b)
                 rt.add(cap, g, self.runner.launches_per_step)
                 rt.qualify(cap, lambda slot: self._replay_equals_eager(slot, b, cap))

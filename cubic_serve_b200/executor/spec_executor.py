@@ -22,7 +22,7 @@ import torch
 
 from ..models.mtp import MtpRunner
 from ..ops import kernels as K
-from .gpu_executor import GpuExecutor, Segment
+from .gpu_executor import GpuExecutor, Segment, capturing
 
 
 class SpeculativeGpuExecutor(GpuExecutor):
@@ -272,7 +272,7 @@ class SpeculativeGpuExecutor(GpuExecutor):
                 restore()
             self.stream.synchronize()
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, stream=self.stream):
+            with capturing(g, self.stream):
                 body()
             restore()
             self._round_graph[key] = g

@@ -119,3 +119,4 @@ def test_review_passes_take_the_general_kernel(graphs):
     runner.ws.check_status()
     assert made and set(made) == {""}
     assert ex.stats["graphed_rounds"] == int(graphs)
+    ex._round_graph.clear()
