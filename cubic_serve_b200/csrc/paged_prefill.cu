@@ -1,53 +1,70 @@
 // Paged GQA attention over the quantized KV cache for portions of prompts, on the tensor cores of tcgen05 (page layout: kv_layout.cuh;
-// row blocks and arithmetic: paged_attn.cu).
+// row blocks: paged_attn.cu).
 //
-// What bounds it.  The general kernel gives a row block (16 MMA rows: 16 / G positions x G heads) a CTA of its own: a prompt's pages
-// are fetched and converted to f16 once per 16 / G positions, and mma.sync re-reads every operand for 16 rows.  Here a CTA takes
-// eight consecutive row blocks -- the 128 rows of one tcgen05 MMA -- and converts a step of 64 tokens once for all of them.
-// Codes stay exact in f16; the scales, one per token and 32 channels, multiply fp32 scores (K) and probabilities before their
-// rounding to f16 (V), as in the general kernel.  So a step makes four score tiles in tensor memory, one per channel group, and four
-// scaled copies of the probabilities; what is left to pay is that arithmetic: 256 fp32 multiply-adds, 256 multiplications, 128
-// packings and 64 exponentials a row and step.
-// One softmax warp a scheduler pays it, and waits for its own tensor-memory loads besides: about 5800 cycles a step.  General kernel -> this one
-// (with 8 us of launch and cold operands), 32 heads over 8: 8 x 1024 tokens 707 -> 513 us, 4 x 256 behind 2048 284 -> 234; 6 bit, 64 over 4,
-// 3 x 500 195 -> 136; one prompt of 331 tokens 29 -> 33, which the caller leaves to the general kernel.  What keeps values that are not finite
-// to those who see them, and scaled probabilities in the range of f16, costs 0.5 % of it.
+// What bounds it: shared memory, then the MMAs.  An item is sixteen consecutive row blocks -- 256 rows, two tiles of one tcgen05 MMA each --
+// of a key / value head; a CTA takes items one after the other and converts a step of 64 tokens once for both tiles.
+// A cached value is a code of at most 8 bits times an fp32 scale, one per token and 32 channels.  The conversion writes it as a sum of two f16
+// (hi + lo, 22 bits and more), so that a step's scores and its output are one chain of MMAs each.  Scales inside the softmax would take
+// four score tiles and four copies of the probabilities, one per channel group (what this kernel did before: 256 multiply-adds, 256 multiplications
+// and 128 packings a row and step instead of 64, 0 and 32; 5800 cycles a step of 128 rows).
+// Powers of two keep hi and lo in the range of f16: one a step for K, undone in the softmax' multiply-add; one for V that grows with
+// the largest scale seen, undone with the output.
+// MMAs of a step take 640 + 512 cycles a tile (measured in a loop of their own); with their operands, raw pages and the conversion's stores shared memory
+// moves about 280 KB a step: 4000 cycles a step of 256 rows where 2 x 5800 were spent.  General kernel -> before -> now, one B200, cold L2, 32 heads
+// over 8, 8 bits: 8 x 1024 tokens 702 -> 520 -> 220 us, 4 x 256 behind 2048 276 -> 233 -> 104, one prompt of 8192 3734 -> 2775 -> 1275, 40 x 20 behind 300
+// 63 -> 103 -> 57; 32 over 4, 4 / 8 bits, 2 x 2048 571 -> 421 -> 193; 64 over 4, 6 bits, 3 x 500 190 -> 131 -> 80.
 //
-// Roles: warps 0-3 own a row a thread (softmax needs no exchange: tensor-memory lane = row); warps 4-7 convert raw pages, which warp 4
-// copies two steps ahead, to the swizzled operands (K as [token][channel], V transposed as [channel][token]); warp 8 issues the MMAs.
-// The scores of step i + 1 are computed while the softmax of step i runs.  Row blocks of several requests may meet in a CTA: it walks
+// Roles: warps 0-7 own a row a thread (softmax needs no exchange: tensor-memory lane = row); warps 8-11 convert raw pages of K to the swizzled operand
+// (hi and lo, [token][channel]), warps 12-15 those of V; warps 16 and 18 issue the MMAs; warp 17 lists the items' requests and copies their
+// pages three steps ahead.  Tensor memory of a tile: scores, probabilities (the A operand of their product), output and the first half of Q's
+// channels; the other half of Q is in shared memory, where an MMA of 64 columns takes 48 cycles instead of 32.
+// The scores of step i + 1 are computed while the softmax of step i runs.  Row blocks of several requests may meet in an item: it walks
 // their steps one request after the other, rows of another request taking part with probability zero.  The output accumulator stays
 // in tensor memory and is rescaled only when a row's maximum has grown by more than a factor of four (2 in the log2 domain): until
-// then probabilities relative to the older maximum are at most 4.  A step with a V scale of which four times is more than f16 holds
-// rescales at any growth, so that scaled probabilities have the range that they have in the general kernel.
-// Every wait is bounded; on a timeout the roles run through without waiting, the status word is set and tensor memory is freed.
+// then probabilities relative to the older maximum are at most 4.
+// Every wait is bounded; on a timeout the roles leave, the status word is set and tensor memory is freed.
 #include "paged_attn.cuh"
 
 namespace cb {
 
-static constexpr int kPfRows = 128;
-static constexpr int kPfBlocks = kPfRows / 16;
+static constexpr int kPfTiles = 2;
+static constexpr int kPfRows = 128;                      // of a tile
+static constexpr int kPfBlocks = kPfTiles * kPfRows / 16;
 static constexpr int kPfPages = 4;                       // pages of a step
 static constexpr int kPfTok = kPfPages * kPageTokens;    // 64
-static constexpr int kPfThreads = 288;
+static constexpr int kPfThreads = 640;
+// registers a thread: at launch, and of the softmax', the conversion's and the other warps after they have shared them out anew
+static constexpr int kPfRegs = 96, kPfRegsSoftmax = 136, kPfRegsConvert = 72, kPfRegsOther = 64;
+static_assert(2 * kPfRegsSoftmax + 2 * kPfRegsConvert + kPfRegsOther <= 5 * kPfRegs, "five warpgroups");
+static constexpr int kPfLists = 4;
+static constexpr int kPfRaw = 3;                         // steps of raw pages
+static constexpr int kPfNotes = 4;                       // steps whose powers of two are kept
+static constexpr int kPfSorted = 512;                    // groups of row blocks that are dealt by their length
 static constexpr float kPfGrowth = 2.f;
-static constexpr float kPfGrowthScale = 65504.f / 4.f;   // largest V scale of a step with probabilities up to 4
-static constexpr uint32_t kPfWild = 1, kPfLarge = 2;     // a V scale of the step is not finite, is finite and above that
-static constexpr uint32_t kPfTmemCols = 512, kPfTmemO = 256;      // four score tiles of 64 columns, then 128 columns of output
+// tensor memory, columns of a tile: scores, probabilities (two f16 a column), channels 0..63 of Q (likewise), output
+static constexpr uint32_t kPfTmemCols = 512, kPfTmemTile = 256, kPfTmemP = 64, kPfTmemQ = 96, kPfTmemO = 128;
+static constexpr int kPfHalf = kPfTok * 128;             // bytes of 64 channels of a step
 
 struct PfRun {
-  int first, end, req, total, pages, steps;              // row blocks [first, end) of the CTA, tokens that the last of them sees
+  int first, end, req, total, pages, steps;              // row blocks [first, end) of the item, tokens that they see, ...
+  int tile_steps[kPfTiles];                              // ... steps that the rows of each tile see something of
+};
+struct PfList {
+  int kvh, runs, steps, tiles;                           // kvh < 0: no more items; tiles: bit mask of those with steps
+  int qstart[kPfBlocks], qcount[kPfBlocks], ctx[kPfBlocks];
+  PfRun run[kPfBlocks];
 };
 struct __align__(1024) PfSmem {
-  uint8_t q[2 * kPfRows * 128];                          // f16 [64-channel half][row][128 B], 16-byte chunk ^ (row & 7)
-  uint8_t p[4][kPfRows * 128];                           // f16 [channel group][row][64 tokens]
-  uint8_t k[2][2 * kPfTok * 128];                        // f16 [stage][64-channel half][token]
-  uint8_t v[2][kD * 128];                                // f16 [stage][channel][64 tokens]
-  float ks[2][4 * kPfTok], vs[2][4 * kPfTok];            // [stage][channel group][token]
-  uint32_t vs_kind[2][2];                                // [stage][half of the tokens] kPfWild, kPfLarge
-  uint64_t raw_full[2], kv_full[2], kv_free[2], s_full, s_free, p_full, pv_done;
-  PfRun run[kPfBlocks];
-  int runs, steps;
+  uint8_t q[kPfTiles][kPfRows * 128];                    // f16, channels 64..127: [row][128 B], 16-byte chunk ^ (row & 7)
+  uint8_t k[2][2][2 * kPfHalf];                          // f16 [stage][hi, lo][64-channel half][token][128 B]
+  uint8_t v[2][2][2 * kPfHalf];                          // likewise
+  float vw[kPfNotes][4 * kPfTok];                        // of a step, [channel group][token]: V scales that are not finite, else 0
+  float k_mul[kPfNotes];                                 // scores are this times what the MMAs give
+  int v_exp[kPfNotes], wild[kPfNotes];                   // output is 2^v_exp times ...; vw is written
+  uint64_t raw_full[kPfRaw], raw_free[kPfRaw], k_full[2], k_free[2], v_full[2], v_free[2], k_note[kPfNotes], v_note[kPfNotes];
+  uint64_t list_full[kPfLists], list_free[kPfLists], q_full[kPfTiles], s_full[kPfTiles], s_free[kPfTiles], p_full[kPfTiles], pv_done[kPfTiles];
+  PfList list[kPfLists];
+  uint16_t order[kPfSorted];                             // groups of row blocks, those that see most first
   uint32_t tmem, abort_word;
 };
 
@@ -63,11 +80,33 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Where a role stands in the CTA's list of steps: runs one after the other.
+__device__ __forceinline__ void tmem_ld_32x1(uint32_t taddr, uint32_t& r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x1(uint32_t taddr, uint32_t r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(r) : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem desc]
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Shared-memory descriptor of an operand whose rows of 128 bytes run along N (or M), 128-byte swizzle: 8 rows of K are 1024 bytes, blocks of 64 columns
+// `block` bytes apart.
+__device__ __forceinline__ uint64_t umma_desc_sw128_n(uint32_t smem_addr, uint32_t block) {
+  return (umma_desc_sw128(smem_addr) & ~(static_cast<uint64_t>(0x3FFF) << 16)) | static_cast<uint64_t>(block >> 4) << 16;
+}
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((min(max(e, -126), 127) + 127) << 23); }
+
+// Where a role stands in an item's list of steps: runs one after the other.
 struct PfWalk {
   int run = 0, step = 0;
-  __device__ __forceinline__ void advance(const PfSmem& sm) {
-    if (++step == sm.run[run].steps) { step = 0; ++run; }
+  __device__ __forceinline__ void advance(const PfList& l) {
+    if (++step == l.run[run].steps) { step = 0; ++run; }
   }
 };
 
@@ -75,35 +114,89 @@ __device__ __forceinline__ uint4 conv8(uint2 w, uint32_t bias) {        // eight
   return make_uint4(u8x2_to_f16x2(w.x, 0x5140u, bias), u8x2_to_f16x2(w.x, 0x5342u, bias), u8x2_to_f16x2(w.y, 0x5140u, bias), u8x2_to_f16x2(w.y, 0x5342u, bias));
 }
 
-// One step's codes and scales into operands.  What a step's tail has beyond `pages` becomes zeros, and so do V scales from `visible`
-// on: those slots may hold anything, and a probability of zero has to stay zero.
-template <int KBITS, int VBITS>
-__device__ __forceinline__ void pf_convert(PfSmem& sm, int b, const uint8_t* raw, int stride, const KvLayout& lay, int pages, int visible, int tid) {
-  constexpr uint32_t kb = KBITS == 8 ? 0x64806480u : KBITS == 6 ? 0x64206420u : 0x64086408u;
-  constexpr uint32_t vb = VBITS == 8 ? 0x64806480u : VBITS == 6 ? 0x64206420u : 0x64086408u;
-  // K: an item is 16 channels (8 bit) or 32 (4 and 6 bit) of a token
-  constexpr int kItems = KBITS == 8 ? kPageTokens * 8 : kPageTokens * 4;
-#pragma unroll 4
-  for (int i = tid; i < kPfPages * kItems; i += 128) {
-    const int page = i / kItems, r = i % kItems, tok = r & 15, blk = r >> 4, sw = tok & 7;
-    uint4* row = reinterpret_cast<uint4*>(sm.k[b] + (KBITS == 8 ? blk >> 2 : blk >> 1) * (kPfTok * 128) + (page * 16 + tok) * 128);
-    const int c = KBITS == 8 ? (blk & 3) * 2 : (blk & 1) * 4;
-    if (page >= pages) {
+// Two codes times their scales sh + sl: the rounded product with sh, and what it left over with the product with sl.  The residual is exact (a code
+// has 8 bits, sh 11), so hi + lo is off by the rounding of sl and of lo: 2^-22 of the value.
+__device__ __forceinline__ void pf_scaled(uint32_t code, uint32_t sh, uint32_t sl, uint32_t& hi, uint32_t& lo) {
+  uint32_t n, r;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(code), "r"(sh));
+  asm("neg.f16x2 %0, %1;" : "=r"(n) : "r"(hi));
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(code), "r"(sh), "r"(n));
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(lo) : "r"(code), "r"(sl), "r"(r));
+}
+__device__ __forceinline__ void pf_scaled8(const uint4& c, uint32_t sh, uint32_t sl, uint4& hi, uint4& lo) {
+  pf_scaled(c.x, sh, sl, hi.x, lo.x);
+  pf_scaled(c.y, sh, sl, hi.y, lo.y);
+  pf_scaled(c.z, sh, sl, hi.z, lo.z);
+  pf_scaled(c.w, sh, sl, hi.w, lo.w);
+}
+// an fp32 scale as a pair of f16, each twice
+__device__ __forceinline__ void pf_split(float s, uint32_t& sh, uint32_t& sl) {
+  sh = pack_f16x2(s, s);
+  const float r = s - __low2float(*reinterpret_cast<const __half2*>(&sh));
+  sl = pack_f16x2(r, r);
+}
+
+// The largest finite scale of a step's visible tokens, as its exponent (at least -100); every warp finds it for itself.  `of`: the thread's scales, of
+// tokens `lane` and `lane` + 32; `odd`: some scale is not finite.
+__device__ __forceinline__ int pf_exponent(const uint8_t* scales, int stride, int visible, int lane, float4 (&of)[2], bool& odd) {
+  uint32_t most = 0;
+  odd = false;
 #pragma unroll
-      for (int j = 0; j < (KBITS == 8 ? 2 : 4); ++j) row[(c + j) ^ sw] = make_uint4(0u, 0u, 0u, 0u);
-      continue;
+  for (int h = 0; h < 2; ++h) {
+    const int tok = lane + 32 * h;
+    of[h] = *reinterpret_cast<const float4*>(scales + (tok >> 4) * stride + (tok & 15) * 16);
+    if (tok >= visible) of[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float f[4] = {of[h].x, of[h].y, of[h].z, of[h].w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t x = __float_as_uint(f[j]) & 0x7FFFFFFFu;
+      if (x < 0x7F800000u) most = max(most, x);
+      else odd = true;
     }
-    const uint8_t* src = raw + page * stride;
-    const uint4 w = *reinterpret_cast<const uint4*>(src + blk * 256 + tok * 16);
+  }
+  odd = __any_sync(0xffffffffu, odd);
+  return max(static_cast<int>(__reduce_max_sync(0xffffffffu, most) >> 23) - 127, -100);
+}
+
+// One step's codes into operands: all of a thread's loads, then its arithmetic (few warps hide nothing).
+// What K holds of tokens that no row sees is masked with their scores.
+template <int KBITS>
+__device__ __forceinline__ void pf_convert_k(uint8_t (&k)[2][2 * kPfHalf], const uint8_t* raw, int stride, const KvLayout& lay, float mul, int tid) {
+  constexpr uint32_t kb = KBITS == 8 ? 0x64806480u : KBITS == 6 ? 0x64206420u : 0x64086408u;
+  // an item is 16 channels (8 bit) or 32 (4 and 6 bit) of a token
+  constexpr int kItems = KBITS == 8 ? kPageTokens * 8 : kPageTokens * 4, kMine = kPfPages * kItems / 128;
+  uint4 x[kMine], xh[kMine];
+  float s[kMine];
+#pragma unroll
+  for (int j = 0; j < kMine; ++j) {
+    const int i = tid + j * 128, r = i % kItems, tok = r & 15, blk = r >> 4;
+    const uint8_t* src = raw + i / kItems * stride;
+    x[j] = *reinterpret_cast<const uint4*>(src + blk * 256 + tok * 16);
+    if constexpr (KBITS == 6) xh[j] = *reinterpret_cast<const uint4*>(src + kPageTokens * kD / 2 + blk * 128 + (tok & 7) * 16);
+    s[j] = *reinterpret_cast<const float*>(src + lay.k_scale_off + tok * 16 + (KBITS == 8 ? blk >> 1 : blk) * 4);
+  }
+#pragma unroll
+  for (int j = 0; j < kMine; ++j) {
+    const int i = tid + j * 128, r = i % kItems, tok = r & 15, blk = r >> 4, sw = tok & 7;
+    const int at = (KBITS == 8 ? blk >> 2 : blk >> 1) * kPfHalf + (i / kItems * 16 + tok) * 128;
+    uint4* row_hi = reinterpret_cast<uint4*>(k[0] + at);
+    uint4* row_lo = reinterpret_cast<uint4*>(k[1] + at);
+    const int c = KBITS == 8 ? (blk & 3) * 2 : (blk & 1) * 4;
+    uint32_t sh, sl;
+    pf_split(s[j] * mul, sh, sl);
+    auto put = [&](int chunk, uint2 codes) {
+      uint4 hi, lo;
+      pf_scaled8(conv8(codes, kb), sh, sl, hi, lo);
+      row_hi[chunk ^ sw] = hi;
+      row_lo[chunk ^ sw] = lo;
+    };
     if constexpr (KBITS == 8) {
-      row[c ^ sw] = conv8(make_uint2(w.x, w.y), kb);
-      row[(c + 1) ^ sw] = conv8(make_uint2(w.z, w.w), kb);
+      put(c, make_uint2(x[j].x, x[j].y));
+      put(c + 1, make_uint2(x[j].z, x[j].w));
     } else {
-      const uint32_t n[4] = {w.x, w.y, w.z, w.w};
+      const uint32_t n[4] = {x[j].x, x[j].y, x[j].z, x[j].w};
       uint32_t lo[4], hi[4];
-      uint4 hb = make_uint4(0u, 0u, 0u, 0u);
-      if constexpr (KBITS == 6) hb = *reinterpret_cast<const uint4*>(src + kPageTokens * kD / 2 + blk * 128 + (tok & 7) * 16);
-      const uint32_t hw[4] = {hb.x, hb.y, hb.z, hb.w};
+      const uint32_t hw[4] = {xh[j].x, xh[j].y, xh[j].z, xh[j].w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         lo[q] = n[q] & 0x0F0F0F0Fu;
@@ -113,80 +206,91 @@ __device__ __forceinline__ void pf_convert(PfSmem& sm, int b, const uint8_t* raw
           hi[q] |= (tok < 8 ? hw[q] >> 2 : hw[q] << 2) & 0x30303030u;
         }
       }
-      row[c ^ sw] = conv8(make_uint2(lo[0], lo[1]), kb);
-      row[(c + 1) ^ sw] = conv8(make_uint2(lo[2], lo[3]), kb);
-      row[(c + 2) ^ sw] = conv8(make_uint2(hi[0], hi[1]), kb);
-      row[(c + 3) ^ sw] = conv8(make_uint2(hi[2], hi[3]), kb);
-    }
-  }
-  // V: lane = token pair of the step; a warp's lanes take four neighbouring chunks (4 channels) in turns, shifted so that neither the
-  // loads nor the stores, one 32-bit pair per channel row, meet in a bank
-  const int lane = tid & 31, page = lane >> 3, pair = lane & 7, j8 = lane >> 2;
-  const uint8_t* src = raw + page * stride + lay.v_code_off;
-#pragma unroll 2
-  for (int c0 = (tid >> 5) * 8; c0 < (tid >> 5) * 8 + 8; c0 += 4)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = c0 + ((j8 + i) & 3), at = c ^ ((pair & 3) << 2);
-      uint4 w = make_uint4(0u, 0u, 0u, 0u);
-      if (page < pages) {
-        if constexpr (VBITS == 8) {
-          w = conv8(*reinterpret_cast<const uint2*>(src + pair * 256 + at * 8), vb);
-        } else {
-          const uint32_t n = *reinterpret_cast<const uint32_t*>(src + pair * 128 + at * 4);
-          uint32_t e = n & 0x0F0F0F0Fu, o = (n >> 4) & 0x0F0F0F0Fu;
-          if constexpr (VBITS == 6) {
-            const uint32_t hw = *reinterpret_cast<const uint32_t*>(src + kPageTokens * kD / 2 + (pair & 3) * 128 + at * 4);
-            e |= (pair < 4 ? hw : hw << 4) & 0x30303030u;
-            o |= (pair < 4 ? hw >> 2 : hw << 2) & 0x30303030u;
-          }
-          w = conv8(make_uint2(prmt(e, o, 0x5140u), prmt(e, o, 0x7362u)), vb);
-        }
-      }
-      uint8_t* dst = sm.v[b] + 4 * c * 128 + (lane & 3) * 4;
-      const int sw = (4 * c) & 7;
-      *reinterpret_cast<uint32_t*>(dst + ((j8 ^ sw) << 4)) = w.x;
-      *reinterpret_cast<uint32_t*>(dst + 128 + ((j8 ^ (sw + 1)) << 4)) = w.y;
-      *reinterpret_cast<uint32_t*>(dst + 256 + ((j8 ^ (sw + 2)) << 4)) = w.z;
-      *reinterpret_cast<uint32_t*>(dst + 384 + ((j8 ^ (sw + 3)) << 4)) = w.w;
-    }
-  {
-    const int tok = tid & 63, pg = tok >> 4;
-    const bool is_v = tid >= 64;
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (pg < pages && (!is_v || tok < visible))
-      s = *reinterpret_cast<const float4*>(raw + pg * stride + (is_v ? lay.v_scale_off : lay.k_scale_off) + (tok & 15) * 16);
-    float* dst = (is_v ? sm.vs[b] : sm.ks[b]) + tok;
-    dst[0] = s.x; dst[kPfTok] = s.y; dst[2 * kPfTok] = s.z; dst[3 * kPfTok] = s.w;
-    if (is_v) {                                          // both warps of V
-      auto of = [](float x) { return fabsf(x) <= kPfGrowthScale ? 0u : fabsf(x) < INFINITY ? kPfLarge : kPfWild; };
-      const uint32_t kind = __reduce_or_sync(0xffffffffu, of(s.x) | of(s.y) | of(s.z) | of(s.w));
-      if ((tid & 31) == 0) sm.vs_kind[b][(tid >> 5) & 1] = kind;
+      put(c, make_uint2(lo[0], lo[1]));
+      put(c + 1, make_uint2(lo[2], lo[3]));
+      put(c + 2, make_uint2(hi[0], hi[1]));
+      put(c + 3, make_uint2(hi[2], hi[3]));
     }
   }
 }
-
-// A step with a V scale that is not finite: zero times it, and it may be another request's, is not zero.  The warp of the MMAs clears the
-// tokens that a row does not see before it multiplies (in the softmax warps, which have no register left for it, the check alone was 1 % of the kernel).
-// `rb_qcount`, `rb_ctx`: of the CTA's first row block; `blocks`: from there to the last; `i`: the step.
-__device__ __noinline__ void pf_unseen(PfSmem& sm, const int* rb_qcount, const int* rb_ctx, int blocks, int G, int i, int lane) {
-  int run = 0;
-  while (i >= sm.run[run].steps) i -= sm.run[run++].steps;
-  for (int row = lane; row < kPfRows; row += 32) {
-    const int blk = row >> 4, qp = (row & 15) / G;
-    int sees = 0;
-    if (blk >= sm.run[run].first && blk < sm.run[run].end && blk < blocks && qp < rb_qcount[blk]) sees = rb_ctx[blk] + qp - i * kPfTok;
-    for (int c = max(sees, 0) >> 3; c < 8; ++c) {
-      const int keep = min(max(sees - 8 * c, 0), 8);                 // tokens of the chunk
-      for (int cg = 0; cg < 4; ++cg) {
-        uint32_t* at = reinterpret_cast<uint32_t*>(sm.p[cg] + row * 128 + ((c ^ (row & 7)) << 4));
+// V from `visible` on becomes zeros: those slots may hold anything, and a probability of zero has to stay zero.  A scale that is not finite is
+// left out (code times one): pf_wild adds its product for the rows that see it.
+template <int VBITS>
+__device__ __forceinline__ void pf_convert_v(uint8_t (&v)[2][2 * kPfHalf], const uint8_t* raw, int stride, const KvLayout& lay, int visible, float mul, int tid) {
+  constexpr uint32_t vb = VBITS == 8 ? 0x64806480u : VBITS == 6 ? 0x64206420u : 0x64086408u;
+  // an item is 8 channels of a token pair of a page
+  const int c = tid & 15, pair = tid >> 4, at = (2 * c) ^ ((pair & 3) << 2);
+  uint4 x[kPfPages];                                     // 8 bit: the codes; else low nibbles, high bits
+  float s[kPfPages][2];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) at[k] &= keep >= 2 * k + 2 ? 0xFFFFFFFFu : keep == 2 * k + 1 ? 0xFFFFu : 0u;
+  for (int j = 0; j < kPfPages; ++j) {
+    const uint8_t* page = raw + j * stride;
+    const uint8_t* src = page + lay.v_code_off;
+    if constexpr (VBITS == 8) {
+      x[j] = *reinterpret_cast<const uint4*>(src + pair * 256 + at * 8);
+    } else {
+      const uint2 n = *reinterpret_cast<const uint2*>(src + pair * 128 + at * 4);
+      uint2 hw = make_uint2(0u, 0u);
+      if constexpr (VBITS == 6) hw = *reinterpret_cast<const uint2*>(src + kPageTokens * kD / 2 + (pair & 3) * 128 + at * 4);
+      x[j] = make_uint4(n.x, n.y, hw.x, hw.y);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) s[j][h] = *reinterpret_cast<const float*>(page + lay.v_scale_off + (2 * pair + h) * 16 + (c >> 2) * 4);
+  }
+#pragma unroll
+  for (int j = 0; j < kPfPages; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int tok = (j * 8 + pair) * 2 + h;
+      uint4 codes;
+      if constexpr (VBITS == 8) {
+        const uint32_t sel = h ? 0x5341u : 0x5240u;
+        codes = make_uint4(u8x2_to_f16x2(x[j].x, sel, vb), u8x2_to_f16x2(x[j].y, sel, vb), u8x2_to_f16x2(x[j].z, sel, vb), u8x2_to_f16x2(x[j].w, sel, vb));
+      } else {
+        uint2 n = h ? make_uint2((x[j].x >> 4) & 0x0F0F0F0Fu, (x[j].y >> 4) & 0x0F0F0F0Fu) : make_uint2(x[j].x & 0x0F0F0F0Fu, x[j].y & 0x0F0F0F0Fu);
+        if constexpr (VBITS == 6) {
+          auto high = [&](uint32_t w) { return (pair < 4 ? (h ? w >> 2 : w) : (h ? w << 2 : w << 4)) & 0x30303030u; };
+          n.x |= high(x[j].z);
+          n.y |= high(x[j].w);
+        }
+        codes = conv8(n, vb);
+      }
+      const float f = tok >= visible ? 0.f : fabsf(s[j][h]) < INFINITY ? s[j][h] * mul : 1.f;
+      uint32_t sh, sl;
+      uint4 hi, lo;
+      pf_split(f, sh, sl);
+      pf_scaled8(codes, sh, sl, hi, lo);
+      const int to = (c >> 3) * kPfHalf + tok * 128 + (((c & 7) ^ (tok & 7)) << 4);
+      *reinterpret_cast<uint4*>(v[0] + to) = hi;
+      *reinterpret_cast<uint4*>(v[1] + to) = lo;
+    }
+}
+
+// A step with a V scale that is not finite: zero times it, and it may be another request's, is not zero.  The operand has the codes of such
+// tokens alone; the rows that see them get the products here, before the step's own.  `tile`: the warp's lanes of its tile; `v`: the step's hi.
+__device__ __forceinline__ void pf_wild(const float* vw, const uint8_t* v, uint32_t tile, int sees) {
+#pragma unroll 1
+  for (int cg = 0; cg < 4; ++cg)
+#pragma unroll 1
+    for (int tok = 0; tok < kPfTok; ++tok) {
+      const float s = vw[cg * kPfTok + tok];
+      if (s == 0.f) continue;
+      uint32_t pw;
+      tmem_ld_32x1(tile + kPfTmemP + (tok >> 1), pw);
+      tmem_ld_wait();
+      const float2 p2 = __half22float2(*reinterpret_cast<const __half2*>(&pw));
+      const float p = tok & 1 ? p2.y : p2.x;
+#pragma unroll 1
+      for (int ch = cg * 32; ch < cg * 32 + 32; ++ch) {
+        const __half code = *reinterpret_cast<const __half*>(v + (ch >> 6) * kPfHalf + tok * 128 + ((((ch & 63) >> 3) ^ (tok & 7)) << 4) + (ch & 7) * 2);
+        uint32_t o;
+        tmem_ld_32x1(tile + kPfTmemO + ch, o);
+        tmem_ld_wait();
+        if (tok < sees) o = __float_as_uint(__uint_as_float(o) + p * (__half2float(code) * s));
+        tmem_st_32x1(tile + kPfTmemO + ch, o);
+        tmem_st_wait();
       }
     }
-  }
-  fence_proxy_async_smem();
-  __syncwarp();
 }
 
 template <int KBITS, int VBITS>
@@ -196,315 +300,516 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
   PfSmem& sm = *reinterpret_cast<PfSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* raw = reinterpret_cast<uint8_t*>(&sm + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kvh = blockIdx.x;
-  const int rb0 = static_cast<int>(gridDim.y - 1 - blockIdx.y) * kPfBlocks;     // the blocks that see most first
   const int stride = (p.lay.blob_bytes + 127) & ~127;
+  const int groups = (row_blocks + kPfBlocks - 1) / kPfBlocks, ctas = gridDim.x;
+  const long long items = static_cast<long long>(groups) * p.Hkv;
+  const bool sorted = items > ctas && groups <= kPfSorted;
   volatile uint32_t* abort_flag = &sm.abort_word;
   if (tid == 0) {
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kPfRaw; ++b) {
       mbar_init(smem_u32(&sm.raw_full[b]), 1);
-      mbar_init(smem_u32(&sm.kv_full[b]), 4);
-      mbar_init(smem_u32(&sm.kv_free[b]), 1);
+      mbar_init(smem_u32(&sm.raw_free[b]), 8);
     }
-    mbar_init(smem_u32(&sm.s_full), 1);
-    mbar_init(smem_u32(&sm.s_free), 4);
-    mbar_init(smem_u32(&sm.p_full), 4);
-    mbar_init(smem_u32(&sm.pv_done), 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&sm.k_full[b]), 4);
+      mbar_init(smem_u32(&sm.k_free[b]), 1);
+      mbar_init(smem_u32(&sm.v_full[b]), 4);
+      mbar_init(smem_u32(&sm.v_free[b]), 1);
+    }
+    for (int b = 0; b < kPfNotes; ++b) {
+      mbar_init(smem_u32(&sm.k_note[b]), 1);
+      mbar_init(smem_u32(&sm.v_note[b]), 1);
+    }
+    for (int b = 0; b < kPfLists; ++b) {
+      mbar_init(smem_u32(&sm.list_full[b]), 1);
+      mbar_init(smem_u32(&sm.list_free[b]), 18);         // all warps but 17 and 19
+    }
+    for (int t = 0; t < kPfTiles; ++t) {
+      mbar_init(smem_u32(&sm.q_full[t]), 4);
+      mbar_init(smem_u32(&sm.s_full[t]), 1);
+      mbar_init(smem_u32(&sm.s_free[t]), 4);
+      mbar_init(smem_u32(&sm.p_full[t]), 4);
+      mbar_init(smem_u32(&sm.pv_done[t]), 1);
+    }
     sm.abort_word = 0;
     mbar_fence_init();
   }
-  if (warp == 8) {
+  if (warp == 16) {
     tmem_alloc(smem_u32(&sm.tmem), kPfTmemCols);
     tmem_relinquish();
   }
   pdl_wait();
   pdl_launch_dependents();
-  if (tid == 32) {
-    // the CTA's row blocks as runs of one request
-    int n = 0, steps = 0;
-    for (int i = 0; i < kPfBlocks && rb0 + i < row_blocks;) {
-      if (p.rb_qcount[rb0 + i] <= 0) { ++i; continue; }
-      PfRun r;
-      r.first = i;
-      r.req = p.rb_req[rb0 + i];
-      r.total = 0;
-      while (i < kPfBlocks && rb0 + i < row_blocks && p.rb_qcount[rb0 + i] > 0 && p.rb_req[rb0 + i] == r.req) {
-        r.total = max(r.total, p.rb_ctx[rb0 + i] + p.rb_qcount[rb0 + i] - 1);
-        ++i;
-      }
-      r.end = i;
-      r.pages = (r.total + kPageTokens - 1) / kPageTokens;
-      r.steps = (r.pages + kPfPages - 1) / kPfPages;
-      if (r.steps > 0) {
-        sm.run[n++] = r;
-        steps += r.steps;
-      }
+  if (sorted) {
+    // With more items than CTAs the groups are dealt by what their last block sees, to and fro: every CTA finds the same order for itself
+    uint16_t* seen = reinterpret_cast<uint16_t*>(sm.v[0][0]);
+    for (int g = tid; g < groups; g += kPfThreads) {
+      const int last = min(g * kPfBlocks + kPfBlocks, row_blocks) - 1;
+      seen[g] = static_cast<uint16_t>(min((max(p.rb_ctx[last] + p.rb_qcount[last], 0) + kPfTok - 2) / kPfTok, 65535));
     }
-    sm.runs = n;
-    sm.steps = steps;
-  }
-  // rows: thread = row of the MMA
-  const int G = p.G, blk = tid >> 4, rb = rb0 + blk;
-  int qp = 0, hh = 0, limit = 0;
-  __nv_bfloat16* out_row = nullptr;
-  if (warp < 4) {
-    qp = (tid & 15) / G;
-    hh = (tid & 15) - qp * G;
-    const int qcount = rb < row_blocks ? p.rb_qcount[rb] : 0;
-    const bool valid = qp < qcount;
-    const __nv_bfloat16* q = nullptr;
-    if (valid) {
-      limit = p.rb_ctx[rb] + qp;
-      const size_t at = (static_cast<size_t>(p.rb_qstart[rb] + qp) * p.Hq + kvh * G + hh) * kD;
-      q = p.q + at;
-      out_row = p.out + at;
+    __syncthreads();
+    for (int g = tid; g < groups; g += kPfThreads) {
+      const int mine = seen[g];
+      int rank = 0;
+      for (int o = 0; o < groups; ++o) rank += seen[o] > mine || (seen[o] == mine && o > g);
+      sm.order[rank] = static_cast<uint16_t>(g);
     }
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      uint4 w = make_uint4(0u, 0u, 0u, 0u);
-      if (valid) w = reinterpret_cast<const uint4*>(q)[c];
-      uint32_t x[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[j]));
-        x[j] = pack_f16x2(v.x * p.scale_log2, v.y * p.scale_log2);
-      }
-      *reinterpret_cast<uint4*>(sm.q + (c >> 3) * (kPfRows * 128) + tid * 128 + (((c & 7) ^ (tid & 7)) << 4)) = make_uint4(x[0], x[1], x[2], x[3]);
-    }
-    fence_proxy_async_smem();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem;
-  const int steps = sm.steps;
   bool ok = true;
 
-  if (warp == 8) {
-    // ------------------------------------------------------------------ MMAs
-    const bool leader = elect_one();
-    const uint32_t idesc_s = umma_idesc(kPfRows, kPfTok, 0u, 0u), idesc_o = umma_idesc(kPfRows, 32u, 0u, 0u);
-    const uint64_t dq = umma_desc_sw128(smem_u32(sm.q)), dp = umma_desc_sw128(smem_u32(sm.p[0]));
-    const uint64_t dk = umma_desc_sw128(smem_u32(sm.k[0])), dv = umma_desc_sw128(smem_u32(sm.v[0]));
-    auto scores = [&](int i) {
-      const int b = i & 1;
-      if (ok) ok = mbar_wait_park(smem_u32(&sm.kv_full[b]), (i >> 1) & 1, abort_flag);
-      if (ok && i > 0) ok = mbar_wait_park(smem_u32(&sm.s_free), (i - 1) & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      tc_fence_after();
-      if (ok && leader) {
+  if (warp >= 16) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfRegsOther));
+    if (warp == 17) {
+      // ------------------------------------------------------- items and pages
+      int gs = 0;
+      auto publish = [&](int n) {                        // the CTA's n-th item; false: there is none
+        const long long at = static_cast<long long>(n) * ctas + (n & 1 ? ctas - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x));
+        PfList& l = sm.list[n % kPfLists];
+        if (ok && n >= kPfLists) ok = mbar_wait_park(smem_u32(&sm.list_free[n % kPfLists]), (n / kPfLists - 1) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return false;
+        if (at >= items) {                               // no item in this round: there is no further round
+          if (lane == 0) l.kvh = -1;
+        } else {
+          const int rank = static_cast<int>(at / p.Hkv);
+          const int rb0 = (sorted ? sm.order[rank] : groups - 1 - rank) * kPfBlocks;      // the blocks that see most first
+          int cnt = 0, req = -1, sees = 0, ctx = 0;
+          if (lane < kPfBlocks) {
+            if (rb0 + lane < row_blocks) {
+              cnt = max(p.rb_qcount[rb0 + lane], 0);
+              req = p.rb_req[rb0 + lane];
+              ctx = p.rb_ctx[rb0 + lane];
+              l.qstart[lane] = p.rb_qstart[rb0 + lane];
+            }
+            l.qcount[lane] = cnt;
+            l.ctx[lane] = ctx;
+            if (cnt > 0) sees = max(ctx + cnt - 1, 0);
+          }
+          const int req_before = __shfl_up_sync(0xffffffffu, req, 1), cnt_before = __shfl_up_sync(0xffffffffu, cnt, 1);
+          const bool on = lane > 0 && cnt > 0 && cnt_before > 0 && req_before == req;     // goes on with the run of the block before it
+          uint32_t starts = __ballot_sync(0xffffffffu, cnt > 0 && !on);
+          const uint32_t goes_on = __ballot_sync(0xffffffffu, on);
+          int runs = 0, steps = 0, tiles = 0;
+          while (starts) {
+            const int s = __ffs(starts) - 1;
+            starts &= starts - 1;
+            const int end = s + __ffs(~(goes_on >> (s + 1)));
+            const bool in = lane >= s && lane < end;
+            PfRun r;
+            r.first = s;
+            r.end = end;
+            r.req = __shfl_sync(0xffffffffu, req, s);
+            r.total = 0;
 #pragma unroll
-        for (int cg = 0; cg < 4; ++cg)
-#pragma unroll
-          for (int k = 0; k < 2; ++k)
-            umma_f16(tmem + cg * kPfTok, dq + ((cg >> 1) * (kPfRows * 128) >> 4) + (cg & 1) * 4 + k * 2,
-                     dk + ((b * 2 + (cg >> 1)) * (kPfTok * 128) >> 4) + (cg & 1) * 4 + k * 2, idesc_s, k > 0);
-        tc_commit(smem_u32(&sm.s_full));
-      }
-      __syncwarp();
-    };
-    if (steps > 0) scores(0);
-    for (int i = 0; i < steps; ++i) {
-      if (i + 1 < steps) scores(i + 1);
-      const int b = i & 1;
-      if (ok) ok = mbar_wait_park(smem_u32(&sm.p_full), i & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      if ((sm.vs_kind[b][0] | sm.vs_kind[b][1]) & kPfWild) pf_unseen(sm, p.rb_qcount + rb0, p.rb_ctx + rb0, row_blocks - rb0, p.G, i, lane);
-      tc_fence_after();
-      if (ok && leader) {
-#pragma unroll
-        for (int cg = 0; cg < 4; ++cg)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f16(tmem + kPfTmemO + cg * 32, dp + (cg * (kPfRows * 128) >> 4) + k * 2, dv + ((b * kD + cg * 32) * 128 >> 4) + k * 2, idesc_o, i > 0 || k > 0);
-        tc_commit(smem_u32(&sm.kv_free[b]));
-        tc_commit(smem_u32(&sm.pv_done));
-      }
-      __syncwarp();
-    }
-  } else if (warp >= 4) {
-    // ------------------------------------------------------------ conversion
-    const int ct = tid - 128;
-    PfWalk ahead, at;
-    // lanes 0..3 of warp 4 copy a page of a step each
-    auto issue = [&](int i) {
-      const PfRun& r = sm.run[ahead.run];
-      const int n = min(kPfPages, r.pages - ahead.step * kPfPages), b = i & 1;
-      if (lane == 0) mbar_expect_tx(smem_u32(&sm.raw_full[b]), n * p.lay.blob_bytes);
-      __syncwarp();
-      if (lane < n) {
-        const int page = p.page_table[static_cast<size_t>(r.req) * p.max_pages + ahead.step * kPfPages + lane];
-        bulk_g2s(smem_u32(raw + (b * kPfPages + lane) * stride), p.cache + (static_cast<size_t>(page) * p.Hkv + kvh) * p.lay.blob_bytes, p.lay.blob_bytes,
-                 smem_u32(&sm.raw_full[b]));
-      }
-      ahead.advance(sm);
-    };
-    int issued = 0;
-    if (warp == 4)
-      for (; issued < 2 && issued < steps; ++issued) issue(issued);
-    for (int i = 0; i < steps; ++i) {
-      const int b = i & 1;
-      const PfRun& r = sm.run[at.run];
-      if (ok) ok = mbar_wait_park(smem_u32(&sm.raw_full[b]), (i >> 1) & 1, abort_flag);
-      if (ok && i >= 2) ok = mbar_wait_park(smem_u32(&sm.kv_free[b]), ((i >> 1) - 1) & 1, abort_flag);
-      pf_convert<KBITS, VBITS>(sm, b, raw + b * kPfPages * stride, stride, p.lay, min(kPfPages, r.pages - at.step * kPfPages), r.total - at.step * kPfTok, ct);
-      at.advance(sm);
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sm.kv_full[b]));
-      asm volatile("bar.sync 2, 128;" ::: "memory");     // the raw pages have been read by all four warps
-      if (warp == 4 && i + 2 < steps && __all_sync(0xffffffffu, ok)) {
-        issue(i + 2);
-        ++issued;
-      }
-    }
-    if (warp == 4 && *abort_flag) {                      // copies in flight land (for a bounded time) before the CTA goes
-      const long long t0 = clock64();
-      for (int i = max(0, issued - 2); i < issued; ++i)
-        while (!mbar_try_wait(smem_u32(&sm.raw_full[i & 1]), (i >> 1) & 1) && clock64() - t0 < kWaitBudgetCycles / 8) {
+            for (int t = 0; t < kPfTiles; ++t) {
+              const int most = static_cast<int>(__reduce_max_sync(0xffffffffu, in && lane / 8 == t ? static_cast<uint32_t>(sees) : 0u));
+              r.tile_steps[t] = (most + kPfTok - 1) / kPfTok;
+              if (most > 0) tiles |= 1 << t;
+              r.total = max(r.total, most);
+            }
+            r.pages = (r.total + kPageTokens - 1) / kPageTokens;
+            r.steps = (r.pages + kPfPages - 1) / kPfPages;
+            if (r.steps > 0) {
+              if (lane == 0) l.run[runs] = r;
+              ++runs;
+              steps += r.steps;
+            }
+          }
+          if (lane == 0) {
+            l.kvh = static_cast<int>(at % p.Hkv);
+            l.runs = runs;
+            l.steps = steps;
+            l.tiles = tiles;
+          }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm.list_full[n % kPfLists]));
+        return at < items;
+      };
+      bool more = publish(0);
+      for (int it = 0; more && ok; ++it) {
+        const PfList& l = sm.list[it % kPfLists];
+        const int steps = l.steps, kvh = l.kvh;
+        bool next = false;
+        PfWalk w;
+        for (int i = 0; i < steps; ++i, ++gs) {
+          const int b = gs % kPfRaw;
+          if (ok && gs >= kPfRaw) ok = mbar_wait_park(smem_u32(&sm.raw_free[b]), (gs / kPfRaw - 1) & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const PfRun& r = l.run[w.run];
+          const int n = min(kPfPages, r.pages - w.step * kPfPages);
+          if (lane == 0) mbar_expect_tx(smem_u32(&sm.raw_full[b]), n * p.lay.blob_bytes);
+          __syncwarp();
+          if (lane < n) {
+            const int page = p.page_table[static_cast<size_t>(r.req) * p.max_pages + w.step * kPfPages + lane];
+            bulk_g2s(smem_u32(raw + (b * kPfPages + lane) * stride), p.cache + (static_cast<size_t>(page) * p.Hkv + kvh) * p.lay.blob_bytes, p.lay.blob_bytes,
+                     smem_u32(&sm.raw_full[b]));
+          }
+          w.advance(l);
+          if (i == min(1, steps - 1)) next = publish(it + 1);
+        }
+        if (steps == 0) next = publish(it + 1);
+        more = next;
+      }
+      if (*abort_flag) {                                 // copies in flight land (for a bounded time) before the CTA goes
+        const long long t0 = clock64();
+        for (int i = max(0, gs - kPfRaw); i < gs; ++i)
+          while (!mbar_try_wait(smem_u32(&sm.raw_full[i % kPfRaw]), (i / kPfRaw) & 1) && clock64() - t0 < kWaitBudgetCycles / 8) {
+          }
+      }
+    } else if (warp != 19) {
+      // ---------------------------------------------------------------- MMAs
+      // Warp 16 issues those of the scores, warp 18 those of the output: what one waits for does not hold up the other
+      const bool leader = elect_one(), is_s = warp == 16;
+      const uint32_t idesc_s = umma_idesc(kPfRows, kPfTok, 0u, 0u), idesc_o = umma_idesc(kPfRows, kD, 0u, 0u) | 1u << 16;      // V: channels are contiguous
+      const uint64_t dq = umma_desc_sw128(smem_u32(sm.q[0])), dk = umma_desc_sw128(smem_u32(sm.k[0][0])), dv = umma_desc_sw128_n(smem_u32(sm.v[0][0]), kPfHalf);
+      int gs = 0;                                        // steps of earlier items
+      int n[kPfTiles] = {0, 0};                          // steps per tile
+      uint32_t q_phase = 0;                              // bit = tile
+      for (int it = 0;; ++it) {
+        const PfList& l = sm.list[it % kPfLists];
+        if (ok) ok = mbar_wait_park(smem_u32(&sm.list_full[it % kPfLists]), (it / kPfLists) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok || l.kvh < 0) break;
+        const int steps = l.steps;
+        uint32_t q_new = 3;                              // tiles whose Q of this item has not been waited for
+        PfWalk w;
+        for (int i = 0; i < steps; ++i, ++gs) {
+          const int b = gs & 1;
+          if (ok) ok = mbar_wait_park(smem_u32(is_s ? &sm.k_full[b] : &sm.v_full[b]), (gs >> 1) & 1, abort_flag);
+#pragma unroll
+          for (int t = 0; t < kPfTiles; ++t) {
+            if (w.step >= l.run[w.run].tile_steps[t]) continue;
+            const uint32_t tile = tmem + t * kPfTmemTile;
+            if (is_s) {
+              if (q_new >> t & 1) {
+                if (ok) ok = mbar_wait_park(smem_u32(&sm.q_full[t]), q_phase >> t & 1, abort_flag);
+                q_new ^= 1u << t;
+                q_phase ^= 1u << t;
+              }
+              if (ok && n[t] > 0) ok = mbar_wait_park(smem_u32(&sm.s_free[t]), (n[t] - 1) & 1, abort_flag);
+            } else {
+              if (ok) ok = mbar_wait_park(smem_u32(&sm.p_full[t]), n[t] & 1, abort_flag);
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            ++n[t];
+            tc_fence_after();
+            if (ok && leader) {
+              if (is_s) {
+#pragma unroll
+                for (int part = 0; part < 2; ++part) {
+                  const uint64_t k0 = dk + ((b * 2 + part) * (2 * kPfHalf) >> 4);
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) umma_f16_ts(tile, tile + kPfTmemQ + k * 8, k0 + k * 2, idesc_s, part > 0 || k > 0);
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) umma_f16(tile, dq + (t * (kPfRows * 128) >> 4) + k * 2, k0 + (kPfHalf >> 4) + k * 2, idesc_s, 1);
+                }
+                tc_commit(smem_u32(&sm.s_full[t]));
+              } else {
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+#pragma unroll
+                  for (int k = 0; k < 4; ++k)
+                    umma_f16_ts(tile + kPfTmemO, tile + kPfTmemP + k * 8, dv + ((b * 2 + part) * (2 * kPfHalf) >> 4) + k * (16 * 128 >> 4), idesc_o, 1);
+                tc_commit(smem_u32(&sm.pv_done[t]));
+              }
+            }
+            __syncwarp();
+          }
+          if (ok && leader) tc_commit(smem_u32(is_s ? &sm.k_free[b] : &sm.v_free[b]));
+          __syncwarp();
+          w.advance(l);
+        }
+        if (lane == 0) mbar_arrive(smem_u32(&sm.list_free[it % kPfLists]));
+      }
+    }
+  } else if (warp >= 8) {
+    // ------------------------------------------------------------ conversion
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfRegsConvert));
+    // warps 8-11 convert K, warps 12-15 V: scores run a step ahead of their softmax, and wait for no conversion of V
+    const bool is_v = warp >= 12;
+    const int ct = tid & 127;
+    int gs = 0, v_exp = 0;
+    for (int it = 0;; ++it) {
+      const PfList& l = sm.list[it % kPfLists];
+      if (ok) ok = mbar_wait_park(smem_u32(&sm.list_full[it % kPfLists]), (it / kPfLists) & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok || l.kvh < 0) break;
+      const int steps = l.steps;
+      PfWalk w;
+      for (int i = 0; i < steps; ++i, ++gs) {
+        const int b = gs & 1, slot = gs % kPfRaw, note = gs % kPfNotes, visible = l.run[w.run].total - w.step * kPfTok;
+        w.advance(l);
+        if (ok) ok = mbar_wait_park(smem_u32(&sm.raw_full[slot]), (gs / kPfRaw) & 1, abort_flag);
+        if (ok && gs >= 2) ok = mbar_wait_park(smem_u32(is_v ? &sm.v_free[b] : &sm.k_free[b]), ((gs >> 1) - 1) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        const uint8_t* pages = raw + slot * kPfPages * stride;
+        float4 scale[2];
+        bool odd;
+        const int e = pf_exponent(pages + (is_v ? p.lay.v_scale_off : p.lay.k_scale_off), stride, visible, lane, scale, odd);
+        if (!is_v) {
+          if (ct == 0) {
+            sm.k_mul[note] = pow2f(e - 5);                               // codes times scales below 2^13
+            mbar_arrive(smem_u32(&sm.k_note[note]));
+          }
+          pf_convert_k<KBITS>(sm.k[b], pages, stride, p.lay, pow2f(5 - e), ct);
+        } else {
+          if (i == 0 || e - 7 > v_exp) v_exp = e - 3;                    // below 2^11, to be changed when they pass 2^15
+          if (warp == 12) {
+            if (odd) {
+              auto of = [](float x) { return fabsf(x) < INFINITY ? 0.f : x; };
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                float* at = sm.vw[note] + lane + 32 * h;
+                at[0] = of(scale[h].x); at[kPfTok] = of(scale[h].y); at[2 * kPfTok] = of(scale[h].z); at[3 * kPfTok] = of(scale[h].w);
+              }
+            }
+            __syncwarp();
+            if (lane == 0) {
+              sm.v_exp[note] = v_exp;
+              sm.wild[note] = odd;
+              mbar_arrive(smem_u32(&sm.v_note[note]));
+            }
+          }
+          pf_convert_v<VBITS>(sm.v[b], pages, stride, p.lay, visible, pow2f(-v_exp), ct);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(smem_u32(is_v ? &sm.v_full[b] : &sm.k_full[b]));
+          mbar_arrive(smem_u32(&sm.raw_free[slot]));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm.list_free[it % kPfLists]));
     }
   } else {
     // --------------------------------------------------------------- softmax
-    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    float m = -INFINITY, l = 0.f;
-    PfWalk at;
-    for (int i = 0; i < steps; ++i) {
-      const int b = i & 1, tok0 = at.step * kPfTok;
-      const PfRun& r = sm.run[at.run];
-      const int sees = (blk >= r.first && blk < r.end) ? limit - tok0 : 0;       // tokens of the step that this row sees
-      at.advance(sm);
-      if (ok) ok = mbar_wait_park(smem_u32(&sm.kv_full[b]), (i >> 1) & 1, abort_flag);      // the scales
-      if (ok) ok = mbar_wait_park(smem_u32(&sm.s_full), i & 1, abort_flag);
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPfRegsSoftmax));
+    const int t = warp >> 2, row = tid & 127, blk = tid >> 4;
+    const uint32_t tile = tmem + t * kPfTmemTile + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const int qp = (tid & 15) / p.G, hh = (tid & 15) - qp * p.G;
+    struct Row {
+      __nv_bfloat16* out;                                // null: not a query
+      int limit;                                         // tokens that it sees
+    };
+    // the row of the thread in item `it`, and Q of its tile; false: no more items
+    auto begin = [&](int it, Row& r) {
+      const PfList& l = sm.list[it % kPfLists];
+      if (ok) ok = mbar_wait_park(smem_u32(&sm.list_full[it % kPfLists]), (it / kPfLists) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
-      tc_fence_after();
-      float2 s[kPfTok / 2];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t a[4][16];
-#pragma unroll
-        for (int cg = 0; cg < 4; ++cg) tmem_ld_32x16(tmem + lane_base + cg * kPfTok + c * 16, a[cg]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int cg = 0; cg < 4; ++cg) {
-            const float4 k = *reinterpret_cast<const float4*>(sm.ks[b] + cg * kPfTok + c * 16 + j * 4);
-            const float2 x = make_float2(__uint_as_float(a[cg][4 * j]), __uint_as_float(a[cg][4 * j + 1])), y = make_float2(__uint_as_float(a[cg][4 * j + 2]), __uint_as_float(a[cg][4 * j + 3]));
-            float2& s0 = s[c * 8 + 2 * j];
-            float2& s1 = s[c * 8 + 2 * j + 1];
-            s0 = cg == 0 ? __fmul2_rn(x, make_float2(k.x, k.y)) : __ffma2_rn(x, make_float2(k.x, k.y), s0);
-            s1 = cg == 0 ? __fmul2_rn(y, make_float2(k.z, k.w)) : __ffma2_rn(y, make_float2(k.z, k.w), s1);
-          }
+      r.out = nullptr;
+      r.limit = 0;
+      if (!ok || l.kvh < 0) return false;
+      const __nv_bfloat16* q = nullptr;
+      if (qp < l.qcount[blk]) {
+        r.limit = l.ctx[blk] + qp;
+        const size_t at = (static_cast<size_t>(l.qstart[blk] + qp) * p.Hq + l.kvh * p.G + hh) * kD;
+        q = p.q + at;
+        r.out = p.out + at;
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sm.s_free));
-      if (sees < kPfTok) {
+      if (l.tiles >> t & 1) {
+        uint32_t x[32];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            uint4 u = make_uint4(0u, 0u, 0u, 0u);
+            if (q != nullptr) u = reinterpret_cast<const uint4*>(q)[h * 8 + c];
+            const uint32_t in[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&in[j]));
+              x[c * 4 + j] = pack_f16x2(f.x * p.scale_log2, f.y * p.scale_log2);
+            }
+          }
+          if (h == 0) {
+            tmem_st_32x32(tile + kPfTmemQ, x);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<uint4*>(sm.q[t] + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+          }
+        }
+        tmem_st_wait();
+        fence_proxy_async_smem();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm.q_full[t]));
+      }
+      return true;
+    };
+    int gs = 0, n = 0;                                   // steps of earlier items; steps that this tile took part in
+    Row cur;
+    bool more = begin(0, cur);
+    for (int it = 0; more; ++it) {
+      const PfList& l = sm.list[it % kPfLists];
+      const int steps = l.steps;
+      const bool part = l.tiles >> t & 1;
+      float m = -INFINITY, sum = 0.f;
+      int v_exp = 0;
+      bool first = true;
+      if (part) {                                        // output starts at zero
+        uint32_t z[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) z[j] = 0u;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_st_32x32(tile + kPfTmemO + c * 32, z);
+        tmem_st_wait();
+      }
+      PfWalk w;
+      for (int i = 0; i < steps; ++i, ++gs) {
+        const PfRun& r = l.run[w.run];
+        const int note = gs % kPfNotes, tok0 = w.step * kPfTok;
+        const bool skip = w.step >= r.tile_steps[t];
+        const int sees = (blk >= r.first && blk < r.end) ? cur.limit - tok0 : 0;       // tokens of the step that this row sees
+        w.advance(l);
+        if (skip) continue;
+        if (ok) ok = mbar_wait_park(smem_u32(&sm.s_full[t]), n & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        tc_fence_after();
+        uint32_t a[2][32];
+        tmem_ld_32x32(tile, a[0]);
+        tmem_ld_32x32(tile + 32, a[1]);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm.s_free[t]));
+        // a note is written again four steps later, after MMAs that are issued after this step's softmax
+        if (ok) ok = mbar_wait_park(smem_u32(&sm.k_note[note]), (gs / kPfNotes) & 1, abort_flag);
+        if (ok) ok = mbar_wait_park(smem_u32(&sm.v_note[note]), (gs / kPfNotes) & 1, abort_flag);
+        if (sees < kPfTok) {
+#pragma unroll
+          for (int j = 0; j < kPfTok; ++j)
+            if (j >= sees) a[j >> 5][j & 31] = 0xFF800000u;                             // -inf
+        }
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int j = 0; j < kPfTok; ++j) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(a[j >> 5][j & 31]));
+        const float mul = sm.k_mul[note], top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * mul;
+        float alpha = 1.f;
+        bool grew = top > m + kPfGrowth || (m == -INFINITY && top > m);
+        if (grew) {
+          alpha = fast_exp2(m - top);
+          m = top;
+          sum *= alpha;
+        }
+        const int e = sm.v_exp[note];
+        if (first) v_exp = e;
+        if (e != v_exp) {
+          alpha *= pow2f(v_exp - e);
+          v_exp = e;
+          grew = true;
+        }
+        const float use = m == -INFINITY ? 0.f : m;
+        const float2 less = make_float2(-use, -use), mul2 = make_float2(mul, mul);
+        float2 part_sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        uint32_t pr[32];
 #pragma unroll
         for (int j = 0; j < kPfTok / 2; ++j) {
-          if (2 * j >= sees) s[j].x = -INFINITY;
-          if (2 * j + 1 >= sees) s[j].y = -INFINITY;
+          const float2 d = __ffma2_rn(make_float2(__uint_as_float(a[j >> 4][2 * j & 31]), __uint_as_float(a[j >> 4][(2 * j + 1) & 31])), mul2, less);
+          const float2 x = make_float2(fast_exp2(d.x), fast_exp2(d.y));
+          part_sum[j & 1] = __fadd2_rn(part_sum[j & 1], x);
+          pr[j] = pack_f16x2(x.x, x.y);
         }
-      }
-      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int j = 0; j < kPfTok / 2; ++j) mx[j & 3] = fmaxf(mx[j & 3], fmaxf(s[j].x, s[j].y));
-      const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      float alpha = 1.f;
-      const bool grew = top > m + ((sm.vs_kind[b][0] | sm.vs_kind[b][1]) & kPfLarge ? 0.f : kPfGrowth) || (m == -INFINITY && top > m);
-      if (grew) {
-        alpha = fast_exp2(m - top);
-        m = top;
-        l *= alpha;
-      }
-      const float use = m == -INFINITY ? 0.f : m;
-      const float2 less = make_float2(-use, -use);
-      float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-      for (int j = 0; j < kPfTok / 2; ++j) {
-        const float2 d = __fadd2_rn(s[j], less);
-        s[j] = make_float2(fast_exp2(d.x), fast_exp2(d.y));
-        sum[j & 1] = __fadd2_rn(sum[j & 1], s[j]);
-      }
-      l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
-      // the previous product has read the probabilities and written the output
-      if (ok && i > 0) ok = mbar_wait_park(smem_u32(&sm.pv_done), (i - 1) & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      if (i > 0 && __any_sync(0xffffffffu, grew)) {
+        sum += (part_sum[0].x + part_sum[0].y) + (part_sum[1].x + part_sum[1].y);
+        // the previous product has read the probabilities and written the output
+        if (ok && !first) ok = mbar_wait_park(smem_u32(&sm.pv_done[t]), (n - 1) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
+        tmem_st_32x32(tile + kPfTmemP, pr);
+        if (!first && __any_sync(0xffffffffu, grew)) {
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32(tile + kPfTmemO + c * 32, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+            tmem_st_32x32(tile + kPfTmemO + c * 32, o);
+          }
+        }
+        tmem_st_wait();
+        if (sm.wild[note]) {
+          if (ok) ok = mbar_wait_park(smem_u32(&sm.v_full[gs & 1]), (gs >> 1) & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          pf_wild(sm.vw[note], sm.v[gs & 1][0], tile, sees);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm.p_full[t]));
+        first = false;
+        ++n;
+      }
+      // the next item's Q while the last product runs (all of this item's scores are there)
+      Row next;
+      more = begin(it + 1, next);
+      if (!part) {                                       // no row of the tile sees a token
+        if (cur.out != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) reinterpret_cast<uint4*>(cur.out)[j] = make_uint4(0u, 0u, 0u, 0u);
+        }
+      } else {
+        if (ok) ok = mbar_wait_park(smem_u32(&sm.pv_done[t]), (n - 1) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        tc_fence_after();
+        const float inv = sum > 0.f ? 1.f / sum : sum == 0.f ? 0.f : sum;               // NaN stays
+        const float up = pow2f(v_exp);
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           uint32_t o[32];
-          tmem_ld_32x32(tmem + lane_base + kPfTmemO + c * 32, o);
+          tmem_ld_32x32(tile + kPfTmemO + c * 32, o);
           tmem_ld_wait();
+          if (cur.out != nullptr) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-          tmem_st_32x32(tmem + lane_base + kPfTmemO + c * 32, o);
-        }
-        tmem_st_wait();
-      }
+            for (int j = 0; j < 4; ++j) {
+              uint32_t x[4];
 #pragma unroll
-      for (int cg = 0; cg < 4; ++cg)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const float4 v0 = *reinterpret_cast<const float4*>(sm.vs[b] + cg * kPfTok + c * 8), v1 = *reinterpret_cast<const float4*>(sm.vs[b] + cg * kPfTok + c * 8 + 4);
-          const float2 w0 = __fmul2_rn(s[4 * c], make_float2(v0.x, v0.y)), w1 = __fmul2_rn(s[4 * c + 1], make_float2(v0.z, v0.w));
-          const float2 w2 = __fmul2_rn(s[4 * c + 2], make_float2(v1.x, v1.y)), w3 = __fmul2_rn(s[4 * c + 3], make_float2(v1.z, v1.w));
-          *reinterpret_cast<uint4*>(sm.p[cg] + tid * 128 + ((c ^ (tid & 7)) << 4)) =
-              make_uint4(pack_f16x2(w0.x, w0.y), pack_f16x2(w1.x, w1.y), pack_f16x2(w2.x, w2.y), pack_f16x2(w3.x, w3.y));
-        }
-      fence_proxy_async_smem();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sm.p_full));
-    }
-    if (steps == 0) {                                    // no row sees a token
-      if (out_row != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) reinterpret_cast<uint4*>(out_row)[j] = make_uint4(0u, 0u, 0u, 0u);
-      }
-    } else {
-      if (ok) ok = mbar_wait_park(smem_u32(&sm.pv_done), (steps - 1) & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t o[32];
-        tmem_ld_32x32(tmem + lane_base + kPfTmemO + c * 32, o);
-        tmem_ld_wait();
-        if (out_row != nullptr) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[k] = pack_bf16x2(__uint_as_float(o[8 * j + 2 * k]) * inv, __uint_as_float(o[8 * j + 2 * k + 1]) * inv);
-            *reinterpret_cast<uint4*>(out_row + c * 32 + j * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+              for (int k = 0; k < 4; ++k) x[k] = pack_bf16x2(__uint_as_float(o[8 * j + 2 * k]) * inv * up, __uint_as_float(o[8 * j + 2 * k + 1]) * inv * up);
+              *reinterpret_cast<uint4*>(cur.out + c * 32 + j * 8) = make_uint4(x[0], x[1], x[2], x[3]);
+            }
           }
         }
+        tc_fence_before();
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm.list_free[it % kPfLists]));
+      cur = next;
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) tmem_dealloc(tmem, kPfTmemCols);
+  if (warp == 16) tmem_dealloc(tmem, kPfTmemCols);
   if (tid == 0 && sm.abort_word) atomicExch(p.status, static_cast<uint32_t>(kErrBarrierTimeout));
 }
 
 template <int KB, int VB>
 static int launch_prefill(const AttnParams& p, int row_blocks, cudaStream_t st) {
   const int stride = (p.lay.blob_bytes + 127) & ~127;
-  const size_t smem = sizeof(PfSmem) + 1024 + static_cast<size_t>(2) * kPfPages * stride;
-  static bool configured[64] = {};
+  const size_t smem = sizeof(PfSmem) + 1024 + static_cast<size_t>(kPfRaw) * kPfPages * stride;
+  static int sms[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -18;
-  if (!configured[dev]) {
+  if (!sms[dev]) {
     cudaError_t e = cudaFuncSetAttribute(paged_prefill_kernel<KB, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    int n = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return static_cast<int>(e);
-    configured[dev] = true;
+    // the warps' new shares come out of the registers that the block was launched with
+    cudaFuncAttributes at;
+    e = cudaFuncGetAttributes(&at, paged_prefill_kernel<KB, VB>);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (at.numRegs < kPfRegs) return -19;
+    sms[dev] = n;
   }
-  return static_cast<int>(launch(paged_prefill_kernel<KB, VB>, dim3(p.Hkv, (row_blocks + kPfBlocks - 1) / kPfBlocks), dim3(kPfThreads), smem, st, p, row_blocks));
+  const long long items = static_cast<long long>((row_blocks + kPfBlocks - 1) / kPfBlocks) * p.Hkv;
+  return static_cast<int>(launch(paged_prefill_kernel<KB, VB>, dim3(static_cast<unsigned>(items < sms[dev] ? items : sms[dev])), dim3(kPfThreads), smem, st, p, row_blocks));
 }
 
 }  // namespace cb

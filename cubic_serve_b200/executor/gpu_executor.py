@@ -144,17 +144,17 @@ class BatchBuilder:
 
     def _prompts(self, blocks: list[int]) -> tuple[int, int]:
         """The longest run of neighbouring segments with at least four row blocks each, as row blocks ``[lo, hi)`` for the prompt
-        kernel (a CTA takes eight blocks and walks the steps of one request at a time; with fewer of a request most of its rows
-        idle), if that is the faster one by a tenth of its estimated time.
+        kernel (a CTA takes sixteen blocks and walks the steps of one request at a time; with fewer of a request most of its rows
+        idle), if a bound of its time is a tenth below the general kernel's.
 
-        Prompt kernel: 3 us a step of 64 tokens, and as much as four steps around them for every CTA; CTAs start last blocks first, so that
-        with more of them than SMs the step ends with the longest, with one that starts late behind the load before it, or with two that
-        have to share an SM.  General kernel: 0.128 us a page and SM, 2.1 us a CTA and SM, 0.06 us a page of the longest split, and
+        The bound of the prompt kernel's time: 3 us a step of 64 tokens and eight blocks, and as much as four steps around them, in CTAs that start last
+        blocks first, so that with more of them than SMs the step ends with the longest, with one that starts late behind the load before it, or
+        with two that have to share an SM.  The kernel takes 2.1 us a step of sixteen blocks, so that what passes gains; what does not pass by
+        little would too (one prompt of 331 tokens 23 against 24 us, 40 x 20 tokens behind 300 57 against 63), what is far from it does not (one of 64 behind
+        4000 136 against 64).  General kernel: 0.128 us a page and SM, 2.1 us a CTA and SM, 0.06 us a page of the longest split, and
         14.5 us for its launch, which is there anyway when there are other row blocks and twice when they are on both sides.
         Fitted to 180 steps of 8 shapes of heads (1 to 32 key / value heads, groups of 1 to 16; 1 to 40 portions of 20 to 6000 tokens behind 0
-        to 8000): mean errors 3 and 7 %; without the margin some steps would be up to 1.26 times slower than with the general kernel, with
-        it none is, nor of 60 steps that have decode or review rows beside the portions (2 % at most).  E.g. 32 over 8 heads: 8 x 1024 tokens
-        513 against 707 us, one prompt of 331 33 against 29, 40 x 20 tokens behind 300 106 against 67.  (One B200.)"""
+        to 8000).  E.g. 32 over 8 heads: 8 x 1024 tokens 220 against 702 us, 4 x 256 behind 2048 104 against 276.  (One B200.)"""
         best, at, lo, first, of = (0, 0), 0, 0, 0, (0, 0)
         for i, n in enumerate(blocks + [0]):
             if n < 4:

@@ -153,6 +153,49 @@ def test_prompt_form_has_the_range_of_f16_for_scales(kb, vb, top):
     assert torch.isfinite(want.float()).all() and _close(_run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1), want)
 
 
+@pytest.mark.parametrize("kb,vb,group,hkv", [(8, 8, 4, 8), (6, 6, 16, 4), (4, 8, 1, 16)])
+@pytest.mark.parametrize("portions", [[(0, 700), (33, 1), (900, 301), (0, 64), (5, 300)], [(63, 9000)], [(64 * i, 65) for i in range(20)]])
+def test_prompt_form_with_more_items_than_ctas(kb, vb, group, hkv, portions):
+    """A CTA takes several items of 256 rows, of unequal length, one after the other; 9000 tokens make more groups than are sorted."""
+    qb = 16 // group
+    if group == 1:
+        portions = [(s, 4 * n) for s, n in portions if n < 9000] or [(0, 2600)]
+    cache, table = _cache([s + n for s, n in portions], hkv, kb, vb, kb + group)
+    T = sum(n for _, n in portions)
+    q = torch.randn(T, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(5)).bfloat16()
+    blocks, t = [], 0
+    for r, (s, n) in enumerate(portions):
+        blocks += [(r, t + i, min(qb, n - i), s + i + 1) for i in range(0, n, qb)]
+        t += n
+    assert -(-len(blocks) // 16) * hkv > torch.cuda.get_device_properties(0).multi_processor_count
+    want = _run("", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
+    assert _close(_run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1), want)
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (4, 6)])
+@pytest.mark.parametrize("low,high", [(-6, 6), (-20, 0), (0, 30), (60, 100), (-110, -98)])
+def test_prompt_form_with_scales_of_any_size(kb, vb, low, high):
+    """V scales of 2^low to 2^high, larger from page to page: the powers of two that keep the operands in the range of f16 change on the way.
+    (Results below 2^-126 would not be normal numbers.)"""
+    hkv, group, n = 1, 4, 200
+    cache, table = _cache([n], hkv, kb, vb, 13)
+    pages = table[0, :13].tolist()
+    factor = torch.tensor([2.0 ** round(low + (high - low) * i / 12) for i in range(13)], dtype=torch.float64)
+    for i, page in enumerate(pages):
+        s = _scales(cache, kb, vb)[page]
+        s.copy_((s.double() * factor[i].item()).float())
+    q = torch.randn(n, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(6)).bfloat16()
+    blocks = [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)]
+    got = _run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
+    k, v = (torch.cat([eager.decode_cache_page(cache[p, 0].cpu(), D, kb, vb)[i] for p in pages])[:n].double() for i in (0, 1))
+    z = torch.einsum("thd,sd->ths", q.cpu().double(), k) * 0.05
+    z.masked_fill_(torch.arange(n)[None, None] > torch.arange(n)[:, None, None], float("-inf"))
+    ref = torch.einsum("ths,sd->thd", z.softmax(-1), v)
+    # relative to a power of two near the row's scale, so that _close's own arithmetic stays in range
+    unit = torch.exp2(ref.abs().amax(-1, keepdim=True).log2().floor())
+    assert _close((got.cpu().double() / unit), ref / unit)
+
+
 @pytest.mark.parametrize("form,splits", [("", 1), ("decode", 1), ("decode", 4), ("prefill", 1)])
 def test_rows_that_see_no_token_are_zero(form, splits):
     """Alone in their CTA and beside rows that see something."""
