@@ -20,8 +20,11 @@
 //
 // Reference counterparts: ops/cuda/linear_attention/causal_conv_native.cu:13, gated_delta_native.cu:36,
 // gated_delta_coefficients_native.cu:17 and the oracle ops/eager/hybrid.py:255-548 (fp32 recurrence branch).
+#include "launch.cuh"
+#include "mma.cuh"
 #include "ptx.cuh"
 #include "segments.cuh"
+#include <limits.h>
 #include <type_traits>
 
 namespace cb {
@@ -185,6 +188,7 @@ struct GdnDeltaParams {
   float eps_norm;             // RMSNorm epsilon
   float eps_l2;               // L2-normalisation epsilon
   int commit;                 // 0: the state is read but not written back (speculative review pass)
+  int most;                   // segments of more rows are left out (gdn_delta_chunk_kernel takes them)
   GdnSegments seg;
 };
 
@@ -207,7 +211,7 @@ gdn_delta_kernel(const GdnDeltaParams p) {
   const int head = blockIdx.x;
   const int s = blockIdx.y;
   const int n = p.seg.count[s];
-  if (n <= 0) return;
+  if (n <= 0 || n > p.most) return;
   const int row0 = p.seg.row0[s];
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -366,6 +370,650 @@ gdn_delta_kernel(const GdnDeltaParams p) {
       *reinterpret_cast<float4*>(sp + (4 * i) * kGdnDim + 32 * c) = make_float4(S[i][c][0].x, S[i][c][0].y, S[i][c][1].x, S[i][c][1].y);
 }
 
+// ------------------------------------------------------------------------------------------------- chunks of long segments
+// The recurrence above has one token after the other: about 1900 cycles each, whatever the machine has idle.  Segments of kGdnChunk tokens and
+// more are taken in chunks of 32 on the tensor cores.  With G the running product of the decays of a chunk and S its state at the start,
+//     Delta = (I + L)^-1 beta (V - G K S^T),   L[t][s] = beta_t G_t / G_s (k_t . k_s) for s < t
+//     o_t = G_t S q_t + sum over s <= t of G_t / G_s (q_t . k_s) Delta_s,      S <- G_end S + sum of G_end / G_s Delta_s k_s^T
+// so that a chunk's chain is a dozen dependent products instead of 32 reductions.  (I + L)^-1 is taken by blocks of 16 tokens: the two blocks on the
+// diagonal are inverted, the one below them is applied between.
+//
+// A value row (a row of S, a column of V, Delta and o) never meets another before the output norm: a warp holds 16 rows of S in registers and
+// walks the chunk alone, everything transposed ([value row][token]), so that a product's accumulators are the next one's A operand
+// without a shuffle.  Operands are f16: normalised k and q are bf16 below one; what is computed in fp32 (S, Delta, L, the inverses, q . k) is
+// split in two f16 behind a power of two that puts its largest at 2^13 (22 bits); Delta as it enters the state in three.  Sums with what is larger than
+// the product (inverse less one, decayed state) are fp32 multiply-adds outside the tensor cores, which cut their sums off.
+// Decay ratios are products of their factors, as in the recurrence: no logarithm, no quotient.
+// Against 64 bits (331 rows, random decays): outputs 2.8982e-3 either way; the state 0.99e-7 against 0.77e-7 of the recurrence, with slow decays
+// and similar keys 5.9e-7 against 7.7e-7 (640 rows), with large values 9.2e-7 against 10.4e-7 (320).
+//
+// A CTA is a head of a segment: warps 0-7 walk the chunks, warps 8-15 prepare the next chunk's operands and norm and store the last one's outputs
+// meanwhile.
+// What bounds it: the chain of a chunk (about 10000 cycles, of which its MMAs take 3500) and its preparation, which takes as long beside it.
+// One row after the other -> in chunks, 32 heads, one B200: segments of 1000, 536, 823, 359 and 646 rows 1013 -> 247 us, one of 1750 924 -> 380, one of 331
+// 307 -> 94, one of 32 34 -> 28, 16 of 256 1040 -> 249.
+// A chunk with a key, query, value or coefficient that is not finite is walked token by token: zero times it, in a row before it, is not zero.
+static constexpr int kGdnChunk = 32;
+static constexpr int kGdnChunkThreads = 512, kGdnPrepareThreads = 256;
+// registers a thread: at launch, and of the walking and the preparing warps after they have shared them out anew
+static constexpr int kGdnRegs = 128, kGdnRegsWalk = 184, kGdnRegsPrepare = 72;
+static_assert(2 * kGdnRegsWalk + 2 * kGdnRegsPrepare <= 4 * kGdnRegs, "four warpgroups");
+struct GdnOperands {
+  uint8_t q[kGdnChunk * 256], k[kGdnChunk * 256];        // f16 [token][128], 16-byte chunk ^ (token & 7)
+  __half inv[2][2][16 * 16];                             // [block][hi, lo] inverses of the blocks on the diagonal, less one
+  __half l10[2][16 * 16];                                // [hi, lo] block of L below the diagonal
+  __half a[3][2][16 * 16];                               // [block 00, 10, 11][hi, lo] q . k with ratios
+  float4 coef[kGdnChunk];                                // beta_t, G_t, G_end / G_t, decay
+  __nv_bfloat16 o[kGdnChunk][kGdnDim];
+  float squares[8][kGdnChunk];                           // [warp][token]
+  int wild;
+};
+struct __align__(128) GdnChunkSmem {
+  GdnOperands op[2];                                     // [parity of the chunk]
+  __nv_bfloat16 raw[2][kGdnChunk * kGdnDim];             // next chunk: q, k
+  __nv_bfloat16 v[3][kGdnChunk * kGdnDim];               // chunk modulo 3
+  float ratio[kGdnChunk][kGdnChunk];                     // [t][s] G_t / G_s, s <= t
+  float low[2][16][16];                                  // blocks on the diagonal of L
+};
+static constexpr float kGdnUp = 4096.f;                  // of L, the inverses and q . k: entries of at most about one
+
+template <int kThreads>
+__device__ __forceinline__ void gdn_bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
+template <int kThreads>
+__device__ __forceinline__ void gdn_bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
+
+// Two rows of 16 f16 a 16-byte chunk apart would meet in a bank: chunk ^ (row >> 2 & 1).
+__device__ __forceinline__ int gdn_at16(int row, int col) { return row * 16 + ((((col >> 3) ^ (row >> 2)) & 1) << 3) + (col & 7); }
+
+__device__ __forceinline__ void gdn_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t gdn_pack(float x, float y) {
+  const __half2 h = __floats2half2_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ void gdn_split(float x, float y, uint32_t& hi, uint32_t& lo) {
+  hi = gdn_pack(x, y);
+  const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = gdn_pack(x - h.x, y - h.y);
+}
+__device__ __forceinline__ float gdn_pow2(int e) { return __int_as_float((e + 127) << 23); }
+// Exponent of the largest finite magnitude that the warp holds (`most`: the thread's, as bits); 0 and small ones count as 2^-100.
+__device__ __forceinline__ int gdn_exponent(uint32_t most) {
+  return min(max(static_cast<int>(__reduce_max_sync(0xffffffffu, most) >> 23) - 127, -100), 110);
+}
+__device__ __forceinline__ uint32_t gdn_bits(float x) {
+  const uint32_t b = __float_as_uint(x) & 0x7FFFFFFFu;
+  return b < 0x7F800000u ? b : 0u;
+}
+// Accumulators of 16 value rows x 16 tokens (two n-tiles) -> the A operand over those tokens, times 2^(13 - e); returns 2^(e - 13)
+__device__ __forceinline__ float gdn_operand(const float (&x)[2][4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+  uint32_t most = 0;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) most = max(most, gdn_bits(x[j][i]));
+  const int e = gdn_exponent(most);
+  const float up = gdn_pow2(13 - e);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    gdn_split(x[j][0] * up, x[j][1] * up, hi[2 * j], lo[2 * j]);
+    gdn_split(x[j][2] * up, x[j][3] * up, hi[2 * j + 1], lo[2 * j + 1]);
+  }
+  return gdn_pow2(e - 13);
+}
+// d[n-tile] = x (hi, lo) times a block of 16 x 16 (hi, lo), [column token][row token]
+__device__ __forceinline__ void gdn_block(float (&d)[2][4], const uint32_t (&hi)[4], const uint32_t (&lo)[4], const __half (&m)[2][16 * 16], int lane) {
+  uint32_t bh[4], bl[4];
+  const int row = (lane & 7) + ((lane >> 4) << 3), col = ((lane >> 3) & 1) << 3;      // matrices: (n 0, k 0) (n 0, k 8) (n 8, k 0) (n 8, k 8)
+  ldsm4(bh, smem_u32(&m[0][gdn_at16(row, col)]));
+  ldsm4(bl, smem_u32(&m[1][gdn_at16(row, col)]));
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[j][i] = 0.f;
+    gdn_mma(d[j], lo, bh[2 * j], bh[2 * j + 1]);
+    gdn_mma(d[j], hi, bl[2 * j], bl[2 * j + 1]);
+    gdn_mma(d[j], hi, bh[2 * j], bh[2 * j + 1]);
+  }
+}
+
+// grid (Hv, segments).  Named barriers: 1 + parity: a chunk's operands are there; 3 + parity: it has been walked; 5: among the preparing warps.
+__global__ void __launch_bounds__(kGdnChunkThreads, 1)
+gdn_delta_chunk_kernel(const GdnDeltaParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
+  extern __shared__ __align__(128) uint8_t gdn_smem[];
+  GdnChunkSmem& sm = *reinterpret_cast<GdnChunkSmem*>(gdn_smem);
+  const int head = blockIdx.x, s = blockIdx.y;
+  const int n = p.seg.count[s];
+  if (n < kGdnChunk) return;
+  const int row0 = p.seg.row0[s], chunks = (n + kGdnChunk - 1) / kGdnChunk;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kGdnRegsPrepare));
+    constexpr int kTokens = kGdnChunk / 8;               // tokens of a warp
+    const int tid = threadIdx.x & 255, w = warp - 8;
+    const int khead = head / (p.Hv / p.Hk);
+    const __nv_bfloat16* qg = p.qkv + khead * kGdnDim;
+    const __nv_bfloat16* kg = p.qkv + (p.Hk + khead) * kGdnDim;
+    const __nv_bfloat16* vg = p.qkv + (2 * p.Hk + head) * kGdnDim;
+    const float neg_exp_a = -__expf(p.a_log[head]), dtb = p.dt_bias[head];
+    const float4 nw = make_float4(p.norm_w[4 * lane], p.norm_w[4 * lane + 1], p.norm_w[4 * lane + 2], p.norm_w[4 * lane + 3]);
+    __nv_bfloat16 bb = __float2bfloat16(0.f), aa = bb;   // b and a of token `lane` of the chunk to be prepared
+    auto fetch = [&](int i) {                            // rows past the segment's become zeros
+      const int t0 = i * kGdnChunk;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int t = j * 16 + (tid >> 4), col = (tid & 15) * 8;
+        const bool in = t0 + t < n;
+        const size_t r = static_cast<size_t>(row0 + (in ? t0 + t : 0)) * p.ldqkv + col;
+        cp_async16(smem_u32(&sm.raw[0][t * kGdnDim + col]), qg + r, in);
+        cp_async16(smem_u32(&sm.raw[1][t * kGdnDim + col]), kg + r, in);
+        cp_async16(smem_u32(&sm.v[i % 3][t * kGdnDim + col]), vg + r, in);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      if (t0 + lane < n) {
+        const size_t r = static_cast<size_t>(row0 + t0 + lane) * p.ldba + head;
+        bb = p.ba[r];
+        aa = p.ba[r + p.Hv];
+      }
+    };
+    fetch(0);
+    for (int i = 0; i < chunks + 2; ++i) {
+      GdnOperands& op = sm.op[i & 1];
+      if (i >= 2) {
+        // ---- gated RMSNorm of chunk i - 2: a lane has four value rows
+        const int t0 = (i - 2) * kGdnChunk + w * kTokens, here = min(n - t0, kTokens);
+        uint2 z[kTokens];
+#pragma unroll
+        for (int j = 0; j < kTokens; ++j) {
+          z[j] = make_uint2(0u, 0u);
+          if (j < here) z[j] = *reinterpret_cast<const uint2*>(p.z + static_cast<size_t>(row0 + t0 + j) * p.ldz + head * kGdnDim + 4 * lane);
+        }
+        gdn_bar_sync<kGdnChunkThreads>(3 + (i & 1));
+        float ss = op.squares[lane >> 2][w * kTokens + (lane & 3)];                       // lane = warp, token
+#pragma unroll
+        for (int sh = 4; sh < 32; sh <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, sh);
+        const float norm = rsqrtf(ss * (1.f / kGdnDim) + p.eps_norm);
+#pragma unroll
+        for (int j = 0; j < kTokens; ++j) {
+          const float inv = __shfl_sync(0xffffffffu, norm, j);
+          const uint2 x = *reinterpret_cast<const uint2*>(&op.o[w * kTokens + j][4 * lane]);
+          auto gated = [&](uint32_t ow, uint32_t zw, float w0, float w1) {
+            const float2 ob = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ow)), zz = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw));
+            const uint32_t nb = pack_bf16x2(ob.x * inv, ob.y * inv);
+            const float2 normed = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&nb));
+            return pack_bf16x2(normed.x * w0 * silu_fast(zz.x), normed.y * w1 * silu_fast(zz.y));
+          };
+          if (j < here)
+            *reinterpret_cast<uint2*>(p.out + static_cast<size_t>(row0 + t0 + j) * p.ldo + head * kGdnDim + 4 * lane) = make_uint2(gated(x.x, z[j].x, nw.x, nw.y), gated(x.y, z[j].y, nw.z, nw.w));
+        }
+      }
+      if (i >= chunks) continue;
+      float beta = 0.f, decay = 1.f;                     // of token `lane`: every warp has them
+      if (i * kGdnChunk + lane < n) {
+        const float x = __bfloat162float(aa) + dtb;
+        const float softplus = x > 20.f ? x : log1pf(__expf(x));
+        beta = 1.f / (1.f + __expf(-__bfloat162float(bb)));
+        decay = __expf(neg_exp_a * softplus);
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (tid == 0) op.wild = 0;
+      gdn_bar_sync<kGdnPrepareThreads>(5);
+      // ---- operands: normalised q and k (rounded to bf16 as the oracle stores them) in f16; a lane has four channels of the warp's tokens
+      bool wild = !(fabsf(beta) < INFINITY) || !(fabsf(decay) < INFINITY);
+      {
+        constexpr int kRows = 2 * kTokens;               // q and k of every token
+        uint2 x[kRows];
+        float sum[kRows];
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) x[j] = *reinterpret_cast<const uint2*>(&sm.raw[j & 1][(w * kTokens + (j >> 1)) * kGdnDim + 4 * lane]);
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) {
+          const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[j].x)), f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[j].y));
+          sum[j] = fmaf(f0.x, f0.x, f0.y * f0.y) + fmaf(f1.x, f1.x, f1.y * f1.y);
+        }
+        // the sums over the warp, dealt to the lanes: half of them stay with each half of the lanes, three times
+#pragma unroll
+        for (int m = kRows / 2, o = 16; m >= 1; m >>= 1, o >>= 1)
+#pragma unroll
+          for (int j = 0; j < m; ++j) {
+            const bool upper = lane & o;
+            const float send = upper ? sum[j] : sum[j + m], keep = upper ? sum[j + m] : sum[j];
+            sum[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 2);
+        sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 1);
+        wild |= !(sum[0] < INFINITY);                    // an element that is not finite, or too large for its square
+        const float inv = rsqrtf(sum[0] + p.eps_l2);
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) {
+          const float f = __shfl_sync(0xffffffffu, inv, 4 * j);
+          auto norm = [&](uint32_t v) {
+            const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
+            const uint32_t nb = pack_bf16x2(e.x * f, e.y * f);
+            const float2 r = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&nb));
+            return gdn_pack(r.x, r.y);
+          };
+          const int t = w * kTokens + (j >> 1);
+          *reinterpret_cast<uint2*>((j & 1 ? op.k : op.q) + t * 256 + (((lane >> 1) ^ (t & 7)) << 4) + (lane & 1) * 8) = make_uint2(norm(x[j].x), norm(x[j].y));
+        }
+      }
+      {
+        uint32_t top = 0;                                // an exponent of all ones overflows into the sign's place
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint4 x = reinterpret_cast<const uint4*>(sm.v[i % 3])[j * 256 + tid];
+          top |= ((x.x & 0x7F807F80u) + 0x00800080u) | ((x.y & 0x7F807F80u) + 0x00800080u) | ((x.z & 0x7F807F80u) + 0x00800080u) | ((x.w & 0x7F807F80u) + 0x00800080u);
+        }
+        wild |= (top & 0x80008000u) != 0;
+      }
+      if (__any_sync(0xffffffffu, wild) && lane == 0) op.wild = 1;
+      // ---- ratios of the decays, lane = s: products of 1, 2, 4, .. decays behind token s, put together by the bits of the distance
+      {
+        float run[5];
+        const float behind = __shfl_down_sync(0xffffffffu, decay, 1);
+        run[0] = lane < 31 ? behind : 1.f;
+#pragma unroll
+        for (int k = 1; k < 5; ++k) {
+          const float x = __shfl_down_sync(0xffffffffu, run[k - 1], 1 << (k - 1));
+          run[k] = run[k - 1] * (lane + (1 << (k - 1)) < 32 ? x : 1.f);
+        }
+        auto ratio = [&](int t) {
+          const int dist = t - lane;
+          int at = lane;
+          float r = 1.f;
+#pragma unroll
+          for (int k = 0; k < 5; ++k) {
+            const float x = __shfl_sync(0xffffffffu, run[k], at);
+            if (dist >> k & 1) {
+              r *= x;
+              at += 1 << k;
+            }
+          }
+          return dist >= 0 ? r : 0.f;
+        };
+        float r = 0.f;
+#pragma unroll
+        for (int j = 0; j < kTokens; ++j) {
+          r = ratio(w * kTokens + j);
+          sm.ratio[w * kTokens + j][lane] = r;
+        }
+        if (w == 7) {
+          float G = decay;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const float x = __shfl_up_sync(0xffffffffu, G, o);
+            if (lane >= o) G *= x;
+          }
+          op.coef[lane] = make_float4(beta, G, r, decay);
+        }
+      }
+      gdn_bar_sync<kGdnPrepareThreads>(5);
+      if (i + 1 < chunks) fetch(i + 1);
+      // ---- k . k and q . k of the chunk: three blocks x (k, q) x two n-tiles of keys; k . k of the blocks on the diagonal first
+      for (int task = w; task < 12; task += 8) {
+        const int is_q = task >= 6, in = is_q ? task - 6 : task, nt = in & 1, blk = (in >> 1) == 0 ? 0 : (in >> 1) == 1 ? 2 : 1, tb = blk > 0, sb = blk > 1;
+        const uint32_t abase = smem_u32(is_q ? op.q : op.k) + (tb * 16 + (lane & 15)) * 256, bbase = smem_u32(op.k) + (sb * 16 + nt * 8 + (lane & 7)) * 256;
+        float d[2][4] = {};
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          uint32_t a0[4], a1[4], b[4];
+          ldsm4(a0, abase + (((2 * k + (lane >> 4)) ^ (lane & 7)) << 4));
+          ldsm4(a1, abase + (((2 * k + 2 + (lane >> 4)) ^ (lane & 7)) << 4));
+          ldsm4(b, bbase + (((2 * k + (lane >> 3)) ^ (lane & 7)) << 4));
+          gdn_mma(d[0], a0, b[0], b[1]);
+          gdn_mma(d[1], a1, b[2], b[3]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int tr = g + 8 * h, t = tb * 16 + tr, sc = nt * 8 + 2 * c;
+          const float2 ratio = *reinterpret_cast<const float2*>(&sm.ratio[t][sb * 16 + sc]);
+          float x = (d[0][2 * h] + d[1][2 * h]) * ratio.x, y = (d[0][2 * h + 1] + d[1][2 * h + 1]) * ratio.y;
+          const float bt = __shfl_sync(0xffffffffu, beta, t);
+          if (!is_q) {
+            x *= bt;
+            y *= bt;
+            if (blk != 1) {
+              *reinterpret_cast<float2*>(&sm.low[sb][tr][sc]) = make_float2(x, y);        // what is not below the diagonal is not read
+              continue;
+            }
+          }
+          uint32_t hi, lo;
+          gdn_split(x * kGdnUp, y * kGdnUp, hi, lo);
+          __half (&to)[2][16 * 16] = is_q ? op.a[blk] : op.l10;
+          *reinterpret_cast<uint32_t*>(&to[0][gdn_at16(tr, sc)]) = hi;
+          *reinterpret_cast<uint32_t*>(&to[1][gdn_at16(tr, sc)]) = lo;
+        }
+      }
+      gdn_bar_sync<kGdnPrepareThreads>(5);
+      // ---- one warp inverts the blocks on the diagonal: their four 8 x 8 blocks on the diagonal, lane = block, column, then what is left of each,
+      // -inverse x block x inverse
+      if (w == 7) {
+        {
+          const int o = (lane >> 3 & 1) * 8, col = lane & 7;
+          float (&m)[16][16] = sm.low[lane >> 4];
+          float x[8];
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            float l[8];
+#pragma unroll
+            for (int j = 0; j < r; j += 4) *reinterpret_cast<float4*>(l + j) = *reinterpret_cast<const float4*>(&m[o + r][o + j]);
+            float acc = r == col ? 1.f : 0.f, acc2 = 0.f;
+#pragma unroll
+            for (int j = 0; j < r; j += 2) {
+              acc = fmaf(-l[j], x[j], acc);
+              if (j + 1 < r) acc2 = fmaf(-l[j + 1], x[j + 1], acc2);
+            }
+            x[r] = acc + acc2;
+          }
+          __syncwarp();
+#pragma unroll
+          for (int r = 0; r < 8; ++r) m[o + r][o + col] = x[r];
+          __syncwarp();
+        }
+        const int blk = lane >> 4, row = lane >> 1 & 7, half = (lane & 1) * 4;      // a lane has four columns of a row of the lower left block
+        float (&m)[16][16] = sm.low[blk];
+        auto times = [&](const float (&left)[8], int top, int first) {              // left . m[top + ..][first + half ..]
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 y = *reinterpret_cast<const float4*>(&m[top + j][first + half]);
+            acc = make_float4(fmaf(left[j], y.x, acc.x), fmaf(left[j], y.y, acc.y), fmaf(left[j], y.z, acc.z), fmaf(left[j], y.w, acc.w));
+          }
+          return acc;
+        };
+        float left[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) left[j] = m[8 + row][j];
+        const float4 lt = times(left, 0, 0);
+        __syncwarp();
+        *reinterpret_cast<float4*>(&m[8 + row][half]) = lt;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) left[j] = m[8 + row][8 + j];
+        const float4 t = times(left, 8, 0);
+        __syncwarp();
+        auto put = [&](int r, int col, float x, float y) {
+          uint32_t hi, lo;
+          gdn_split(x * kGdnUp, y * kGdnUp, hi, lo);
+          *reinterpret_cast<uint32_t*>(&op.inv[blk][0][gdn_at16(r, col)]) = hi;
+          *reinterpret_cast<uint32_t*>(&op.inv[blk][1][gdn_at16(r, col)]) = lo;
+        };
+        put(8 + row, half, -t.x, -t.y);
+        put(8 + row, half + 2, -t.z, -t.w);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {                    // the blocks on the diagonal, less one, and the zeros beside them
+          const int r = q * 8 + row;
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            const int cl = half + j;
+            put(r, q * 8 + cl, row > cl ? m[r][q * 8 + cl] : 0.f, row > cl + 1 ? m[r][q * 8 + cl + 1] : 0.f);
+            if (q == 0) put(r, 8 + cl, 0.f, 0.f);
+          }
+        }
+      }
+      gdn_bar_arrive<kGdnChunkThreads>(1 + (i & 1));
+    }
+    return;
+  }
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kGdnRegsWalk));
+  float* sp = p.state + ((static_cast<size_t>(p.seg.slot[s]) * p.Hv + head) * kGdnDim + warp * 16 + g) * kGdnDim + 2 * c;
+  float S[16][4];                                        // [8 key columns][rows g: 2 c, 2 c + 1; rows g + 8: the same]
+  const bool resumed = p.seg.pos0[s] > 0;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    float2 x = make_float2(0.f, 0.f), y = x;
+    if (resumed) {
+      x = *reinterpret_cast<const float2*>(sp + 8 * j);
+      y = *reinterpret_cast<const float2*>(sp + 8 * kGdnDim + 8 * j);
+    }
+    S[j][0] = x.x; S[j][1] = x.y; S[j][2] = y.x; S[j][3] = y.y;
+  }
+  for (int i = 0; i < chunks; ++i) {
+    GdnOperands& op = sm.op[i & 1];
+    const __nv_bfloat16* vs = sm.v[i % 3] + warp * 16 + g;
+    float o[2][2][4];                                    // [16 tokens][n-tile][value rows g, g + 8 x tokens 2 c, 2 c + 1], without 1 / sqrt(d_k)
+    gdn_bar_sync<kGdnChunkThreads>(1 + (i & 1));
+    if (!op.wild) {
+      // ---- S k and S q
+      float u[2][2][4];
+      float down;
+      {
+        float x[2][2][4];
+        uint32_t most = 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) most = max(most, gdn_bits(S[j][q]));
+        const int e = gdn_exponent(most);
+        const float up = gdn_pow2(13 - e);
+        down = gdn_pow2(e - 13);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) u[h][j][q] = o[h][j][q] = x[h][j][q] = 0.f;
+        const int brow = (lane & 7) + ((lane >> 4) << 3);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          uint32_t hi[4], lo[4];
+          gdn_split(S[2 * k][0] * up, S[2 * k][1] * up, hi[0], lo[0]);
+          gdn_split(S[2 * k][2] * up, S[2 * k][3] * up, hi[1], lo[1]);
+          gdn_split(S[2 * k + 1][0] * up, S[2 * k + 1][1] * up, hi[2], lo[2]);
+          gdn_split(S[2 * k + 1][2] * up, S[2 * k + 1][3] * up, hi[3], lo[3]);
+          const uint32_t at = brow * 256 + (((2 * k + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t bk[4], bq[4];
+            ldsm4(bk, smem_u32(op.k) + at + h * 16 * 256);
+            ldsm4(bq, smem_u32(op.q) + at + h * 16 * 256);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              gdn_mma(x[h][j], lo, bk[2 * j], bk[2 * j + 1]);
+              gdn_mma(o[h][j], lo, bq[2 * j], bq[2 * j + 1]);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              gdn_mma(x[h][j], hi, bk[2 * j], bk[2 * j + 1]);
+              gdn_mma(o[h][j], hi, bq[2 * j], bq[2 * j + 1]);
+            }
+            if (k & 1) {                                 // the tensor cores cut their sums off: short ones, added here
+#pragma unroll
+              for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                  u[h][j][r] += x[h][j][r];
+                  x[h][j][r] = 0.f;
+                }
+            }
+          }
+        }
+      }
+      // ---- beta (v - G S k), G S q
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int t = h * 16 + j * 8 + 2 * c + q;
+            const float2 bg = *reinterpret_cast<const float2*>(&op.coef[t]);
+            const float f = down * bg.y;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              u[h][j][2 * r + q] = fmaf(-u[h][j][2 * r + q], f, __bfloat162float(vs[t * kGdnDim + 8 * r])) * bg.x;
+              o[h][j][2 * r + q] *= f;
+            }
+          }
+      // ---- Delta (in place of u) of tokens 0..15, then of 16..31
+      uint32_t hi[4], lo[4];
+      float d[2][4];
+      auto add = [&](float (&x)[2][4], float f) {        // x += f d
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[j][q] = fmaf(f, d[j][q], x[j][q]);
+      };
+      constexpr float kDown = 1.f / kGdnUp;
+      float f = gdn_operand(u[0], hi, lo) * kDown;
+      gdn_block(d, hi, lo, op.inv[0], lane);
+      add(u[0], f);
+      f = gdn_operand(u[0], hi, lo) * kDown;
+      gdn_block(d, hi, lo, op.l10, lane);
+      add(u[1], -f);
+      gdn_block(d, hi, lo, op.a[0], lane);
+      add(o[0], f);
+      gdn_block(d, hi, lo, op.a[1], lane);
+      add(o[1], f);
+      f = gdn_operand(u[1], hi, lo) * kDown;
+      gdn_block(d, hi, lo, op.inv[1], lane);
+      add(u[1], f);
+      f = gdn_operand(u[1], hi, lo) * kDown;
+      gdn_block(d, hi, lo, op.a[2], lane);
+      add(o[1], f);
+      // ---- the state: G_end S plus the products of the chunk, which the tensor cores sum from zero
+      const float end = op.coef[kGdnChunk - 1].y;
+      uint32_t first[2][4], second[2][4], third[2][4], most = 0;
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float r0 = op.coef[b * 16 + j * 8 + 2 * c].z, r1 = op.coef[b * 16 + j * 8 + 2 * c + 1].z;
+          u[b][j][0] *= r0; u[b][j][1] *= r1;
+          u[b][j][2] *= r0; u[b][j][3] *= r1;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) most = max(most, gdn_bits(u[b][j][q]));
+        }
+      const int e = gdn_exponent(most);
+      const float up = gdn_pow2(13 - e), fs = gdn_pow2(e - 13);
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int at = 2 * j + r;
+            float x = u[b][j][2 * r] * up, y = u[b][j][2 * r + 1] * up;
+            const uint32_t coarse = pack_bf16x2(x, y);
+            first[b][at] = gdn_pack(__uint_as_float(coarse << 16), __uint_as_float(coarse & 0xFFFF0000u));
+            const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&first[b][at]));
+            x -= f2.x;
+            y -= f2.y;
+            gdn_split(x, y, second[b][at], third[b][at]);
+          }
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        uint32_t kb[2][4];                               // (tokens 0, columns 0) (tokens 8, columns 0) (tokens 0, columns 8) (tokens 8, columns 8)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const int t = b * 16 + (lane & 15);
+          ldsm4_t(kb[b], smem_u32(op.k) + t * 256 + (((j + (lane >> 4)) ^ (t & 7)) << 4));
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          // products of the first parts have 16 bits: kept apart from the rest, 2^-8 of them, their sum loses next to nothing
+          float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            gdn_mma(x, first[b], kb[b][2 * q], kb[b][2 * q + 1]);
+            gdn_mma(y, third[b], kb[b][2 * q], kb[b][2 * q + 1]);
+            gdn_mma(y, second[b], kb[b][2 * q], kb[b][2 * q + 1]);
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) S[j + q][r] = fmaf(fs, x[r], fmaf(fs, y[r], S[j + q][r] * end));
+        }
+      }
+    } else {
+      // ---- token by token
+#pragma unroll 1
+      for (int t = 0; t < kGdnChunk; ++t) {
+        const float4 co = op.coef[t];
+        float m0 = 0.f, m1 = 0.f, r0 = 0.f, r1 = 0.f, kq = 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int at = t * 256 + ((j ^ (t & 7)) << 4) + c * 4;
+          const float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + at)), q = __half22float2(*reinterpret_cast<const __half2*>(op.q + at));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) S[j][i] *= co.w;
+          m0 = fmaf(S[j][0], k.x, fmaf(S[j][1], k.y, m0));
+          m1 = fmaf(S[j][2], k.x, fmaf(S[j][3], k.y, m1));
+          r0 = fmaf(S[j][0], q.x, fmaf(S[j][1], q.y, r0));
+          r1 = fmaf(S[j][2], q.x, fmaf(S[j][3], q.y, r1));
+          kq = fmaf(k.x, q.x, fmaf(k.y, q.y, kq));
+        }
+#pragma unroll
+        for (int sh = 1; sh < 4; sh <<= 1) {
+          m0 += __shfl_xor_sync(0xffffffffu, m0, sh);
+          m1 += __shfl_xor_sync(0xffffffffu, m1, sh);
+          r0 += __shfl_xor_sync(0xffffffffu, r0, sh);
+          r1 += __shfl_xor_sync(0xffffffffu, r1, sh);
+          kq += __shfl_xor_sync(0xffffffffu, kq, sh);
+        }
+        const float d0 = (__bfloat162float(vs[t * kGdnDim]) - m0) * co.x, d1 = (__bfloat162float(vs[t * kGdnDim + 8]) - m1) * co.x;
+        r0 = fmaf(d0, kq, r0);
+        r1 = fmaf(d1, kq, r1);
+        if (i * kGdnChunk + t < n) {                     // behind the segment's end nothing happens to the state
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + t * 256 + ((j ^ (t & 7)) << 4) + c * 4));
+            S[j][0] = fmaf(d0, k.x, S[j][0]); S[j][1] = fmaf(d0, k.y, S[j][1]);
+            S[j][2] = fmaf(d1, k.x, S[j][2]); S[j][3] = fmaf(d1, k.y, S[j][3]);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+              if (h * 16 + j * 8 + 2 * c + q == t) { o[h][j][q] = r0; o[h][j][2 + q] = r1; }
+      }
+    }
+    // ---- outputs (stored in bf16 by the oracle) and the warp's sums of their squares
+    float sq[2][2][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int t = h * 16 + j * 8 + 2 * c + q;
+          const __nv_bfloat16 x = __float2bfloat16(o[h][j][q] * 0.08838834764831845f), y = __float2bfloat16(o[h][j][2 + q] * 0.08838834764831845f);
+          op.o[t][warp * 16 + g] = x;
+          op.o[t][warp * 16 + g + 8] = y;
+          const float xf = __bfloat162float(x), yf = __bfloat162float(y);
+          sq[h][j][q] = fmaf(xf, xf, yf * yf);
+        }
+#pragma unroll
+    for (int sh = 4; sh < 32; sh <<= 1)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) sq[h][j][q] += __shfl_xor_sync(0xffffffffu, sq[h][j][q], sh);
+    if (g == 0) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) *reinterpret_cast<float2*>(&op.squares[warp][h * 16 + j * 8 + 2 * c]) = make_float2(sq[h][j][0], sq[h][j][1]);
+    }
+    gdn_bar_arrive<kGdnChunkThreads>(3 + (i & 1));
+  }
+  if (!p.commit) return;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    *reinterpret_cast<float2*>(sp + 8 * j) = make_float2(S[j][0], S[j][1]);
+    *reinterpret_cast<float2*>(sp + 8 * kGdnDim + 8 * j) = make_float2(S[j][2], S[j][3]);
+  }
+}
+
 // out = x * sigmoid(gate): the output gate of the hybrid family's full-attention layers (bf16, in place allowed)
 __global__ void __launch_bounds__(256)
 sigmoid_gate_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ gate, int ldg,
@@ -436,6 +1084,7 @@ struct CbGdnDelta {
   int Hk, Hv;
   float eps_norm, eps_l2;
   int commit;
+  int longest;      // rows of the longest segment, or a bound of them (the rows of the step)
 };
 
 int cb_gdn_delta(const CbGdnDelta* a, const CbGdnSegments* seg, void* stream) {
@@ -454,6 +1103,28 @@ int cb_gdn_delta(const CbGdnDelta* a, const CbGdnSegments* seg, void* stream) {
   p.commit = a->commit;
   p.seg = cb::GdnSegments{static_cast<const int*>(seg->row0), static_cast<const int*>(seg->count),
                           static_cast<const int*>(seg->slot), static_cast<const int*>(seg->pos0)};
+  // Segments of a chunk and more go to the kernel of chunks; what is shorter keeps the bits that its rows have one by one (speculative rounds).  The
+  // chunks read rows in 16 bytes and write outputs and states in eight.
+  auto aligned = [](const void* x, int ld, int bytes) { return (reinterpret_cast<uintptr_t>(x) | static_cast<uintptr_t>(2ll * ld)) % bytes == 0; };
+  const bool chunks = a->longest >= cb::kGdnChunk && aligned(a->qkv, a->ldqkv, 16) && aligned(a->z, a->ldz, 8) && aligned(a->out, a->ldo, 8) && reinterpret_cast<uintptr_t>(a->state) % 8 == 0;
+  p.most = chunks ? cb::kGdnChunk - 1 : INT_MAX;
+  if (chunks) {
+    static bool configured[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -18;
+    if (!configured[dev]) {
+      const cudaError_t e = cudaFuncSetAttribute(cb::gdn_delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(cb::GdnChunkSmem)));
+      if (e != cudaSuccess) return static_cast<int>(e);
+      // the warps' new shares come out of the registers that the block was launched with
+      cudaFuncAttributes at;
+      const cudaError_t e2 = cudaFuncGetAttributes(&at, cb::gdn_delta_chunk_kernel);
+      if (e2 != cudaSuccess) return static_cast<int>(e2);
+      if (at.numRegs < cb::kGdnRegs) return -19;
+      configured[dev] = true;
+    }
+    const cudaError_t e = cb::launch(cb::gdn_delta_chunk_kernel, dim3(a->Hv, seg->num), dim3(cb::kGdnChunkThreads), sizeof(cb::GdnChunkSmem), static_cast<cudaStream_t>(stream), p);
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
   dim3 grid(a->Hv, seg->num);
   cb::gdn_delta_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return static_cast<int>(cudaGetLastError());

@@ -330,7 +330,7 @@ class BatchBuilder:
                          rb_qstart=d["rb_qstart"], rb_qcount=d["rb_qcount"], rb_ctx=d["rb_ctx"],
                          logit_rows=d["logit_rows"], attn_splits=splits,
                          attn_decode=decode, attn_prompts=prompts,
-                         segments=K.GdnSegments(d["seg_row0"], d["seg_count"], d["seg_slot"], d["seg_pos0"], nseg),
+                         segments=K.GdnSegments(d["seg_row0"], d["seg_count"], d["seg_slot"], d["seg_pos0"], nseg, max((len(s.token_ids) for s in segs), default=1)),
                          positions_hw=(d["positions_h"], d["positions_w"]) if axes else None,
                          embeds=[(first, feat.to(self.device, torch.bfloat16, non_blocking=True))
                                  for first, feat in embeds] or None), rows

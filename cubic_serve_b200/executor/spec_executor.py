@@ -423,7 +423,7 @@ class SpeculativeGpuExecutor(GpuExecutor):
             i32 = dict(dtype=torch.int32, device=dev)
             fold = K.GdnSegments(torch.arange(R, **i32) * (Kd + 1), (self.accepted[:R] + 1).to(torch.int32),
                                  torch.tensor([s.request_slot for s in segs], **i32),
-                                 torch.tensor([s.start for s in segs], **i32), R)
+                                 torch.tensor([s.start for s in segs], **i32), R, Kd + 1)
             self._fold_launches = r.fold_gdn(fold, T)
         return hidden
 

@@ -741,12 +741,14 @@ def moe_combine(y: torch.Tensor, sc: MoeScratch, tokens: int, out: torch.Tensor,
 @dataclass
 class GdnSegments:
     """A step's token rows grouped by request: rows ``[row0, row0 + count)`` of state slot ``slot``, the first at
-    absolute position ``pos0`` (0 = the request starts here, from zero state).  int32 device tensors of length >= num."""
+    absolute position ``pos0`` (0 = the request starts here, from zero state).  int32 device tensors of length >= num.
+    ``longest``: a bound of the counts, if the caller knows one below the rows of the step (0: it does not)."""
     row0: torch.Tensor
     count: torch.Tensor
     slot: torch.Tensor
     pos0: torch.Tensor
     num: int
+    longest: int = 0
 
     def struct(self) -> "native.GdnSegmentsStruct":
         s = native.GdnSegmentsStruct()
@@ -787,6 +789,7 @@ def gdn_delta(qkv: torch.Tensor, z: torch.Tensor, ba: torch.Tensor, a_log: torch
     d.a_log, d.dt_bias, d.norm_w, d.state = a_log.data_ptr(), dt_bias.data_ptr(), norm_w.data_ptr(), state.data_ptr()
     d.out, d.ldo, d.Hk, d.Hv, d.eps_norm, d.eps_l2 = out.data_ptr(), out.stride(0), hk, hv, eps_norm, eps_l2
     d.commit = int(commit)
+    d.longest = int(seg.longest or qkv.shape[0])
     st = seg.struct()
     native.check(native.lib().cb_gdn_delta(ctypes.byref(d), ctypes.byref(st), _stream()), "cb_gdn_delta")
     return out

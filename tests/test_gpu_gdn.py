@@ -79,6 +79,84 @@ def test_gdn_delta_matches_oracle_and_chunks_compose(hk, hv):
     assert torch.equal(out2, out[:6]) and torch.equal(st2[3], st_dev[3])
 
 
+def _delta_case(counts, pos0, hk, hv, seed):
+    g = torch.Generator().manual_seed(seed)
+    T = sum(counts)
+    qkv = (torch.randn(T, (2 * hk + hv) * 128, generator=g) * 0.7).to(torch.bfloat16).to(DEV)
+    z = torch.randn(T, hv * 128, generator=g).to(torch.bfloat16).to(DEV)
+    ba = torch.randn(T, 2 * hv, generator=g).to(torch.bfloat16).to(DEV)
+    a_log, dt_bias = (torch.randn(hv, generator=g).to(DEV) * 0.5 - 2 * (seed % 2) for _ in range(2))
+    norm_w = 1 + 0.1 * torch.randn(128, generator=g).to(DEV)
+    state = torch.randn(len(counts), hv, 128, 128, generator=g).to(DEV) * 0.05
+    return qkv, z, ba, a_log, dt_bias, norm_w, state
+
+
+def _delta(case, counts, pos0, hk, hv, at_once):
+    """Segments whole, or ``at_once`` rows a launch: 31 and fewer are walked row by row."""
+    from cubic_serve_b200.ops import kernels as K
+    qkv, z, ba, a_log, dt_bias, norm_w, state = case
+    state, out = state.clone(), torch.full((qkv.shape[0], hv * 128), 9.0, dtype=torch.bfloat16, device=DEV)
+    if at_once is None:
+        K.gdn_delta(qkv, z, ba, a_log, dt_bias, norm_w, state, _segments(K, counts, list(range(len(counts))), pos0), out, hk, hv)
+        return out, state
+    r = 0
+    for i, n in enumerate(counts):
+        for o in range(0, n, at_once):
+            e = slice(r + o, r + min(n, o + at_once))
+            K.gdn_delta(qkv[e], z[e], ba[e], a_log, dt_bias, norm_w, state, _segments(K, [e.stop - e.start], [i], [pos0[i] + o]), out[e], hk, hv)
+        r += n
+    return out, state
+
+
+@pytest.mark.parametrize("hk,hv", [(1, 1), (2, 6)])
+@pytest.mark.parametrize("counts", [[32], [31, 33, 1, 0, 64], [63, 65, 5, 331]])
+def test_gdn_delta_chunks(hk, hv, counts):
+    """Segments in chunks of 32 against the row-by-row kernel: sums of 2^-24 each in another order, up to a hundred of which add up."""
+    pos0 = [7 * (i % 2) for i in range(len(counts))]
+    for seed in (0, 1):
+        case = _delta_case(counts, pos0, hk, hv, seed)
+        out, state = _delta(case, counts, pos0, hk, hv, None)
+        want, want_state = _delta(case, counts, pos0, hk, hv, 31)
+        assert _rel(out, want) < 2e-3                       # some results round to the other bf16
+        r = 0
+        for i, n in enumerate(counts):
+            assert _rel(state[i], want_state[i]) < 2.0 ** -18
+            if n < 32:
+                assert torch.equal(out[r:r + n], want[r:r + n]) and torch.equal(state[i], want_state[i])
+            r += n
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "beta"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_gdn_delta_chunks_keep_what_is_not_finite_behind_it(what, bad):
+    """Rows before the one that is not finite, and other segments, have the bits that they have without it; the rest as row by row."""
+    counts, pos0, hk, hv, at = [70, 40], [0, 0], 1, 2, 45
+    case = _delta_case(counts, pos0, hk, hv, 0)
+    clean, _ = _delta(case, counts, pos0, hk, hv, None)
+    column = {"q": 3, "k": 128 + 3, "v": 256 + 3}
+    (case[2] if what == "beta" else case[0])[at, column.get(what, 0)] = bad
+    out, state = _delta(case, counts, pos0, hk, hv, None)
+    want, want_state = _delta(case, counts, pos0, hk, hv, 31)
+    assert torch.equal(out[:32], clean[:32]) and torch.equal(out[70:], clean[70:])
+    assert _rel(out[32:at], clean[32:at]) < 2e-3
+    assert torch.equal(torch.isfinite(out), torch.isfinite(want)) and torch.equal(torch.isfinite(state), torch.isfinite(want_state))
+
+
+def test_gdn_delta_chunks_of_rows_that_are_not_aligned():
+    """Rows that start anywhere are walked one by one; a review pass leaves the state."""
+    from cubic_serve_b200.ops import kernels as K
+    counts, hk, hv = [50], 1, 2
+    case = _delta_case(counts, [0], hk, hv, 3)
+    wide = torch.zeros(50, 4 * 128 + 1, dtype=torch.bfloat16, device=DEV)
+    wide[:, 1:] = case[0]
+    a, sa = _delta((wide[:, 1:], *case[1:]), counts, [0], hk, hv, None)
+    b, sb = _delta(case, counts, [0], hk, hv, 31)
+    assert torch.equal(a, b) and torch.equal(sa, sb)
+    state, out = case[6].clone(), torch.empty_like(a)
+    K.gdn_delta(*case[:6], state, _segments(K, counts, [0], [0]), out, hk, hv, commit=False)
+    assert torch.equal(state, case[6]) and _rel(out, b) < 2e-3
+
+
 def test_sigmoid_gate():
     from cubic_serve_b200.ops import kernels as K
     x = torch.randn(37, 256).to(torch.bfloat16).to(DEV)
