@@ -19,7 +19,8 @@
 //
 // Measured, weights not in L2 (floor = packed bytes / 6.65 TB/s), Cubic weights, 8 rows: 24576 x 4096 22.3 us (floor 9.5, tcgen05
 // kernels 34), 4096 x 12288 12.8 (4.7, 21.5), 6144 x 4096 9.1 (2.4, 14.8), 4096 x 4096 6.4 (1.6, 10.1); bf16 50688 x 4096 65 (62,
-// 98).  What is left above the floor is the decode (integer pipe 38 % busy, four warps a scheduler that issue in 37 % of the cycles) and
+// 98).  Block-scaled e4m3 weights have nothing to decode either: their chunks and those of the e4m3 activations are the operands of m16n8k32;
+// 128 experts of 3072 x 4096, eight rows each, 267 us (floor 246, tcgen05 kernel 409), 4096 x 1536 145 (123, 289).  What is left above the floor is the decode (integer pipe 38 % busy, four warps a scheduler that issue in 37 % of the cycles) and
 // 5 us of start, last loads and the sum of the parts.
 #include "wq_gemm_common.cuh"
 #include "launch.cuh"
@@ -35,22 +36,23 @@ struct SkinnyParams {
   WqGemmParams g;
   int its;                    // iterations of a tile: K / columns of an iteration
   int grid;
+  int experts;                // fp8: stacked matrices
 };
 
 template <int FMT, int NB>
 struct SnShape {
-  static constexpr bool kBf16 = FMT == kFmtBf16;
+  static constexpr bool kBf16 = FMT == kFmtBf16, kFp8 = FMT == kFmtFp8Block, kDirect = kBf16 || kFp8;     // direct: weights as [N, K] rows
   static constexpr int kRows = NB * 8;
   static constexpr int kCols = kBf16 ? 64 : 128;                // K columns of a warp and iteration
   static constexpr int kSteps = kCols / 32;                     // eight columns of every row and lane at a time
-  static constexpr int kXTile = kRows * 128;                    // 64 columns
-  static constexpr int kXBytes = 2 * kCols / 64 * kXTile;
+  static constexpr int kXTile = kRows * 128, kXTileCols = kFp8 ? 128 : 64;
+  static constexpr int kXBytes = 2 * kCols / kXTileCols * kXTile;
   static constexpr int kSeg = kTileN * 16 + 64;                 // 32 columns of the tile's codes
-  static constexpr int kCodes = kBf16 ? 2 * kATileBytes : 8 * kSeg;
+  static constexpr int kCodes = kDirect ? 2 * kATileBytes : 8 * kSeg;
   static constexpr int kMetaSeg = FMT == kFmtCubic4 ? kMetaBytesCubic : kTileN * 4 + 32;
-  static constexpr int kMetaSegs = kBf16 ? 0 : FMT == kFmtCubic4 ? 2 : 8;
+  static constexpr int kMetaSegs = kDirect ? 0 : FMT == kFmtCubic4 ? 2 : 8;
   static constexpr int kStage = (kXBytes + kCodes + kMetaSegs * kMetaSeg + 1023) & ~1023;
-  static constexpr uint32_t kTx = kXBytes + (kBf16 ? 2 * kATileBytes : 4 * kCodeBytes + (FMT == kFmtCubic4 ? 2 * kMetaBytesCubic : 4 * kMetaBytes));
+  static constexpr uint32_t kTx = kXBytes + (kDirect ? 2 * kATileBytes : 4 * kCodeBytes + (FMT == kFmtCubic4 ? 2 * kMetaBytesCubic : 4 * kMetaBytes));
   static constexpr int kRed = kRows * kSnRedStride * 4;
   static constexpr int kFit = (112 * 1024 - 1024 - 128 - kRed) / kStage;      // two CTAs per SM
   static constexpr int kStages = kFit > kSnMaxStages ? kSnMaxStages : kFit;
@@ -61,6 +63,13 @@ struct SnShape {
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -139,6 +148,9 @@ __device__ __forceinline__ void sn_load_weights(const SkinnyParams& p, const CUt
   if constexpr (Sh::kBf16) {
 #pragma unroll
     for (int kg = 0; kg < 2; ++kg) tma_load_2d(dst + kg * kATileBytes, tw, (it * 2 + kg) * 64, s.n_tile * kTileN, bar);
+  } else if constexpr (Sh::kFp8) {
+#pragma unroll
+    for (int kg = 0; kg < 2; ++kg) tma_load_2d(dst + kg * kATileBytes, tw, (it * 2 + kg) * 128, (s.expert * p.g.n_tiles + s.n_tile) * kTileN, bar);
   } else {
     const int kb = it * 4;
     const uint8_t* src = p.g.codes + s.expert * p.g.group_code_stride + (static_cast<size_t>(s.n_tile) * p.g.k_blocks + kb) * kCodeBytes;
@@ -161,7 +173,7 @@ template <int FMT, int NB>
 __device__ __forceinline__ void sn_load_x(const CUtensorMap* tx, const SnSegment& s, int it, uint32_t stage, uint32_t bar) {
   using Sh = SnShape<FMT, NB>;
 #pragma unroll
-  for (int i = 0; i < 2 * Sh::kCols / 64; ++i) tma_load_2d(stage + i * Sh::kXTile, tx, it * 2 * Sh::kCols + i * 64, s.m0, bar);
+  for (int i = 0; i < 2 * Sh::kCols / Sh::kXTileCols; ++i) tma_load_2d(stage + i * Sh::kXTile, tx, it * 2 * Sh::kCols + i * Sh::kXTileCols, s.m0, bar);
 }
 
 __device__ __forceinline__ uint4 lds16(uint32_t a) {
@@ -247,6 +259,45 @@ __device__ __forceinline__ void sn_compute(float (&acc)[2][NB][4], uint32_t stag
         }
     }
   }
+}
+
+// One iteration of a warp with e4m3 weights and activations: the 128 columns of its half are a scale block, whose product is summed from zero
+// and joins the accumulators times the block's scale.  Lane t takes the chunks 2 t and 2 t + 1 of every row.
+template <int NB>
+__device__ __forceinline__ void sn_compute_fp8(float (&acc)[2][NB][4], uint32_t stage, int nb_used, int rg, int kg, int g, int t, float scale) {
+  using Sh = SnShape<kFmtFp8Block, NB>;
+  const uint32_t arow = stage + Sh::kXBytes + kg * kATileBytes + (rg * 32 + g) * 128, xa = stage + kg * Sh::kXTile + g * 128;
+  float part[2][NB][4];
+#pragma unroll
+  for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) part[rt][nb][c] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t o = ((2 * t + j) ^ g) << 4;
+    uint4 b[NB];
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb)
+      if (NB == 1 || nb < nb_used) b[nb] = lds16(xa + nb * 1024 + o);
+#pragma unroll
+    for (int rt = 0; rt < 2; ++rt) {
+      const uint4 l = lds16(arow + 2 * rt * 1024 + o), u = lds16(arow + (2 * rt + 1) * 1024 + o);
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+        if (NB == 1 || nb < nb_used) {
+          mma_e4m3(part[rt][nb], l.x, u.x, l.y, u.y, b[nb].x, b[nb].y);
+          mma_e4m3(part[rt][nb], l.z, u.z, l.w, u.w, b[nb].z, b[nb].w);
+        }
+    }
+  }
+#pragma unroll
+  for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[rt][nb][c] = fmaf(scale, part[rt][nb][c], acc[rt][nb][c]);
 }
 
 __device__ __forceinline__ void sn_bar() { asm volatile("bar.sync 1, %0;" ::"r"(kSnConsumers) : "memory"); }
@@ -352,15 +403,27 @@ wq_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[r][n][c] = 0.f;
     const int nb_used = (seg.rows + 7) >> 3;
+    const float* block_scale = nullptr;
+    if constexpr (Sh::kFp8) block_scale = p.g.row_scale + (static_cast<size_t>(seg.expert) * p.g.n_tiles + seg.n_tile) * p.g.k_blocks + kg;
     for (int it = seg.it; it < seg.it_end; ++it) {
+      float scale = 0.f;
+      if constexpr (Sh::kFp8) scale = __ldg(block_scale + 2 * it);
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait_park(smem_u32(&full[slot]), phase, abort_flag));
-      sn_compute<FMT, NB>(acc, ring + slot * Sh::kStage, nb_used, rg, kg, g, t);
+      if constexpr (Sh::kFp8) sn_compute_fp8<NB>(acc, ring + slot * Sh::kStage, nb_used, rg, kg, g, t, scale);
+      else sn_compute<FMT, NB>(acc, ring + slot * Sh::kStage, nb_used, rg, kg, g, t);
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&empty[slot]));
       if (++slot == S) { slot = 0; phase ^= 1u; }
     }
     // the two column halves meet in shared memory as [batch row][feature]
     float* mine = red + (2 * t) * kSnRedStride + rg * 32 + g;
+    float xs[NB][2];                           // scales of the activation rows
+    if constexpr (Sh::kFp8) {
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) xs[nb][c] = nb * 8 + 2 * t + c < seg.rows ? p.g.col_scale[seg.m0 + nb * 8 + 2 * t + c] : 0.f;
+    }
     auto each = [&](auto&& f) {
 #pragma unroll
       for (int rt = 0; rt < 2; ++rt)
@@ -368,7 +431,7 @@ wq_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         for (int nb = 0; nb < NB; ++nb)
           if (NB == 1 || nb < nb_used)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) f(mine[(nb * 8 + (c & 1)) * kSnRedStride + rt * 16 + (c >> 1) * 8], acc[rt][nb][c]);
+            for (int c = 0; c < 4; ++c) f(mine[(nb * 8 + (c & 1)) * kSnRedStride + rt * 16 + (c >> 1) * 8], acc[rt][nb][c] * (Sh::kFp8 ? xs[nb][c & 1] : 1.f));
     };
     sn_bar();                                  // the previous segment's sums have been read: nothing else holds a warp back that is a run ahead
     if (kg == 1) each([](float& m, float v) { m = v; });
@@ -413,8 +476,9 @@ template <int FMT, int NB>
 static int launch_skinny(SkinnyParams p, const void* x, int ldx, int max_grid, cudaStream_t stream) {
   using Sh = SnShape<FMT, NB>;
   CUtensorMap tx, tw;
-  if (make_tmap_bf16(&tx, x, p.g.M, p.g.K, ldx, Sh::kRows) != 0) return -20;
+  if ((Sh::kFp8 ? make_tmap_u8(&tx, x, p.g.M, p.g.K, ldx, Sh::kRows) : make_tmap_bf16(&tx, x, p.g.M, p.g.K, ldx, Sh::kRows)) != 0) return -20;
   tw = tx;
+  if (Sh::kFp8 && make_tmap_u8(&tw, p.g.codes, static_cast<uint64_t>(p.g.N) * p.experts, p.g.K, p.g.K, kTileN) != 0) return -21;
   if (FMT == kFmtBf16 && make_tmap_bf16(&tw, p.g.codes, p.g.N, p.g.K, p.g.K, kTileN) != 0) return -21;
   static bool configured[64] = {};
   int dev = 0;
@@ -447,9 +511,10 @@ static int launch_skinny_rows(const SkinnyParams& p, const void* x, int ldx, int
 
 static int skinny(int fmt, const void* x, int ldx, const void* codes, const void* meta, void* y, int ldy, const void* residual, float alpha, int M, int N, int K,
                   int group_k, int swiglu, const void* tiles, int rows, size_t code_stride, size_t meta_stride, void* workspace, long long workspace_bytes,
-                  void* counters, void* status, void* stream) {
-  if (fmt != kFmtBf16 && fmt != kFmtCubic4 && fmt != kFmtAffine4 && fmt != kFmtNvfp4) return -11;
-  if (M <= 0 || N <= 0 || K <= 0 || K % (fmt == kFmtBf16 ? 128 : 256) != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return -10;
+                  void* counters, void* status, void* stream, const void* x_scale = nullptr, int experts = 1) {
+  if (fmt != kFmtBf16 && fmt != kFmtCubic4 && fmt != kFmtAffine4 && fmt != kFmtNvfp4 && fmt != kFmtFp8Block) return -11;
+  if (M <= 0 || N <= 0 || K <= 0 || K % (fmt == kFmtBf16 ? 128 : 256) != 0 || ldx % (fmt == kFmtFp8Block ? 16 : 8) != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return -10;
+  if (fmt == kFmtFp8Block && (!x_scale || !meta || swiglu || (reinterpret_cast<uintptr_t>(codes) & 15) != 0 || experts <= 0 || (tiles && N % kTileN != 0))) return -15;
   if (fmt == kFmtCubic4 && group_k % 128 != 0) return -12;
   if (rows <= 0 || rows > 32) return -17;
   if (swiglu && (residual || (N % 32) != 0 || ldy < N / 2)) return -51;
@@ -467,7 +532,10 @@ static int skinny(int fmt, const void* x, int ldx, const void* codes, const void
   p.g.status = static_cast<uint32_t*>(status);
   p.g.M = M; p.g.N = N; p.g.K = K; p.g.ldy = ldy; p.g.alpha = alpha;
   p.g.swiglu = swiglu;
-  p.g.k_blocks = K / kBlockK;
+  p.experts = experts;
+  p.g.row_scale = static_cast<const float*>(meta);
+  p.g.col_scale = static_cast<const float*>(x_scale);
+  p.g.k_blocks = K / (fmt == kFmtFp8Block ? 128 : kBlockK);
   p.g.meta_k_blocks = fmt == kFmtCubic4 ? group_k / kBlockK : 1;
   p.g.meta_blocks = (p.g.k_blocks + p.g.meta_k_blocks - 1) / p.g.meta_k_blocks;
   p.g.n_tiles = (N + kTileN - 1) / kTileN;
@@ -485,6 +553,7 @@ static int skinny(int fmt, const void* x, int ldx, const void* codes, const void
     case kFmtCubic4: return launch_skinny_rows<kFmtCubic4>(p, x, ldx, rows, max_grid, st);
     case kFmtAffine4: return launch_skinny_rows<kFmtAffine4>(p, x, ldx, rows, max_grid, st);
     case kFmtNvfp4: return launch_skinny_rows<kFmtNvfp4>(p, x, ldx, rows, max_grid, st);
+    case kFmtFp8Block: return launch_skinny_rows<kFmtFp8Block>(p, x, ldx, rows, max_grid, st);
     default: return launch_skinny_rows<kFmtBf16>(p, x, ldx, rows, max_grid, st);
   }
 }
@@ -503,9 +572,21 @@ int cb_wq_gemm_skinny(int fmt, const void* x, int ldx, const void* codes, const 
 // The grouped form over a device work list {count, then {expert, first row, rows}}: `rows` (<= 32) rows of an item at a time.
 int cb_wq_gemm_skinny_grouped(int fmt, const void* x, int ldx, const void* codes, const void* meta, void* y, int ldy, float alpha, int total_rows, int N, int K,
                               int group_k, int swiglu, const void* tiles, int rows, long long code_stride, long long meta_stride, void* status, void* stream) {
-  if (!tiles || fmt == cb::kFmtBf16) return -40;
+  if (!tiles || fmt == cb::kFmtBf16 || fmt == cb::kFmtFp8Block) return -40;
   return cb::skinny(fmt, x, ldx, codes, meta, y, ldy, nullptr, alpha, total_rows, N, K, group_k, swiglu, tiles, rows, static_cast<size_t>(code_stride),
                     static_cast<size_t>(meta_stride), nullptr, 0, nullptr, status, stream);
+}
+
+// Block-scaled e4m3 weights [N, K] times e4m3 activations with a scale a row, for M <= 32, or over a work list as above (`experts` matrices stacked
+// in `wq` and `w_scale`, N a multiple of 128).  K a multiple of 256, rows of `xq` 16 bytes apart or a multiple.
+int cb_wq_gemm_skinny_fp8(const void* xq, int ldx, const void* x_scale, const void* wq, const void* w_scale, void* y, int ldy, const void* residual, int M, int N, int K,
+                          void* workspace, long long workspace_bytes, void* counters, void* status, void* stream) {
+  return cb::skinny(cb::kFmtFp8Block, xq, ldx, wq, w_scale, y, ldy, residual, 1.f, M, N, K, K, 0, nullptr, M, 0, 0, workspace, workspace_bytes, counters, status, stream, x_scale);
+}
+int cb_wq_gemm_skinny_fp8_grouped(const void* xq, int ldx, const void* x_scale, const void* wq, const void* w_scale, void* y, int ldy, int total_rows, int N, int K,
+                                  const void* tiles, int rows, int experts, void* status, void* stream) {
+  if (!tiles) return -40;
+  return cb::skinny(cb::kFmtFp8Block, xq, ldx, wq, w_scale, y, ldy, nullptr, 1.f, total_rows, N, K, K, 0, tiles, rows, 0, 0, nullptr, 0, nullptr, status, stream, x_scale, experts);
 }
 
 }  // extern "C"

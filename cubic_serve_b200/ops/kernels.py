@@ -164,6 +164,8 @@ def skinny_fits(w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = Non
         whole = w.k % 128 == 0
     elif w.fmt in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
         whole = w.k % 256 == 0 and (w.fmt != FMT_CUBIC4 or w.group_k % 128 == 0)
+    elif w.fmt == FMT_FP8_BLOCK:             # ``x``: the e4m3 activations
+        whole = w.k % 256 == 0 and x.stride(0) % 16 == 0 and w.codes.data_ptr() % 16 == 0
     else:
         return False
     if not whole or x.stride(0) % 8 or x.data_ptr() % 16:
@@ -183,7 +185,8 @@ def use_skinny(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | Non
     grows with the rows where the tcgen05 kernels' stays: 4-bit weights of 24576 x 4096 take 22 / 26 / 43 us at 8 / 16 / 32 rows
     against 34 / 34 / 35, 4096 x 4096 6.4 / 8.2 / 14 against 10.1 / 10.2 / 10.6.  bf16 weights have nothing to decode: with more
     weight tiles than SMs they stream at 65 / 68 / 74 us against 98 / 98 / 102 (50688 x 4096), with fewer the split tiles of the
-    other kernel are as good from 16 rows on (8.0 / 10.4 against 9.2 / 9.2, 4096 x 4096).  (One B200, weights not in L2.)
+    other kernel are as good from 16 rows on (8.0 / 10.4 against 9.2 / 9.2, 4096 x 4096).  Block-scaled e4m3 weights of 9216 x 4096
+    take 13.7 / 16.6 / 27.4 us at 8 / 16 / 32 rows against 17.8 / 17.9 / 18.3.  (One B200, weights not in L2.)
     The thresholds live in the operator configuration (``few_rows_*``); an installed plan comes before them."""
     if m > 32:
         return False
@@ -205,7 +208,9 @@ SKINNY_ROWS_PER_EXPERT: int | None = None
 
 def skinny_rows_per_expert() -> int:
     """6 / 12 / 16 / 24 rows of 128 experts of 1536 x 2048 (NVFP4) take 82 / 103 / 107 / 134 us against 125 us of the tcgen05 kernel at
-    any of them."""
+    any of them.  1 / 8 / 12 / 16 / 24 rows of 128 experts with block-scaled e4m3 weights of 3072 x 4096 take 173 / 267 / 346 / 411 / 571 us
+    against 270 / 409 / 410 / 411 / 419 (the tcgen05 kernel sets up a tile for each of its CTAs), of 4096 x 1536 96 / 145 / 182 / 210 / 281 against
+    190 / 289 / 290 / 290 / 297."""
     from .strategies import active
     return active().moe.few_rows_per_expert if SKINNY_ROWS_PER_EXPERT is None else SKINNY_ROWS_PER_EXPERT
 
@@ -300,6 +305,11 @@ def _wq_gemm_fp8(x, w: PackedWeight, out, residual, splits, ws: Workspace, link,
     # scales; block scales and explicit split factors stay on the per-tile kernel
     # (measured: the fp8 loop is bound by the L2 -> SM operand feed in both kernels; CTA pairs pay off for deep K at
     # prefill sizes -- 4096 x 4096 x 12288: 153 us against 176 us -- and nowhere else, stream-K at decode sizes ties)
+    if splits is None and min_units is None and link is None and not swiglu and w.fmt == FMT_FP8_BLOCK and use_skinny(m, w, a.q, out, residual, ws):
+        code = l.cb_wq_gemm_skinny_fp8(a.q.data_ptr(), a.q.stride(0), a.scale.data_ptr(), w.codes.data_ptr(), w.meta.data_ptr(), out.data_ptr(), out.stride(0),
+                                       _ptr(residual), m, w.n, k, ws.gemm.data_ptr(), ws.gemm.numel(), ws.gemm_counters.data_ptr(), ws.status.data_ptr(), _stream())
+        native.check(code, "cb_wq_gemm_skinny_fp8")
+        return out
     stream_k = (splits is None and w.fmt == FMT_FP8 and link is None
                 and (min_units is not None or (m >= 2048 and k >= 8192 and (-(-w.n // 128)) % 2 == 0)))
     if stream_k and min_units is None:
@@ -706,6 +716,14 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
         # the routed rows (plus the slack rows a work item's tile may touch) are quantized per token, then one grouped
         # launch over the stacked e4m3 experts
         a = fp8_quantize(x[:min(x.shape[0], rows + sc.mb)], ws)
+        if (w.fmt == FMT_FP8_BLOCK and rows / sc.experts <= skinny_rows_per_expert() and not swiglu and w.n % 128 == 0
+                and skinny_fits(w, a.q, out)):
+            # sixteen rows at a time: with fewer of an expert a tile of eight is no faster (1 row: 175 against 173 us)
+            code = native.lib().cb_wq_gemm_skinny_fp8_grouped(a.q.data_ptr(), a.q.stride(0), a.scale.data_ptr(), w.codes.data_ptr(), w.meta.data_ptr(),
+                                                              out.data_ptr(), out.stride(0), rows, w.n, w.k, sc.tiles.data_ptr(), 16, w.codes.shape[0],
+                                                              ws.status.data_ptr(), _stream())
+            native.check(code, "cb_wq_gemm_skinny_fp8_grouped")
+            return out
         code = native.lib().cb_wq_gemm_fp8_grouped(a.q.data_ptr(), a.q.stride(0), a.scale.data_ptr(), w.codes.data_ptr(),
                                                    w.meta.data_ptr(), int(w.fmt == FMT_FP8_BLOCK), out.data_ptr(),
                                                    out.stride(0), rows, w.n, w.k,

@@ -273,6 +273,10 @@ def _declare(l: ctypes.CDLL) -> None:
     l.cb_wq_gemm_skinny.restype = i
     l.cb_wq_gemm_skinny_grouped.argtypes = [i, vp, i, vp, vp, vp, i, f, i, i, i, i, i, vp, i, ll, ll, vp, vp]
     l.cb_wq_gemm_skinny_grouped.restype = i
+    l.cb_wq_gemm_skinny_fp8.argtypes = [vp, i, vp, vp, vp, vp, i, vp, i, i, i, vp, ll, vp, vp, vp]
+    l.cb_wq_gemm_skinny_fp8.restype = i
+    l.cb_wq_gemm_skinny_fp8_grouped.argtypes = [vp, i, vp, vp, vp, vp, i, i, i, i, vp, i, i, vp, vp]
+    l.cb_wq_gemm_skinny_fp8_grouped.restype = i
     l.cb_tp_reduce_norm.argtypes = [vp, vp]
     l.cb_tp_reduce_norm.restype = i
     l.cb_tp_wait.argtypes = [vp, vp, ctypes.c_uint, i, vp, vp]

@@ -96,3 +96,53 @@ def test_skinny_grouped_gemm(tokens, skew):
         K.SKINNY_ROWS_PER_EXPERT = limit
     # two chained products: a flipped rounding of an activation moves a result by a part of a bf16 step
     assert ((got.float() - want.float()).norm() / want.float().norm()).item() < 2e-3
+
+
+@pytest.mark.parametrize("n,k", [(128, 256), (200, 768), (1000, 1280), (9216, 1024)])
+def test_skinny_gemm_of_block_scaled_fp8(n, k):
+    from cubic_serve_b200.ops import kernels as K
+    g = torch.Generator(device=DEV).manual_seed(n)
+    w = wq_pack.pack_fp8_block((torch.randn(n, k, device=DEV, generator=g) * 100).clamp_(-448, 448).to(torch.float8_e4m3fn),
+                               torch.rand(-(-n // 128), -(-k // 128), device=DEV, generator=g) + 0.5)
+    dense = w.codes.view(torch.float8_e4m3fn).double() * w.meta.double().repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)[:, :k]
+    for m in (1, 8, 9, 16):
+        x, res = torch.randn(m, k, device=DEV, generator=g).bfloat16(), torch.randn(m, n, device=DEV, generator=g).bfloat16()
+        a = K.fp8_quantize(x, out=K.Fp8Act(torch.empty(m, k, dtype=torch.uint8, device=DEV), torch.empty(m, device=DEV)))
+        ref = (a.q.view(torch.float8_e4m3fn).double() * a.scale.double()[:, None]) @ dense.t()
+        out = torch.full((m, n + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+        assert K.use_skinny(m, w, a.q)
+        K.wq_gemm(a, w, out=out[:, :n])
+        assert (out[:, n:] == 7).all()
+        assert ((out[:, :n].double() - ref).norm() / ref.norm()).item() < 2.0 ** -9       # one rounding to bf16
+        assert _close(out[:, :n], K.wq_gemm(a, w, splits=1), k)
+        assert _close(K.wq_gemm(a, w, residual=res), K.wq_gemm(a, w, residual=res, splits=1), k)
+    K.workspace(torch.device(DEV, 0)).check_status()
+    assert not K.workspace(torch.device(DEV, 0)).gemm_counters.any()
+
+
+@pytest.mark.parametrize("counts", [[1], [0, 5, 16, 17, 0, 40, 3], [16] * 9])
+def test_skinny_grouped_block_scaled_fp8(counts):
+    """Experts with no, few and more rows than a pass takes, rows behind the last untouched."""
+    from cubic_serve_b200.ops import kernels as K, native
+    E, n, k, T = len(counts), 256, 512, sum(counts)
+    g = torch.Generator(device=DEV).manual_seed(E)
+    codes = (torch.randn(E * n, k, device=DEV, generator=g) * 100).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    scale = torch.rand(E * n // 128, k // 128, device=DEV, generator=g) + 0.5
+    a = K.fp8_quantize(torch.randn(T, k, device=DEV, generator=g).bfloat16())
+    items, at = [], 0
+    for e, c in enumerate(counts):
+        items += [(e, at, c)] if c else []
+        at += c
+    tiles = torch.tensor([len(items)] + [v for i in items for v in i], dtype=torch.int32, device=DEV)
+    ws = K.workspace(torch.device(DEV, 0))
+    dense = codes.double() * scale.double().repeat_interleave(128, 0).repeat_interleave(128, 1)
+    x = a.q.view(torch.float8_e4m3fn).double() * a.scale.double()[:, None]
+    for rows in (8, 16, 32):
+        out = torch.full((T + 4, n), 7.0, device=DEV, dtype=torch.bfloat16)
+        native.check(native.lib().cb_wq_gemm_skinny_fp8_grouped(a.q.data_ptr(), k, a.scale.data_ptr(), codes.data_ptr(), scale.data_ptr(), out.data_ptr(), n, T, n, k,
+                                                                tiles.data_ptr(), rows, E, ws.status.data_ptr(), K._stream()), "grouped")
+        assert (out[T:] == 7).all()
+        for e, first, c in items:
+            ref = x[first:first + c] @ dense[e * n:(e + 1) * n].t()
+            assert ((out[first:first + c].double() - ref).norm() / ref.norm()).item() < 2.0 ** -9
+    ws.check_status()
