@@ -215,11 +215,36 @@ def skinny_rows_per_expert() -> int:
     return active().moe.few_rows_per_expert if SKINNY_ROWS_PER_EXPERT is None else SKINNY_ROWS_PER_EXPERT
 
 
-def _wq_gemm_skinny(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, residual: torch.Tensor | None, ws: "Workspace", swiglu: bool) -> torch.Tensor:
-    code = native.lib().cb_wq_gemm_skinny(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(), out.stride(0),
+def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None, residual: torch.Tensor | None = None, ws: "Workspace | None" = None) -> bool:
+    """Which batches of 4-bit weights the kernel with decoded tiles in tensor memory takes (``csrc/wq_gemm_ts.cu``): up to 128 rows of whole
+    units of 128 columns.  Its time hardly grows with the rows, but a tile's parts are summed behind a start of 3 us, so it wants six and a half units an SM.
+    8 / 16 / 48 / 128 rows, few-row or per-tile and persistent kernels -> this one: 24576 x 4096
+    27.4 / 31.3 / 38.7 / 44.5 -> 22.4 / 23.0 / 26.9 / 36.9 us, 4096 x 12288 17.2 / 20.2 / 25.5 / 28.3 -> 15.6 / 15.9 / 17.5 / 22.6, 6144 x 4096
+    13.2 / 14.7 / 18.9 / 21.4 -> 12.1 / 12.4 / 13.9 / 18.9, 4096 x 4096 10.0 / 12.1 / 13.2 / 15.5 -> 10.2 / 10.5 / 11.9 / 15.8; 5120 x 2048 (NVFP4)
+    9.2 / 11.2 / 11.3 / 13.3 -> 10.0 / 10.2 / 11.7 / 15.7.  (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration.)"""
+    if m > 128 or w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
+        return False
+    from .strategies import active
+    g = active().gemm
+    if m > g.tensor_memory_rows or w.k % 128 or (w.fmt == FMT_CUBIC4 and w.group_k % 128) or x.stride(0) % 8 or x.data_ptr() % 16:
+        return False
+    if out is not None and out.stride(0) % 4 == 0 and (out.data_ptr() | (0 if residual is None else residual.data_ptr())) % 8:
+        return False
+    sms = sm_count(x.device) if x.is_cuda else 148
+    if 2 * -(-w.n // 128) * (w.k // 128) < 13 * sms:
+        return False
+    if ws is not None:
+        parts = 2 * sms * -(-m // 16) * 16 * 128 * 4
+        return parts <= ws.gemm.numel() and -(-w.n // 128) <= ws.gemm_counters.numel()
+    return True
+
+
+def _wq_gemm_skinny(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, residual: torch.Tensor | None, ws: "Workspace", swiglu: bool,
+                    entry: str = "cb_wq_gemm_skinny") -> torch.Tensor:
+    code = getattr(native.lib(), entry)(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(), out.stride(0),
                                           _ptr(residual), float(w.alpha), x.shape[0], w.n, w.k, w.group_k, int(swiglu), ws.gemm.data_ptr(),
                                           ws.gemm.numel(), ws.gemm_counters.data_ptr(), ws.status.data_ptr(), _stream())
-    native.check(code, "cb_wq_gemm_skinny")
+    native.check(code, entry)
     return out
 
 
@@ -335,9 +360,9 @@ def wq_gemm(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = None,
             ws: Workspace | None = None, link=None, min_units: int | None = None) -> torch.Tensor:
     """``out[M, N] = x[M, K] @ W[N, K]^T * alpha (+ residual)`` with W in packed form.
 
-    Three kernels: one CTA per (weight tile, K split) (``csrc/wq_gemm.cu``), the persistent stream-K kernel
-    (``csrc/wq_gemm_sk.cu``), and one for few rows (``csrc/wq_gemm_skinny.cu``).  With neither ``splits`` nor ``min_units`` given an
-    installed plan decides, else ``use_skinny`` and ``use_stream_k``.  ``splits`` forces the first with that split-K factor; ``min_units`` forces the
+    Four kernels: one CTA per (weight tile, K split) (``csrc/wq_gemm.cu``), the persistent stream-K kernel
+    (``csrc/wq_gemm_sk.cu``), and two for few rows (``csrc/wq_gemm_ts.cu``, ``csrc/wq_gemm_skinny.cu``).  With neither ``splits`` nor ``min_units`` given an
+    installed plan decides, else ``use_ts``, ``use_skinny`` and ``use_stream_k``.  ``splits`` forces the first with that split-K factor; ``min_units`` forces the
     second (0 = its own schedule, > 0 = the smallest run of k-blocks a CTA is dealt).
     """
     assert isinstance(x, Fp8Act) or (x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1)
@@ -356,6 +381,8 @@ def wq_gemm(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = None,
         tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:0") if TUNED_PLANS else None
         if tuned is not None:
             splits, min_units = (None, 0) if tuned[0] else (tuned[1], None)
+        elif use_ts(m, w, x, out, residual, ws):
+            return _wq_gemm_skinny(x, w, out, residual, ws, False, "cb_wq_gemm_ts")
         elif use_skinny(m, w, x, out, residual, ws):
             return _wq_gemm_skinny(x, w, out, residual, ws, False)
     l = native.lib()
@@ -407,6 +434,8 @@ def wq_gemm_act(x: torch.Tensor, w: PackedWeight, out: torch.Tensor | None = Non
         tuned = TUNED_PLANS.get(f"{w.fmt}:{m}:{w.n}:{k}:1") if TUNED_PLANS else None
         if tuned is not None:
             splits, min_units = (None, 0) if tuned[0] else (tuned[1], None)
+        elif use_ts(m, w, x, out, None, ws):
+            return _wq_gemm_skinny(x, w, out, None, ws, True, "cb_wq_gemm_ts")
         elif use_skinny(m, w, x, out, None, ws):
             return _wq_gemm_skinny(x, w, out, None, ws, True)
     l = native.lib()

@@ -146,3 +146,50 @@ def test_skinny_grouped_block_scaled_fp8(counts):
             ref = x[first:first + c] @ dense[e * n:(e + 1) * n].t()
             assert ((out[first:first + c].double() - ref).norm() / ref.norm()).item() < 2.0 ** -9
     ws.check_status()
+
+
+@pytest.mark.parametrize("fmt", ["cubic", "affine", "nvfp4"])
+@pytest.mark.parametrize("n,k", [
+    (128, 128),            # one tile, one unit
+    (200, 1152),           # nine parts of a tile with 72 rows of padding
+    (5120, 2048),          # parts of uneven length
+    (10000, 1024),         # runs that straddle tiles
+    (24576, 512),          # whole tiles between parts
+])
+def test_gemm_with_decoded_tiles_in_tensor_memory(fmt, n, k):
+    from cubic_serve_b200.ops import kernels as K
+    w = _weight(fmt, n, k, n + k)
+    dense = wq_pack.unpack_to_dense(w)[:n]
+    g = torch.Generator(device=DEV).manual_seed(2)
+    ws = K.workspace(torch.device(DEV, 0))
+    for m in (1, 16, 17, 33, 128):
+        wide = torch.randn(m, k + 64, device=DEV, generator=g).bfloat16()
+        x, res = wide[:, :k], torch.randn(m, n, device=DEV, generator=g).bfloat16()
+        ref = x.float() @ dense.t()
+        out = torch.full((m, n + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+        K._wq_gemm_skinny(x, w, out[:, :n], None, ws, False, "cb_wq_gemm_ts")
+        assert (out[:, n:] == 7).all()
+        assert _close(out[:, :n], K.wq_gemm(x, w, splits=1), k)
+        assert ((out[:, :n].float() - ref).norm() / ref.norm()).item() < 6e-3        # rounding of decode arithmetic and result
+        got = [K._wq_gemm_skinny(x, w, torch.empty(m, n, device=DEV, dtype=torch.bfloat16), res, ws, False, "cb_wq_gemm_ts") for _ in range(2)]
+        assert _close(got[0], K.wq_gemm(x, w, residual=res, splits=1), k) and torch.equal(*got)      # parts are summed in their order
+        if n % 128 == 0:
+            act = wq_pack.swiglu_interleave(w)
+            plain = wq_pack.PackedWeight(act.fmt, act.n, act.k, act.group_k, act.codes, act.meta, act.alpha)
+            gu = torch.empty(m, n, device=DEV, dtype=torch.bfloat16)
+            gu[:, wq_pack.swiglu_row_order(n // 2).to(DEV)] = K._wq_gemm_skinny(x, plain, torch.empty_like(gu), None, ws, False, "cb_wq_gemm_ts")
+            assert torch.equal(K._wq_gemm_skinny(x, act, torch.empty(m, n // 2, device=DEV, dtype=torch.bfloat16), None, ws, True, "cb_wq_gemm_ts"), K.swiglu(gu))
+    ws.check_status()
+    assert not ws.gemm_counters.any()
+
+
+def test_gemm_with_decoded_tiles_in_tensor_memory_refuses_what_it_does_not_take():
+    from cubic_serve_b200.ops import kernels as K
+    from cubic_serve_b200.ops.native import NativeLibraryError
+    ws = K.workspace(torch.device(DEV, 0))
+    w = _weight("affine", 128, 128, 0)
+    for m, weight in ((129, w), (8, _weight("affine", 128, 192, 0)), (8, _weight("bf16", 128, 128, 0))):
+        x = torch.zeros(m, weight.k, device=DEV, dtype=torch.bfloat16)
+        assert not K.use_ts(m, weight, x)
+        with pytest.raises(NativeLibraryError):
+            K._wq_gemm_skinny(x, weight, torch.empty(m, 128, device=DEV, dtype=torch.bfloat16), None, ws, False, "cb_wq_gemm_ts")
