@@ -146,7 +146,7 @@ class MoeLayer:
         t, h = x.shape
         sc = self.ensure_scratch(runner.max_tokens if runner is not None else t, h, x.device)
         ws = runner.ws if runner is not None else None
-        sc.mb = K.rows_per_work_item(t * self.top_k, self.num_experts, self.least_rows)
+        sc.mb = K.rows_per_work_item(t * self.top_k, self.num_experts, self.least_rows, (self.gate_up, self.down), self.expert_count)
         logits = K.wq_gemm(x, self.router, out=self.logits[:t], ws=ws)
         K.moe_route(logits, x, self.top_k, sc, self.normalize, self.expert_lo, self.expert_count)
         rows = t * self.top_k

@@ -207,8 +207,8 @@ SKINNY_ROWS_PER_EXPERT: int | None = None
 
 
 def skinny_rows_per_expert() -> int:
-    """6 / 12 / 16 / 24 rows of 128 experts of 1536 x 2048 (NVFP4) take 82 / 103 / 107 / 134 us against 125 us of the tcgen05 kernel at
-    any of them.  1 / 8 / 12 / 16 / 24 rows of 128 experts with block-scaled e4m3 weights of 3072 x 4096 take 173 / 267 / 346 / 411 / 571 us
+    """6 / 12 / 16 / 24 rows of 128 experts of 1536 x 2048 (NVFP4) take 82 / 103 / 107 / 134 us against 125 us of the per-tile tcgen05 kernel at
+    any of them (``use_ts_grouped`` comes first).  1 / 8 / 12 / 16 / 24 rows of 128 experts with block-scaled e4m3 weights of 3072 x 4096 take 173 / 267 / 346 / 411 / 571 us
     against 270 / 409 / 410 / 411 / 419 (the tcgen05 kernel sets up a tile for each of its CTAs), of 4096 x 1536 96 / 145 / 182 / 210 / 281 against
     190 / 289 / 290 / 290 / 297."""
     from .strategies import active
@@ -218,10 +218,9 @@ def skinny_rows_per_expert() -> int:
 def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None, residual: torch.Tensor | None = None, ws: "Workspace | None" = None) -> bool:
     """Which batches of 4-bit weights the kernel with decoded tiles in tensor memory takes (``csrc/wq_gemm_ts.cu``): up to 128 rows of whole
     units of 128 columns.  Its time hardly grows with the rows, but a tile's parts are summed behind a start of 3 us, so it wants six and a half units an SM.
-    8 / 16 / 48 / 128 rows, few-row or per-tile and persistent kernels -> this one: 24576 x 4096
-    27.4 / 31.3 / 38.7 / 44.5 -> 22.4 / 23.0 / 26.9 / 36.9 us, 4096 x 12288 17.2 / 20.2 / 25.5 / 28.3 -> 15.6 / 15.9 / 17.5 / 22.6, 6144 x 4096
-    13.2 / 14.7 / 18.9 / 21.4 -> 12.1 / 12.4 / 13.9 / 18.9, 4096 x 4096 10.0 / 12.1 / 13.2 / 15.5 -> 10.2 / 10.5 / 11.9 / 15.8; 5120 x 2048 (NVFP4)
-    9.2 / 11.2 / 11.3 / 13.3 -> 10.0 / 10.2 / 11.7 / 15.7.  (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration.)"""
+    8 / 48 / 128 rows, few-row or per-tile and persistent kernels -> this one: 24576 x 4096 27.4 / 38.7 / 44.5 -> 21.9 / 24.0 / 29.7 us,
+    4096 x 12288 17.2 / 25.5 / 28.3 -> 15.7 / 17.9 / 22.3, 6144 x 4096 13.2 / 18.9 / 21.4 -> 11.7 / 13.6 / 18.8, 4096 x 4096
+    10.0 / 13.2 / 15.5 -> 10.3 / 12.3 / 16.0; 5120 x 2048 (NVFP4) 9.2 / 11.3 / 13.3 -> 9.8 / 11.9 / 16.3.  (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration.)"""
     if m > 128 or w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
         return False
     from .strategies import active
@@ -237,6 +236,18 @@ def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = 
         parts = 2 * sms * -(-m // 16) * 16 * 128 * 4
         return parts <= ws.gemm.numel() and -(-w.n // 128) <= ws.gemm_counters.numel()
     return True
+
+
+def use_ts_grouped(rows: int, w: PackedWeight, experts: int, mb: int) -> bool:
+    """Which launches over 4-bit experts that kernel takes: work items of up to 128 rows.  A CTA has whole tiles, so that it wants two of them
+    for every SM.  128 experts (NVFP4), few-row kernel (above 16 rows an expert: per-tile kernel in items of its best size) -> this one, at 16 / 32 / 64 / 128
+    routes and 2 / 6 / 24 / 64 / 256 rows an expert: 1536 x 2048 19.0 / 26.9 / 38.9 / 53 and 76 / 85 / 134 / 137 / 299 -> 19.4 / 26.1 / 37.5 / 50 and
+    67 / 73 / 78 / 93 / 251 us, 2048 x 768 10.9 / 13.9 / 22.6 / 34 and 40 / 48 / 88 / 102 / 287 -> 11.4 / 13.7 / 20.8 / 28 and 36 / 41 / 43 / 51 / 132.
+    (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration.)"""
+    if w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4) or w.k % 128 or (w.fmt == FMT_CUBIC4 and w.group_k % 128):
+        return False
+    from .strategies import active
+    return mb <= active().gemm.tensor_memory_rows and min(experts, rows) * -(-w.n // 128) >= 2 * (sm_count(w.codes.device) if w.codes.is_cuda else 148)
 
 
 def _wq_gemm_skinny(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, residual: torch.Tensor | None, ws: "Workspace", swiglu: bool,
@@ -704,8 +715,10 @@ class MoeScratch:
         return min(self.max_items, rows // self.mb + min(self.local_experts, rows))
 
 
-def rows_per_work_item(rows: int, experts: int, least: int) -> int:
-    """Rows of a work item of the grouped tcgen05 GEMM for ``rows`` routes over ``experts``.  A work item's weights are decoded once
+def rows_per_work_item(rows: int, experts: int, least: int, weights: tuple[PackedWeight, ...] = (), local: int = 0) -> int:
+    """Rows of a work item of the grouped tcgen05 GEMMs for ``rows`` routes over ``experts``.  Items that hold 128 rows where ``use_ts_grouped`` takes the
+    launches over ``weights`` of the ``local`` experts (1536 x 2048, 256 / 64 rows an expert, items of 64 / 96 / 128 rows: 296 / 262 / 251 and
+    109 / 96 / 93 us).  Else a work item's weights are decoded once
     whatever its rows, and the decode sets the pace up to 200 of them, so an item should hold all rows of an expert with an
     average load (three standard deviations of a random routing above the mean), or an even part of them.  Gate / up and down of
     128 experts (1536 x 2048, 2048 x 768, NVFP4), items of 64 rows -> of this size: 1024 tokens 188 + 109 -> 137 + 92 us (96),
@@ -718,6 +731,8 @@ def rows_per_work_item(rows: int, experts: int, least: int) -> int:
     want = mean + 3.0 * math.sqrt(mean)
     if want <= least:
         return least
+    if least <= 128 and weights and all(use_ts_grouped(rows, w, local, 128) for w in weights):
+        return 128
     return max(least, -(-math.ceil(want / math.ceil(want / 256)) // 16) * 16)
 
 
@@ -759,6 +774,12 @@ def wq_gemm_grouped(x: torch.Tensor, w: PackedWeight, out: torch.Tensor, rows: i
                                                    sc.tiles.data_ptr(), sc.items(rows), sc.mb, w.codes.shape[0], int(swiglu),
                                                    ws.status.data_ptr(), _stream())
         native.check(code, "cb_wq_gemm_fp8_grouped")
+        return out
+    if use_ts_grouped(rows, w, sc.local_experts, sc.mb) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+        code = native.lib().cb_wq_gemm_ts_grouped(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), _ptr(w.meta), out.data_ptr(), out.stride(0),
+                                                  float(w.alpha), rows, w.n, w.k, w.group_k, int(swiglu), sc.tiles.data_ptr(), sc.items(rows), sc.mb,
+                                                  code_stride, meta_stride, ws.status.data_ptr(), _stream())
+        native.check(code, "cb_wq_gemm_ts_grouped")
         return out
     per = rows / sc.experts                  # routes of all experts, wherever they live
     if per <= skinny_rows_per_expert() and w.fmt != FMT_BF16 and skinny_fits(w, x, out):

@@ -275,6 +275,8 @@ def _declare(l: ctypes.CDLL) -> None:
     l.cb_wq_gemm_skinny_grouped.restype = i
     l.cb_wq_gemm_ts.argtypes = list(l.cb_wq_gemm_skinny.argtypes)
     l.cb_wq_gemm_ts.restype = i
+    l.cb_wq_gemm_ts_grouped.argtypes = [i, vp, i, vp, vp, vp, i, f, i, i, i, i, i, vp, i, i, ll, ll, vp, vp]
+    l.cb_wq_gemm_ts_grouped.restype = i
     l.cb_wq_gemm_skinny_fp8.argtypes = [vp, i, vp, vp, vp, vp, i, vp, i, i, i, vp, ll, vp, vp, vp]
     l.cb_wq_gemm_skinny_fp8.restype = i
     l.cb_wq_gemm_skinny_fp8_grouped.argtypes = [vp, i, vp, vp, vp, vp, i, i, i, i, vp, i, i, vp, vp]

@@ -105,3 +105,16 @@ def test_rows_of_an_expert_count_over_all_ranks(calls, ranks, tokens, entry):
     sc = K.MoeScratch(tokens, 8, 256, 128, local, 32, "cpu", experts=32)
     K.wq_gemm_grouped(torch.zeros(rows, 256, dtype=torch.bfloat16), w, torch.empty(rows, 128, dtype=torch.bfloat16), rows, sc, 16, 16, _ws())
     assert calls.made.pop()[0] == entry
+
+
+@pytest.mark.parametrize("routes,mb,n,k,fmt,entry", [
+    (24, 32, 1536, 2048, wq_pack.FMT_NVFP4, "cb_wq_gemm_skinny_grouped"), (25, 32, 1536, 2048, wq_pack.FMT_NVFP4, "cb_wq_gemm_ts_grouped"),
+    (4096, 128, 1536, 2048, wq_pack.FMT_CUBIC4, "cb_wq_gemm_ts_grouped"), (4096, 144, 1536, 2048, wq_pack.FMT_CUBIC4, "cb_wq_gemm_grouped"),
+    (4096, 128, 384, 2048 + 64, wq_pack.FMT_AFFINE4, "cb_wq_gemm_grouped"), (4096, 128, 384, 2048, wq_pack.FMT_BF16, "cb_wq_gemm_grouped")])
+def test_experts_with_two_tiles_for_every_sm(calls, routes, mb, n, k, fmt, entry):
+    w = wq_pack.PackedWeight(fmt, n, k, 128, torch.zeros(128, 16), torch.zeros(128, 16), 1.0)
+    sc = SimpleNamespace(experts=128, local_experts=128, mb=mb, tiles=torch.zeros(1, dtype=torch.int32), items=lambda rows: rows)
+    K.wq_gemm_grouped(torch.zeros(routes, k, dtype=torch.bfloat16), w, torch.empty(routes, n, dtype=torch.bfloat16), routes, sc, 16, 16, _ws())
+    assert calls.made.pop()[0] == entry
+    assert K.rows_per_work_item(4096, 64, 64, (w,), 128) == (128 if n * k == 1536 * 2048 and fmt != wq_pack.FMT_BF16 else 96)
+    assert K.rows_per_work_item(1024, 64, 64, (w,), 128) == 64 and K.rows_per_work_item(4096, 64, 160, (w,), 128) == 160

@@ -183,6 +183,43 @@ def test_gemm_with_decoded_tiles_in_tensor_memory(fmt, n, k):
     assert not ws.gemm_counters.any()
 
 
+@pytest.mark.parametrize("mb", [16, 48, 128])
+@pytest.mark.parametrize("fmt", ["cubic", "affine", "nvfp4"])
+def test_grouped_gemm_with_decoded_tiles_in_tensor_memory(fmt, mb):
+    """Experts with no, few and many rows (an item full, one row over, several items, a short last tile), fewer and more tiles than SMs."""
+    from cubic_serve_b200.models.moe import stack_experts
+    from cubic_serve_b200.ops import kernels as K, native
+    ws = K.workspace(torch.device(DEV, 0))
+    for counts, n, k in (([1], 128, 128), ([0, 5, 16, 17, 0, 129, 3, 300], 320, 640), ([40] * 30, 1280, 256)):
+        T, g = sum(counts), torch.Generator(device=DEV).manual_seed(mb)
+        each = [_weight(fmt, n, k, e) for e in range(len(counts))]
+        w, cs, ms = stack_experts(each)
+        x = torch.randn(T, k + 64, device=DEV, generator=g).bfloat16()[:, :k]
+        items, at = [], 0
+        for e, c in enumerate(counts):
+            items += [(e, at + o, min(mb, c - o)) for o in range(0, c, mb)]
+            at += c
+        tiles = torch.tensor([len(items)] + [v for i in items for v in i], dtype=torch.int32, device=DEV)
+
+        def run(w, out, act):
+            native.check(native.lib().cb_wq_gemm_ts_grouped(w.fmt, x.data_ptr(), x.stride(0), w.codes.data_ptr(), K._ptr(w.meta), out.data_ptr(), out.stride(0), w.alpha,
+                                                            T, n, k, w.group_k, act, tiles.data_ptr(), len(items) + 2, mb, cs, ms, ws.status.data_ptr(), K._stream()), "grouped")
+            return out
+        out = run(w, torch.full((T + 4, n + 3), 7.0, device=DEV, dtype=torch.bfloat16), 0)
+        assert (out[T:] == 7).all() and (out[:, n:] == 7).all()
+        at = 0
+        for e, c in enumerate(counts):
+            if c:
+                assert _close(out[at:at + c, :n], K.wq_gemm(x[at:at + c], each[e], splits=1), k)
+            at += c
+        if n % 128 == 0:
+            act = wq_pack.swiglu_interleave(w, stacked=True)
+            gu = torch.empty(T, n, device=DEV, dtype=torch.bfloat16)
+            gu[:, wq_pack.swiglu_row_order(n // 2).to(DEV)] = run(act, torch.empty_like(gu), 0)
+            assert torch.equal(run(act, torch.empty(T, n // 2, device=DEV, dtype=torch.bfloat16), 1), K.swiglu(gu))
+    ws.check_status()
+
+
 def test_gemm_with_decoded_tiles_in_tensor_memory_refuses_what_it_does_not_take():
     from cubic_serve_b200.ops import kernels as K
     from cubic_serve_b200.ops.native import NativeLibraryError
