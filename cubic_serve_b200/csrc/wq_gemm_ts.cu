@@ -1,4 +1,4 @@
-// Weight-quantized GEMM of up to 128 batch rows, of one matrix or of each expert of a work list: y[M, N] = x[M, K] * W[N, K]^T, 4-bit weights
+// Weight-quantized GEMM of batch rows in blocks of up to 128, of one matrix or of each expert of a work list: y[M, N] = x[M, K] * W[N, K]^T, 4-bit weights
 // (packed weight layout and decode arithmetic: wq_gemm_common.cuh).
 //
 // What bounds it.  The other tcgen05 kernels write a decoded tile to shared memory, in a stage that also holds the activation tile and (per-tile
@@ -11,9 +11,12 @@
 // 21.9 / 24.0 / 29.7 us (floor 8.7), 4096 x 12288 17.2 / 25.5 / 28.3 -> 15.7 / 17.9 / 22.3 (4.3), 6144 x 4096 13.2 / 18.9 / 21.4 -> 11.7 / 13.6 / 18.8
 // (2.2).  About 8 us of each are start (4300 cycles to the first codes), the last run's sums and the sum of parts.  128 experts (NVFP4) of 1536 x 2048,
 // 6 / 24 / 64 / 256 rows an expert: 85 / 134 / 137 / 299 -> 73 / 78 / 93 / 251 us (35 us of codes; at 256 rows 125 us of MMAs), 2048 x 768
-// 48 / 88 / 102 / 287 -> 41 / 43 / 51 / 132.  Pairs of CTAs (half of the activation tile each) measured the same or slower at every size.
+// 48 / 88 / 102 / 287 -> 41 / 43 / 51 / 132.  Blocks of rows decode a tile once each: 24576 x 4096 at 256 / 331 / 512 rows, single cold launches,
+// 57.5 / 89.5 / 93.1 -> 48.8 / 64.3 / 83.5 us.  Up to 24 rows the decode's integer pipe is half busy and its latency the rest (a unit in 740 cycles, 490
+// instructions a scheduler), at 128 rows a unit takes 1150 cycles of which the MMAs are 517.  What did not help: pairs of CTAs with half of the activation
+// tile each (256 rows: 51.4 us), MMAs on each half of a unit while the other is decoded (8 rows: 25.9 us, the one thread's rounds double).
 //
-// Split.  One CTA per SM.  One matrix: the units of all weight tiles are dealt evenly, a tile in a few runs whose fp32 sums the last one to arrive
+// Split.  One CTA per SM.  One matrix: the units of all weight tiles (of each block of rows in turn) are dealt evenly, a tile in a few runs whose fp32 sums the last one to arrive
 // adds in the order of K (deterministic).  Work list: whole tiles, every CTA every so many.  Roles: warps 0-3 epilogue (from one of two accumulators
 // while the next run fills the other one; a lane has a feature, results leave from its registers: staged in shared memory for wider stores they set
 // the pace of short K, 2048 x 768 at 256 rows 230 us), warp 4 codes, warp 7 their tables, warp 5 MMAs, warp 6 activations, warps 8-23 decode: group g
@@ -43,6 +46,7 @@ struct __align__(16) TsCtl {
 // A run of units of one tile.
 struct TsRun {
   int tile, kb, kb_end, part, parts;
+  int sum;                                       // counter of the tile's (and block of rows') parts
   int expert, m0, rows;                          // batch rows [m0, m0 + rows)
 };
 // The deal; every role walks the same list.  Work list: tile c, c + CTAs, .. of its items, whole.  p.splits > 0: CTA c has part c % splits of
@@ -50,11 +54,12 @@ struct TsRun {
 template <bool GROUPED>
 struct TsWalk {
   uint32_t u, u_end, total;
+  int m_blocks;
   int tile, tiles, e, m0, rows;                  // work list: the next tile, its item
-  __device__ __forceinline__ TsWalk(const WqGemmParams& p) {
+  __device__ __forceinline__ TsWalk(const WqGemmParams& p, int m_blocks_) : m_blocks(m_blocks_) {
     const uint32_t cta = blockIdx.x, ctas = gridDim.x;
     const uint32_t kbs = static_cast<uint32_t>(p.k_blocks);
-    total = static_cast<uint32_t>(p.tiles) * kbs;
+    total = static_cast<uint32_t>(GROUPED ? p.tiles : p.tiles * m_blocks) * kbs;
     if constexpr (GROUPED) {
       tiles = p.group_tiles[0] * p.tiles;
       tile = static_cast<int>(cta);
@@ -80,7 +85,7 @@ struct TsWalk {
       if (tile >= tiles) return false;
       r.tile = tile % p.tiles;
       r.kb = 0; r.kb_end = p.k_blocks;
-      r.part = 0; r.parts = 1;
+      r.part = 0; r.parts = 1; r.sum = 0;
       r.expert = e; r.m0 = m0; r.rows = rows;
       tile += static_cast<int>(gridDim.x);
       if (tile < tiles) item(p);                 // on its way while this tile is worked on
@@ -88,13 +93,18 @@ struct TsWalk {
     } else {
       if (u >= u_end) return false;
       const uint32_t kbs = static_cast<uint32_t>(p.k_blocks), t = u / kbs, first = t * kbs, end = min(u_end, first + kbs);
-      r.tile = static_cast<int>(t);
+      r.tile = r.sum = static_cast<int>(t);
       r.kb = static_cast<int>(u - first);
       r.kb_end = static_cast<int>(end - first);
       r.expert = 0; r.m0 = 0; r.rows = p.M;
+      if (p.M > p.mb) {                          // blocks of rows, those of a weight tile in turn
+        r.tile = static_cast<int>(t) / m_blocks;
+        r.m0 = (r.sum - r.tile * m_blocks) * p.mb;
+        r.rows = min(p.mb, p.M - r.m0);
+      }
       if (p.splits > 0) {
         r.parts = p.splits;
-        r.part = static_cast<int>(blockIdx.x) - r.tile * p.splits;
+        r.part = static_cast<int>(blockIdx.x) - r.sum * p.splits;
       } else {
         // CTA that owns unit v: the largest c with floor(total * c / ctas) <= v
         const uint32_t ctas = gridDim.x, c0 = ((first + 1u) * ctas - 1u) / total, c1 = ((first + kbs) * ctas - 1u) / total;
@@ -230,7 +240,7 @@ __device__ __forceinline__ void ts_out(const WqGemmParams& p, const TsRun& run, 
 // mb: most batch rows of a run, rounded up to 16
 template <int FMT, bool GROUPED>
 __global__ void __launch_bounds__(kTsThreads, 1)
-wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ WqGemmParams p, const int box, const int boxes) {
+wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ WqGemmParams p, const int m_blocks, const int box, const int boxes) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr uint32_t kC = ts_codes() + ts_meta(FMT);
   const uint32_t box_bytes = static_cast<uint32_t>(box) * 128u, x_half = box_bytes * boxes, x_bytes = 2 * x_half;
@@ -269,7 +279,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   pdl_launch_dependents();
   if constexpr (GROUPED) pdl_wait();             // the work list is written by the routing kernels
   const uint32_t tmem = ctl.tmem;
-  TsWalk<GROUPED> walk(p);
+  TsWalk<GROUPED> walk(p, m_blocks);
   TsRun run;
   bool ok = true;
 
@@ -383,7 +393,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       more = walk.next(p, next);
       const int b = runs & 1, used = runs >> 1;
       // (from lane 0: what the MMAs take has to be known to be the same in all lanes, or every one of them moves it to uniform registers)
-      const uint32_t acc = tmem_u + b * 128, idesc = __shfl_sync(0xffffffffu, umma_idesc(kTileN, static_cast<uint32_t>(GROUPED ? (run.rows + 15) & ~15 : p.mb), 1u, 1u), 0);
+      const uint32_t acc = tmem_u + b * 128, idesc = __shfl_sync(0xffffffffu, umma_idesc(kTileN, static_cast<uint32_t>((run.rows + 15) & ~15), 1u, 1u), 0);
       if (used > 0) ok = mbar_wait_park(smem_u32(&ctl.acc_empty[b]), (used - 1) & 1, abort_flag);
       for (int kb = run.kb; kb < run.kb_end; ++kb) {
         ok = __all_sync(0xffffffffu, ok && mbar_wait_park(smem_u32(&ctl.full[s]), phase, abort_flag));
@@ -438,10 +448,10 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         if (helped) asm volatile("bar.sync 2, 640;" ::: "memory");
         else ts_bar();
         if (threadIdx.x == 0) {
-          const uint32_t prev = atom_add_acq_rel_gpu(p.counters + run.tile, 1u);
+          const uint32_t prev = atom_add_acq_rel_gpu(p.counters + run.sum, 1u);
           if (prev == static_cast<uint32_t>(run.parts) - 1u) {
-            p.counters[run.tile] = 0;
-            ctl.sum_tile[ctl.sums] = run.tile;
+            p.counters[run.sum] = 0;
+            ctl.sum_tile[ctl.sums] = run.sum;
             ctl.sum_part[ctl.sums] = run.part;
             ctl.sum_parts[ctl.sums] = run.parts;
             ++ctl.sums;                          // the first and the last run of a CTA are all that can be parts
@@ -458,7 +468,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   }
   // tiles in parts that are complete with this CTA's: summed by all threads, two parts (most weights have no more) of several places in flight
   for (int d = 0; !GROUPED && d < ctl.sums; ++d) {
-    const int parts = ctl.sum_parts[d], tile = ctl.sum_tile[d], c0 = static_cast<int>(blockIdx.x) - ctl.sum_part[d], shift = p.swiglu ? 4 : 5;
+    const int parts = ctl.sum_parts[d], t = ctl.sum_tile[d], tile = t / m_blocks, m0 = (t - tile * m_blocks) * p.mb, c0 = static_cast<int>(blockIdx.x) - ctl.sum_part[d], shift = p.swiglu ? 4 : 5;
     auto part = [&](int q, int at) { return __ldcg(reinterpret_cast<const float4*>(ts_slot(p, c0 + q, q) + at)); };
     auto out = [&](int i, auto sum) {
       const int m = i >> shift, j = i & ((1 << shift) - 1);
@@ -466,12 +476,12 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         float4 g = sum(m * kTileN + act_gate_col(j * 4)), u = sum(m * kTileN + act_gate_col(j * 4) + 16);
         g.x *= p.alpha; g.y *= p.alpha; g.z *= p.alpha; g.w *= p.alpha;
         u.x *= p.alpha; u.y *= p.alpha; u.z *= p.alpha; u.w *= p.alpha;
-        store_act4(p, m, tile, j * 4, g, u);
+        store_act4(p, m0 + m, tile, j * 4, g, u);
       } else {
-        sk_store4<FMT>(p, m, tile * kTileN + j * 4, sum(i * 4));
+        sk_store4<FMT>(p, m0 + m, tile * kTileN + j * 4, sum(i * 4));
       }
     };
-    const int n = p.M << shift;
+    const int n = min(p.mb, p.M - m0) << shift;
     if (parts == 2) {
       for (int i = threadIdx.x; i < n; i += 2 * kTsThreads) {
         const int i2 = i + kTsThreads;
@@ -511,7 +521,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 }
 
 template <int FMT, bool GROUPED>
-static int launch_ts(const CUtensorMap& tx, const WqGemmParams& p, int box, int boxes, int grid, size_t smem, cudaStream_t stream) {
+static int launch_ts(const CUtensorMap& tx, const WqGemmParams& p, int m_blocks, int box, int boxes, int grid, size_t smem, cudaStream_t stream) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -18;
@@ -520,7 +530,7 @@ static int launch_ts(const CUtensorMap& tx, const WqGemmParams& p, int box, int 
     if (e != cudaSuccess) return static_cast<int>(e);
     configured[dev] = true;
   }
-  return static_cast<int>(launch(wq_gemm_ts_kernel<FMT, GROUPED>, dim3(static_cast<unsigned>(grid)), dim3(kTsThreads), smem, stream, tx, p, box, boxes));
+  return static_cast<int>(launch(wq_gemm_ts_kernel<FMT, GROUPED>, dim3(static_cast<unsigned>(grid)), dim3(kTsThreads), smem, stream, tx, p, m_blocks, box, boxes));
 }
 
 // A matrix (mb = M), or with `items` the experts of a work list of at most `max_items` items of at most mb rows
@@ -553,14 +563,16 @@ static int ts_gemm(int fmt, const void* x, int ldx, const void* codes, const voi
   p.group_tiles = static_cast<const int*>(items);
   p.group_code_stride = code_stride;
   p.group_meta_stride = meta_stride;
-  const long long units = static_cast<long long>(p.tiles) * p.k_blocks, most = items ? static_cast<long long>(max_items) * p.tiles : units;
+  const int m_blocks = items ? 1 : (M + p.mb - 1) / p.mb;
+  const long long units = static_cast<long long>(p.tiles) * m_blocks * p.k_blocks, most = items ? static_cast<long long>(max_items) * p.tiles : units;
   if (units * sms[dev] >= (1ll << 32) || most * p.k_blocks >= (1ll << 31)) return -19;
   if (!items && (!workspace || !counters || workspace_bytes < 2ll * sms[dev] * p.mb * kTileN * 4)) return -13;
   int grid = static_cast<int>(most < sms[dev] ? most : sms[dev]);
   // Few tiles: parts of one tile each, so that a CTA has one run and joins one sum
-  if (!items && 2 * p.tiles <= grid) {
-    p.splits = grid / p.tiles < p.k_blocks ? grid / p.tiles : p.k_blocks;
-    grid = p.splits * p.tiles;
+  const int all = p.tiles * m_blocks;
+  if (!items && 2 * all <= grid) {
+    p.splits = grid / all < p.k_blocks ? grid / all : p.k_blocks;
+    grid = p.splits * all;
   }
   const int box = p.mb < kTsBox ? p.mb : kTsBox, boxes = (p.mb + box - 1) / box;
   const size_t kC = ts_codes() + ts_meta(fmt), xb = static_cast<size_t>(kTsSlots) * box * boxes * 256;
@@ -572,7 +584,7 @@ static int ts_gemm(int fmt, const void* x, int ldx, const void* codes, const voi
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto go = [&](auto f) {
     constexpr int F = decltype(f)::value;
-    return items ? launch_ts<F, true>(tx, p, box, boxes, grid, smem, st) : launch_ts<F, false>(tx, p, box, boxes, grid, smem, st);
+    return items ? launch_ts<F, true>(tx, p, m_blocks, box, boxes, grid, smem, st) : launch_ts<F, false>(tx, p, m_blocks, box, boxes, grid, smem, st);
   };
   switch (fmt) {
     case kFmtCubic4: return go(std::integral_constant<int, kFmtCubic4>());
@@ -585,10 +597,13 @@ static int ts_gemm(int fmt, const void* x, int ldx, const void* codes, const voi
 
 extern "C" {
 
-// Arguments as cb_wq_gemm_skinny; 4-bit weights, M <= 128, K a multiple of 128.  `workspace`: two fp32 tiles of the rows rounded up to 16 for every SM.
+// Arguments as cb_wq_gemm_skinny; 4-bit weights, K a multiple of 128; M in blocks of one size of up to 128 rows.
+// `workspace`: two fp32 tiles of a block's rows rounded up to 16 for every SM; `counters`: one for every weight tile and block.
 int cb_wq_gemm_ts(int fmt, const void* x, int ldx, const void* codes, const void* meta, void* y, int ldy, const void* residual, float alpha, int M, int N, int K,
                   int group_k, int swiglu, void* workspace, long long workspace_bytes, void* counters, void* status, void* stream) {
-  return cb::ts_gemm(fmt, x, ldx, codes, meta, y, ldy, residual, alpha, M, M, N, K, group_k, swiglu, nullptr, 0, 0, 0, workspace, workspace_bytes, counters, status, stream);
+  if (M <= 0) return -10;
+  const int blocks = (M + 127) / 128, mb = (M + blocks - 1) / blocks;
+  return cb::ts_gemm(fmt, x, ldx, codes, meta, y, ldy, residual, alpha, M, mb, N, K, group_k, swiglu, nullptr, 0, 0, 0, workspace, workspace_bytes, counters, status, stream);
 }
 
 // The grouped form over a device work list {count, then {expert, first row, rows}} of at most `max_items` items of at most `mb` <= 128 rows.

@@ -216,25 +216,36 @@ def skinny_rows_per_expert() -> int:
 
 
 def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None, residual: torch.Tensor | None = None, ws: "Workspace | None" = None) -> bool:
-    """Which batches of 4-bit weights the kernel with decoded tiles in tensor memory takes (``csrc/wq_gemm_ts.cu``): up to 128 rows of whole
-    units of 128 columns.  Its time hardly grows with the rows, but a tile's parts are summed behind a start of 3 us, so it wants six and a half units an SM.
-    8 / 48 / 128 rows, few-row or per-tile and persistent kernels -> this one: 24576 x 4096 27.4 / 38.7 / 44.5 -> 21.9 / 24.0 / 29.7 us,
-    4096 x 12288 17.2 / 25.5 / 28.3 -> 15.7 / 17.9 / 22.3, 6144 x 4096 13.2 / 18.9 / 21.4 -> 11.7 / 13.6 / 18.8, 4096 x 4096
-    10.0 / 13.2 / 15.5 -> 10.3 / 12.3 / 16.0; 5120 x 2048 (NVFP4) 9.2 / 11.3 / 13.3 -> 9.8 / 11.9 / 16.3.  (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration.)"""
-    if m > 128 or w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
+    """Which batches of 4-bit weights the kernel with decoded tiles in tensor memory takes (``csrc/wq_gemm_ts.cu``): whole units of 128 columns,
+    in blocks of up to 128 rows.  Its time hardly grows with the rows of a block, but a tile's parts are summed behind a start of 3 us: up to 128 rows it
+    wants six and a half units an SM.  8 / 48 / 128 rows, few-row or per-tile and persistent kernels -> this one: 24576 x 4096 27.4 / 38.7 / 44.5 ->
+    21.9 / 24.0 / 29.7 us, 4096 x 12288 17.2 / 25.5 / 28.3 -> 15.7 / 17.9 / 22.3, 6144 x 4096 13.2 / 18.9 / 21.4 -> 11.7 / 13.6 / 18.8, 4096 x 4096
+    10.0 / 13.2 / 15.5 -> 10.3 / 12.3 / 16.0; 5120 x 2048 (NVFP4) 9.2 / 11.3 / 13.3 -> 9.8 / 11.9 / 16.3.
+
+    129 to 512 rows: the other kernels decode a tile once for 256 rows and do the same work for 331 as for 512, here it is done for blocks of one size; from
+    28 units an SM, or where every tile has parts of its own.  In a loop over many weights, at the clocks that it settles at, 192 / 256 / 331 / 512 rows:
+    24576 x 4096 52.6 / 63.9 / 98.2 / 107.5 -> 52.0 / 57.8 / 77.1 / 104.2 us, 4096 x 12288 29.6 / 33.1 / 52.6 / 57.0 -> 27.7 / 30.7 / 41.1 / 54.6,
+    6144 x 4096 at 331 / 512 32.8 / 33.6 -> 24.2 / 31.4, 4096 x 4096 at 192 / 256 15.0 / 16.4 -> 12.7 / 14.2.  The lines: 4096 x 4096 at 512 rows (27.7 units)
+    23.4 against 24.3 here, 8192 x 2048 (NVFP4) at 256 (13.8) 16.1 against 19.8; at 768 / 1024 rows 24576 x 4096 150.2 / 189.1 against 150.3 / 196.2,
+    and prompts of 4096 rows whose projections took this kernel were 3 % slower although each alone was up to a tenth faster (cold, single launches).
+    (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration: fewer than 128 also keep it from more rows.)"""
+    if w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
         return False
     from .strategies import active
-    g = active().gemm
-    if m > g.tensor_memory_rows or w.k % 128 or (w.fmt == FMT_CUBIC4 and w.group_k % 128) or x.stride(0) % 8 or x.data_ptr() % 16:
+    most = active().gemm.tensor_memory_rows
+    if m > (most if most < 128 else 512) or w.k % 128 or (w.fmt == FMT_CUBIC4 and w.group_k % 128) or x.stride(0) % 8 or x.data_ptr() % 16:
         return False
     if out is not None and out.stride(0) % 4 == 0 and (out.data_ptr() | (0 if residual is None else residual.data_ptr())) % 8:
         return False
     sms = sm_count(x.device) if x.is_cuda else 148
-    if 2 * -(-w.n // 128) * (w.k // 128) < 13 * sms:
+    blocks = -(-m // 128)
+    tiles = -(-w.n // 128) * blocks
+    units = tiles * (w.k // 128)
+    if 2 * units < 13 * sms or m > 128 and units < 28 * sms and 2 * tiles > sms:
         return False
     if ws is not None:
-        parts = 2 * sms * -(-m // 16) * 16 * 128 * 4
-        return parts <= ws.gemm.numel() and -(-w.n // 128) <= ws.gemm_counters.numel()
+        parts = 2 * sms * -(-(-(-m // blocks)) // 16) * 16 * 128 * 4
+        return parts <= ws.gemm.numel() and tiles <= ws.gemm_counters.numel()
     return True
 
 

@@ -35,7 +35,7 @@ class GemmPolicy:
     pair_min_blocks: int = 80           # ... when every pair gets at least this many k-blocks (else one CTA per tile)
     few_rows_quantized: int = 16        # kernel without decoded tiles up to this many batch rows (0: never), 4-bit and block-scaled 8-bit weights ...
     few_rows_bf16: int = 8              # ... bf16 weights
-    tensor_memory_rows: int = 128       # 4-bit weights: kernel with decoded tiles in tensor memory up to this many batch rows, or rows of a work item (0: never)
+    tensor_memory_rows: int = 128       # 4-bit weights: kernel with decoded tiles in tensor memory up to this many batch rows (128: more in blocks), or rows of a work item (0: never)
     few_rows_bf16_streamed: int = 32    # ... bf16 weights with more tiles than SMs (lm_head)
 
 

@@ -118,3 +118,22 @@ def test_experts_with_two_tiles_for_every_sm(calls, routes, mb, n, k, fmt, entry
     assert calls.made.pop()[0] == entry
     assert K.rows_per_work_item(4096, 64, 64, (w,), 128) == (128 if n * k == 1536 * 2048 and fmt != wq_pack.FMT_BF16 else 96)
     assert K.rows_per_work_item(1024, 64, 64, (w,), 128) == 64 and K.rows_per_work_item(4096, 64, 160, (w,), 128) == 160
+
+
+@pytest.mark.parametrize("n,k,rows,others", [(24576, 4096, (129, 331, 512), (513, 8192)), (6144, 4096, (331, 512), (200, 600)), (4096, 4096, (129, 256), (331, 512)),
+                                            (2048, 4096, (200, 512), (513, 768)), (512, 1024, (), (129, 512))])
+def test_batches_of_more_rows_than_a_block(n, k, rows, others):
+    """28 units an SM, or parts of a tile's own, up to 512 rows: on both sides of the lines."""
+    w, ws = SimpleNamespace(fmt=wq_pack.FMT_NVFP4, n=n, k=k, group_k=16), _ws()
+    takes = lambda m, ws=ws: K.use_ts(m, w, torch.empty(m, k, dtype=torch.bfloat16), ws=ws)  # noqa: E731
+    assert all(takes(m) for m in rows) and not any(takes(m) for m in others)
+    for m in rows[:1]:
+        blocks = -(-m // 128)
+        need, tiles = 2 * 148 * -(-(-(-m // blocks)) // 16) * 16 * 512, n // 128 * blocks
+        assert takes(m, _ws(gemm=need, counters=tiles)) and not takes(m, _ws(gemm=need - 1)) and not takes(m, _ws(counters=tiles - 1))
+    old = strategies.active()
+    try:
+        strategies.install(strategies.operator_config_from_dict({"gemm": {"tensor_memory_rows": 112}}))
+        assert not any(takes(m) for m in rows)
+    finally:
+        strategies.install(old)

@@ -183,6 +183,36 @@ def test_gemm_with_decoded_tiles_in_tensor_memory(fmt, n, k):
     assert not ws.gemm_counters.any()
 
 
+@pytest.mark.parametrize("n,k", [
+    (200, 1152),           # parts of a block's tile of their own, 72 rows of padding
+    (3000, 640),           # whole tiles and parts
+    (128, 128),            # a unit a tile
+])
+@pytest.mark.parametrize("fmt", ["cubic", "affine", "nvfp4"])
+def test_gemm_with_decoded_tiles_in_tensor_memory_in_blocks_of_rows(fmt, n, k):
+    """The smallest second block, blocks of one size and a shorter last one, many blocks."""
+    from cubic_serve_b200.ops import kernels as K
+    w = _weight(fmt, n, k, n + k)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    ws = K.workspace(torch.device(DEV, 0))
+    for m in (129, 256, 331, 1030):
+        x, res = torch.randn(m, k, device=DEV, generator=g).bfloat16(), torch.randn(m, n, device=DEV, generator=g).bfloat16()
+        out = torch.full((m + 2, n + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+        K._wq_gemm_skinny(x, w, out[:m, :n], None, ws, False, "cb_wq_gemm_ts")
+        assert (out[:, n:] == 7).all() and (out[m:] == 7).all()
+        assert _close(out[:m, :n], K.wq_gemm(x, w, splits=1), k)
+        got = [K._wq_gemm_skinny(x, w, torch.empty(m, n, device=DEV, dtype=torch.bfloat16), res, ws, False, "cb_wq_gemm_ts") for _ in range(2)]
+        assert _close(got[0], K.wq_gemm(x, w, residual=res, splits=1), k) and torch.equal(*got)
+        if n % 128 == 0:
+            act = wq_pack.swiglu_interleave(w)
+            plain = wq_pack.PackedWeight(act.fmt, act.n, act.k, act.group_k, act.codes, act.meta, act.alpha)
+            gu = torch.empty(m, n, device=DEV, dtype=torch.bfloat16)
+            gu[:, wq_pack.swiglu_row_order(n // 2).to(DEV)] = K._wq_gemm_skinny(x, plain, torch.empty_like(gu), None, ws, False, "cb_wq_gemm_ts")
+            assert torch.equal(K._wq_gemm_skinny(x, act, torch.empty(m, n // 2, device=DEV, dtype=torch.bfloat16), None, ws, True, "cb_wq_gemm_ts"), K.swiglu(gu))
+    ws.check_status()
+    assert not ws.gemm_counters.any()
+
+
 @pytest.mark.parametrize("mb", [16, 48, 128])
 @pytest.mark.parametrize("fmt", ["cubic", "affine", "nvfp4"])
 def test_grouped_gemm_with_decoded_tiles_in_tensor_memory(fmt, mb):
@@ -225,7 +255,7 @@ def test_gemm_with_decoded_tiles_in_tensor_memory_refuses_what_it_does_not_take(
     from cubic_serve_b200.ops.native import NativeLibraryError
     ws = K.workspace(torch.device(DEV, 0))
     w = _weight("affine", 128, 128, 0)
-    for m, weight in ((129, w), (8, _weight("affine", 128, 192, 0)), (8, _weight("bf16", 128, 128, 0))):
+    for m, weight in ((0, w), (8, _weight("affine", 128, 192, 0)), (8, _weight("bf16", 128, 128, 0))):
         x = torch.zeros(m, weight.k, device=DEV, dtype=torch.bfloat16)
         assert not K.use_ts(m, weight, x)
         with pytest.raises(NativeLibraryError):
