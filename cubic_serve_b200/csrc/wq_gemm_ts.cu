@@ -43,6 +43,8 @@ struct __align__(16) TsCtl {
   uint32_t tmem, abort_word;
 };
 
+// Forms, each a kernel of its own: what blocks of rows add to every role's walk costs a matrix of one block 0.5 us (4096 x 12288 at 8 rows 16.3 against 15.7)
+static constexpr int kTsOneBlock = 0, kTsGrouped = 1, kTsRowBlocks = 2;
 // A run of units of one tile.
 struct TsRun {
   int tile, kb, kb_end, part, parts;
@@ -51,15 +53,16 @@ struct TsRun {
 };
 // The deal; every role walks the same list.  Work list: tile c, c + CTAs, .. of its items, whole.  p.splits > 0: CTA c has part c % splits of
 // tile c / splits; else the units of all tiles are dealt evenly.
-template <bool GROUPED>
+template <int FORM>
 struct TsWalk {
+  static constexpr bool GROUPED = FORM == kTsGrouped, BLOCKS = FORM == kTsRowBlocks;
   uint32_t u, u_end, total;
   int m_blocks;
   int tile, tiles, e, m0, rows;                  // work list: the next tile, its item
   __device__ __forceinline__ TsWalk(const WqGemmParams& p, int m_blocks_) : m_blocks(m_blocks_) {
     const uint32_t cta = blockIdx.x, ctas = gridDim.x;
     const uint32_t kbs = static_cast<uint32_t>(p.k_blocks);
-    total = static_cast<uint32_t>(GROUPED ? p.tiles : p.tiles * m_blocks) * kbs;
+    total = static_cast<uint32_t>(BLOCKS ? p.tiles * m_blocks : p.tiles) * kbs;
     if constexpr (GROUPED) {
       tiles = p.group_tiles[0] * p.tiles;
       tile = static_cast<int>(cta);
@@ -97,7 +100,7 @@ struct TsWalk {
       r.kb = static_cast<int>(u - first);
       r.kb_end = static_cast<int>(end - first);
       r.expert = 0; r.m0 = 0; r.rows = p.M;
-      if (p.M > p.mb) {                          // blocks of rows, those of a weight tile in turn
+      if constexpr (BLOCKS) {                    // those of a weight tile in turn
         r.tile = static_cast<int>(t) / m_blocks;
         r.m0 = (r.sum - r.tile * m_blocks) * p.mb;
         r.rows = min(p.mb, p.M - r.m0);
@@ -238,9 +241,10 @@ __device__ __forceinline__ void ts_out(const WqGemmParams& p, const TsRun& run, 
 
 // k_blocks counts units here, meta_k_blocks units of a table; tiles: weight tiles of a matrix; c_stages: depth of the code ring;
 // mb: most batch rows of a run, rounded up to 16
-template <int FMT, bool GROUPED>
+template <int FMT, int FORM>
 __global__ void __launch_bounds__(kTsThreads, 1)
 wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ WqGemmParams p, const int m_blocks, const int box, const int boxes) {
+  constexpr bool GROUPED = FORM == kTsGrouped, BLOCKS = FORM == kTsRowBlocks;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr uint32_t kC = ts_codes() + ts_meta(FMT);
   const uint32_t box_bytes = static_cast<uint32_t>(box) * 128u, x_half = box_bytes * boxes, x_bytes = 2 * x_half;
@@ -279,7 +283,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   pdl_launch_dependents();
   if constexpr (GROUPED) pdl_wait();             // the work list is written by the routing kernels
   const uint32_t tmem = ctl.tmem;
-  TsWalk<GROUPED> walk(p, m_blocks);
+  TsWalk<FORM> walk(p, m_blocks);
   TsRun run;
   bool ok = true;
 
@@ -393,7 +397,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       more = walk.next(p, next);
       const int b = runs & 1, used = runs >> 1;
       // (from lane 0: what the MMAs take has to be known to be the same in all lanes, or every one of them moves it to uniform registers)
-      const uint32_t acc = tmem_u + b * 128, idesc = __shfl_sync(0xffffffffu, umma_idesc(kTileN, static_cast<uint32_t>((run.rows + 15) & ~15), 1u, 1u), 0);
+      const uint32_t acc = tmem_u + b * 128, idesc = __shfl_sync(0xffffffffu, umma_idesc(kTileN, static_cast<uint32_t>(FORM == kTsOneBlock ? p.mb : (run.rows + 15) & ~15), 1u, 1u), 0);
       if (used > 0) ok = mbar_wait_park(smem_u32(&ctl.acc_empty[b]), (used - 1) & 1, abort_flag);
       for (int kb = run.kb; kb < run.kb_end; ++kb) {
         ok = __all_sync(0xffffffffu, ok && mbar_wait_park(smem_u32(&ctl.full[s]), phase, abort_flag));
@@ -468,7 +472,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   }
   // tiles in parts that are complete with this CTA's: summed by all threads, two parts (most weights have no more) of several places in flight
   for (int d = 0; !GROUPED && d < ctl.sums; ++d) {
-    const int parts = ctl.sum_parts[d], t = ctl.sum_tile[d], tile = t / m_blocks, m0 = (t - tile * m_blocks) * p.mb, c0 = static_cast<int>(blockIdx.x) - ctl.sum_part[d], shift = p.swiglu ? 4 : 5;
+    const int parts = ctl.sum_parts[d], t = ctl.sum_tile[d], tile = BLOCKS ? t / m_blocks : t, m0 = BLOCKS ? (t - tile * m_blocks) * p.mb : 0, c0 = static_cast<int>(blockIdx.x) - ctl.sum_part[d], shift = p.swiglu ? 4 : 5;
     auto part = [&](int q, int at) { return __ldcg(reinterpret_cast<const float4*>(ts_slot(p, c0 + q, q) + at)); };
     auto out = [&](int i, auto sum) {
       const int m = i >> shift, j = i & ((1 << shift) - 1);
@@ -481,7 +485,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         sk_store4<FMT>(p, m0 + m, tile * kTileN + j * 4, sum(i * 4));
       }
     };
-    const int n = min(p.mb, p.M - m0) << shift;
+    const int n = (BLOCKS ? min(p.mb, p.M - m0) : p.M) << shift;
     if (parts == 2) {
       for (int i = threadIdx.x; i < n; i += 2 * kTsThreads) {
         const int i2 = i + kTsThreads;
@@ -520,17 +524,17 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   if (threadIdx.x == 0 && ctl.abort_word) atomicExch(p.status, static_cast<uint32_t>(kErrBarrierTimeout));
 }
 
-template <int FMT, bool GROUPED>
+template <int FMT, int FORM>
 static int launch_ts(const CUtensorMap& tx, const WqGemmParams& p, int m_blocks, int box, int boxes, int grid, size_t smem, cudaStream_t stream) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -18;
   if (!configured[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(wq_gemm_ts_kernel<FMT, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    const cudaError_t e = cudaFuncSetAttribute(wq_gemm_ts_kernel<FMT, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured[dev] = true;
   }
-  return static_cast<int>(launch(wq_gemm_ts_kernel<FMT, GROUPED>, dim3(static_cast<unsigned>(grid)), dim3(kTsThreads), smem, stream, tx, p, m_blocks, box, boxes));
+  return static_cast<int>(launch(wq_gemm_ts_kernel<FMT, FORM>, dim3(static_cast<unsigned>(grid)), dim3(kTsThreads), smem, stream, tx, p, m_blocks, box, boxes));
 }
 
 // A matrix (mb = M), or with `items` the experts of a work list of at most `max_items` items of at most mb rows
@@ -584,7 +588,9 @@ static int ts_gemm(int fmt, const void* x, int ldx, const void* codes, const voi
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto go = [&](auto f) {
     constexpr int F = decltype(f)::value;
-    return items ? launch_ts<F, true>(tx, p, m_blocks, box, boxes, grid, smem, st) : launch_ts<F, false>(tx, p, m_blocks, box, boxes, grid, smem, st);
+    if (items) return launch_ts<F, kTsGrouped>(tx, p, m_blocks, box, boxes, grid, smem, st);
+    if (m_blocks > 1) return launch_ts<F, kTsRowBlocks>(tx, p, m_blocks, box, boxes, grid, smem, st);
+    return launch_ts<F, kTsOneBlock>(tx, p, m_blocks, box, boxes, grid, smem, st);
   };
   switch (fmt) {
     case kFmtCubic4: return go(std::integral_constant<int, kFmtCubic4>());
