@@ -33,7 +33,7 @@ class GemmPolicy:
     fuse_swiglu: bool = True            # SwiGLU in the epilogue of the gate/up GEMM (weight rows re-ordered at load)
     cta_pairs: bool = True              # persistent kernel on CTA pairs (cta_group::2) above stream_k_max_rows ...
     pair_min_blocks: int = 80           # ... when every pair gets at least this many k-blocks (else one CTA per tile)
-    few_rows_quantized: int = 16        # kernel without decoded tiles up to this many batch rows (0: never), 4-bit and block-scaled 8-bit weights ...
+    few_rows_quantized: int = 16        # kernel without decoded tiles up to this many batch rows (0: never), small 4-bit and block-scaled 8-bit weights ...
     few_rows_bf16: int = 8              # ... bf16 weights
     tensor_memory_rows: int = 128       # 4-bit weights: kernel with decoded tiles in tensor memory up to this many batch rows (128: more in blocks), or rows of a work item (0: never)
     few_rows_bf16_streamed: int = 32    # ... bf16 weights with more tiles than SMs (lm_head)
@@ -51,7 +51,7 @@ class MoePolicy:
     rows_per_item_large: int = 64
     large_routes_per_expert: int = 32
     rows_per_item_by_load: bool = True  # larger work items where a step gives an expert more rows; false: exactly the above
-    few_rows_per_expert: int = 16       # mean rows of an expert up to which 4-bit and block-scaled 8-bit experts take the kernel without decoded tiles (0: never)
+    few_rows_per_expert: int = 16       # mean rows of an expert up to which block-scaled 8-bit experts, and 4-bit ones of few tiles, take the kernel without decoded tiles (0: never)
 
 
 @dataclass(frozen=True)
