@@ -38,7 +38,11 @@ static constexpr int kPfRegs = 96, kPfRegsSoftmax = 136, kPfRegsConvert = 72, kP
 static_assert(2 * kPfRegsSoftmax + 2 * kPfRegsConvert + kPfRegsOther <= 5 * kPfRegs, "five warpgroups");
 static constexpr int kPfLists = 4;
 static constexpr int kPfRaw = 3;                         // steps of raw pages
-static constexpr int kPfNotes = 4;                       // steps whose powers of two are kept
+// Steps whose powers of two are kept.  Nothing else orders the note of step g + kPfNotes behind the reads of step g's: a tile that sees nothing of the
+// steps behind g holds back neither their scores nor k_free.  It holds back v_free of step g alone, whose product waits for the tile's probabilities,
+// and that reaches the conversion of K by way of the raw pages: note of K (s) <- raw_full (s) <- raw_free (s - kPfRaw) <- V of s - kPfRaw
+// converted <- v_free (s - kPfRaw - 2) <- p_full of every tile that takes part in it.
+static constexpr int kPfNotes = kPfRaw + 2;
 static constexpr int kPfSorted = 512;                    // groups of row blocks that are dealt by their length
 static constexpr float kPfGrowth = 2.f;
 // tensor memory, columns of a tile: scores, probabilities (two f16 a column), channels 0..63 of Q (likewise), output
@@ -681,7 +685,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm.s_free[t]));
-        // a note is written again four steps later, after MMAs that are issued after this step's softmax
+        // (a note is written again after this step's product, which waits for what follows: kPfNotes)
         if (ok) ok = mbar_wait_park(smem_u32(&sm.k_note[note]), (gs / kPfNotes) & 1, abort_flag);
         if (ok) ok = mbar_wait_park(smem_u32(&sm.v_note[note]), (gs / kPfNotes) & 1, abort_flag);
         if (sees < kPfTok) {

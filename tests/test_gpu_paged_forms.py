@@ -196,6 +196,29 @@ def test_prompt_form_with_scales_of_any_size(kb, vb, low, high):
     assert _close((got.cpu().double() / unit), ref / unit)
 
 
+@pytest.mark.parametrize("kb,vb,hkv", [(8, 8, 8), (4, 6, 16)])
+def test_prompt_form_with_one_tile_ahead_of_the_other(kb, vb, hkv):
+    """Items whose first tile sees one step and whose second sees many, the other way round, and with padding for a tile; several of a CTA."""
+    group, qb = 4, 4
+    kinds = [[(0, 32), (2000, 32)], [(700, 32), None], [(1500, 32), (3, 32)], [None, (64, 32)], [(0, 7), (129, 25), (900, 32)]]
+    portions, blocks, t = [], [], 0
+    for i in range(30):
+        for portion in kinds[i % 5]:
+            if portion is None:
+                blocks += [(0, 0, 0, 0)] * 8
+                continue
+            s, n = portion
+            blocks += [(len(portions), t + o, min(qb, n - o), s + o + 1) for o in range(0, n, qb)]
+            portions.append(portion)
+            t += n
+        blocks += [(0, 0, 0, 0)] * (-len(blocks) % 16)
+    assert len(blocks) // 16 * hkv > torch.cuda.get_device_properties(0).multi_processor_count
+    cache, table = _cache([s + n for s, n in portions], hkv, kb, vb, 17)
+    q = torch.randn(t, group * hkv, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(7)).bfloat16()
+    want = _run("", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1)
+    assert _close(_run("prefill", q, cache, table, blocks, group * hkv, hkv, kb, vb, 1), want)
+
+
 @pytest.mark.parametrize("form,splits", [("", 1), ("decode", 1), ("decode", 4), ("prefill", 1)])
 def test_rows_that_see_no_token_are_zero(form, splits):
     """Alone in their CTA and beside rows that see something."""
