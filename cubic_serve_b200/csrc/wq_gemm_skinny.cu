@@ -20,8 +20,8 @@
 // Large 4-bit weights go to wq_gemm_ts.cu.  Measured, weights not in L2 (floor = packed bytes / 6.65 TB/s), Cubic weights, 8 rows: 24576 x 4096
 // 22.3 us (floor 9.5, tcgen05 kernels with decoded tiles in shared memory 34), 4096 x 12288 12.8 (4.7, 21.5), 6144 x 4096 9.1 (2.4, 14.8), 4096 x 4096
 // 6.4 (1.6, 10.1); bf16 50688 x 4096 65 (62, 98).  Block-scaled e4m3 weights have nothing to decode either: their chunks and those of the e4m3
-// activations are the operands of m16n8k32; 128 experts of 3072 x 4096, eight rows each, 267 us (floor 246, tcgen05 kernel 409), 4096 x 1536 145
-// (123, 289).  What is left above the floor of 4-bit weights is the decode (integer pipe 38 % busy, four warps a scheduler that issue in 37 % of
+// activations are the operands of m16n8k16 once they are f16; 128 experts of 3072 x 4096, eight rows each, 263 us (floor 246, tcgen05 kernel 409),
+// 4096 x 1536 140 (123, 289).  What is left above the floor of 4-bit weights is the decode (integer pipe 38 % busy, four warps a scheduler that issue in 37 % of
 // the cycles) and 5 us of start, last loads and the sum of the parts.
 #include "wq_gemm_common.cuh"
 #include "launch.cuh"
@@ -68,11 +68,15 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_f16_f32(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// four e4m3 values -> two pairs of f16 (exact)
+__device__ __forceinline__ void e4m3_to_f16(uint32_t w, uint32_t& lo, uint32_t& hi) {
+  asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, a;\n\tcvt.rn.f16x2.e4m3x2 %1, b;\n\t}" : "=r"(lo), "=r"(hi) : "r"(w));
 }
 
 // A run of iterations of one tile.
@@ -263,42 +267,60 @@ __device__ __forceinline__ void sn_compute(float (&acc)[2][NB][4], uint32_t stag
 }
 
 // One iteration of a warp with e4m3 weights and activations: the 128 columns of its half are a scale block, whose product is summed from zero
-// and joins the accumulators times the block's scale.  Lane t takes the chunks 2 t and 2 t + 1 of every row.
+// and joins the accumulators times the block's scale.  Lane t takes the chunks 2 t and 2 t + 1 of every row.  Both operands become f16, which has
+// every e4m3 value: a weight is converted once for sixteen batch rows and an activation once for the warp's 32 features, where m16n8k32 of e4m3
+// took as long as if it converted both for each product.  128 experts of 3072 x 4096, 16 rows each, 411 -> 394 us, of 4096 x 1536 210 -> 185; 1024 routes
+// on 8 of them (128 rows each, in eight passes) 162 + 90 -> 125 + 72, where the tcgen05 kernel takes 120 + 96.
 template <int NB>
 __device__ __forceinline__ void sn_compute_fp8(float (&acc)[2][NB][4], uint32_t stage, int nb_used, int rg, int kg, int g, int t, float scale) {
   using Sh = SnShape<kFmtFp8Block, NB>;
   const uint32_t arow = stage + Sh::kXBytes + kg * kATileBytes + (rg * 32 + g) * 128, xa = stage + kg * Sh::kXTile + g * 128;
-  float part[2][NB][4];
+  constexpr int W = NB < 2 ? NB : 2;
 #pragma unroll
-  for (int rt = 0; rt < 2; ++rt)
+  for (int n0 = 0; n0 < NB; n0 += W) {
+    if (n0 > 0 && n0 >= nb_used) break;
+    float part[2][W][4];
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
+    for (int rt = 0; rt < 2; ++rt)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) part[rt][nb][c] = 0.f;
+      for (int nb = 0; nb < W; ++nb)
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const uint32_t o = ((2 * t + j) ^ g) << 4;
-    uint4 b[NB];
+        for (int c = 0; c < 4; ++c) part[rt][nb][c] = 0.f;
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
-      if (NB == 1 || nb < nb_used) b[nb] = lds16(xa + nb * 1024 + o);
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t o = ((2 * t + j) ^ g) << 4;
+      uint32_t b[W][8];
 #pragma unroll
-    for (int rt = 0; rt < 2; ++rt) {
-      const uint4 l = lds16(arow + 2 * rt * 1024 + o), u = lds16(arow + (2 * rt + 1) * 1024 + o);
-#pragma unroll
-      for (int nb = 0; nb < NB; ++nb)
-        if (NB == 1 || nb < nb_used) {
-          mma_e4m3(part[rt][nb], l.x, u.x, l.y, u.y, b[nb].x, b[nb].y);
-          mma_e4m3(part[rt][nb], l.z, u.z, l.w, u.w, b[nb].z, b[nb].w);
+      for (int nb = 0; nb < W; ++nb)
+        if (NB == 1 || n0 + nb < nb_used) {
+          const uint4 x = lds16(xa + (n0 + nb) * 1024 + o);
+          e4m3_to_f16(x.x, b[nb][0], b[nb][1]);
+          e4m3_to_f16(x.y, b[nb][2], b[nb][3]);
+          e4m3_to_f16(x.z, b[nb][4], b[nb][5]);
+          e4m3_to_f16(x.w, b[nb][6], b[nb][7]);
         }
+#pragma unroll
+      for (int rt = 0; rt < 2; ++rt) {
+        const uint4 l = lds16(arow + 2 * rt * 1024 + o), u = lds16(arow + (2 * rt + 1) * 1024 + o);
+        const uint32_t lw[4] = {l.x, l.y, l.z, l.w}, uw[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          uint32_t a0, a1, a2, a3;
+          e4m3_to_f16(lw[w], a0, a2);
+          e4m3_to_f16(uw[w], a1, a3);
+#pragma unroll
+          for (int nb = 0; nb < W; ++nb)
+            if (NB == 1 || n0 + nb < nb_used) mma_f16_f32(part[rt][nb], a0, a1, a2, a3, b[nb][2 * w], b[nb][2 * w + 1]);
+        }
+      }
     }
+#pragma unroll
+    for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+      for (int nb = 0; nb < W; ++nb)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[rt][n0 + nb][c] = fmaf(scale, part[rt][nb][c], acc[rt][n0 + nb][c]);
   }
-#pragma unroll
-  for (int rt = 0; rt < 2; ++rt)
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[rt][nb][c] = fmaf(scale, part[rt][nb][c], acc[rt][nb][c]);
 }
 
 __device__ __forceinline__ void sn_bar() { asm volatile("bar.sync 1, %0;" ::"r"(kSnConsumers) : "memory"); }

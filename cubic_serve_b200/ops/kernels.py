@@ -208,9 +208,12 @@ SKINNY_ROWS_PER_EXPERT: int | None = None
 
 def skinny_rows_per_expert() -> int:
     """6 / 12 / 16 / 24 rows of 128 experts of 1536 x 2048 (NVFP4) take 82 / 103 / 107 / 134 us against 125 us of the per-tile tcgen05 kernel at
-    any of them (``use_ts_grouped`` comes first).  1 / 8 / 12 / 16 / 24 rows of 128 experts with block-scaled e4m3 weights of 3072 x 4096 take 173 / 267 / 346 / 411 / 571 us
-    against 270 / 409 / 410 / 411 / 419 (the tcgen05 kernel sets up a tile for each of its CTAs), of 4096 x 1536 96 / 145 / 182 / 210 / 281 against
-    190 / 289 / 290 / 290 / 297."""
+    any of them (``use_ts_grouped`` comes first).  1 / 8 / 12 / 16 rows of 128 experts with block-scaled e4m3 weights of 3072 x 4096 take 173 / 263 / 319 / 394 us
+    against 270 / 409 / 410 / 411 (the tcgen05 kernel sets up a tile for each of its CTAs), of 4096 x 1536 96 / 141 / 166 / 186 against 190 / 290 / 292 / 295.
+    The mean decides, because the loads are known on the device alone: an expert with more rows takes a pass for each sixteen, where an item of the other
+    kernel holds 32.  256 / 512 / 1024 / 2048 routes, all on eight of the experts: 51 / 73 / 124 / 217 and 26 / 40 / 72 / 122 us against 47 / 71 / 120 / 215 and
+    45 / 63 / 96 / 162; 1024 routes on 32 150 and 79 against 125 and 103, 2048 on 64 267 and 130 against 224 and 172.  The two launches of a layer together take
+    as long or less in each of these.  (Weights not in L2, one B200.)"""
     from .strategies import active
     return active().moe.few_rows_per_expert if SKINNY_ROWS_PER_EXPERT is None else SKINNY_ROWS_PER_EXPERT
 

@@ -260,3 +260,69 @@ def test_gemm_with_decoded_tiles_in_tensor_memory_refuses_what_it_does_not_take(
         assert not K.use_ts(m, weight, x)
         with pytest.raises(NativeLibraryError):
             K._wq_gemm_skinny(x, weight, torch.empty(m, 128, device=DEV, dtype=torch.bfloat16), None, ws, False, "cb_wq_gemm_ts")
+
+
+def _moe_layer(weight, E, H, I, skew, tokens):
+    """A layer of experts with eight routes a token, and rows for it; with ``skew`` every token goes to the same eight experts."""
+    from cubic_serve_b200.models.moe import MoeLayer, stack_experts
+    gu, c0, m0 = stack_experts([weight(2 * I, H, e) for e in range(E)])
+    dn, c1, m1 = stack_experts([weight(H, I, 100 + e) for e in range(E)])
+    router = torch.randn(E, H, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)) * 0.1
+    x = torch.randn(tokens, H, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4)).bfloat16()
+    if skew:
+        x[:, 0] = 8.0
+        router[:8, 0] += 10.0
+    return MoeLayer(wq_pack.pack_bf16(router), gu, dn, (c0, m0, c1, m1), E, 8, 0, E, True), x
+
+
+def _same_by_other_kernels(layer, x, monkeypatch, change, entries):
+    """``layer.forward(x)`` calls the first of ``entries``, under ``change`` the second, with the same results."""
+    from cubic_serve_b200.ops import kernels as K, native
+    called, lib = [], native.lib()
+
+    class Spy:
+        def __getattr__(self, name):
+            if "grouped" in name:
+                called.append(name)
+            return getattr(lib, name)
+    monkeypatch.setattr(K.native, "lib", lambda spy=Spy(): spy)
+    got = layer.forward(x).clone()
+    change()
+    want = layer.forward(x).clone()
+    K.workspace(torch.device(DEV, 0)).check_status()
+    assert called == [entries[0]] * 2 + [entries[1]] * 2
+    # two chained products: a flipped rounding of an activation moves a result by a part of a bf16 step
+    assert torch.isfinite(got).all() and ((got.float() - want.float()).norm() / want.float().norm()).item() < 2e-3
+
+
+@pytest.mark.parametrize("skew", [False, True])
+@pytest.mark.parametrize("tokens", [1, 60, 120])
+def test_layer_of_block_scaled_experts(tokens, skew, monkeypatch):
+    """Few rows an expert on average, with ``skew`` many of eight that take several passes."""
+    from cubic_serve_b200.ops import kernels as K
+    g = torch.Generator(device=DEV).manual_seed(5)
+
+    def weight(n, k, seed):
+        return wq_pack.pack_fp8_block((torch.randn(n, k, device=DEV, generator=g) * 100).clamp_(-448, 448).to(torch.float8_e4m3fn),
+                                      (torch.rand(-(-n // 128), -(-k // 128), device=DEV, generator=g) + 0.5) * 2e-4)
+    layer, x = _moe_layer(weight, 64, 512, 256, skew, tokens)
+    _same_by_other_kernels(layer, x, monkeypatch, lambda: monkeypatch.setattr(K, "SKINNY_ROWS_PER_EXPERT", 0),
+                           ("cb_wq_gemm_skinny_fp8_grouped", "cb_wq_gemm_fp8_grouped"))
+
+
+@pytest.mark.parametrize("skew", [False, True])
+@pytest.mark.parametrize("fmt", ["cubic", "nvfp4"])
+@pytest.mark.parametrize("tokens", [30, 512, 1100])
+def test_layer_of_4_bit_experts_in_tensor_memory(fmt, tokens, skew, monkeypatch):
+    """Small work items, and items of 128 rows: the load of an expert is above the least ones."""
+    from cubic_serve_b200.ops import kernels as K, strategies
+    layer, x = _moe_layer(lambda n, k, seed: _weight(fmt, n, k, seed), 64, 640, 384, skew, tokens)
+    old = strategies.active()
+    try:
+        _same_by_other_kernels(layer, x, monkeypatch, lambda: strategies.install(strategies.operator_config_from_dict({"gemm": {"tensor_memory_rows": 0}})),
+                               ("cb_wq_gemm_ts_grouped", "cb_wq_gemm_skinny_grouped" if tokens == 30 and K.skinny_fits(layer.down, x, x) else "cb_wq_gemm_grouped"))
+        strategies.install(old)
+        layer.forward(x)
+        assert layer.scratch.mb == (32 if tokens == 30 else 128)
+    finally:
+        strategies.install(old)
