@@ -220,16 +220,24 @@ def skinny_rows_per_expert() -> int:
 
 def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None, residual: torch.Tensor | None = None, ws: "Workspace | None" = None) -> bool:
     """Which batches of 4-bit weights the kernel with decoded tiles in tensor memory takes (``csrc/wq_gemm_ts.cu``): whole units of 128 columns,
-    in blocks of up to 128 rows.  Its time hardly grows with the rows of a block, but a tile's parts are summed behind a start of 3 us: up to 128 rows it
-    wants six and a half units an SM.  8 / 48 / 128 rows, few-row or per-tile and persistent kernels -> this one: 24576 x 4096 27.4 / 38.7 / 44.5 ->
-    21.9 / 24.0 / 29.7 us, 4096 x 12288 17.2 / 25.5 / 28.3 -> 15.7 / 17.9 / 22.3, 6144 x 4096 13.2 / 18.9 / 21.4 -> 11.7 / 13.6 / 18.8, 4096 x 4096
-    10.0 / 13.2 / 15.5 -> 10.3 / 12.3 / 16.0; 5120 x 2048 (NVFP4) 9.2 / 11.3 / 13.3 -> 9.8 / 11.9 / 16.3.
+    in blocks of up to 128 rows.  Its time hardly grows with the rows of a block, but it starts for 3 us, and where a tile is dealt to several CTAs their
+    sums of the block's rows are added up at the end.  Few-row kernel up to 16 rows, then per-tile and persistent kernels -> this one, 8 / 16 / 32 / 64 / 96 / 128
+    rows, Cubic weights (the other formats within 5 %): 24576 x 4096 27.7 / 31.7 / 37.9 / 39.8 / - / 44.2 -> 22.5 / 22.4 / 23.2 / 25.5 / - / 30.4 us, 6144 x 4096
+    13.0 / 15.0 / 18.3 / 19.5 / 20.5 / 21.3 -> 11.7 / 11.9 / 13.0 / 14.5 / 16.3 / 18.7, 5120 x 4096 11.8 / 14.1 / 15.0 / 16.1 / 17.0 / 18.0 -> 11.5 / 11.7 / 12.8 / 14.1 / 15.7 / 17.9,
+    4096 x 4096 10.4 / 11.8 / 12.8 / 13.7 / 14.7 / 15.9 -> 10.6 / 10.5 / 11.9 / 13.0 / 14.3 / 16.3, 8192 x 2048 9.5 / 11.3 / 12.7 / 13.6 / 14.4 / 15.4 -> 10.3 / 10.6 / 11.0 / 12.1 / 13.1 / 14.3,
+    14336 x 1024 9.6 / 11.1 / 11.3 / 12.1 / 12.7 / 13.5 -> 11.2 / 11.4 / 12.8 / 13.7 / 16.3 / 20.5.
+    - Up to 8 rows the few-row kernel has next to nothing to do but to read: eight and a half units an SM (5120 x 4096 has 8.6, 4608 x 4096 7.8: 10.3 against
+      10.5).  From 9 rows, which take it a second pass, six and a half (8192 x 2048 has 6.9, 14336 x 1024 6.1).
+    - From 65 rows the sums count.  Tiles of several parts of their own: up to 480 rows times parts (4096 x 4096 at 96: 384), or ten units a part (2560 x 9728 has
+      10.9, at 128 rows 20.6 -> 20.8; 3584 x 5120 8, 16.9 -> 17.9; 1024 x 16384 7.1, 21.7 -> 28.6).  Tiles dealt across their borders: ten units an SM from 97 rows (6144 x
+      4096 has 10.4, 10240 x 2048 8.6: 18.5 -> 18.2 at 96, 19.5 -> 21.3 at 128).
 
     129 to 512 rows: the other kernels decode a tile once for 256 rows and do the same work for 331 as for 512, here it is done for blocks of one size; from
     28 units an SM, or where every tile has parts of its own.  In a loop over many weights, at the clocks that it settles at, 192 / 256 / 331 / 512 rows:
     24576 x 4096 52.6 / 63.9 / 98.2 / 107.5 -> 52.0 / 57.8 / 77.1 / 104.2 us, 4096 x 12288 29.6 / 33.1 / 52.6 / 57.0 -> 27.7 / 30.7 / 41.1 / 54.6,
     6144 x 4096 at 331 / 512 32.8 / 33.6 -> 24.2 / 31.4, 4096 x 4096 at 192 / 256 15.0 / 16.4 -> 12.7 / 14.2.  The lines: 4096 x 4096 at 512 rows (27.7 units)
-    23.4 against 24.3 here, 8192 x 2048 (NVFP4) at 256 (13.8) 16.1 against 19.8; at 768 / 1024 rows 24576 x 4096 150.2 / 189.1 against 150.3 / 196.2,
+    23.4 against 24.3 here, 8192 x 2048 (NVFP4) at 256 (13.8) 16.1 against 19.8; parts of their own up to 1000 rows of a block times parts (1024 x 8192 at 192: 864,
+    18.0 -> 17.6, at 256: 1152, 19.8 -> 20.9; single cold launches); at 768 / 1024 rows 24576 x 4096 150.2 / 189.1 against 150.3 / 196.2,
     and prompts of 4096 rows whose projections took this kernel were 3 % slower although each alone was up to a tenth faster (cold, single launches).
     (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration: fewer than 128 also keep it from more rows.)"""
     if w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
@@ -244,10 +252,20 @@ def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = 
     blocks = -(-m // 128)
     tiles = -(-w.n // 128) * blocks
     units = tiles * (w.k // 128)
-    if 2 * units < 13 * sms or m > 128 and units < 28 * sms and 2 * tiles > sms:
+    own = sms // tiles if 2 * tiles <= sms else 0          # parts of a tile, if every one has some of its own
+    rows = -(-m // blocks)
+    if 2 * units < (17 if m <= 8 else 13) * sms:
+        return False
+    if m > 128:
+        if rows * own > 1000 if own else units < 28 * sms:
+            return False
+    elif m > 64 and own:
+        if rows * own > 480 and units < 10 * own * tiles:
+            return False
+    elif m > 96 and units < 10 * sms:
         return False
     if ws is not None:
-        parts = 2 * sms * -(-(-(-m // blocks)) // 16) * 16 * 128 * 4
+        parts = 2 * sms * -(-rows // 16) * 16 * 128 * 4
         return parts <= ws.gemm.numel() and tiles <= ws.gemm_counters.numel()
     return True
 
