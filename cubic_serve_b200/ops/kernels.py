@@ -239,12 +239,13 @@ def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = 
     23.4 against 24.3 here, 8192 x 2048 (NVFP4) at 256 (13.8) 16.1 against 19.8; parts of their own up to 1000 rows of a block times parts (1024 x 8192 at 192: 864,
     18.0 -> 17.6, at 256: 1152, 19.8 -> 20.9; single cold launches); at 768 / 1024 rows 24576 x 4096 150.2 / 189.1 against 150.3 / 196.2,
     and prompts of 4096 rows whose projections took this kernel were 3 % slower although each alone was up to a tenth faster (cold, single launches).
-    (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration: fewer than 128 also keep it from more rows.)"""
+    (Weights not in L2, one B200; ``tensor_memory_rows`` and ``tensor_memory_rows_in_blocks`` in the operator configuration.)"""
     if w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4):
         return False
     from .strategies import active
-    most = active().gemm.tensor_memory_rows
-    if m > (most if most < 128 else 512) or w.k % 128 or (w.fmt == FMT_CUBIC4 and w.group_k % 128) or x.stride(0) % 8 or x.data_ptr() % 16:
+    g = active().gemm
+    most = g.tensor_memory_rows if m <= 128 or g.tensor_memory_rows < 128 else g.tensor_memory_rows_in_blocks
+    if m > most or w.k % 128 or (w.fmt == FMT_CUBIC4 and w.group_k % 128) or x.stride(0) % 8 or x.data_ptr() % 16:
         return False
     if out is not None and out.stride(0) % 4 == 0 and (out.data_ptr() | (0 if residual is None else residual.data_ptr())) % 8:
         return False

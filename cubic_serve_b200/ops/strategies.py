@@ -35,7 +35,8 @@ class GemmPolicy:
     pair_min_blocks: int = 80           # ... when every pair gets at least this many k-blocks (else one CTA per tile)
     few_rows_quantized: int = 16        # kernel without decoded tiles up to this many batch rows (0: never), small 4-bit and block-scaled 8-bit weights ...
     few_rows_bf16: int = 8              # ... bf16 weights
-    tensor_memory_rows: int = 128       # 4-bit weights: kernel with decoded tiles in tensor memory up to this many batch rows (128: more in blocks), or rows of a work item (0: never)
+    tensor_memory_rows: int = 128       # 4-bit weights: kernel with decoded tiles in tensor memory up to this many batch rows, or rows of a work item (0: never) ...
+    tensor_memory_rows_in_blocks: int = 512     # ... and, if those are 128, up to this many in blocks of up to 128 (128 and fewer: never)
     few_rows_bf16_streamed: int = 32    # ... bf16 weights with more tiles than SMs (lm_head)
 
 
@@ -70,6 +71,8 @@ class OperatorConfig:
             raise ValueError("gemm.few_rows_* must be in [0, 32]")
         if not 0 <= g.tensor_memory_rows <= 128:
             raise ValueError("gemm.tensor_memory_rows must be in [0, 128]")
+        if g.tensor_memory_rows_in_blocks < 0:
+            raise ValueError("gemm.tensor_memory_rows_in_blocks must not be negative")
         if a.target_ctas < 1 or not 1 <= a.max_splits <= 64:
             raise ValueError("attention policy out of range")
         for v in (m.rows_per_item_small, m.rows_per_item_large):

@@ -147,3 +147,16 @@ def test_lines_of_the_kernel_with_tiles_in_tensor_memory(n, k, takes, others):
     w = SimpleNamespace(fmt=wq_pack.FMT_CUBIC4, n=n, k=k, group_k=128)
     use = {m: K.use_ts(m, w, torch.empty(m, k, dtype=torch.bfloat16), ws=_ws()) for m in takes + others}
     assert use == {m: m in takes for m in takes + others}
+
+
+def test_blocks_of_rows_have_a_limit_of_their_own():
+    w, ws, old = SimpleNamespace(fmt=wq_pack.FMT_CUBIC4, n=24576, k=4096, group_k=128), _ws(), strategies.active()
+    takes = lambda m: K.use_ts(m, w, torch.empty(m, 4096, dtype=torch.bfloat16), ws=ws)  # noqa: E731
+    try:
+        for most, rows, others in ((0, (1, 128), (129, 512)), (300, (128, 129, 300), (301, 512)), (700, (128, 512, 700), (701,))):
+            strategies.install(strategies.operator_config_from_dict({"gemm": {"tensor_memory_rows_in_blocks": most}}))
+            assert all(takes(m) for m in rows) and not any(takes(m) for m in others)
+        with pytest.raises(ValueError):
+            strategies.install(strategies.operator_config_from_dict({"gemm": {"tensor_memory_rows_in_blocks": -1}}))
+    finally:
+        strategies.install(old)
