@@ -4,11 +4,14 @@
 // What bounds it: shared memory, then the MMAs.  An item is sixteen consecutive row blocks -- 256 rows, two tiles of one tcgen05 MMA each --
 // of a key / value head; a CTA takes items one after the other and converts a step of 64 tokens once for both tiles.
 // A cached value is a code of at most 8 bits times an fp32 scale, one per token and 32 channels.  The conversion writes it as a sum of two f16
-// (hi + lo, 22 bits and more), so that a step's scores and its output are one chain of MMAs each.  Scales inside the softmax would take
+// (hi + lo), so that a step's scores and its output are one chain of MMAs each.  Scales inside the softmax would take
 // four score tiles and four copies of the probabilities, one per channel group (what this kernel did before: 256 multiply-adds, 256 multiplications
 // and 128 packings a row and step instead of 64, 0 and 32; 5800 cycles a step of 128 rows).
-// Powers of two keep hi and lo in the range of f16: one a step for K, undone in the softmax' multiply-add; one for V that grows with
-// the largest scale seen, undone with the output.
+// Powers of two keep hi and lo in the range of f16: one a step for K, undone in the softmax' multiply-add; one for V that grows with the
+// largest scale of a run of steps, falls back towards one, and is undone with the output (a row keeps that of its own request's steps).
+// What is 2^-k of the largest scale keeps 22 bits up to k = 6 to 8, then 28 - k; probabilities have 11.  A product's error stays below 2^-18 (V) and 2^-20 (K) as long
+// as the largest scale is below 16 (values of 2000), as far as f16 products of probabilities and scales would go.  Beyond that, and with V
+// scales that are not finite, the rows that see such tokens are computed once more, in fp32 from the pages (pf_row).
 // MMAs of a step take 640 + 512 cycles a tile (measured in a loop of their own); with their operands, raw pages and the conversion's stores shared memory
 // moves about 280 KB a step: 4000 cycles a step of 256 rows where 2 x 5800 were spent.  General kernel -> before -> now, one B200, cold L2, 32 heads
 // over 8, 8 bits: 8 x 1024 tokens 702 -> 520 -> 220 us, 4 x 256 behind 2048 276 -> 233 -> 104, one prompt of 8192 3734 -> 2775 -> 1275, 40 x 20 behind 300
@@ -24,6 +27,7 @@
 // then probabilities relative to the older maximum are at most 4.
 // Every wait is bounded; on a timeout the roles leave, the status word is set and tensor memory is freed.
 #include "paged_attn.cuh"
+#include <limits.h>
 
 namespace cb {
 
@@ -45,6 +49,8 @@ static constexpr int kPfRaw = 3;                         // steps of raw pages
 static constexpr int kPfNotes = kPfRaw + 2;
 static constexpr int kPfSorted = 512;                    // groups of row blocks that are dealt by their length
 static constexpr float kPfGrowth = 2.f;
+static constexpr int kPfLarge = 3;                       // exponent of scales from which on small ones beside them are looked at
+static constexpr int kPfVFall = 80;                      // most by which v_exp falls in a run: outputs in its units stay below 2^(37 + 80)
 // tensor memory, columns of a tile: scores, probabilities (two f16 a column), channels 0..63 of Q (likewise), output
 static constexpr uint32_t kPfTmemCols = 512, kPfTmemTile = 256, kPfTmemP = 64, kPfTmemQ = 96, kPfTmemO = 128;
 static constexpr int kPfHalf = kPfTok * 128;             // bytes of 64 channels of a step
@@ -62,9 +68,9 @@ struct __align__(1024) PfSmem {
   uint8_t q[kPfTiles][kPfRows * 128];                    // f16, channels 64..127: [row][128 B], 16-byte chunk ^ (row & 7)
   uint8_t k[2][2][2 * kPfHalf];                          // f16 [stage][hi, lo][64-channel half][token][128 B]
   uint8_t v[2][2][2 * kPfHalf];                          // likewise
-  float vw[kPfNotes][4 * kPfTok];                        // of a step, [channel group][token]: V scales that are not finite, else 0
   float k_mul[kPfNotes];                                 // scores are this times what the MMAs give
-  int v_exp[kPfNotes], wild[kPfNotes];                   // output is 2^v_exp times ...; vw is written
+  int v_exp[kPfNotes];                                   // output is 2^v_exp times ...
+  int redo[kPfLists][kPfBlocks], redo_least[kPfLists];   // of a run, of all: rows that see more tokens than this are computed once more
   uint64_t raw_full[kPfRaw], raw_free[kPfRaw], k_full[2], k_free[2], v_full[2], v_free[2], k_note[kPfNotes], v_note[kPfNotes];
   uint64_t list_full[kPfLists], list_free[kPfLists], q_full[kPfTiles], s_full[kPfTiles], s_free[kPfTiles], p_full[kPfTiles], pv_done[kPfTiles];
   PfList list[kPfLists];
@@ -140,26 +146,25 @@ __device__ __forceinline__ void pf_split(float s, uint32_t& sh, uint32_t& sl) {
   sl = pack_f16x2(r, r);
 }
 
-// The largest finite scale of a step's visible tokens, as its exponent (at least -100); every warp finds it for itself.  `of`: the thread's scales, of
-// tokens `lane` and `lane` + 32; `odd`: some scale is not finite.
-__device__ __forceinline__ int pf_exponent(const uint8_t* scales, int stride, int visible, int lane, float4 (&of)[2], bool& odd) {
-  uint32_t most = 0;
-  odd = false;
+// The largest magnitude of a token's scales, as bits; FINITE: of those that are
+template <bool FINITE>
+__device__ __forceinline__ uint32_t pf_most(const float4& s) {
+  auto magnitude = [](float x) {
+    const uint32_t b = __float_as_uint(x) & 0x7FFFFFFFu;
+    return !FINITE || b < 0x7F800000u ? b : 0u;
+  };
+  return max(max(magnitude(s.x), magnitude(s.y)), max(magnitude(s.z), magnitude(s.w)));
+}
+__device__ __forceinline__ int pf_exponent(uint32_t magnitude) { return max(static_cast<int>(magnitude >> 23) - 127, -100); }
+
+// The scales of a step's tokens `lane` and `lane` + 32, zeros from `visible` on
+__device__ __forceinline__ void pf_scales(const uint8_t* scales, int stride, int visible, int lane, float4 (&of)[2]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int tok = lane + 32 * h;
     of[h] = *reinterpret_cast<const float4*>(scales + (tok >> 4) * stride + (tok & 15) * 16);
     if (tok >= visible) of[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float f[4] = {of[h].x, of[h].y, of[h].z, of[h].w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t x = __float_as_uint(f[j]) & 0x7FFFFFFFu;
-      if (x < 0x7F800000u) most = max(most, x);
-      else odd = true;
-    }
   }
-  odd = __any_sync(0xffffffffu, odd);
-  return max(static_cast<int>(__reduce_max_sync(0xffffffffu, most) >> 23) - 127, -100);
 }
 
 // One step's codes into operands: all of a thread's loads, then its arithmetic (few warps hide nothing).
@@ -217,8 +222,7 @@ __device__ __forceinline__ void pf_convert_k(uint8_t (&k)[2][2 * kPfHalf], const
     }
   }
 }
-// V from `visible` on becomes zeros: those slots may hold anything, and a probability of zero has to stay zero.  A scale that is not finite is
-// left out (code times one): pf_wild adds its product for the rows that see it.
+// V from `visible` on becomes zeros: those slots may hold anything, and a probability of zero has to stay zero.  Likewise where a scale is not finite.
 template <int VBITS>
 __device__ __forceinline__ void pf_convert_v(uint8_t (&v)[2][2 * kPfHalf], const uint8_t* raw, int stride, const KvLayout& lay, int visible, float mul, int tid) {
   constexpr uint32_t vb = VBITS == 8 ? 0x64806480u : VBITS == 6 ? 0x64206420u : 0x64086408u;
@@ -259,7 +263,8 @@ __device__ __forceinline__ void pf_convert_v(uint8_t (&v)[2][2 * kPfHalf], const
         }
         codes = conv8(n, vb);
       }
-      const float f = tok >= visible ? 0.f : fabsf(s[j][h]) < INFINITY ? s[j][h] * mul : 1.f;
+      float f = s[j][h] * mul;
+      if (tok >= visible || !(fabsf(f) < INFINITY)) f = 0.f;
       uint32_t sh, sl;
       uint4 hi, lo;
       pf_split(f, sh, sl);
@@ -270,31 +275,87 @@ __device__ __forceinline__ void pf_convert_v(uint8_t (&v)[2][2 * kPfHalf], const
     }
 }
 
-// A step with a V scale that is not finite: zero times it, and it may be another request's, is not zero.  The operand has the codes of such
-// tokens alone; the rows that see them get the products here, before the step's own.  `tile`: the warp's lanes of its tile; `v`: the step's hi.
-__device__ __forceinline__ void pf_wild(const float* vw, const uint8_t* v, uint32_t tile, int sees) {
+// Codes of the channels 4 lane .. 4 lane + 3 of a token of a page, a byte each, with their bias
+template <int BITS>
+__device__ __forceinline__ uint32_t pf_codes_k(const uint8_t* k, int tok, int lane) {
+  if constexpr (BITS == 8) return *reinterpret_cast<const uint32_t*>(k + (lane >> 2) * 256 + tok * 16 + (lane & 3) * 4);
+  const int blk = lane >> 3, high = lane >> 2 & 1, t = lane & 3;
+  uint32_t x = *reinterpret_cast<const uint32_t*>(k + blk * 256 + tok * 16 + t * 4) >> (4 * high) & 0x0F0F0F0Fu;
+  if constexpr (BITS == 6) {
+    const uint32_t w = *reinterpret_cast<const uint32_t*>(k + kPageTokens * kD / 2 + blk * 128 + (tok & 7) * 16 + t * 4);
+    x |= (tok < 8 ? (high ? w >> 2 : w) : (high ? w << 2 : w << 4)) & 0x30303030u;
+  }
+  return x;
+}
+template <int BITS>
+__device__ __forceinline__ uint32_t pf_codes_v(const uint8_t* v, int tok, int lane) {
+  const int pair = tok >> 1, odd = tok & 1, at = lane ^ ((pair & 3) << 2);
+  if constexpr (BITS == 8) {
+    const uint2 w = *reinterpret_cast<const uint2*>(v + pair * 256 + at * 8);
+    return prmt(w.x, w.y, odd ? 0x7531u : 0x6420u);
+  }
+  uint32_t x = *reinterpret_cast<const uint32_t*>(v + pair * 128 + at * 4) >> (4 * odd) & 0x0F0F0F0Fu;
+  if constexpr (BITS == 6) {
+    const uint32_t w = *reinterpret_cast<const uint32_t*>(v + kPageTokens * kD / 2 + (pair & 3) * 128 + at * 4);
+    x |= (pair < 4 ? (odd ? w >> 2 : w) : (odd ? w << 2 : w << 4)) & 0x30303030u;
+  }
+  return x;
+}
+
+// A row in fp32, by a warp whose lanes have four channels each: `limit` tokens of request `req`, the query at `q` (result likewise in `out`).
+// About 100 cycles a token and row where the MMAs take an eighth of one: for caches whose scales lie far apart.
+template <int KBITS, int VBITS>
+__device__ __forceinline__ void pf_row(const AttnParams& p, int req, int kvh, int limit, const __nv_bfloat16* q, __nv_bfloat16* out, int lane) {
+  constexpr int kTok = 4;                                // tokens at a time, of one page
+  constexpr float kBias = 1 << (KBITS - 1), vBias = 1 << (VBITS - 1);
+  const uint2 qw = reinterpret_cast<const uint2*>(q)[lane];
+  const float2 q01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qw.x)), q23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qw.y));
+  const float qf[4] = {q01.x * p.scale_log2, q01.y * p.scale_log2, q23.x * p.scale_log2, q23.y * p.scale_log2};
+  float m = -INFINITY, sum = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-  for (int cg = 0; cg < 4; ++cg)
-#pragma unroll 1
-    for (int tok = 0; tok < kPfTok; ++tok) {
-      const float s = vw[cg * kPfTok + tok];
-      if (s == 0.f) continue;
-      uint32_t pw;
-      tmem_ld_32x1(tile + kPfTmemP + (tok >> 1), pw);
-      tmem_ld_wait();
-      const float2 p2 = __half22float2(*reinterpret_cast<const __half2*>(&pw));
-      const float p = tok & 1 ? p2.y : p2.x;
-#pragma unroll 1
-      for (int ch = cg * 32; ch < cg * 32 + 32; ++ch) {
-        const __half code = *reinterpret_cast<const __half*>(v + (ch >> 6) * kPfHalf + tok * 128 + ((((ch & 63) >> 3) ^ (tok & 7)) << 4) + (ch & 7) * 2);
-        uint32_t o;
-        tmem_ld_32x1(tile + kPfTmemO + ch, o);
-        tmem_ld_wait();
-        if (tok < sees) o = __float_as_uint(__uint_as_float(o) + p * (__half2float(code) * s));
-        tmem_st_32x1(tile + kPfTmemO + ch, o);
-        tmem_st_wait();
-      }
+  for (int t0 = 0; t0 < limit; t0 += kTok) {
+    const int page = p.page_table[static_cast<size_t>(req) * p.max_pages + t0 / kPageTokens], tok0 = t0 % kPageTokens;
+    const uint8_t* blob = p.cache + (static_cast<size_t>(page) * p.Hkv + kvh) * p.lay.blob_bytes;
+    uint32_t kc[kTok], vc[kTok];
+    float ks[kTok], vs[kTok], z[kTok];
+#pragma unroll
+    for (int j = 0; j < kTok; ++j) {
+      kc[j] = pf_codes_k<KBITS>(blob, tok0 + j, lane);
+      vc[j] = pf_codes_v<VBITS>(blob + p.lay.v_code_off, tok0 + j, lane);
+      ks[j] = *reinterpret_cast<const float*>(blob + p.lay.k_scale_off + (tok0 + j) * 16 + (lane >> 3) * 4);
+      vs[j] = *reinterpret_cast<const float*>(blob + p.lay.v_scale_off + (tok0 + j) * 16 + (lane >> 3) * 4);
     }
+    float top = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kTok; ++j) {
+      float d = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) d = fmaf(qf[c], static_cast<float>(kc[j] >> (8 * c) & 255u) - kBias, d);
+      d *= ks[j];
+#pragma unroll
+      for (int o2 = 16; o2 > 0; o2 >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o2);
+      z[j] = t0 + j < limit ? d : -INFINITY;
+      top = fmaxf(top, z[j]);
+    }
+    if (top > m) {
+      const float alpha = fast_exp2(m - top);
+      m = top;
+      sum *= alpha;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[c] *= alpha;
+    }
+    const float use = m == -INFINITY ? 0.f : m;
+#pragma unroll
+    for (int j = 0; j < kTok; ++j) {
+      if (t0 + j >= limit) break;
+      const float pr = fast_exp2(z[j] - use);
+      sum += pr;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[c] = fmaf(pr, (static_cast<float>(vc[j] >> (8 * c) & 255u) - vBias) * vs[j], o[c]);
+    }
+  }
+  const float inv = sum > 0.f ? 1.f / sum : sum == 0.f ? 0.f : sum;
+  reinterpret_cast<uint2*>(out)[lane] = make_uint2(pack_bf16x2(o[0] * inv, o[1] * inv), pack_bf16x2(o[2] * inv, o[3] * inv));
 }
 
 template <int KBITS, int VBITS>
@@ -376,6 +437,8 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
         if (ok && n >= kPfLists) ok = mbar_wait_park(smem_u32(&sm.list_free[n % kPfLists]), (n / kPfLists - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) return false;
+        if (lane < kPfBlocks) sm.redo[n % kPfLists][lane] = INT_MAX;
+        if (lane == 0) sm.redo_least[n % kPfLists] = INT_MAX;
         if (at >= items) {                               // no item in this round: there is no further round
           if (lane == 0) l.kvh = -1;
         } else {
@@ -538,7 +601,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
     // warps 8-11 convert K, warps 12-15 V: scores run a step ahead of their softmax, and wait for no conversion of V
     const bool is_v = warp >= 12;
     const int ct = tid & 127;
-    int gs = 0, v_exp = 0;
+    int gs = 0, v_exp = 0, v_top = 0;                    // v_top: largest of the run
     for (int it = 0;; ++it) {
       const PfList& l = sm.list[it % kPfLists];
       if (ok) ok = mbar_wait_park(smem_u32(&sm.list_full[it % kPfLists]), (it / kPfLists) & 1, abort_flag);
@@ -548,6 +611,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
       PfWalk w;
       for (int i = 0; i < steps; ++i, ++gs) {
         const int b = gs & 1, slot = gs % kPfRaw, note = gs % kPfNotes, visible = l.run[w.run].total - w.step * kPfTok;
+        const int run = w.run, tok0 = w.step * kPfTok;
         w.advance(l);
         if (ok) ok = mbar_wait_park(smem_u32(&sm.raw_full[slot]), (gs / kPfRaw) & 1, abort_flag);
         if (ok && gs >= 2) ok = mbar_wait_park(smem_u32(is_v ? &sm.v_free[b] : &sm.k_free[b]), ((gs >> 1) - 1) & 1, abort_flag);
@@ -555,29 +619,51 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
         if (!ok) break;
         const uint8_t* pages = raw + slot * kPfPages * stride;
         float4 scale[2];
-        bool odd;
-        const int e = pf_exponent(pages + (is_v ? p.lay.v_scale_off : p.lay.k_scale_off), stride, visible, lane, scale, odd);
+        pf_scales(pages + (is_v ? p.lay.v_scale_off : p.lay.k_scale_off), stride, visible, lane, scale);
+        uint32_t most = __reduce_max_sync(0xffffffffu, max(pf_most<false>(scale[0]), pf_most<false>(scale[1])));       // (every warp for itself)
+        const bool odd = most >= 0x7F800000u;                            // some are not finite
+        if (odd) most = __reduce_max_sync(0xffffffffu, max(pf_most<true>(scale[0]), pf_most<true>(scale[1])));
+        const int e = pf_exponent(most);
+        auto redo_from = [&](int tok) {                                  // rows that see more than `tok` tokens of the run
+          atomicMin(&sm.redo[it % kPfLists][run], tok);
+          atomicMin(&sm.redo_least[it % kPfLists], tok);
+        };
         if (!is_v) {
-          if (ct == 0) {
-            sm.k_mul[note] = pow2f(e - 5);                               // codes times scales below 2^13
-            mbar_arrive(smem_u32(&sm.k_note[note]));
+          // codes times scales below 2^13
+          if (warp == 8) {
+            if (e > kPfLarge) {
+              const uint32_t of[2] = {pf_most<true>(scale[0]), pf_most<true>(scale[1])};
+              if (__any_sync(0xffffffffu, (of[0] != 0 && pf_exponent(of[0]) < e - 8) || (of[1] != 0 && pf_exponent(of[1]) < e - 8)) && lane == 0) redo_from(tok0);
+            }
+            if (lane == 0) {
+              sm.k_mul[note] = pow2f(e - 5);
+              mbar_arrive(smem_u32(&sm.k_note[note]));
+            }
           }
           pf_convert_k<KBITS>(sm.k[b], pages, stride, p.lay, pow2f(5 - e), ct);
         } else {
-          if (i == 0 || e - 7 > v_exp) v_exp = e - 3;                    // below 2^11, to be changed when they pass 2^15
+          // below 2^11, to be changed when they pass 2^15, or when the scales fall below 2^v_exp and that is more than one
+          if (tok0 == 0) {
+            v_exp = v_top = e - 3;
+          } else if (e - 7 > v_exp || (v_exp > kPfLarge - 3 && e < v_exp && most != 0)) {
+            v_exp = max(e - 3, v_top - kPfVFall);
+            v_top = max(v_top, v_exp);
+          }
           if (warp == 12) {
-            if (odd) {
-              auto of = [](float x) { return fabsf(x) < INFINITY ? 0.f : x; };
+            if (odd || v_exp > kPfLarge - 3) {                           // tokens with a scale that is not finite, or below 2^-8 beside large ones
+              const float least = v_exp > kPfLarge - 3 ? pow2f(v_exp - 8) : 0.f;
+              bool out[2] = {false, false};
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
-                float* at = sm.vw[note] + lane + 32 * h;
-                at[0] = of(scale[h].x); at[kPfTok] = of(scale[h].y); at[2 * kPfTok] = of(scale[h].z); at[3 * kPfTok] = of(scale[h].w);
+                const float f[4] = {scale[h].x, scale[h].y, scale[h].z, scale[h].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) out[h] |= !(fabsf(f[j]) < INFINITY) || (f[j] != 0.f && fabsf(f[j]) < least);
               }
+              const uint32_t lo = __ballot_sync(0xffffffffu, out[0]), hi = __ballot_sync(0xffffffffu, out[1]);
+              if ((lo | hi) != 0 && lane == 0) redo_from(tok0 + (lo != 0 ? __ffs(lo) - 1 : 31 + __ffs(hi)));
             }
-            __syncwarp();
             if (lane == 0) {
               sm.v_exp[note] = v_exp;
-              sm.wild[note] = odd;
               mbar_arrive(smem_u32(&sm.v_note[note]));
             }
           }
@@ -705,9 +791,8 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
           sum *= alpha;
         }
         const int e = sm.v_exp[note];
-        if (first) v_exp = e;
-        if (e != v_exp) {
-          alpha *= pow2f(v_exp - e);
+        if (sees > 0 && e != v_exp) {                    // (rows of other requests keep theirs: nothing is added to their outputs)
+          alpha = v_exp - e < -126 ? 0.f : alpha * pow2f(v_exp - e);
           v_exp = e;
           grew = true;
         }
@@ -740,11 +825,6 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
           }
         }
         tmem_st_wait();
-        if (sm.wild[note]) {
-          if (ok) ok = mbar_wait_park(smem_u32(&sm.v_full[gs & 1]), (gs >> 1) & 1, abort_flag);
-          ok = __all_sync(0xffffffffu, ok);
-          pf_wild(sm.vw[note], sm.v[gs & 1][0], tile, sees);
-        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm.p_full[t]));
@@ -781,6 +861,21 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
           }
         }
         tc_fence_before();
+        if (*const_cast<volatile int*>(&sm.redo_least[it % kPfLists]) != INT_MAX && ok) {
+          // (what later steps still add to `redo` is beyond what the rows of this tile see)
+          __syncwarp();                                  // a row's result is written again by other lanes
+          int req = 0, from = INT_MAX;
+          for (int i = 0; i < l.runs; ++i)
+            if (blk >= l.run[i].first && blk < l.run[i].end) {
+              req = l.run[i].req;
+              from = *const_cast<volatile int*>(&sm.redo[it % kPfLists][i]);
+            }
+          for (uint32_t rows = __ballot_sync(0xffffffffu, cur.out != nullptr && cur.limit > from); rows; rows &= rows - 1) {
+            const int of = __ffs(rows) - 1;
+            const long long at = __shfl_sync(0xffffffffu, static_cast<long long>(cur.out - p.out), of);
+            pf_row<KBITS, VBITS>(p, __shfl_sync(0xffffffffu, req, of), l.kvh, __shfl_sync(0xffffffffu, cur.limit, of), p.q + at, p.out + at, lane);
+          }
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm.list_free[it % kPfLists]));

@@ -196,6 +196,124 @@ def test_prompt_form_with_scales_of_any_size(kb, vb, low, high):
     assert _close((got.cpu().double() / unit), ref / unit)
 
 
+def _scale_views(cache, kb, vb):
+    """K and V scales of the cache as floats [page][head][token of the page][group]."""
+    lay = eager.blob_layout(D, kb, vb)
+    return [cache[:, :, lay[a]:lay[b]].view(torch.float32).view(cache.shape[0], cache.shape[1], 16, D // 32)
+            for a, b in (("k_scale", "v_code"), ("v_scale", "bytes"))]
+
+
+def _request(cache, table, r, n, kb, vb):
+    """K and V of the first ``n`` tokens of a request with one key / value head, in 64 bits."""
+    pages = [eager.decode_cache_page(cache[p, 0].cpu(), D, kb, vb) for p in table[r, :-(-n // 16)].tolist()]
+    return [torch.cat([page[i] for page in pages])[:n].double() for i in (0, 1)]
+
+
+def _softmax_of(q, k, v, first):
+    """Rows [T, G, D] of positions first, first + 1, .. against keys and values, in 64 bits."""
+    z = torch.einsum("thd,sd->ths", q.cpu().double(), k) * 0.05
+    z.masked_fill_(torch.arange(k.shape[0])[None, None] > (first + torch.arange(q.shape[0]))[:, None, None], float("-inf"))
+    return torch.einsum("ths,sd->thd", z.softmax(-1), v)
+
+
+def _close_in_groups(got, ref):
+    """As ``_close`` in every row and channel group, whatever the size of its values."""
+    got, ref = got.cpu().double().unflatten(-1, (-1, 32)), ref.unflatten(-1, (-1, 32))
+    unit = torch.exp2(ref.abs().amax(-1, keepdim=True).clamp_min(1e-300).log2().floor())
+    return torch.isfinite(got).all() and _close(got / unit, ref / unit)
+
+
+def _sharp(k, rows, group, seed):
+    """Queries that see next to nothing but the key of their own position."""
+    g = torch.Generator().manual_seed(seed)
+    unit = k[-rows:] / k[-rows:].norm(dim=-1, keepdim=True).clamp_min(1e-30)
+    return (unit[:, None] * 6000 + torch.randn(rows, group, D, generator=g)).bfloat16().to(DEV)
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (4, 6), (6, 4)])
+@pytest.mark.parametrize("first,last", [(6, -6), (12, -2), (30, 0), (60, -2), (-10, -14), (0, 40)])
+def test_prompt_form_with_v_scales_that_fall(kb, vb, first, last):
+    """V scales that shrink (or grow) from page to page, seen by rows that attend to their own position: what was large before is no measure
+    of what comes."""
+    group, n = 4, 600
+    cache, table = _cache([n], 1, kb, vb, 19)
+    for i, page in enumerate(table[0].tolist()):
+        _scale_views(cache, kb, vb)[1][page] *= 2.0 ** round(first + (last - first) * i / table.shape[1])
+    k, v = _request(cache, table, 0, n, kb, vb)
+    q = _sharp(k, n, group, 8)
+    got = _run("prefill", q, cache, table, [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)], group, 1, kb, vb, 1)
+    assert _close_in_groups(got, _softmax_of(q, k, v, 0))
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (4, 6)])
+@pytest.mark.parametrize("apart", [12, 24, 30, 60, -24, -60])
+def test_prompt_form_with_requests_of_other_scales_in_an_item(kb, vb, apart):
+    """Requests whose V scales are far from their neighbours' in the same item: each has the result that it has by itself."""
+    group, portions = 4, [(0, 12), (20, 21), (0, 9), (130, 22), (3, 40), (64, 30)]
+    cache, table = _cache([s + n for s, n in portions], 1, kb, vb, 20)
+    for r, (s, n) in enumerate(portions):
+        _scale_views(cache, kb, vb)[1][table[r, :-(-(s + n) // 16)].long()] *= 2.0 ** (apart * (r % 2))
+    T = sum(n for _, n in portions)
+    q = torch.randn(T, group, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(9)).bfloat16()
+    blocks, t = [], 0
+    for r, (s, n) in enumerate(portions):
+        blocks += [(r, t + i, min(4, n - i), s + i + 1) for i in range(0, n, 4)]
+        t += n
+    got = _run("prefill", q, cache, table, blocks, group, 1, kb, vb, 1)
+    t = 0
+    for r, (s, n) in enumerate(portions):
+        assert _close_in_groups(got[t:t + n], _softmax_of(q[t:t + n], *_request(cache, table, r, s + n, kb, vb), s))
+        t += n
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (8, 6), (8, 4)])
+@pytest.mark.parametrize("up,down", [(0, 6), (0, 11), (12, 11), (12, 20), (40, 20), (100, 60)])
+def test_prompt_form_with_v_scales_apart_in_a_step(kb, vb, up, down):
+    """Tokens, and channel groups of a token, far below others of the same step, alone or before them.  (2^-28 of scales of ordinary size is
+    nothing to a product of a probability and a scale in f16 either.)"""
+    group, n = 4, 150
+    cache, table = _cache([n], 1, kb, vb, 21)
+    g = torch.Generator().manual_seed(down)
+    for at in range(n):
+        factor = 2.0 ** up * torch.where(torch.rand(D // 32, generator=g) < (0.5 if at >= 10 else 1.1), 2.0 ** -down, 1.0)
+        _scale_views(cache, kb, vb)[1][int(table[0, at // 16]), 0, at % 16] *= factor.to(DEV)
+    k, v = _request(cache, table, 0, n, kb, vb)
+    q = torch.cat([_sharp(k, n, 2, 10), torch.randn(n, 2, D, generator=g).bfloat16().to(DEV)], 1).contiguous()
+    got = _run("prefill", q, cache, table, [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)], group, 1, kb, vb, 1)
+    assert _close_in_groups(got, _softmax_of(q, k, v, 0))
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (6, 8), (4, 8)])
+@pytest.mark.parametrize("up,at", [(9, 40), (24, 40), (40, 63), (100, 0), (100, 100)])
+def test_prompt_form_with_a_key_far_above_the_others(kb, vb, up, at):
+    """One token's K scales far above those of its step: rows before it, and rows that it is nothing to, have the scores of the others."""
+    group, n = 4, 130
+    cache, table = _cache([n], 1, kb, vb, 22)
+    _scale_views(cache, kb, vb)[0][int(table[0, at // 16]), 0, at % 16] *= 2.0 ** up
+    k, v = _request(cache, table, 0, n, kb, vb)
+    g = torch.Generator().manual_seed(up)
+    q = torch.randn(n, group, D, generator=g).bfloat16()
+    # half of the rows look away from it
+    q[:, 2:] = torch.where(((q[:, 2:].double() * k[at]).sum(-1, keepdim=True) > 0), -q[:, 2:], q[:, 2:])
+    q = q.to(DEV)
+    got = _run("prefill", q, cache, table, [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)], group, 1, kb, vb, 1)
+    assert _close_in_groups(got, _softmax_of(q, k, v, 0))
+
+
+@pytest.mark.parametrize("kb,vb", [(8, 8), (4, 6)])
+def test_prompt_form_with_k_scales_apart(kb, vb):
+    """K scales of the tokens of a step 2^-40 to 1 of each other."""
+    group, n = 4, 200
+    cache, table = _cache([n], 1, kb, vb, 23)
+    ks, g = _scale_views(cache, kb, vb)[0], torch.Generator().manual_seed(1)
+    for at in range(n):
+        ks[int(table[0, at // 16]), 0, at % 16] *= 2.0 ** -int(torch.randint(0, 41, (1,), generator=g))
+    k, v = _request(cache, table, 0, n, kb, vb)
+    q = torch.randn(n, group, D, generator=g).bfloat16().to(DEV)
+    got = _run("prefill", q, cache, table, [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)], group, 1, kb, vb, 1)
+    assert _close_in_groups(got, _softmax_of(q, k, v, 0))
+
+
 @pytest.mark.parametrize("kb,vb,hkv", [(8, 8, 8), (4, 6, 16)])
 def test_prompt_form_with_one_tile_ahead_of_the_other(kb, vb, hkv):
     """Items whose first tile sees one step and whose second sees many, the other way round, and with padding for a tile; several of a CTA."""
