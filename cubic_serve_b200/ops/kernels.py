@@ -226,11 +226,12 @@ def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = 
     13.0 / 15.0 / 18.3 / 19.5 / 20.5 / 21.3 -> 11.7 / 11.9 / 13.0 / 14.5 / 16.3 / 18.7, 5120 x 4096 11.8 / 14.1 / 15.0 / 16.1 / 17.0 / 18.0 -> 11.5 / 11.7 / 12.8 / 14.1 / 15.7 / 17.9,
     4096 x 4096 10.4 / 11.8 / 12.8 / 13.7 / 14.7 / 15.9 -> 10.6 / 10.5 / 11.9 / 13.0 / 14.3 / 16.3, 8192 x 2048 9.5 / 11.3 / 12.7 / 13.6 / 14.4 / 15.4 -> 10.3 / 10.6 / 11.0 / 12.1 / 13.1 / 14.3,
     14336 x 1024 9.6 / 11.1 / 11.3 / 12.1 / 12.7 / 13.5 -> 11.2 / 11.4 / 12.8 / 13.7 / 16.3 / 20.5.
-    - Up to 8 rows the few-row kernel has next to nothing to do but to read: eight and a half units an SM (5120 x 4096 has 8.6, 4608 x 4096 7.8: 10.3 against
-      10.5).  From 9 rows, which take it a second pass, six and a half (8192 x 2048 has 6.9, 14336 x 1024 6.1).
-    - From 65 rows the sums count.  Tiles of several parts of their own: up to 480 rows times parts (4096 x 4096 at 96: 384), or ten units a part (2560 x 9728 has
-      10.9, at 128 rows 20.6 -> 20.8; 3584 x 5120 8, 16.9 -> 17.9; 1024 x 16384 7.1, 21.7 -> 28.6).  Tiles dealt across their borders: ten units an SM from 97 rows (6144 x
-      4096 has 10.4, 10240 x 2048 8.6: 18.5 -> 18.2 at 96, 19.5 -> 21.3 at 128).
+    - Six and a half units an SM (8192 x 2048 has 6.9, 14336 x 1024 6.1).  Alone, the matrices between that and eight and a half lose 2 to 8 % at up to 8 rows; in a
+      step their codes are on the way before the attention in front of them is done: 4096 x 4096 behind it, one request behind 700 tokens 1008 us a step of 12
+      layers against 1018 with the few-row kernel, 7 behind 2100 1133 against 1146; at 100 and 112 rows 1789 and 1824 against 1806 and 1831 with the per-tile kernel.
+    - From 65 rows the sums count.  Tiles of several parts of their own: up to 800 rows times parts (4096 x 4096 at 128: 512, 2048 x 8192 at 96: 864, 17.1 -> 17.7),
+      or ten units a part (2560 x 9728 has 10.9, at 128 rows 20.6 -> 20.8; 1024 x 16384 7.1, 21.7 -> 28.6).  Tiles dealt across their borders: ten units an SM from 97 rows
+      (6144 x 4096 has 10.4, 10240 x 2048 8.6: 18.5 -> 18.2 at 96, 19.5 -> 21.3 at 128).
 
     129 to 512 rows: the other kernels decode a tile once for 256 rows and do the same work for 331 as for 512, here it is done for blocks of one size; from
     28 units an SM, or where every tile has parts of its own.  In a loop over many weights, at the clocks that it settles at, 192 / 256 / 331 / 512 rows:
@@ -255,13 +256,13 @@ def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = 
     units = tiles * (w.k // 128)
     own = sms // tiles if 2 * tiles <= sms else 0          # parts of a tile, if every one has some of its own
     rows = -(-m // blocks)
-    if 2 * units < (17 if m <= 8 else 13) * sms:
+    if 2 * units < 13 * sms:
         return False
     if m > 128:
         if rows * own > 1000 if own else units < 28 * sms:
             return False
     elif m > 64 and own:
-        if rows * own > 480 and units < 10 * own * tiles:
+        if rows * own > 800 and units < 10 * own * tiles:
             return False
     elif m > 96 and units < 10 * sms:
         return False
