@@ -381,8 +381,8 @@ gdn_delta_kernel(const GdnDeltaParams p) {
 // A value row (a row of S, a column of V, Delta and o) never meets another before the output norm: a warp holds 16 rows of S in registers and
 // walks the chunk alone, everything transposed ([value row][token]), so that a product's accumulators are the next one's A operand
 // without a shuffle.  Operands are f16: normalised k and q are bf16 below one; what is computed in fp32 (S, Delta, L, the inverses, q . k) is
-// split in two f16 behind a power of two that puts its largest at 2^13 (22 bits); Delta as it enters the state in three.  Sums with what is larger than
-// the product (inverse less one, decayed state) are fp32 multiply-adds outside the tensor cores, which cut their sums off.
+// split in two f16 behind a power of two that puts the largest of its value row at 2^13 (22 bits); Delta as it enters the state in three.  Sums with what is
+// larger than the product (inverse less one, decayed state) are fp32 multiply-adds outside the tensor cores, which cut their sums off.
 // Decay ratios are products of their factors, as in the recurrence: no logarithm, no quotient.
 // Against 64 bits (331 rows, random decays): outputs 2.8982e-3 either way; the state 0.99e-7 against 0.77e-7 of the recurrence, with slow decays
 // and similar keys 5.9e-7 against 7.7e-7 (640 rows), with large values 9.2e-7 against 10.4e-7 (320).
@@ -392,7 +392,8 @@ gdn_delta_kernel(const GdnDeltaParams p) {
 // What bounds it: the chain of a chunk (about 10000 cycles, of which its MMAs take 3500) and its preparation, which takes as long beside it.
 // One row after the other -> in chunks, 32 heads, one B200: segments of 1000, 536, 823, 359 and 646 rows 1013 -> 247 us, one of 1750 924 -> 380, one of 331
 // 307 -> 94, one of 32 34 -> 28, 16 of 256 1040 -> 249.
-// A chunk with a key, query, value or coefficient that is not finite is walked token by token: zero times it, in a row before it, is not zero.
+// A chunk with a key, query, value or coefficient that is not finite is walked token by token: zero times it, in a row before it, is not zero.  Likewise, by
+// a warp for itself, one whose state or Delta is not.
 static constexpr int kGdnChunk = 32;
 static constexpr int kGdnChunkThreads = 512, kGdnPrepareThreads = 256;
 // registers a thread: at launch, and of the walking and the preparing warps after they have shared them out anew
@@ -441,29 +442,33 @@ __device__ __forceinline__ void gdn_split(float x, float y, uint32_t& hi, uint32
   lo = gdn_pack(x - h.x, y - h.y);
 }
 __device__ __forceinline__ float gdn_pow2(int e) { return __int_as_float((e + 127) << 23); }
-// Exponent of the largest finite magnitude that the warp holds (`most`: the thread's, as bits); 0 and small ones count as 2^-100.
-__device__ __forceinline__ int gdn_exponent(uint32_t most) {
-  return min(max(static_cast<int>(__reduce_max_sync(0xffffffffu, most) >> 23) - 127, -100), 110);
+__device__ __forceinline__ uint32_t gdn_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+// The largest magnitudes, as bits, of the value rows g and g + 8 of the warp's fragments (`most`: what the thread has of them): the four lanes of a row
+__device__ __forceinline__ void gdn_row_max(uint32_t (&most)[2]) {
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) most[r] = max(most[r], __shfl_xor_sync(0xffffffffu, most[r], o));
 }
-__device__ __forceinline__ uint32_t gdn_bits(float x) {
-  const uint32_t b = __float_as_uint(x) & 0x7FFFFFFFu;
-  return b < 0x7F800000u ? b : 0u;
-}
-// Accumulators of 16 value rows x 16 tokens (two n-tiles) -> the A operand over those tokens, times 2^(13 - e); returns 2^(e - 13)
-__device__ __forceinline__ float gdn_operand(const float (&x)[2][4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-  uint32_t most = 0;
+// Its exponent; 0 and small ones count as 2^-85
+__device__ __forceinline__ int gdn_exponent(uint32_t magnitude) { return max(static_cast<int>(magnitude >> 23) - 127, -85); }
+// Accumulators of 16 value rows x 16 tokens (two n-tiles) -> the A operand over those tokens, each row times its 2^(13 - e); down: 2^(e - 13) of the rows
+__device__ __forceinline__ void gdn_operand(const float (&x)[2][4], uint32_t (&hi)[4], uint32_t (&lo)[4], float (&down)[2]) {
+  uint32_t most[2];
+  float up[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) most[r] = max(max(gdn_bits(x[0][2 * r]), gdn_bits(x[0][2 * r + 1])), max(gdn_bits(x[1][2 * r]), gdn_bits(x[1][2 * r + 1])));
+  gdn_row_max(most);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int e = gdn_exponent(most[r]);
+    up[r] = gdn_pow2(13 - e);
+    down[r] = gdn_pow2(e - 13);
+  }
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) most = max(most, gdn_bits(x[j][i]));
-  const int e = gdn_exponent(most);
-  const float up = gdn_pow2(13 - e);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    gdn_split(x[j][0] * up, x[j][1] * up, hi[2 * j], lo[2 * j]);
-    gdn_split(x[j][2] * up, x[j][3] * up, hi[2 * j + 1], lo[2 * j + 1]);
-  }
-  return gdn_pow2(e - 13);
+    for (int r = 0; r < 2; ++r) gdn_split(x[j][2 * r] * up[r], x[j][2 * r + 1] * up[r], hi[2 * j + r], lo[2 * j + r]);
 }
 // d[n-tile] = x (hi, lo) times a block of 16 x 16 (hi, lo), [column token][row token]
 __device__ __forceinline__ void gdn_block(float (&d)[2][4], const uint32_t (&hi)[4], const uint32_t (&lo)[4], const __half (&m)[2][16 * 16], int lane) {
@@ -779,20 +784,26 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
     const __nv_bfloat16* vs = sm.v[i % 3] + warp * 16 + g;
     float o[2][2][4];                                    // [16 tokens][n-tile][value rows g, g + 8 x tokens 2 c, 2 c + 1], without 1 / sqrt(d_k)
     gdn_bar_sync<kGdnChunkThreads>(1 + (i & 1));
-    if (!op.wild) {
+    uint32_t most[2] = {0, 0};
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) most[q >> 1] = max(most[q >> 1], gdn_bits(S[j][q]));
+    gdn_row_max(most);
+    // what is not finite in the warp's rows of the state, or in what the chunk adds to them, is walked with too
+    bool walk = op.wild || __any_sync(0xffffffffu, max(most[0], most[1]) >= 0x7F800000u);
+    if (!walk) {
       // ---- S k and S q
       float u[2][2][4];
-      float down;
+      float down[2];
       {
-        float x[2][2][4];
-        uint32_t most = 0;
+        float x[2][2][4], up[2];
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) most = max(most, gdn_bits(S[j][q]));
-        const int e = gdn_exponent(most);
-        const float up = gdn_pow2(13 - e);
-        down = gdn_pow2(e - 13);
+        for (int r = 0; r < 2; ++r) {
+          const int e = gdn_exponent(most[r]);
+          up[r] = gdn_pow2(13 - e);
+          down[r] = gdn_pow2(e - 13);
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -803,10 +814,8 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           uint32_t hi[4], lo[4];
-          gdn_split(S[2 * k][0] * up, S[2 * k][1] * up, hi[0], lo[0]);
-          gdn_split(S[2 * k][2] * up, S[2 * k][3] * up, hi[1], lo[1]);
-          gdn_split(S[2 * k + 1][0] * up, S[2 * k + 1][1] * up, hi[2], lo[2]);
-          gdn_split(S[2 * k + 1][2] * up, S[2 * k + 1][3] * up, hi[3], lo[3]);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) gdn_split(S[2 * k + (r >> 1)][2 * (r & 1)] * up[r & 1], S[2 * k + (r >> 1)][2 * (r & 1) + 1] * up[r & 1], hi[r], lo[r]);
           const uint32_t at = brow * 256 + (((2 * k + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -844,92 +853,103 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
           for (int q = 0; q < 2; ++q) {
             const int t = h * 16 + j * 8 + 2 * c + q;
             const float2 bg = *reinterpret_cast<const float2*>(&op.coef[t]);
-            const float f = down * bg.y;
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
+              const float f = down[r] * bg.y;
               u[h][j][2 * r + q] = fmaf(-u[h][j][2 * r + q], f, __bfloat162float(vs[t * kGdnDim + 8 * r])) * bg.x;
               o[h][j][2 * r + q] *= f;
             }
           }
       // ---- Delta (in place of u) of tokens 0..15, then of 16..31
       uint32_t hi[4], lo[4];
-      float d[2][4];
-      auto add = [&](float (&x)[2][4], float f) {        // x += f d
+      float d[2][4], f[2];
+      auto add = [&](float (&x)[2][4], float sign) {     // x += d
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) x[j][q] = fmaf(f, d[j][q], x[j][q]);
+          for (int q = 0; q < 4; ++q) x[j][q] = fmaf(sign * (1.f / kGdnUp) * f[q >> 1], d[j][q], x[j][q]);
       };
-      constexpr float kDown = 1.f / kGdnUp;
-      float f = gdn_operand(u[0], hi, lo) * kDown;
+      gdn_operand(u[0], hi, lo, f);
       gdn_block(d, hi, lo, op.inv[0], lane);
-      add(u[0], f);
-      f = gdn_operand(u[0], hi, lo) * kDown;
+      add(u[0], 1.f);
+      gdn_operand(u[0], hi, lo, f);
       gdn_block(d, hi, lo, op.l10, lane);
-      add(u[1], -f);
+      add(u[1], -1.f);
       gdn_block(d, hi, lo, op.a[0], lane);
-      add(o[0], f);
+      add(o[0], 1.f);
       gdn_block(d, hi, lo, op.a[1], lane);
-      add(o[1], f);
-      f = gdn_operand(u[1], hi, lo) * kDown;
+      add(o[1], 1.f);
+      gdn_operand(u[1], hi, lo, f);
       gdn_block(d, hi, lo, op.inv[1], lane);
-      add(u[1], f);
-      f = gdn_operand(u[1], hi, lo) * kDown;
+      add(u[1], 1.f);
+      gdn_operand(u[1], hi, lo, f);
       gdn_block(d, hi, lo, op.a[2], lane);
-      add(o[1], f);
+      add(o[1], 1.f);
       // ---- the state: G_end S plus the products of the chunk, which the tensor cores sum from zero
       const float end = op.coef[kGdnChunk - 1].y;
-      uint32_t first[2][4], second[2][4], third[2][4], most = 0;
+      uint32_t first[2][4], second[2][4], third[2][4];
+      most[0] = most[1] = 0;
 #pragma unroll
       for (int b = 0; b < 2; ++b)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const float r0 = op.coef[b * 16 + j * 8 + 2 * c].z, r1 = op.coef[b * 16 + j * 8 + 2 * c + 1].z;
-          u[b][j][0] *= r0; u[b][j][1] *= r1;
-          u[b][j][2] *= r0; u[b][j][3] *= r1;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) most = max(most, gdn_bits(u[b][j][q]));
-        }
-      const int e = gdn_exponent(most);
-      const float up = gdn_pow2(13 - e), fs = gdn_pow2(e - 13);
-#pragma unroll
-      for (int b = 0; b < 2; ++b)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const int at = 2 * j + r;
-            float x = u[b][j][2 * r] * up, y = u[b][j][2 * r + 1] * up;
-            const uint32_t coarse = pack_bf16x2(x, y);
-            first[b][at] = gdn_pack(__uint_as_float(coarse << 16), __uint_as_float(coarse & 0xFFFF0000u));
-            const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&first[b][at]));
-            x -= f2.x;
-            y -= f2.y;
-            gdn_split(x, y, second[b][at], third[b][at]);
+          for (int q = 0; q < 4; ++q) {
+            u[b][j][q] *= q & 1 ? r1 : r0;
+            most[q >> 1] = max(most[q >> 1], gdn_bits(u[b][j][q]));
           }
+        }
+      gdn_row_max(most);
+      walk = __any_sync(0xffffffffu, max(most[0], most[1]) >= 0x7F800000u);
+      if (!walk) {
+        float up[2], fs[2];
 #pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        uint32_t kb[2][4];                               // (tokens 0, columns 0) (tokens 8, columns 0) (tokens 0, columns 8) (tokens 8, columns 8)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int t = b * 16 + (lane & 15);
-          ldsm4_t(kb[b], smem_u32(op.k) + t * 256 + (((j + (lane >> 4)) ^ (t & 7)) << 4));
+        for (int r = 0; r < 2; ++r) {
+          const int e = gdn_exponent(most[r]);
+          up[r] = gdn_pow2(13 - e);
+          fs[r] = gdn_pow2(e - 13);
         }
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          // products of the first parts have 16 bits: kept apart from the rest, 2^-8 of them, their sum loses next to nothing
-          float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const int at = 2 * j + r;
+              float x = u[b][j][2 * r] * up[r], y = u[b][j][2 * r + 1] * up[r];
+              const uint32_t coarse = pack_bf16x2(x, y);
+              first[b][at] = gdn_pack(__uint_as_float(coarse << 16), __uint_as_float(coarse & 0xFFFF0000u));
+              const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&first[b][at]));
+              x -= f2.x;
+              y -= f2.y;
+              gdn_split(x, y, second[b][at], third[b][at]);
+            }
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          uint32_t kb[2][4];                             // (tokens 0, columns 0) (tokens 8, columns 0) (tokens 0, columns 8) (tokens 8, columns 8)
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
-            gdn_mma(x, first[b], kb[b][2 * q], kb[b][2 * q + 1]);
-            gdn_mma(y, third[b], kb[b][2 * q], kb[b][2 * q + 1]);
-            gdn_mma(y, second[b], kb[b][2 * q], kb[b][2 * q + 1]);
+            const int t = b * 16 + (lane & 15);
+            ldsm4_t(kb[b], smem_u32(op.k) + t * 256 + (((j + (lane >> 4)) ^ (t & 7)) << 4));
           }
 #pragma unroll
-          for (int r = 0; r < 4; ++r) S[j + q][r] = fmaf(fs, x[r], fmaf(fs, y[r], S[j + q][r] * end));
+          for (int q = 0; q < 2; ++q) {
+            // products of the first parts have 16 bits: kept apart from the rest, 2^-8 of them, their sum loses next to nothing
+            float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              gdn_mma(x, first[b], kb[b][2 * q], kb[b][2 * q + 1]);
+              gdn_mma(y, third[b], kb[b][2 * q], kb[b][2 * q + 1]);
+              gdn_mma(y, second[b], kb[b][2 * q], kb[b][2 * q + 1]);
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) S[j + q][r] = fmaf(fs[r >> 1], x[r], fmaf(fs[r >> 1], y[r], S[j + q][r] * end));
+          }
         }
       }
-    } else {
+    }
+    if (walk) {
       // ---- token by token
 #pragma unroll 1
       for (int t = 0; t < kGdnChunk; ++t) {
@@ -938,7 +958,7 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int at = t * 256 + ((j ^ (t & 7)) << 4) + c * 4;
-          const float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + at)), q = __half22float2(*reinterpret_cast<const __half2*>(op.q + at));
+          float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + at)), q = __half22float2(*reinterpret_cast<const __half2*>(op.q + at));
 #pragma unroll
           for (int i = 0; i < 4; ++i) S[j][i] *= co.w;
           m0 = fmaf(S[j][0], k.x, fmaf(S[j][1], k.y, m0));
@@ -961,7 +981,7 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
         if (i * kGdnChunk + t < n) {                     // behind the segment's end nothing happens to the state
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + t * 256 + ((j ^ (t & 7)) << 4) + c * 4));
+            float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + t * 256 + ((j ^ (t & 7)) << 4) + c * 4));
             S[j][0] = fmaf(d0, k.x, S[j][0]); S[j][1] = fmaf(d0, k.y, S[j][1]);
             S[j][2] = fmaf(d1, k.x, S[j][2]); S[j][3] = fmaf(d1, k.y, S[j][3]);
           }

@@ -142,6 +142,45 @@ def test_gdn_delta_chunks_keep_what_is_not_finite_behind_it(what, bad):
     assert torch.equal(torch.isfinite(out), torch.isfinite(want)) and torch.equal(torch.isfinite(state), torch.isfinite(want_state))
 
 
+def _row_errors(a, b, dim=-1):
+    a, b = a.double(), b.double()
+    return ((a - b).norm(dim=dim) / b.norm(dim=dim).clamp_min(1e-300)).max().item()
+
+
+@pytest.mark.parametrize("low,high", [(-24, 0), (-60, 20), (90, 116)])
+def test_gdn_delta_chunks_of_value_rows_of_any_size(low, high):
+    """Value rows (rows of the state, columns of V) 2^low to 2^high of each other: each has its own precision, as row by row."""
+    counts, pos0, hk, hv = [100, 33], [7, 0], 1, 2
+    case = list(_delta_case(counts, pos0, hk, hv, 1))
+    size = torch.exp2(torch.linspace(low, high, 128, device=DEV).round()).roll(5)
+    case[0] = torch.cat([case[0][:, :256], (case[0][:, 256:].view(-1, hv, 128) * size).view(-1, hv * 128)], 1).bfloat16()
+    case[6] = case[6] * size[:, None]
+    out, state = _delta(case, counts, pos0, hk, hv, None)
+    want, want_state = _delta(case, counts, pos0, hk, hv, 31)
+    assert torch.isfinite(state).all() and _row_errors(state, want_state) < 2.0 ** -18
+    assert torch.equal(torch.isfinite(out), torch.isfinite(want))
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.2e38])
+@pytest.mark.parametrize("where", ["state", "v"])
+def test_gdn_delta_chunks_that_do_not_stay_finite(where, value):
+    """A state that is not finite, or values that become so on the way (the same key with values of either sign): as row by row."""
+    counts, pos0, hk, hv = [70, 40], [7, 0], 1, 2
+    case = _delta_case(counts, pos0, hk, hv, 1)
+    if where == "state":
+        case[6][0, 1, 17, 5] = value
+    else:
+        case[0][20:24, 128:256] = case[0][20, 128:256]
+        case[0][20:24, 256 + 9] = torch.tensor([value, -value, value, -value]).bfloat16()
+        case[2][20:24, :hv] = 20.0
+        case[3].fill_(-20.0)
+    out, state = _delta(case, counts, pos0, hk, hv, None)
+    want, want_state = _delta(case, counts, pos0, hk, hv, 31)
+    assert torch.equal(torch.isfinite(state), torch.isfinite(want_state)) and torch.equal(torch.isfinite(out), torch.isfinite(want))
+    rows = torch.isfinite(want_state).all(-1)
+    assert rows.sum() >= rows.numel() - 2 and _row_errors(state[rows], want_state[rows]) < 2.0 ** -18
+
+
 def test_gdn_delta_chunks_of_rows_that_are_not_aligned():
     """Rows that start anywhere are walked one by one; a review pass leaves the state."""
     from cubic_serve_b200.ops import kernels as K
