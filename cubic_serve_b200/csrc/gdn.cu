@@ -380,7 +380,7 @@ gdn_delta_kernel(const GdnDeltaParams p) {
 //
 // A value row (a row of S, a column of V, Delta and o) never meets another before the output norm: a warp holds 16 rows of S in registers and
 // walks the chunk alone, everything transposed ([value row][token]), so that a product's accumulators are the next one's A operand
-// without a shuffle.  Operands are f16: normalised k and q are bf16 below one; what is computed in fp32 (S, Delta, L, the inverses, q . k) is
+// without a shuffle.  Operands are f16: normalised k and q, bf16 of at most one, behind 2^15 (all bits down to 2^-32); what is computed in fp32 (S, Delta, L, the inverses, q . k) is
 // split in two f16 behind a power of two that puts the largest of its value row at 2^13 (22 bits); Delta as it enters the state in three.  Sums with what is
 // larger than the product (inverse less one, decayed state) are fp32 multiply-adds outside the tensor cores, which cut their sums off.
 // Decay ratios are products of their factors, as in the recurrence: no logarithm, no quotient.
@@ -417,6 +417,8 @@ struct __align__(128) GdnChunkSmem {
   float low[2][16][16];                                  // blocks on the diagonal of L
 };
 static constexpr float kGdnUp = 4096.f;                  // of L, the inverses and q . k: entries of at most about one
+static constexpr float kGdnKeyUp = 32768.f;              // of normalised q and k: elements of at most one, with all bits of bf16 down to 2^-32
+static constexpr float kGdnKeyDown = 1.f / kGdnKeyUp;
 
 template <int kThreads>
 __device__ __forceinline__ void gdn_bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
@@ -602,7 +604,7 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
             const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
             const uint32_t nb = pack_bf16x2(e.x * f, e.y * f);
             const float2 r = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&nb));
-            return gdn_pack(r.x, r.y);
+            return gdn_pack(r.x * kGdnKeyUp, r.y * kGdnKeyUp);
           };
           const int t = w * kTokens + (j >> 1);
           *reinterpret_cast<uint2*>((j & 1 ? op.k : op.q) + t * 256 + (((lane >> 1) ^ (t & 7)) << 4) + (lane & 1) * 8) = make_uint2(norm(x[j].x), norm(x[j].y));
@@ -678,7 +680,8 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
         for (int h = 0; h < 2; ++h) {
           const int tr = g + 8 * h, t = tb * 16 + tr, sc = nt * 8 + 2 * c;
           const float2 ratio = *reinterpret_cast<const float2*>(&sm.ratio[t][sb * 16 + sc]);
-          float x = (d[0][2 * h] + d[1][2 * h]) * ratio.x, y = (d[0][2 * h + 1] + d[1][2 * h + 1]) * ratio.y;
+          constexpr float down = kGdnKeyDown * kGdnKeyDown;
+          float x = (d[0][2 * h] + d[1][2 * h]) * down * ratio.x, y = (d[0][2 * h + 1] + d[1][2 * h + 1]) * down * ratio.y;
           const float bt = __shfl_sync(0xffffffffu, beta, t);
           if (!is_q) {
             x *= bt;
@@ -802,7 +805,7 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
         for (int r = 0; r < 2; ++r) {
           const int e = gdn_exponent(most[r]);
           up[r] = gdn_pow2(13 - e);
-          down[r] = gdn_pow2(e - 13);
+          down[r] = gdn_pow2(e - 13) * kGdnKeyDown;
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h)
@@ -908,7 +911,7 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
         for (int r = 0; r < 2; ++r) {
           const int e = gdn_exponent(most[r]);
           up[r] = gdn_pow2(13 - e);
-          fs[r] = gdn_pow2(e - 13);
+          fs[r] = gdn_pow2(e - 13) * kGdnKeyDown;
         }
 #pragma unroll
         for (int b = 0; b < 2; ++b)
@@ -959,6 +962,8 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
         for (int j = 0; j < 16; ++j) {
           const int at = t * 256 + ((j ^ (t & 7)) << 4) + c * 4;
           float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + at)), q = __half22float2(*reinterpret_cast<const __half2*>(op.q + at));
+          k.x *= kGdnKeyDown; k.y *= kGdnKeyDown;
+          q.x *= kGdnKeyDown; q.y *= kGdnKeyDown;
 #pragma unroll
           for (int i = 0; i < 4; ++i) S[j][i] *= co.w;
           m0 = fmaf(S[j][0], k.x, fmaf(S[j][1], k.y, m0));
@@ -982,6 +987,7 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             float2 k = __half22float2(*reinterpret_cast<const __half2*>(op.k + t * 256 + ((j ^ (t & 7)) << 4) + c * 4));
+            k.x *= kGdnKeyDown; k.y *= kGdnKeyDown;
             S[j][0] = fmaf(d0, k.x, S[j][0]); S[j][1] = fmaf(d0, k.y, S[j][1]);
             S[j][2] = fmaf(d1, k.x, S[j][2]); S[j][3] = fmaf(d1, k.y, S[j][3]);
           }

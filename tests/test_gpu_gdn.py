@@ -181,6 +181,21 @@ def test_gdn_delta_chunks_that_do_not_stay_finite(where, value):
     assert rows.sum() >= rows.numel() - 2 and _row_errors(state[rows], want_state[rows]) < 2.0 ** -18
 
 
+@pytest.mark.parametrize("small", [-12, -18, -22])
+def test_gdn_delta_chunks_of_keys_with_small_elements(small):
+    """Elements of normalised q and k far below one (all bits of bf16 down to 2^-32): the columns of the state that they write, and what they read of
+    columns that are as much larger."""
+    counts, pos0, hk, hv = [64, 40], [7, 0], 1, 2
+    case = _delta_case(counts, pos0, hk, hv, 1)
+    size = torch.where(torch.arange(128, device=DEV) % 4 == 1, 2.0 ** small, 1.0)
+    case[0][:, :256] = (case[0][:, :256].view(-1, 2, 128) * size).view(-1, 256)
+    case[6].mul_(1 / size)
+    out, state = _delta(case, counts, pos0, hk, hv, None)
+    want, want_state = _delta(case, counts, pos0, hk, hv, 31)
+    assert _rel(out, want) < 2e-3 and _row_errors(state[1], want_state[1], -2) < 2.0 ** -14       # columns; the second request starts from zero
+    assert _row_errors(state[0] * size, want_state[0] * size) < 2.0 ** -18
+
+
 def test_gdn_delta_chunks_of_rows_that_are_not_aligned():
     """Rows that start anywhere are walked one by one; a review pass leaves the state."""
     from cubic_serve_b200.ops import kernels as K
