@@ -383,15 +383,18 @@ gdn_delta_kernel(const GdnDeltaParams p) {
 // without a shuffle.  Operands are f16: normalised k and q, bf16 of at most one, behind 2^15 (all bits down to 2^-32); what is computed in fp32 (S, Delta, L, the inverses, q . k) is
 // split in two f16 behind a power of two that puts the largest of its value row at 2^13 (22 bits); Delta as it enters the state in three.  Sums with what is
 // larger than the product (inverse less one, decayed state) are fp32 multiply-adds outside the tensor cores, which cut their sums off.
-// Decay ratios are products of their factors, as in the recurrence: no logarithm, no quotient.
-// Against 64 bits (331 rows, random decays): outputs 2.8982e-3 either way; the state 0.99e-7 against 0.77e-7 of the recurrence, with slow decays
-// and similar keys 5.9e-7 against 7.7e-7 (640 rows), with large values 9.2e-7 against 10.4e-7 (320).
+// Decay ratios are products of their factors, as in the recurrence: no logarithm, no quotient; they, and Delta on its way into the state, carry what a
+// rounding leaves over.
+// Against 64 bits, the recurrence -> this (relative error of the state; outputs, rounded to bf16, 2.9e-3 either way): random decays 0.74 -> 0.60e-7 (32 rows), 0.72 -> 0.63e-7
+// (331), slow ones 13.1 -> 12.0e-7 (1000; the decays themselves), none 2.9 -> 1.4e-7 (640) and with values 2^-24 to 1 of each other 2.7 -> 1.3e-7 (320).  It grows faster with the
+// likeness of a chunk's keys, as Delta is the product with an inverse: a mean cosine of 0.84 without decay 4.0 -> 2.9e-7, with random decays 0.77 -> 0.79e-7, of 0.99 without
+// decay 3.9 -> 5.2e-7 (keys of random projections behind the convolution: 0.11).
 //
 // A CTA is a head of a segment: warps 0-7 walk the chunks, warps 8-15 prepare the next chunk's operands and norm and store the last one's outputs
 // meanwhile.
-// What bounds it: the chain of a chunk (about 10000 cycles, of which its MMAs take 3500) and its preparation, which takes as long beside it.
-// One row after the other -> in chunks, 32 heads, one B200: segments of 1000, 536, 823, 359 and 646 rows 1013 -> 247 us, one of 1750 924 -> 380, one of 331
-// 307 -> 94, one of 32 34 -> 28, 16 of 256 1040 -> 249.
+// What bounds it: the chain of a chunk (6.9 us at 1.9 GHz, about 13000 cycles, of which its MMAs take 3500) and its preparation, which takes as long beside it.
+// One row after the other -> in chunks, 32 heads, one B200: segments of 1000, 536, 823, 359 and 646 rows 1013 -> 254 us, one of 1750 924 -> 382, one of 331
+// 307 -> 93, one of 32 34 -> 28, 16 of 256 1040 -> 254.
 // A chunk with a key, query, value or coefficient that is not finite is walked token by token: zero times it, in a row before it, is not zero.  Likewise, by
 // a warp for itself, one whose state or Delta is not.
 static constexpr int kGdnChunk = 32;
@@ -620,44 +623,43 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
         wild |= (top & 0x80008000u) != 0;
       }
       if (__any_sync(0xffffffffu, wild) && lane == 0) op.wild = 1;
-      // ---- ratios of the decays, lane = s: products of 1, 2, 4, .. decays behind token s, put together by the bits of the distance
+      // ---- ratios of the decays, lane = s: the products behind token s up to the warp's first token, and a decay more for each of its others.  With what the
+      // products leave over (in doubles the chunk took 7 % longer)
       {
-        float run[5];
-        const float behind = __shfl_down_sync(0xffffffffu, decay, 1);
-        run[0] = lane < 31 ? behind : 1.f;
-#pragma unroll
-        for (int k = 1; k < 5; ++k) {
-          const float x = __shfl_down_sync(0xffffffffu, run[k - 1], 1 << (k - 1));
-          run[k] = run[k - 1] * (lane + (1 << (k - 1)) < 32 ? x : 1.f);
-        }
-        auto ratio = [&](int t) {
-          const int dist = t - lane;
-          int at = lane;
-          float r = 1.f;
-#pragma unroll
-          for (int k = 0; k < 5; ++k) {
-            const float x = __shfl_sync(0xffffffffu, run[k], at);
-            if (dist >> k & 1) {
-              r *= x;
-              at += 1 << k;
-            }
-          }
-          return dist >= 0 ? r : 0.f;
+        float r = lane <= w * kTokens ? decay : 1.f, rest = 0.f;
+        auto times = [](float& x, float& x_rest, float y, float y_rest) {
+          const float z = x * y;
+          x_rest = fmaf(x, y_rest, fmaf(x_rest, y, fmaf(x, y, -z)));
+          x = z;
         };
-        float r = 0.f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float x = __shfl_down_sync(0xffffffffu, r, o), y = __shfl_down_sync(0xffffffffu, rest, o);
+          if (lane + o < 32) times(r, rest, x, y);
+        }
+        r = __shfl_down_sync(0xffffffffu, r, 1);
+        rest = __shfl_down_sync(0xffffffffu, rest, 1);
 #pragma unroll
         for (int j = 0; j < kTokens; ++j) {
-          r = ratio(w * kTokens + j);
-          sm.ratio[w * kTokens + j][lane] = r;
+          const int t = w * kTokens + j;
+          if (j > 0) times(r, rest, __shfl_sync(0xffffffffu, decay, t), 0.f);
+          if (lane == t) {
+            r = 1.f;
+            rest = 0.f;
+          }
+          sm.ratio[t][lane] = lane <= t ? r + rest : 0.f;
         }
-        if (w == 7) {
-          float G = decay;
+        if (w == 7) op.coef[lane].z = r + rest;
+        if (w == 6) {
+          float G = decay, G_rest = 0.f;
 #pragma unroll
           for (int o = 1; o < 32; o <<= 1) {
-            const float x = __shfl_up_sync(0xffffffffu, G, o);
-            if (lane >= o) G *= x;
+            const float x = __shfl_up_sync(0xffffffffu, G, o), y = __shfl_up_sync(0xffffffffu, G_rest, o);
+            if (lane >= o) times(G, G_rest, x, y);
           }
-          op.coef[lane] = make_float4(beta, G, r, decay);
+          op.coef[lane].x = beta;
+          op.coef[lane].y = G + G_rest;
+          op.coef[lane].w = decay;
         }
       }
       gdn_bar_sync<kGdnPrepareThreads>(5);
@@ -797,7 +799,8 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
     bool walk = op.wild || __any_sync(0xffffffffu, max(most[0], most[1]) >= 0x7F800000u);
     if (!walk) {
       // ---- S k and S q
-      float u[2][2][4];
+      constexpr float kToGrid = 1.5f * 8589934592.f;     // added and subtracted: multiples of 2^10
+      float u[2][2][4], rest[2][2][4];                   // u + rest is Delta, when all is done
       float down[2];
       {
         float x[2][2][4], up[2];
@@ -858,12 +861,13 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
             const float2 bg = *reinterpret_cast<const float2*>(&op.coef[t]);
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-              const float f = down[r] * bg.y;
-              u[h][j][2 * r + q] = fmaf(-u[h][j][2 * r + q], f, __bfloat162float(vs[t * kGdnDim + 8 * r])) * bg.x;
+              const float f = down[r] * bg.y, x = fmaf(-u[h][j][2 * r + q], f, __bfloat162float(vs[t * kGdnDim + 8 * r])), y = x * bg.x;
+              u[h][j][2 * r + q] = y;
+              rest[h][j][2 * r + q] = fmaf(x, bg.x, -y);
               o[h][j][2 * r + q] *= f;
             }
           }
-      // ---- Delta (in place of u) of tokens 0..15, then of 16..31
+      // ---- Delta (u + rest) of tokens 0..15, then of 16..31: what is smaller is added up beside u, so that u is rounded once
       uint32_t hi[4], lo[4];
       float d[2][4], f[2];
       auto add = [&](float (&x)[2][4], float sign) {     // x += d
@@ -872,19 +876,38 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) x[j][q] = fmaf(sign * (1.f / kGdnUp) * f[q >> 1], d[j][q], x[j][q]);
       };
+      auto sum = [&](float (&x)[2][4], float (&y)[2][4]) {                        // x + y in x, what that leaves over in y
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float z = x[j][q] + y[j][q], part = z - x[j][q];
+            y[j][q] = (x[j][q] - (z - part)) + (y[j][q] - part);
+            x[j][q] = z;
+          }
+      };
       gdn_operand(u[0], hi, lo, f);
       gdn_block(d, hi, lo, op.inv[0], lane);
-      add(u[0], 1.f);
+      add(rest[0], 1.f);
+      sum(u[0], rest[0]);
       gdn_operand(u[0], hi, lo, f);
       gdn_block(d, hi, lo, op.l10, lane);
-      add(u[1], -1.f);
+      add(rest[1], -1.f);
       gdn_block(d, hi, lo, op.a[0], lane);
       add(o[0], 1.f);
       gdn_block(d, hi, lo, op.a[1], lane);
       add(o[1], 1.f);
-      gdn_operand(u[1], hi, lo, f);
+      {
+        float x[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[j][q] = u[1][j][q] + rest[1][j][q];
+        gdn_operand(x, hi, lo, f);
+      }
       gdn_block(d, hi, lo, op.inv[1], lane);
-      add(u[1], 1.f);
+      add(rest[1], 1.f);
+      sum(u[1], rest[1]);
       gdn_operand(u[1], hi, lo, f);
       gdn_block(d, hi, lo, op.a[2], lane);
       add(o[1], 1.f);
@@ -899,7 +922,9 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
           const float r0 = op.coef[b * 16 + j * 8 + 2 * c].z, r1 = op.coef[b * 16 + j * 8 + 2 * c + 1].z;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            u[b][j][q] *= q & 1 ? r1 : r0;
+            const float r = q & 1 ? r1 : r0, x = u[b][j][q] * r;
+            rest[b][j][q] = fmaf(rest[b][j][q], r, fmaf(u[b][j][q], r, -x));
+            u[b][j][q] = x;
             most[q >> 1] = max(most[q >> 1], gdn_bits(u[b][j][q]));
           }
         }
@@ -921,11 +946,10 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
             for (int r = 0; r < 2; ++r) {
               const int at = 2 * j + r;
               float x = u[b][j][2 * r] * up[r], y = u[b][j][2 * r + 1] * up[r];
-              const uint32_t coarse = pack_bf16x2(x, y);
-              first[b][at] = gdn_pack(__uint_as_float(coarse << 16), __uint_as_float(coarse & 0xFFFF0000u));
-              const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&first[b][at]));
-              x -= f2.x;
-              y -= f2.y;
+              const float xf = x + kToGrid - kToGrid, yf = y + kToGrid - kToGrid;
+              first[b][at] = gdn_pack(xf, yf);
+              x = x - xf + rest[b][j][2 * r] * up[r];
+              y = y - yf + rest[b][j][2 * r + 1] * up[r];
               gdn_split(x, y, second[b][at], third[b][at]);
             }
 #pragma unroll
@@ -938,7 +962,8 @@ gdn_delta_chunk_kernel(const GdnDeltaParams p) {
           }
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            // products of the first parts have 16 bits: kept apart from the rest, 2^-8 of them, their sum loses next to nothing
+            // The tensor cores cut a sum off below its last bit, half a bit too small on average.  First parts are multiples of 2^10: their sums have no more
+            // bits than fit, unless a key's element is below 2^-13; what is cut off the rest, 2^-4 of them, does not count.
             float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int b = 0; b < 2; ++b) {

@@ -196,6 +196,53 @@ def test_gdn_delta_chunks_of_keys_with_small_elements(small):
     assert _row_errors(state[0] * size, want_state[0] * size) < 2.0 ** -18
 
 
+def _delta_in_64_bits(case, hk, hv):
+    """The state behind one segment that goes on from ``case``'s."""
+    qkv, _, ba, a_log, dt_bias, _, state = case
+    n = qkv.shape[0]
+    k = qkv[:, hk * 128:2 * hk * 128].double().view(n, hk, 128)
+    k = (k * (k.square().sum(-1, keepdim=True) + 1e-6).rsqrt()).bfloat16().double().repeat_interleave(hv // hk, 1)
+    v = qkv[:, 2 * hk * 128:].double().view(n, hv, 128)
+    b, a = ba.double().split(hv, -1)
+    decay = (-a_log.double().exp() * torch.nn.functional.softplus(a + dt_bias.double())).exp()
+    s = state[0].double().clone()
+    for t in range(n):
+        s *= decay[t][:, None, None]
+        s += ((v[t] - (s @ k[t].unsqueeze(-1)).squeeze(-1)) * b[t].sigmoid().unsqueeze(-1)).unsqueeze(-1) * k[t].unsqueeze(-2)
+    return s
+
+
+def _away_from_ties(x):
+    """Rows of 128 whose normalised elements are not near a tie of bf16 are kept, the others drawn again."""
+    while True:
+        z = x.double()
+        z = z * (z.square().sum(-1, keepdim=True) + 1e-6).rsqrt()
+        f = torch.frexp(z.abs()).mantissa * 256
+        bad = ((f - f.floor() - 0.5).abs() < 1e-4).any(-1)
+        if not bad.any():
+            return x
+        x[bad] = (x[bad].float() + 0.3 * torch.randn(int(bad.sum()), 128, device=DEV)).bfloat16()
+
+
+@pytest.mark.parametrize("alike", [0.0, 0.4])
+@pytest.mark.parametrize("a,n", [(0.0, 32), (0.0, 331), (1.5, 200), (-5.0, 640), (-200.0, 331)])
+def test_gdn_delta_chunks_are_as_near_to_64_bits_as_rows(a, n, alike):
+    """The state's error against 64 bits is no larger than that of the row-by-row kernel: random, fast, slow and no decay, unlike and similar keys
+    (a cosine of 0.3; see the kernel's comment for more alike ones)."""
+    hk, hv, errors = 2, 4, [[], []]
+    torch.manual_seed(n)
+    for seed in range(3):
+        case = list(_delta_case([n], [7], hk, hv, 2 * seed))
+        g = torch.Generator(device=DEV).manual_seed(seed)
+        qk = torch.randn(n, 2 * hk, 128, device=DEV, generator=g) * (1 - alike) + torch.randn(1, 2 * hk, 128, device=DEV, generator=g) * alike
+        case[0][:, :2 * hk * 128] = _away_from_ties(qk.bfloat16()).view(n, -1)
+        case[3] = torch.full((hv,), a, device=DEV) + (0.3 * torch.randn(hv, device=DEV, generator=g) if a > -100 else 0)
+        exact = _delta_in_64_bits(case, hk, hv)
+        for at_once, e in zip((None, 31), errors):
+            e.append(_rel(_delta(case, [n], [7], hk, hv, at_once)[1][0].double(), exact))
+    assert sum(errors[0]) <= sum(errors[1])
+
+
 def test_gdn_delta_chunks_of_rows_that_are_not_aligned():
     """Rows that start anywhere are walked one by one; a review pass leaves the state."""
     from cubic_serve_b200.ops import kernels as K
