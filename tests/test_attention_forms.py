@@ -84,6 +84,14 @@ def test_prompts_take_the_kernel_that_was_measured_faster(hq, hkv, portions, pro
     assert b.attn_prompts == ((0, b.num_row_blocks) if prompt else (0, 0)) and not b.attn_decode
 
 
+@pytest.mark.parametrize("hq,hkv,portions,prompt", [
+    (32, 32, [(0, 64)] * 5, False), (32, 32, [(0, 64), (0, 40), (0, 33), (0, 64), (0, 51)], False), (16, 1, [(0, 26 - i % 19) for i in range(40)], False),
+    (32, 8, [(0, 64)] * 8, True)])
+def test_short_prompts_take_the_kernel_that_was_measured_faster(hq, hkv, portions, prompt):
+    b = _fill(portions, hq, hkv)
+    assert b.attn_prompts == ((0, b.num_row_blocks) if prompt else (0, 0))
+
+
 @pytest.mark.parametrize("hq,hkv,portions,prompts", [
     (32, 8, [(1000, 1)] * 64 + [(0, 512)] * 2, (64, 320)), (32, 4, [(700, 1)] * 20 + [(0, 512)] * 2 + [(700, 1)] * 20, (0, 0)),
     (16, 1, [(1000, 4)] * 32 + [(0, 1024)] * 4, (0, 0)),               # the long review CTAs would start last
