@@ -120,25 +120,6 @@ struct TsWalk {
   }
 };
 
-__device__ __forceinline__ void ts_umma_bf16(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void ts_tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
-      "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]),
-      "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-
 // Bytes of a unit's codes and tables
 __host__ __device__ constexpr int ts_codes() { return 2 * kCodeBytes; }
 __host__ __device__ constexpr int ts_meta(int fmt) { return fmt == kFmtCubic4 ? kMetaBytesCubic : 2 * kMetaBytes; }
@@ -302,13 +283,13 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       if (!ok) break;
       tc_fence_after();
       const uint32_t to = tmem + kTsTmemA + grp * 64 + (static_cast<uint32_t>(quad * 32) << 16);
-      ts_tmem_st32(to, out);
+      tmem_st_32x32(to, out);
       uint32_t out2[32];
       ts_decode<FMT>(cs + c * kC, 1, row, out2);
-      ts_tmem_st32(to + 32, out2);
+      tmem_st_32x32(to + 32, out2);
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl.c_empty[c]));
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl.full[grp]));
@@ -409,7 +390,7 @@ wq_gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              ts_umma_bf16(acc, tmem_u + kTsTmemA + s * 64 + h * 32 + k * 8, d + (h * x_half >> 4) + k * 2, idesc, kb > run.kb || h > 0 || k > 0);
+              umma_f16_ts(acc, tmem_u + kTsTmemA + s * 64 + h * 32 + k * 8, d + (h * x_half >> 4) + k * 2, idesc, kb > run.kb || h > 0 || k > 0);
           tc_commit(smem_u32(&ctl.empty[s]));
         }
         __syncwarp();
