@@ -254,10 +254,10 @@ def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = 
     blocks = -(-m // 128)
     tiles = -(-w.n // 128) * blocks
     units = tiles * (w.k // 128)
+    if 2 * units < 13 * sms:                               # (no rows: none)
+        return False
     own = sms // tiles if 2 * tiles <= sms else 0          # parts of a tile, if every one has some of its own
     rows = -(-m // blocks)
-    if 2 * units < 13 * sms:
-        return False
     if m > 128:
         if rows * own > 1000 if own else units < 28 * sms:
             return False

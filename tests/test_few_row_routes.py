@@ -141,7 +141,7 @@ def test_batches_of_more_rows_than_a_block(n, k, rows, others):
 
 @pytest.mark.parametrize("n,k,takes,others", [
     (4096, 4096, (1, 8, 64, 128, 129, 256), (257,)), (6144, 4096, (1, 8, 96, 128), (129,)), (8192, 2048, (1, 64, 128), (129,)), (10240, 2048, (1, 64, 96), (97, 128)),
-    (14336, 1024, (), (1, 9, 64, 128)), (2560, 9728, (1, 128), ()), (3584, 5120, (9, 96, 128), ()), (2048, 8192, (1, 64, 88), (89, 128)),
+    (14336, 1024, (), (0, 1, 9, 64, 128)), (2560, 9728, (1, 128), ()), (3584, 5120, (9, 96, 128), ()), (2048, 8192, (1, 64, 88), (89, 128)),
     (1024, 16384, (1, 9, 64), (65, 128)), (1024, 8192, (129, 192, 257, 512), (64, 128, 256))])
 def test_lines_of_the_kernel_with_tiles_in_tensor_memory(n, k, takes, others):
     w = SimpleNamespace(fmt=wq_pack.FMT_CUBIC4, n=n, k=k, group_k=128)
