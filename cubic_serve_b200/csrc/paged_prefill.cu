@@ -10,12 +10,12 @@
 // Powers of two keep hi and lo in the range of f16: one a step for K, undone in the softmax' multiply-add; one for V that grows with the
 // largest scale of a run of steps, falls back towards one, and is undone with the output (a row keeps that of its own request's steps).
 // What is 2^-k of the largest scale keeps 22 bits up to k = 6 to 8, then 28 - k; probabilities have 11.  A product's error stays below 2^-18 (V) and 2^-20 (K) as long
-// as the largest scale is below 16 (values of 2000), as far as f16 products of probabilities and scales would go.  Beyond that, and with V
-// scales that are not finite, the rows that see such tokens are computed once more, in fp32 from the pages (pf_row).
+// as the largest scale is below 16 (values of 2000), as far as f16 products of probabilities and scales would go.  Beyond that the rows
+// that see such tokens are computed once more, in fp32 from the pages (pf_row); what values with scales that are not finite contribute is added (pf_odd).
 // MMAs of a step take 640 + 512 cycles a tile (measured in a loop of their own); with their operands, raw pages and the conversion's stores shared memory
 // moves about 280 KB a step: 4000 cycles a step of 256 rows where 2 x 5800 were spent.  General kernel -> before -> now, one B200, cold L2, 32 heads
-// over 8, 8 bits: 8 x 1024 tokens 702 -> 520 -> 220 us, 4 x 256 behind 2048 276 -> 233 -> 104, one prompt of 8192 3734 -> 2775 -> 1275, 40 x 20 behind 300
-// 63 -> 103 -> 57; 32 over 4, 4 / 8 bits, 2 x 2048 571 -> 421 -> 193; 64 over 4, 6 bits, 3 x 500 190 -> 131 -> 80.
+// over 8, 8 bits: 8 x 1024 tokens 702 -> 520 -> 219 us, 4 x 256 behind 2048 276 -> 233 -> 104, one prompt of 8192 3734 -> 2775 -> 1252, 40 x 20 behind 300
+// 63 -> 103 -> 56, 8 x 64 26 -> 15 -> 17; 32 over 4, 4 / 8 bits, 2 x 2048 571 -> 421 -> 194; 64 over 4, 6 bits, 3 x 500 190 -> 131 -> 76.
 //
 // Roles: warps 0-7 own a row a thread (softmax needs no exchange: tensor-memory lane = row); warps 8-11 convert raw pages of K to the swizzled operand
 // (hi and lo, [token][channel]), warps 12-15 those of V; warps 16 and 18 issue the MMAs; warp 17 lists the items' requests and copies their
@@ -70,7 +70,8 @@ struct __align__(1024) PfSmem {
   uint8_t v[2][2][2 * kPfHalf];                          // likewise
   float k_mul[kPfNotes];                                 // scores are this times what the MMAs give
   int v_exp[kPfNotes];                                   // output is 2^v_exp times ...
-  int redo[kPfLists][kPfBlocks], redo_least[kPfLists];   // of a run, of all: rows that see more tokens than this are computed once more
+  // tokens of a run: rows that see more are computed once more [0], have values with scales that are not finite added [1]; the least of all
+  int redo[kPfLists][2][kPfBlocks], redo_least[kPfLists];
   uint64_t raw_full[kPfRaw], raw_free[kPfRaw], k_full[2], k_free[2], v_full[2], v_free[2], k_note[kPfNotes], v_note[kPfNotes];
   uint64_t list_full[kPfLists], list_free[kPfLists], q_full[kPfTiles], s_full[kPfTiles], s_free[kPfTiles], p_full[kPfTiles], pv_done[kPfTiles];
   PfList list[kPfLists];
@@ -331,6 +332,79 @@ __device__ __forceinline__ void pf_row(const AttnParams& p, int req, int kvh, in
   reinterpret_cast<uint2*>(out)[lane] = make_uint2(pack_bf16x2(o[0] * inv, o[1] * inv), pack_bf16x2(o[2] * inv, o[3] * inv));
 }
 
+// Adds to the rows of a warp (a lane has one: its request, how many tokens it sees, where its query and result are, its maximum and the reciprocal of its
+// sum) what tokens from `from` on whose V scales are not finite contribute; the operands have left them out.  Rows of a request look for them together.
+template <int KBITS, int VBITS>
+__device__ __forceinline__ void pf_odd(const AttnParams& p, int kvh, int req, int from, int limit, long long at, float m, float inv, int lane) {
+  constexpr float kBias = 1 << (KBITS - 1), vBias = 1 << (VBITS - 1);
+  constexpr int kScan = 4;
+#pragma unroll 1
+  for (uint32_t left = __ballot_sync(0xffffffffu, limit > from); left;) {
+    const int rq = __shfl_sync(0xffffffffu, req, __ffs(left) - 1);
+    const bool mine = (left >> lane & 1) != 0 && req == rq;
+    uint32_t rows = __ballot_sync(0xffffffffu, mine);
+    left &= ~rows;
+    const int most = __reduce_max_sync(0xffffffffu, mine ? limit : 0), least = __reduce_min_sync(0xffffffffu, mine ? from : INT_MAX);
+    auto blob_of = [&](int tok) {
+      return p.cache + (static_cast<size_t>(p.page_table[static_cast<size_t>(rq) * p.max_pages + tok / kPageTokens]) * p.Hkv + kvh) * p.lay.blob_bytes;
+    };
+    auto next = [&](int t) {                               // the first of them from t on, or `most`
+#pragma unroll 1
+      for (int t0 = t & ~31; t0 < most; t0 += 32 * kScan) {
+        bool odd[kScan];                                   // the lane's token of every 32
+#pragma unroll
+        for (int j = 0; j < kScan; ++j) {
+          const int tok = t0 + 32 * j + lane;
+          float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (tok >= t && tok < most) f = *reinterpret_cast<const float4*>(blob_of(tok) + p.lay.v_scale_off + tok % kPageTokens * 16);
+          odd[j] = !(fabsf(f.x) < INFINITY && fabsf(f.y) < INFINITY && fabsf(f.z) < INFINITY && fabsf(f.w) < INFINITY);
+        }
+#pragma unroll
+        for (int j = 0; j < kScan; ++j) {
+          const uint32_t toks = __ballot_sync(0xffffffffu, odd[j]);
+          if (toks) return t0 + 32 * j + __ffs(toks) - 1;
+        }
+      }
+      return most;
+    };
+#pragma unroll 1
+    for (int t = next(least); t < most && rows != 0; t = next(t + 1)) {
+      const int tok = t % kPageTokens;
+      const uint8_t* blob = blob_of(t);
+      const uint32_t kc = pf_codes_k<KBITS>(blob, tok, lane), vc = pf_codes_v<VBITS>(blob + p.lay.v_code_off, tok, lane);
+      const float ks = *reinterpret_cast<const float*>(blob + p.lay.k_scale_off + tok * 16 + (lane >> 3) * 4) * p.scale_log2;
+      const float vs = *reinterpret_cast<const float*>(blob + p.lay.v_scale_off + tok * 16 + (lane >> 3) * 4);
+      const bool add = !(fabsf(vs) < INFINITY);
+#pragma unroll 1
+      for (uint32_t see = rows & __ballot_sync(0xffffffffu, limit > t); see; see &= see - 1) {
+        const int of = __ffs(see) - 1;
+        const long long to = __shfl_sync(0xffffffffu, at, of);
+        const float top = __shfl_sync(0xffffffffu, m, of), scale = __shfl_sync(0xffffffffu, inv, of);
+        const uint2 qw = reinterpret_cast<const uint2*>(p.q + to)[lane];
+        uint2* out = reinterpret_cast<uint2*>(p.out + to) + lane;
+        const uint2 w = *out;
+        auto two = [](uint32_t x) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x)); };
+        const float2 q01 = two(qw.x), q23 = two(qw.y), o01 = two(w.x), o23 = two(w.y);
+        const float qf[4] = {q01.x, q01.y, q23.x, q23.y};
+        float o[4] = {o01.x, o01.y, o23.x, o23.y}, z = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) z = fmaf(qf[c], static_cast<float>(kc >> (8 * c) & 255u) - kBias, z);
+        z *= ks;
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o2);
+        if (add) {
+          const float pr = fast_exp2(z - (top == -INFINITY ? 0.f : top)) * scale;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) o[c] = fmaf(pr, (static_cast<float>(vc >> (8 * c) & 255u) - vBias) * vs, o[c]);
+          *out = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+        }
+        // (NaN stays: behind it there is nothing to add)
+        if (__all_sync(0xffffffffu, o[0] != o[0] && o[1] != o[1] && o[2] != o[2] && o[3] != o[3])) rows &= ~(1u << of);
+      }
+    }
+  }
+}
+
 template <int KBITS, int VBITS>
 __global__ void __launch_bounds__(kPfThreads, 1)
 paged_prefill_kernel(const AttnParams p, const int row_blocks) {
@@ -410,7 +484,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
         if (ok && n >= kPfLists) ok = mbar_wait_park(smem_u32(&sm.list_free[n % kPfLists]), (n / kPfLists - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) return false;
-        if (lane < kPfBlocks) sm.redo[n % kPfLists][lane] = INT_MAX;
+        sm.redo[n % kPfLists][lane / kPfBlocks][lane % kPfBlocks] = INT_MAX;
         if (lane == 0) sm.redo_least[n % kPfLists] = INT_MAX;
         if (at >= items) {                               // no item in this round: there is no further round
           if (lane == 0) l.kvh = -1;
@@ -597,8 +671,8 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
         const bool odd = most >= 0x7F800000u;                            // some are not finite
         if (odd) most = __reduce_max_sync(0xffffffffu, max(pf_most<true>(scale[0]), pf_most<true>(scale[1])));
         const int e = pf_exponent(most);
-        auto redo_from = [&](int tok) {                                  // rows that see more than `tok` tokens of the run
-          atomicMin(&sm.redo[it % kPfLists][run], tok);
+        auto redo_from = [&](int what, int tok) {                        // rows that see more than `tok` tokens of the run
+          atomicMin(&sm.redo[it % kPfLists][what][run], tok);
           atomicMin(&sm.redo_least[it % kPfLists], tok);
         };
         if (!is_v) {
@@ -606,7 +680,7 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
           if (warp == 8) {
             if (e > kPfLarge) {
               const uint32_t of[2] = {pf_most<true>(scale[0]), pf_most<true>(scale[1])};
-              if (__any_sync(0xffffffffu, (of[0] != 0 && pf_exponent(of[0]) < e - 8) || (of[1] != 0 && pf_exponent(of[1]) < e - 8)) && lane == 0) redo_from(tok0);
+              if (__any_sync(0xffffffffu, (of[0] != 0 && pf_exponent(of[0]) < e - 8) || (of[1] != 0 && pf_exponent(of[1]) < e - 8)) && lane == 0) redo_from(0, tok0);
             }
             if (lane == 0) {
               sm.k_mul[note] = pow2f(e - 5);
@@ -623,17 +697,20 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
             v_top = max(v_top, v_exp);
           }
           if (warp == 12) {
-            if (odd || v_exp > kPfLarge - 3) {                           // tokens with a scale that is not finite, or below 2^-8 beside large ones
+            if (odd || v_exp > kPfLarge - 3) {
               const float least = v_exp > kPfLarge - 3 ? pow2f(v_exp - 8) : 0.f;
-              bool out[2] = {false, false};
+#pragma unroll 1
+              for (int what = 0; what < 2; ++what) {                     // tokens with a scale below 2^-8 beside large ones, with one that is not finite
+                bool out[2] = {false, false};
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const float f[4] = {scale[h].x, scale[h].y, scale[h].z, scale[h].w};
+                for (int h = 0; h < 2; ++h) {
+                  const float f[4] = {scale[h].x, scale[h].y, scale[h].z, scale[h].w};
 #pragma unroll
-                for (int j = 0; j < 4; ++j) out[h] |= !(fabsf(f[j]) < INFINITY) || (f[j] != 0.f && fabsf(f[j]) < least);
+                  for (int j = 0; j < 4; ++j) out[h] |= what == 0 ? f[j] != 0.f && fabsf(f[j]) < least : !(fabsf(f[j]) < INFINITY);
+                }
+                const uint32_t lo = __ballot_sync(0xffffffffu, out[0]), hi = __ballot_sync(0xffffffffu, out[1]);
+                if ((lo | hi) != 0 && lane == 0) redo_from(what, tok0 + (lo != 0 ? __ffs(lo) - 1 : 31 + __ffs(hi)));
               }
-              const uint32_t lo = __ballot_sync(0xffffffffu, out[0]), hi = __ballot_sync(0xffffffffu, out[1]);
-              if ((lo | hi) != 0 && lane == 0) redo_from(tok0 + (lo != 0 ? __ffs(lo) - 1 : 31 + __ffs(hi)));
             }
             if (lane == 0) {
               sm.v_exp[note] = v_exp;
@@ -837,17 +914,21 @@ paged_prefill_kernel(const AttnParams p, const int row_blocks) {
         if (*const_cast<volatile int*>(&sm.redo_least[it % kPfLists]) != INT_MAX && ok) {
           // (what later steps still add to `redo` is beyond what the rows of this tile see)
           __syncwarp();                                  // a row's result is written again by other lanes
-          int req = 0, from = INT_MAX;
+          int req = 0, from[2] = {INT_MAX, INT_MAX};
           for (int i = 0; i < l.runs; ++i)
             if (blk >= l.run[i].first && blk < l.run[i].end) {
               req = l.run[i].req;
-              from = *const_cast<volatile int*>(&sm.redo[it % kPfLists][i]);
+              for (int what = 0; what < 2; ++what) from[what] = *const_cast<volatile int*>(&sm.redo[it % kPfLists][what][i]);
             }
-          for (uint32_t rows = __ballot_sync(0xffffffffu, cur.out != nullptr && cur.limit > from); rows; rows &= rows - 1) {
+          const bool again = cur.out != nullptr && cur.limit > from[0];
+          const long long at = cur.out != nullptr ? cur.out - p.out : 0;
+#pragma unroll 1
+          for (uint32_t rows = __ballot_sync(0xffffffffu, again); rows; rows &= rows - 1) {
             const int of = __ffs(rows) - 1;
-            const long long at = __shfl_sync(0xffffffffu, static_cast<long long>(cur.out - p.out), of);
-            pf_row<KBITS, VBITS>(p, __shfl_sync(0xffffffffu, req, of), l.kvh, __shfl_sync(0xffffffffu, cur.limit, of), p.q + at, p.out + at, lane);
+            const long long to = __shfl_sync(0xffffffffu, at, of);
+            pf_row<KBITS, VBITS>(p, __shfl_sync(0xffffffffu, req, of), l.kvh, __shfl_sync(0xffffffffu, cur.limit, of), p.q + to, p.out + to, lane);
           }
+          pf_odd<KBITS, VBITS>(p, l.kvh, req, from[1], again || cur.out == nullptr ? 0 : cur.limit, at, m, inv, lane);
         }
       }
       __syncwarp();

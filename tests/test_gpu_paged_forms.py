@@ -139,6 +139,30 @@ def test_prompt_form_keeps_values_to_those_who_see_them(kb, vb, bad):
         assert not torch.isfinite(got[sees].float()).all(-1).any()
 
 
+@pytest.mark.parametrize("kb,vb", [(8, 8), (6, 4), (4, 6)])
+def test_prompt_form_with_values_that_are_infinite_in_a_channel_group(kb, vb):
+    """Infinite V scales of one channel group, of one token, of a few far apart, of all from some on: that group of the rows that see them is what
+    the codes say, the other groups and rows keep their results."""
+    group, n = 4, 300
+    cache, table = _cache([n], 1, kb, vb, 25)
+    q = torch.randn(n, group, D, device=DEV, generator=torch.Generator(device=DEV).manual_seed(11)).bfloat16()
+    blocks = [(0, i, min(4, n - i), i + 1) for i in range(0, n, 4)]
+    want = _run("prefill", q, cache, table, blocks, group, 1, kb, vb, 1)
+    for toks in ([77], [3, 130, 299], range(150, n)):
+        hit = cache.clone()
+        for t in toks:
+            _scales(hit, kb, vb)[int(table[0, t // 16]), 0, t % 16, 2] = float("inf")
+        got = _run("prefill", q, hit, table, blocks, group, 1, kb, vb, 1)
+        sees = torch.arange(n, device=DEV) >= min(toks)
+        one = _request(hit, table, 0, n, kb, vb) if len(toks) == 1 else None
+        assert torch.equal(got[~sees], want[~sees]) and not torch.isfinite(got[sees][..., 64:96].float()).any()
+        if one:                                              # infinities by the sign of the token's codes, NaN where those are zero
+            codes = one[1][toks[0], 64:96].float()
+            assert torch.equal(got[sees][..., 64:96].cpu().float().nan_to_num(nan=0), codes.nan_to_num(nan=0).expand(int(sees.sum()), group, 32).nan_to_num(nan=0))
+        for cols in (slice(0, 64), slice(96, 128)):
+            assert _close(got[..., cols], want[..., cols])
+
+
 @pytest.mark.parametrize("kb,vb", [(8, 8), (8, 4)])
 @pytest.mark.parametrize("top", [16000.0, 16400.0, 40000.0, 65000.0])
 def test_prompt_form_has_the_range_of_f16_for_scales(kb, vb, top):
