@@ -14,8 +14,8 @@
 // that see such tokens are computed once more, in fp32 from the pages (pf_row); what values with scales that are not finite contribute is added (pf_odd).
 // MMAs of a step take 640 + 512 cycles a tile (measured in a loop of their own); with their operands, raw pages and the conversion's stores shared memory
 // moves about 280 KB a step: 4000 cycles a step of 256 rows where 2 x 5800 were spent.  General kernel -> before -> now, one B200, cold L2, 32 heads
-// over 8, 8 bits: 8 x 1024 tokens 702 -> 520 -> 219 us, 4 x 256 behind 2048 276 -> 233 -> 104, one prompt of 8192 3734 -> 2775 -> 1252, 40 x 20 behind 300
-// 63 -> 103 -> 56, 8 x 64 26 -> 15 -> 17; 32 over 4, 4 / 8 bits, 2 x 2048 571 -> 421 -> 194; 64 over 4, 6 bits, 3 x 500 190 -> 131 -> 76.
+// over 8, 8 bits: 8 x 1024 tokens 702 -> 520 -> 213 us, 4 x 256 behind 2048 276 -> 233 -> 100, one prompt of 8192 3734 -> 2775 -> 1165, 40 x 20 behind 300
+// 63 -> 103 -> 56, 8 x 64 26 -> 15 -> 17; 32 over 4, 4 / 8 bits, 2 x 2048 571 -> 421 -> 192; 64 over 4, 6 bits, 3 x 500 190 -> 131 -> 79.
 //
 // Roles: warps 0-7 own a row a thread (softmax needs no exchange: tensor-memory lane = row); warps 8-11 convert raw pages of K to the swizzled operand
 // (hi and lo, [token][channel]), warps 12-15 those of V; warps 16 and 18 issue the MMAs; warp 17 lists the items' requests and copies their
@@ -277,7 +277,7 @@ __device__ __forceinline__ uint32_t pf_codes_v(const uint8_t* v, int tok, int la
 }
 
 // A row in fp32, by a warp whose lanes have four channels each: `limit` tokens of request `req`, the query at `q` (result likewise in `out`).
-// About 100 cycles a token and row where the MMAs take an eighth of one: for caches whose scales lie far apart.
+// A hundred times as long as the MMAs (8 x 1024 tokens 23 ms): for caches whose scales are as large and as far apart as no model's.
 template <int KBITS, int VBITS>
 __device__ __forceinline__ void pf_row(const AttnParams& p, int req, int kvh, int limit, const __nv_bfloat16* q, __nv_bfloat16* out, int lane) {
   constexpr int kTok = 4;                                // tokens at a time, of one page

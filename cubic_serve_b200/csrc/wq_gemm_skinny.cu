@@ -17,12 +17,12 @@
 // swizzled 64-column tiles.  (Copies by the consumers themselves, cp.async, spent 27 shared-memory cycles per instruction and a
 // quarter of the issue slots: 30 us instead of 23 at 8 x 24576 x 4096.)
 //
-// Large 4-bit weights go to wq_gemm_ts.cu.  Measured, weights not in L2 (floor = packed bytes / 6.65 TB/s), Cubic weights, 8 rows: 24576 x 4096
-// 22.3 us (floor 9.5, tcgen05 kernels with decoded tiles in shared memory 34), 4096 x 12288 12.8 (4.7, 21.5), 6144 x 4096 9.1 (2.4, 14.8), 4096 x 4096
-// 6.4 (1.6, 10.1); bf16 50688 x 4096 65 (62, 98).  Block-scaled e4m3 weights have nothing to decode either: their chunks and those of the e4m3
+// Large 4-bit weights go to wq_gemm_ts.cu.  Measured, weights not in L2 (floor = packed bytes / 6.65 TB/s), Cubic weights, 8 rows, launches in a row whose
+// starts overlap: 24576 x 4096 24 us (floor 9.5, tcgen05 kernels with decoded tiles in shared memory 34), 4096 x 12288 13.6 (4.7, 21.5), 6144 x 4096 9.5 (2.4,
+// 14.8), 4096 x 4096 6.6 (1.6, 10.1); single launches behind other work 27.7, 17.5, 13.0, 10.4.  bf16 50688 x 4096 65 (62, 98).  Block-scaled e4m3 weights have nothing to decode either: their chunks and those of the e4m3
 // activations are the operands of m16n8k16 once they are f16; 128 experts of 3072 x 4096, eight rows each, 263 us (floor 246, tcgen05 kernel 409),
 // 4096 x 1536 140 (123, 289).  What is left above the floor of 4-bit weights is the decode (integer pipe 38 % busy, four warps a scheduler that issue in 37 % of
-// the cycles) and 5 us of start, last loads and the sum of the parts.
+// the cycles) and 4 to 5 us of start, last loads and the sum of the parts.
 #include "wq_gemm_common.cuh"
 #include "launch.cuh"
 

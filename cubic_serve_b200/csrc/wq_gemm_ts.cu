@@ -7,9 +7,9 @@
 // decoding thread owns a weight row, its 64 decoded columns are one tcgen05.st.  Shared memory then holds nothing but copies, in two rings of
 // their own: codes (10 KB a stage, up to 12 stages, on their way before the previous kernel is done) and activations.  A unit of the pipeline
 // is 128 columns: the one thread that waits, counts and issues copies or MMAs for a stage takes 150 to 200 cycles for it, whatever it moves.
-// Few-row, per-tile or persistent kernel -> this one, Cubic weights not in L2, 8 / 48 / 128 rows, one B200: 24576 x 4096 27.4 / 38.7 / 44.5 ->
-// 21.9 / 24.0 / 29.7 us (floor 8.7), 4096 x 12288 17.2 / 25.5 / 28.3 -> 15.7 / 17.9 / 22.3 (4.3), 6144 x 4096 13.2 / 18.9 / 21.4 -> 11.7 / 13.6 / 18.8
-// (2.2).  About 8 us of each are start (4300 cycles to the first codes), the last run's sums and the sum of parts.  128 experts (NVFP4) of 1536 x 2048,
+// Few-row, per-tile or persistent kernel -> this one, Cubic weights not in L2, single launches behind other work, 8 / 48 / 128 rows, one B200: 24576 x 4096
+// 27.4 / 38.7 / 44.5 -> 21.9 / 24.0 / 29.7 us (floor 8.7), 4096 x 12288 17.2 / 25.5 / 28.3 -> 15.7 / 17.9 / 22.3 (4.3), 6144 x 4096 13.2 / 18.9 / 21.4 -> 11.7 / 13.6 / 18.8
+// (2.2); launches in a row whose starts overlap, 8 rows: 23.9 -> 20.3, 13.6 -> 12.9, 9.5 -> 8.9.  About 8 us of each are start (4300 cycles to the first codes), the last run's sums and the sum of parts.  128 experts (NVFP4) of 1536 x 2048,
 // 6 / 24 / 64 / 256 rows an expert: 85 / 134 / 137 / 299 -> 73 / 78 / 93 / 251 us (35 us of codes; at 256 rows 125 us of MMAs), 2048 x 768
 // 48 / 88 / 102 / 287 -> 41 / 43 / 51 / 132.  Blocks of rows decode a tile once each: 24576 x 4096 at 256 / 331 / 512 rows, single cold launches,
 // 57.5 / 89.5 / 93.1 -> 48.8 / 64.3 / 83.5 us.  Up to 24 rows the decode's integer pipe is half busy and its latency the rest (a unit in 740 cycles, 490

@@ -150,13 +150,13 @@ class BatchBuilder:
         The bound of the prompt kernel's time: 3 us a step of 64 tokens and eight blocks, and as much as four steps around them, in CTAs that start last
         blocks first, so that with more of them than SMs the step ends with the longest, with one that starts late behind the load before it, or
         with two that have to share an SM.  The kernel itself is persistent, deals items of sixteen blocks by their length and takes 2.1 us a step of them: the
-        bound holds back steps that would gain, and few that would not pass it.  General kernel: 0.128 us a page and SM, 2.1 us a CTA and SM, 0.06 us a page
+        bound keeps some steps from it that would gain.  General kernel: 0.128 us a page and SM, 2.1 us a CTA and SM, 0.06 us a page
         of the longest split, and 14.5 us for its launch, which is there anyway when there are other row blocks and twice when they are on both sides;
         7.4 us and 0.018 us a CTA where no row sees more than 64 tokens (640 CTAs 19.3 us, 1024 25.7, 2048 44.1).
         Of 220 random steps of 8 shapes of heads (1 to 32 key / value heads, groups of 1 to 16; 1 to 40 portions of 10 to 6000 tokens behind 0 to 8000) 81 pass: all
-        faster than with the general kernel, 1.08 to 6 times, 2.1 in the mean.  68 of those that do not would be faster too, 57 by more than a tenth: one prompt of
+        faster than with the general kernel, 1.08 times and more, 2.1 in the mean.  68 of those that do not would be faster too, 57 by more than a tenth: one prompt of
         331 tokens 23 against 24 us, 40 x 20 tokens behind 300 56 against 62; others not (one of 64 behind 4000 139 against 64).  E.g. 32 over 8 heads:
-        8 x 1024 tokens 219 against 703 us, 4 x 256 behind 2048 104 against 277.  (One B200.)"""
+        8 x 1024 tokens 213 against 703 us, 4 x 256 behind 2048 100 against 277.  (One B200.)"""
         best, at, lo, first, of = (0, 0), 0, 0, 0, (0, 0)
         for i, n in enumerate(blocks + [0]):
             if n < 4:

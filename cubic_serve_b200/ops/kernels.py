@@ -182,8 +182,8 @@ def skinny_fits(w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = Non
 def use_skinny(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = None, residual: torch.Tensor | None = None,
                ws: "Workspace | None" = None) -> bool:
     """Which batches the kernel without decoded tiles takes.  Its products run on ``mma.sync`` eight rows at a time, so its time
-    grows with the rows where the tcgen05 kernels' stays: 4-bit weights of 24576 x 4096 take 22 / 26 / 43 us at 8 / 16 / 32 rows
-    against 34 / 34 / 35, 4096 x 4096 6.4 / 8.2 / 14 against 10.1 / 10.2 / 10.6.  bf16 weights have nothing to decode: with more
+    grows with the rows where the tcgen05 kernels' stays: 4-bit weights of 24576 x 4096 take 24 / 28 / 43 us at 8 / 16 / 32 rows
+    against 34 / 34 / 35, 4096 x 4096 6.6 / 8.5 / 14 against 10.1 / 10.2 / 10.6 (in a row of launches; ``use_ts`` comes first).  bf16 weights have nothing to decode: with more
     weight tiles than SMs they stream at 65 / 68 / 74 us against 98 / 98 / 102 (50688 x 4096), with fewer the split tiles of the
     other kernel are as good from 16 rows on (8.0 / 10.4 against 9.2 / 9.2, 4096 x 4096).  Block-scaled e4m3 weights of 9216 x 4096
     take 13.7 / 16.6 / 27.4 us at 8 / 16 / 32 rows against 17.8 / 17.9 / 18.3.  (One B200, weights not in L2.)
@@ -229,6 +229,7 @@ def use_ts(m: int, w: PackedWeight, x: torch.Tensor, out: torch.Tensor | None = 
     - Six and a half units an SM (8192 x 2048 has 6.9, 14336 x 1024 6.1).  Alone, the matrices between that and eight and a half lose 2 to 8 % at up to 8 rows; in a
       step their codes are on the way before the attention in front of them is done: 4096 x 4096 behind it, one request behind 700 tokens 1008 us a step of 12
       layers against 1018 with the few-row kernel, 7 behind 2100 1133 against 1146; at 100 and 112 rows 1789 and 1824 against 1806 and 1831 with the per-tile kernel.
+      (Behind 200 tokens, a shorter attention, there is nothing between them at 1 and 2 rows and 0.4 to 1 % the other way at 8; in a row of launches 7.3 against 6.6 us.)
     - From 65 rows the sums count.  Tiles of several parts of their own: up to 800 rows times parts (4096 x 4096 at 128: 512, 2048 x 8192 at 96: 864, 17.1 -> 17.7),
       or ten units a part (2560 x 9728 has 10.9, at 128 rows 20.6 -> 20.8; 1024 x 16384 7.1, 21.7 -> 28.6).  Tiles dealt across their borders: ten units an SM from 97 rows
       (6144 x 4096 has 10.4, 10240 x 2048 8.6: 18.5 -> 18.2 at 96, 19.5 -> 21.3 at 128).
@@ -277,6 +278,7 @@ def use_ts_grouped(rows: int, w: PackedWeight, experts: int, mb: int) -> bool:
     for every SM.  128 experts (NVFP4), few-row kernel (above 16 rows an expert: per-tile kernel in items of its best size) -> this one, at 16 / 32 / 64 / 128
     routes and 2 / 6 / 24 / 64 / 256 rows an expert: 1536 x 2048 19.0 / 26.9 / 38.9 / 53 and 76 / 85 / 134 / 137 / 299 -> 19.4 / 26.1 / 37.5 / 50 and
     67 / 73 / 78 / 93 / 251 us, 2048 x 768 10.9 / 13.9 / 22.6 / 34 and 40 / 48 / 88 / 102 / 287 -> 11.4 / 13.7 / 20.8 / 28 and 36 / 41 / 43 / 51 / 132.
+    A leaning routing gains as well, 256 / 1024 / 8192 / 32768 routes on eight of the experts: 40 / 50 / 100 / 234 -> 13 / 23 / 50 / 159 and 26 / 31 / 73 / 239 -> 9 / 15 / 34 / 114.
     (Weights not in L2, one B200; ``tensor_memory_rows`` in the operator configuration.)"""
     if w.fmt not in (FMT_CUBIC4, FMT_AFFINE4, FMT_NVFP4) or w.k % 128 or (w.fmt == FMT_CUBIC4 and w.group_k % 128):
         return False
